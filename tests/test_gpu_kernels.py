@@ -58,6 +58,47 @@ def test_gemm_fp32_out_and_accumulate(M, N, K):
     assert relerr(acc, base + ref) < 1e-4
 
 
+@pytest.mark.parametrize("tile_n,splits", [(64, 1), (64, 8), (128, 2), (128, 4), (256, 1), (256, 8), (-1, 3), (-1, 7)])
+@pytest.mark.parametrize("M,N,K", [(128, 64, 512), (300, 520, 2500), (1, 8, 520), (257, 136, 1000)])
+def test_gemm_few_tile_kernels(M, N, K, tile_n, splits):
+    """The kernel for few output tiles (K slices summed inside a cluster) and the slices through a workspace, at single
+    and ragged tiles and uneven slices: every operand layout, bf16 / fp32 / accumulating outputs, neighbours of a strided
+    output untouched, same bits on a second run.  bf16 outputs are within half an ulp (2^-9) of the fp32 sum; fp32 sums
+    of K <= 2500 products differ by their order only."""
+    from torchure_b200 import ops
+
+    if tile_n < 0 and M <= 128:
+        pytest.skip("the pair kernel needs more than 128 rows")
+    torch.manual_seed(0)
+    pad = lambda n: (n + 7) // 8 * 8
+    a = torch.randn(M, K, device="cuda").bfloat16()
+    b = torch.randn(N, K, device="cuda").bfloat16()
+    ref = a.double() @ b.double().t()
+
+    def stored(t, mn):
+        t = t.t() if mn else t
+        buf = torch.zeros(t.shape[0], pad(t.shape[1]), dtype=torch.bfloat16, device="cuda")
+        buf[:, :t.shape[1]] = t
+        return buf[:, :t.shape[1]]
+
+    for mode, a_mn, b_mn in ((0, False, False), (0, False, True), (0, True, True), (1, True, True), (2, True, True),
+                             (1, False, False), (2, False, False)):
+        if tile_n < 0 and mode == 2:
+            continue        # accumulating products split K by reduce-add
+        x, y = stored(a, a_mn), stored(b, b_mn)
+        dt = torch.bfloat16 if mode == 0 else torch.float32
+        base = torch.full((M, pad(N) + 8), 3.0, dtype=dt, device="cuda")
+        outs = []
+        for _ in range(2):
+            buf = base.clone()
+            ops.ext().gemm(x, y, buf[:, :N], a_mn, b_mn, mode, splits, tile_n)
+            outs.append(buf)
+        want = ref + 3.0 if mode == 2 else ref
+        assert relerr(outs[0][:, :N].double(), want) < (4e-3 if mode == 0 else 1e-5), (mode, a_mn, b_mn)
+        assert (outs[0][:, N:] == 3.0).all(), "columns beyond N"
+        assert torch.equal(outs[0], outs[1])
+
+
 def test_gemm_strided_views():
     from torchure_b200.ops import kernels
 

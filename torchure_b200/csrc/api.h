@@ -15,15 +15,32 @@ namespace tb {
 //   b_mn == false: B is stored [N, K] (K contiguous)
 //   b_mn == true : B is stored [K, N] (N contiguous)
 // out_mode 0: C bf16 store, 1: C fp32 store, 2: C fp32 += (TMA reduce-add)
+struct GemmPlan {
+  enum Kind { kSingle, kPair, kSmall, kSlices };
+  int kind;
+  int tile_n;         // kSmall: 64, 128 or 256
+  int splits;         // K slices
+  size_t workspace;   // kSlices: bytes the caller provides
+};
+// The kernel and the K split for a problem.  force_splits > 0 fixes the number of K slices; force_tile_n > 0 selects the
+// kernel for few tiles with that tile width, force_tile_n < 0 the slices through a workspace.
+GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_splits, int force_tile_n);
 // Returns 0 or a negative code for an argument error.  `err` is a device int that a kernel sets when
 // one of its bounded waits expires.
 int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-              bool a_mn, bool b_mn, int out_mode, int* err, int num_sms, cudaStream_t stream, int force_splits = 0);
+              bool a_mn, bool b_mn, int out_mode, const GemmPlan& plan, void* workspace, int* err, int num_sms,
+              cudaStream_t stream);
 // CTA pairs the device holds at once (0 before the first pair launch of this process).
 int gemm_pair_capacity();
-// The CTA-pair kernel behind gemm_bf16 (tiles of 256 x 256 on two SMs); `splits` as chosen by gemm_bf16.
+// The CTA-pair kernel behind gemm_bf16 (tiles of 256 x 256 on two SMs).  slice_rows > 0: K slice s stores its tile at row
+// s * slice_rows of C (a multiple of 256) instead of adding into a shared tile.
 int gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-               bool a_mn, bool b_mn, int out_mode, int splits, int* err, int num_sms, cudaStream_t stream);
+               bool a_mn, bool b_mn, int out_mode, int splits, int* err, int num_sms, cudaStream_t stream,
+               int64_t slice_rows);
+// The kernel for few output tiles (tiles of 128 x tile_n, K slices reduced inside a cluster): tile_n 64, 128 or 256,
+// splits a power of two up to 8 and at most the number of 64-wide k-blocks.
+int gemm_small_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+                    bool a_mn, bool b_mn, int out_mode, int tile_n, int splits, int* err, cudaStream_t stream);
 
 // ---- elementwise / normalisation -------------------------------------------------------------
 // h = rmsnorm(x_new) * w with x_new = x (+ y); optional gather x = table[ids].  Writes x_new when y or ids

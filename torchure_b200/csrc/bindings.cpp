@@ -39,7 +39,7 @@ T* opt_mptr(c10::optional<torch::Tensor>& t) {
 }
 
 void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
-          int64_t splits) {
+          int64_t splits, int64_t tile_n) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda(), "gemm: CUDA tensors required");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm: bf16 operands");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2, "gemm: 2-D tensors");
@@ -51,9 +51,13 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   TORCH_CHECK(out_mode == 0 ? out.scalar_type() == torch::kBFloat16 : out.scalar_type() == torch::kFloat32,
               "gemm: output dtype does not match out_mode");
   c10::cuda::CUDAGuard guard(a.device());
+  const tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, (int)out_mode, num_sms(), (int)splits, (int)tile_n);
+  torch::Tensor ws;
+  if (plan.workspace > 0) ws = torch::empty({(int64_t)plan.workspace}, a.options().dtype(torch::kUInt8));
   const int rc = tb::gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0),
-                               b.stride(0), out.stride(0), a_mn, b_mn, (int)out_mode, err_word().data_ptr<int>(),
-                               num_sms(), cur_stream(), (int)splits);
+                               b.stride(0), out.stride(0), a_mn, b_mn, (int)out_mode, plan,
+                               plan.workspace > 0 ? ws.data_ptr() : nullptr, err_word().data_ptr<int>(), num_sms(),
+                               cur_stream());
   TORCH_CHECK(rc == 0, "gemm_bf16 failed with code ", rc);
 }
 
@@ -211,7 +215,7 @@ void register_attn(pybind11::module_& m);
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
         pybind11::arg("b"), pybind11::arg("out"), pybind11::arg("a_mn"), pybind11::arg("b_mn"), pybind11::arg("out_mode"),
-        pybind11::arg("splits") = 0);
+        pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0);
   m.def("set_sm_reserve", [](int64_t n) { g_sm_reserve = (int)n; }, "persistent kernels use (SM count - n) CTAs");
   m.def("gemm_pair_capacity", &tb::gemm_pair_capacity, "CTA pairs (2-SM clusters) resident at once; 0 before the first launch");
   m.def("error_word", &error_word, "device int32[4]; [0] is set when a bounded wait of a kernel expired");

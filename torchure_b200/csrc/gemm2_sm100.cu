@@ -14,7 +14,8 @@
 //   Two 256-column accumulators per CTA: the epilogue of tile i overlaps the main loop of tile i + 1.
 //
 // Operand layouts, output modes (bf16 store, fp32 store, fp32 reduce-add) and split-K are those of the single-CTA
-// kernel in gemm_sm100.cu, which remains the path of the fused GEMM + collective kernels and of small problems.
+// kernel in gemm_sm100.cu, which remains the path of the fused GEMM + collective kernels and of wide products of at most
+// 128 rows; problems with few tiles run on gemm_small_sm100.cu (the choice is gemm_plan in gemm_sm100.cu).
 // Every wait is bounded; the two CTAs meet at a cluster barrier before anyone touches a partner's barrier and again
 // before either releases its tensor memory.
 #include "api.h"
@@ -88,7 +89,7 @@ __device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
 template <bool A_MN, bool B_MN, int OUT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int splits, int* err) {
+                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int splits, int slice_rows, int* err) {
   pdl_wait();
   pdl_launch_dependents();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -229,6 +230,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int unit = cluster; unit < num_units && ok; unit += num_clusters) {
       const int tile = unit % num_tiles;
       if ((unit / num_tiles) * kb_per >= num_kb) continue;  // empty K slice
+      const int c_row = (unit / num_tiles) * slice_rows;    // each slice has rows of its own in a workspace
       const int m0 = (tile % num_m) * 2 * BM + static_cast<int>(rank) * BM;
       const int n0 = (tile / num_m) * BN;
       const int acc = it & 1;
@@ -275,8 +277,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (OUT == 2) tma_reduce_add_2d(&tmC, buf, n0 + c * COLS, m0 + q * 32);
-            else tma_store_2d(&tmC, buf, n0 + c * COLS, m0 + q * 32);
+            if (OUT == 2) tma_reduce_add_2d(&tmC, buf, n0 + c * COLS, c_row + m0 + q * 32);
+            else tma_store_2d(&tmC, buf, n0 + c * COLS, c_row + m0 + q * 32);
             tma_commit_group();
           }
         }
@@ -308,7 +310,7 @@ int g_pair_capacity = 0;
 
 template <bool A_MN, bool B_MN, int OUT>
 int launch2(const CUtensorMap& ta, const CUtensorMap& tb_, const CUtensorMap& tc, int M, int N, int K, int splits,
-            int* err, int units, int num_sms, cudaStream_t stream) {
+            int slice_rows, int* err, int units, int num_sms, cudaStream_t stream) {
   auto kern = gemm2_bf16_kernel<A_MN, B_MN, OUT>;
   if (!ensure_dynamic_smem(reinterpret_cast<const void*>(kern), SMEM_BYTES)) return -20;
   cudaLaunchConfig_t cfg{};
@@ -339,16 +341,17 @@ int launch2(const CUtensorMap& ta, const CUtensorMap& tb_, const CUtensorMap& tc
   attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb_, tc, M, N, K, splits, err) == cudaSuccess ? 0 : -21;
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb_, tc, M, N, K, splits, slice_rows, err) == cudaSuccess ? 0 : -21;
 }
 
 }  // namespace
 
 int gemm_pair_capacity() { return g_pair_capacity; }
 
-// Same contract as gemm_bf16 (gemm_sm100.cu), which calls this for problems with more than 128 rows.
+// Same contract as gemm_bf16 (gemm_sm100.cu), which decides between this kernel and the others (gemm_plan).
 int gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-               bool a_mn, bool b_mn, int out_mode, int splits, int* err, int num_sms, cudaStream_t stream) {
+               bool a_mn, bool b_mn, int out_mode, int splits, int* err, int num_sms, cudaStream_t stream,
+               int64_t slice_rows) {
   CUtensorMap ta, tb_, tc;
   int r;
   // K-major operand [R, K]: box 64 (k) x tile rows.  MN-major operand stored [K, R]: box 64 (r) x 64 (k rows).
@@ -356,13 +359,15 @@ int gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64
   if (r) return r;
   r = b_mn ? make_tmap_2d(&tb_, B, 2, K, N, ldb, 64, 64) : make_tmap_2d(&tb_, B, 2, N, K, ldb, BNH, 64);
   if (r) return r - 100;
-  r = out_mode == 0 ? make_tmap_2d(&tc, C, 2, M, N, ldc, 32, 64) : make_tmap_2d(&tc, C, 4, M, N, ldc, 32, 32);
+  // slices with rows of their own: the padding rows up to slice_rows take what the ragged last tile stores
+  const uint64_t c_rows = slice_rows > 0 ? static_cast<uint64_t>(slice_rows) * splits : M;
+  r = out_mode == 0 ? make_tmap_2d(&tc, C, 2, c_rows, N, ldc, 32, 64) : make_tmap_2d(&tc, C, 4, c_rows, N, ldc, 32, 32);
   if (r) return r - 200;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
   const int units = tiles * splits;
 #define TB_GEMM2_CASE(AM, BMN, O) \
   if (a_mn == AM && b_mn == BMN && out_mode == O) \
-    return launch2<AM, BMN, O>(ta, tb_, tc, M, N, K, splits, err, units, num_sms, stream);
+    return launch2<AM, BMN, O>(ta, tb_, tc, M, N, K, splits, static_cast<int>(slice_rows), err, units, num_sms, stream);
   TB_GEMM2_CASE(false, false, 0)
   TB_GEMM2_CASE(false, false, 1)
   TB_GEMM2_CASE(false, false, 2)

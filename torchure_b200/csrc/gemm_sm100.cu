@@ -18,6 +18,7 @@
 #include "comm_device.cuh"
 #include "common.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -487,7 +488,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb_, const CUtensorM
              : -21;
 }
 
-// Problems with more than 128 rows run on CTA pairs (gemm2_sm100.cu) unless TORCHURE_B200_GEMM_PAIR=0.
+// Problems with more than 128 rows run on CTA pairs (gemm2_sm100.cu) or, with few tiles, on the kernel of
+// gemm_small_sm100.cu; TORCHURE_B200_GEMM_PAIR=0 keeps everything on the single-CTA kernel for comparison.
 static bool pair_enabled() {
   static const bool on = [] {
     const char* e = std::getenv("TORCHURE_B200_GEMM_PAIR");
@@ -496,13 +498,171 @@ static bool pair_enabled() {
   return on;
 }
 
-int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-              bool a_mn, bool b_mn, int out_mode, int* err, int num_sms, cudaStream_t stream, int force_splits) {
-  if (M <= 0 || N <= 0 || K <= 0) return -1;
+// C (=, or += in mode 2) the sum of `slices` fp32 matrices that lie `stride` elements apart, in slice order.  One thread
+// per four columns of a row; a bf16 output is rounded once.
+template <int OUT>
+__global__ void __launch_bounds__(256)
+sum_slices_kernel(const float* __restrict__ ws, int64_t stride, int slices, int64_t ldw, void* __restrict__ C, int64_t ldc,
+                  int M, int N) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int groups = (N + 3) >> 2;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  if (i >= static_cast<int64_t>(M) * groups) return;
+  const int64_t row = i / groups;
+  const int col = static_cast<int>(i - row * groups) * 4;
+  const float* p = ws + row * ldw + col;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < slices; ++s) {
+    const float4 x = *reinterpret_cast<const float4*>(p + s * stride);
+    acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+  }
+  const float f[4] = {acc.x, acc.y, acc.z, acc.w};
+  if (OUT == 0) {
+    __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(C) + row * ldc + col;
+    if (col + 4 <= N) {
+      *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (col + e < N) o[e] = __float2bfloat16(f[e]);
+    }
+  } else {
+    float* o = reinterpret_cast<float*>(C) + row * ldc + col;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (col + e < N) o[e] = OUT == 2 ? o[e] + f[e] : f[e];
+  }
+}
+
+static int sum_slices(const float* ws, int64_t stride, int slices, int64_t ldw, void* C, int64_t ldc, int M, int N,
+                      int out_mode, cudaStream_t stream) {
+  if ((reinterpret_cast<uintptr_t>(C) & 15) != 0 || (ldc * (out_mode == 0 ? 2 : 4)) % 16 != 0) return -212;
+  const int64_t threads = static_cast<int64_t>(M) * ((N + 3) / 4);
+  const dim3 grid(static_cast<unsigned>((threads + 255) / 256));
+  auto kern = out_mode == 0 ? sum_slices_kernel<0> : (out_mode == 1 ? sum_slices_kernel<1> : sum_slices_kernel<2>);
+  return launch_pdl(kern, grid, dim3(256), 0, stream, ws, stride, slices, ldw, C, ldc, M, N) == cudaSuccess ? 0 : -21;
+}
+
+// Which kernel a problem runs on, from a model of its time in microseconds.  The constants are fits to measured times on
+// B200 (cold weights, launches back to back from a graph): a fixed part (launch, pipeline fill, last epilogue) plus
+// k-blocks of 64 times the cost of one.
+//   pair kernel, 256 x 256 tiles:            6.9 + 0.30 per k-block and wave  (8 k-blocks 9.0, 16 k-blocks 11.3,
+//                                            128 k-blocks 42.8)
+//   128 x 64 / 128 / 256 tiles, one per CTA: 3.7 / 4.1 / 4.4 + 0.14 / 0.18 / 0.36 per k-block, all of it again per wave
+//                                            (8 k-blocks 4.8 / 5.5 / 7.0, 32 k-blocks 8.0 / 9.0 / 14)
+//   their K slices in a cluster:             + 1 + 0.02 BN log2(S): the exchange of partials (64 x 2: 2.3, 64 x 4: 3.7,
+//                                            128 x 4: 6.3)
+//   K slices through a workspace:            + 4 for the summing kernel + its traffic
+// and, when the operands exceed half of L2, the bytes brought into shared memory at 8.5 TB/s for K slices (2 slices: 12,
+// unsplit: 16): CTAs on different slices share no operand tile, so fewer of their reads meet in L2 (128 x 1024 x 151936 in
+// 8 slices: 912 MB with 64-wide tiles 108 us, 608 MB with 128-wide ones 75; 512 x 512 x 8192, 17 MB of operands, in 4
+// slices: 13.1 us, as the other terms say).
+// Narrow tiles win while the problem is one wave of them (1024 x 512 x 512: 4.8 against 9.1 us; 2048 x 1024 x 4096: 16.2
+// against 25.4), the pair kernel as soon as it fills its 74 SM pairs (4096 x 1024 x 6144: 37.1 against 38.7).
+GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_splits, int force_tile_n) {
+  GemmPlan p{};
+  p.splits = 1;
+  const int num_kb = (K + BK - 1) / BK;
+  auto ceil_div = [](int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); };
   const bool pair = pair_enabled() && M > BM && num_sms >= 2;
+  const int workers = pair ? (gemm_pair_capacity() > 0 ? gemm_pair_capacity() : num_sms / 2) : num_sms;
+  const int64_t tiles = static_cast<int64_t>(ceil_div(M, (pair ? 2 : 1) * BM)) * ceil_div(N, BN);
+  const int64_t slice_rows = static_cast<int64_t>(ceil_div(M, 2 * BM)) * 2 * BM;
+  auto use_slices = [&](int s) {
+    const int per = ceil_div(num_kb, s);
+    p.kind = GemmPlan::kSlices;
+    p.splits = ceil_div(num_kb, per);        // no empty slice
+    p.workspace = static_cast<size_t>(p.splits) * slice_rows * ((N + 3) / 4 * 4) * 4;
+  };
+  if (force_tile_n > 0) {
+    p.kind = GemmPlan::kSmall;
+    p.tile_n = force_tile_n;
+    p.splits = force_splits > 0 ? force_splits : 1;
+    return p;
+  }
+  if (force_tile_n < 0 && pair) {
+    use_slices(force_splits > 0 ? force_splits : 1);
+    return p;
+  }
+  p.kind = pair ? GemmPlan::kPair : GemmPlan::kSingle;
+  if (force_splits > 0) {
+    p.splits = force_splits;
+    return p;
+  }
+  // split-K by reduce-add for fp32 outputs (wgrad: few output tiles, long K): the slice count with the least wave time
+  if (out_mode != 0 && num_kb >= 32 && tiles < 2 * workers) {
+    float best = 1e30f;
+    for (int s = 1; s <= 8 && s * 8 <= num_kb; ++s) {
+      const int waves = ceil_div(tiles * s, workers);
+      const float cost = static_cast<float>(waves) / s + 0.02f * (s - 1);
+      if (cost < best - 1e-6f) { best = cost; p.splits = s; }
+    }
+  }
+  const bool cold = 2ll * (M + N) * K > (64ll << 20);
+  if (!pair_enabled()) return p;      // the comparison switch: the single-CTA kernel for everything
+  float best = pair ? 6.9f + 0.30f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits)
+                    : 5.f + 0.36f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits);
+  if (p.splits > 1 && out_mode == 1) best += 3.f;     // C is cleared first
+  // K slices through a workspace: only where the tiles leave most of the chip idle for a long K
+  if (pair && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
+    const int s = static_cast<int>(workers / tiles) < num_kb / 16 ? static_cast<int>(workers / tiles) : num_kb / 16;
+    if (s > 1) {
+      const float run = std::max(0.30f * ceil_div(num_kb, s), cold ? tiles * num_kb * 65536.f / 8.5e6f : 0.f);
+      const float t = 6.9f + run + 4.f + 2e-6f * s * static_cast<float>(M) * N;
+      if (t < best) { best = t; use_slices(s); }
+    }
+  }
+  static constexpr int kTile[3] = {64, 128, 256};
+  static constexpr float kFixed[3] = {3.7f, 4.1f, 4.4f}, kPerKb[3] = {0.14f, 0.18f, 0.36f};
+  for (int i = 0; i < 3; ++i) {
+    const int64_t t_small = static_cast<int64_t>(ceil_div(M, BM)) * ceil_div(N, kTile[i]);
+    if (t_small > 2 * num_sms) continue;
+    for (int s = 1, lg = 0; s <= 8 && s <= num_kb; s *= 2, ++lg) {
+      // clusters of 4 and 8 leave SMs of a GPC over
+      const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 15 / 16 : num_sms * 7 / 8);
+      const int waves = ceil_div(t_small * s, slots);
+      const float bytes = static_cast<float>(t_small) * num_kb * (A_BYTES + 128 * kTile[i]);
+      const float run = std::max(waves * kPerKb[i] * ceil_div(num_kb, s),
+                                 cold ? bytes / (s == 1 ? 16e6f : (s == 2 ? 12e6f : 8.5e6f)) : 0.f);
+      const float t = waves * kFixed[i] + run + (s > 1 ? 1.f + 0.02f * kTile[i] * lg : 0.f);
+      if (t < best) {
+        best = t;
+        p.kind = GemmPlan::kSmall;
+        p.tile_n = kTile[i];
+        p.splits = s;
+        p.workspace = 0;
+      }
+    }
+  }
+  return p;
+}
+
+int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
+              bool a_mn, bool b_mn, int out_mode, const GemmPlan& plan, void* workspace, int* err, int num_sms,
+              cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return -1;
+  int splits = plan.splits;
+  if (plan.kind == GemmPlan::kSmall)
+    return gemm_small_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, plan.tile_n, splits, err, stream);
+  if (plan.kind == GemmPlan::kSlices) {
+    const int64_t slice_rows = static_cast<int64_t>((M + 2 * BM - 1) / (2 * BM)) * 2 * BM, ldw = (N + 3) / 4 * 4;
+    if (workspace == nullptr) return -4;
+    int rc = gemm2_bf16(A, B, workspace, M, N, K, lda, ldb, ldw, a_mn, b_mn, 1, splits, err, num_sms, stream, slice_rows);
+    if (rc) return rc;
+    return sum_slices(reinterpret_cast<const float*>(workspace), slice_rows * ldw, splits, ldw, C, ldc, M, N, out_mode, stream);
+  }
+  if (splits > 1 && out_mode == 0) return -5;
+  if (splits > 1 && out_mode == 1) {
+    // the slices all add into C: clear it first
+    if (cudaMemset2DAsync(C, static_cast<size_t>(ldc) * 4, 0, static_cast<size_t>(N) * 4, M, stream) != cudaSuccess) return -22;
+    out_mode = 2;
+  }
+  if (plan.kind == GemmPlan::kPair)
+    return gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, splits, err, num_sms, stream, 0);
   CUtensorMap ta, tb_, tc;
   int r;
-  if (!pair) {
   // K-major operand [R, K]: box 64 (k) x tile rows.  MN-major operand stored [K, R]: box 64 (r) x 64 (k rows).
   r = a_mn ? make_tmap_2d(&ta, A, 2, K, M, lda, 64, 64) : make_tmap_2d(&ta, A, 2, M, K, lda, BM, 64);
   if (r) return r;
@@ -510,31 +670,7 @@ int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_
   if (r) return r - 100;
   r = out_mode == 0 ? make_tmap_2d(&tc, C, 2, M, N, ldc, 32, 64) : make_tmap_2d(&tc, C, 4, M, N, ldc, 32, 32);
   if (r) return r - 200;
-  }
-  // work units and workers: 128 x 256 tiles on SMs, or 256 x 256 tiles on SM pairs
-  const int tiles = ((M + (pair ? 2 : 1) * BM - 1) / ((pair ? 2 : 1) * BM)) * ((N + BN - 1) / BN);
-  const int workers = pair ? (gemm_pair_capacity() > 0 ? gemm_pair_capacity() : num_sms / 2) : num_sms;
-  // split-K for fp32 outputs (wgrad: few output tiles, long K): pick the slice count with the least wave time
-  int splits = 1;
-  const int num_kb = (K + BK - 1) / BK;
-  if (force_splits > 0) {
-    splits = force_splits;
-  } else if (out_mode != 0 && num_kb >= 32 && tiles < 2 * workers) {
-    float best = 1e30f;
-    for (int s = 1; s <= 8 && s * 8 <= num_kb; ++s) {
-      const int waves = (tiles * s + workers - 1) / workers;
-      const float cost = static_cast<float>(waves) / s + 0.02f * (s - 1);
-      if (cost < best - 1e-6f) { best = cost; splits = s; }
-    }
-  }
-  if (splits > 1 && out_mode == 1) {
-    // the slices all add into C: clear it first
-    if (cudaMemset2DAsync(C, static_cast<size_t>(ldc) * 4, 0, static_cast<size_t>(N) * 4, M, stream) != cudaSuccess) return -22;
-    out_mode = 2;
-  }
-  if (pair)
-    return gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, splits, err, num_sms, stream);
-  const int units = tiles * splits;
+  const int units = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * splits;
   const int grid = units < num_sms ? units : num_sms;
 #define TB_GEMM_CASE(AM, BMN, O) \
   if (a_mn == AM && b_mn == BMN && out_mode == O) return launch<AM, BMN, O>(ta, tb_, tc, M, N, K, splits, err, grid, stream);
