@@ -143,6 +143,33 @@ def test_add_rmsnorm_fwd_bwd(M, D):
     assert relerr(dw, wa.grad) < 1e-4
 
 
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("M,D", [(1, 1032), (7, 2048), (600, 1280), (3000, 2048), (1200, 2056), (333, 3072), (1201, 4096),
+                                 (50, 4104)])
+def test_rmsnorm_bwd_rows_shared_by_warps(M, D, residual):
+    """Rows of more than 1024 columns: two or four warps per row, ragged last slices, fewer rows than teams, the widths on
+    both sides of each limit.  fp32 sums of D products against fp64: 2^-24 sqrt(D) is 4e-6 at 4096, 1e-5 allowed; the gain
+    gradient sums M rows, 1e-4 as above."""
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(0)
+    x, dh = torch.randn(M, D, device="cuda"), torch.randn(M, D, device="cuda").bfloat16()
+    w = torch.rand(D, device="cuda") + 0.5
+    rstd = torch.rsqrt(x.pow(2).mean(-1) + 1e-6)
+    dx_in = torch.randn(M, D, device="cuda") if residual else None
+    dw = torch.ones(D, device="cuda")
+    dx, dxb = kernels.rmsnorm_bwd(dh, x, w, rstd, dx_in, dw)
+    kernels.check_error()
+    r, xd, gd = rstd.double()[:, None], x.double(), dh.double()
+    xh = xd * r
+    want = r * (gd * w.double() - xh * (gd * w.double() * xh).mean(-1, keepdim=True))
+    if residual:
+        want = want + dx_in.double()
+    assert relerr(dx.double(), want) < 1e-5
+    assert relerr(dxb, dx) < 5e-3
+    assert relerr(dw.double() - 1, (gd * xh).sum(0)) < 1e-4
+
+
 def test_embedding_gather_norm_and_scatter():
     from torchure_b200.ops import kernels, oracle
 

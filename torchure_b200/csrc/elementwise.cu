@@ -274,14 +274,23 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dh, const float* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// rmsnorm backward for D <= 1024, rows staged through shared memory by bulk copies (the scheme of the QK-norm / RoPE
-// backward further down): every warp of one persistent CTA per SM owns one or two row buffers [x fp32 | dh bf16 |
-// dx_in fp32]; while it works on a row the next one is in flight, at no register cost, and the second pass (outputs
-// and gain gradient) re-reads the row from shared memory instead of holding it in registers.  Eight warps of at most
-// 128 registers: the CTA fits beside a 512-thread CTA of a gradient all-reduce kernel.
+// rmsnorm backward, rows staged through shared memory by bulk copies (the scheme of the QK-norm / RoPE backward further
+// down): one persistent CTA per SM; while a row [x fp32 | dh bf16 | dx_in fp32] is worked on the next ones are in flight,
+// at no register cost, and the second pass (outputs and gain gradient) re-reads the row from shared memory instead of
+// holding it in registers.  Eight warps of at most 128 registers: the CTA fits beside a 512-thread CTA of a gradient
+// all-reduce kernel.
+// A row belongs to a team of T warps, each with up to 1024 of its columns (gain and gain-gradient partial of a lane's
+// columns stay in 64 registers): T = 1 up to D = 1024, 2 up to 2048, 4 up to 4096.  The warps of a team meet once per row,
+// where they exchange their dot products through shared memory; behind that barrier every one of them has finished the
+// row before, so its buffer can take the next copy.
+// Bound by memory: 16 bytes per element with residual input and bf16 copy.  Measured on B200: 8192 x 1024 21 us (6.4
+// TB/s in a step); with one warp per row and both passes reading memory 8192 x 2048 took 96 us, now 45 (5.9 TB/s), 4096 x
+// 2560 62, now 29, 4096 x 4096 227, now 47, 512 x 2048 22, now 6.4.
 // ---------------------------------------------------------------------------------------------
 constexpr int RNB_MAX_WARPS = 8;
+constexpr int RNB_MAX_STAGES = 4;
 
+template <int T>
 __global__ void __launch_bounds__(RNB_MAX_WARPS * 32, 2)
 rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __restrict__ x, const float* __restrict__ w,
                           const float* __restrict__ rstd, const float* __restrict__ dx_in, float* __restrict__ dx,
@@ -291,29 +300,32 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
   pdl_launch_dependents();
   constexpr int MAX_VEC = 8;
   extern __shared__ __align__(128) uint8_t rn_smem[];
-  __shared__ uint64_t bars[RNB_MAX_WARPS][2];
+  __shared__ uint64_t bars[RNB_MAX_WARPS][RNB_MAX_STAGES];
+  __shared__ float s_dot[RNB_MAX_WARPS / T][2][T];
   const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int wid = threadIdx.x >> 5;
+  const int teams = (blockDim.x >> 5) / T, team = wid / T, part = wid % T;
   const int nvec = D >> 2;
-  uint8_t* buf = rn_smem + static_cast<size_t>(wid) * stages * stage_bytes;
+  const int part_vec = T == 1 ? nvec : (nvec + T - 1) / T;   // float4 columns of a warp: [v0, v1)
+  const int v0 = part * part_vec, v1 = min(nvec, v0 + part_vec);
+  uint8_t* buf = rn_smem + static_cast<size_t>(team) * stages * stage_bytes;
   const int off_dh = D * 4, off_in = D * 6;
-  if (lane == 0) {
-    mbar_init(&bars[wid][0], 1);
-    mbar_init(&bars[wid][1], 1);
+  if (part == 0 && lane < stages) {
+    mbar_init(&bars[team][lane], 1);
     fence_barrier_init();
   }
   __syncthreads();
   float4 wv[MAX_VEC], dw_acc[MAX_VEC];
 #pragma unroll
   for (int j = 0; j < MAX_VEC; ++j) {
-    const int i = lane + j * 32;
-    wv[j] = i < nvec ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int i = v0 + lane + j * 32;
+    wv[j] = i < v1 ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     dw_acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const uint32_t tx_bytes = static_cast<uint32_t>(D * (dx_in ? 10 : 6));
-  auto issue = [&](int row, int stage) {
+  auto issue = [&](int row, int stage) {   // by the team's first warp
     uint8_t* dst = buf + stage * stage_bytes;
-    uint64_t* bar = &bars[wid][stage];
+    uint64_t* bar = &bars[team][stage];
     if (lane == 0) mbar_expect_tx(bar, tx_bytes);
     __syncwarp();
     const int64_t off = static_cast<int64_t>(row) * D;
@@ -321,27 +333,31 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
     else if (lane == 1) bulk_load_1d(dst + off_dh, dh + off, static_cast<uint32_t>(D * 2), bar);
     else if (lane == 2 && dx_in) bulk_load_1d(dst + off_in, dx_in + off, static_cast<uint32_t>(D * 4), bar);
   };
-  const int row0 = blockIdx.x * warps + wid, row_step = gridDim.x * warps;
-  const bool two = stages == 2;
+  const int row0 = blockIdx.x * teams + team, row_step = gridDim.x * teams;
   bool ok = true;
-  if (two && row0 < M) issue(row0, 0);
+  if (part == 0)
+    for (int s = 0; s < stages - 1; ++s)
+      if (row0 + s * row_step < M) issue(row0 + s * row_step, s);
   float r_next = row0 < M ? rstd[row0] : 0.f;
-  int k = 0;
+  int k = 0, stage = 0;
+  uint32_t phase = 0;
   for (int row = row0; row < M; row += row_step, ++k) {
-    const int stage = two ? (k & 1) : 0;
-    if (!two) issue(row, 0);
-    else if (row + row_step < M) issue(row + row_step, stage ^ 1);
+    // the buffer of the row before this one takes the row `stages - 1` ahead; a team has to meet first (below)
+    const int ahead = row + (stages - 1) * row_step;
+    const int free_stage = stage == 0 ? stages - 1 : stage - 1;
+    if (T == 1 && ahead < M) issue(ahead, free_stage);
     const float r = r_next;
     if (row + row_step < M) r_next = rstd[row + row_step];
-    if (!mbar_wait(&bars[wid][stage], (two ? (k >> 1) : k) & 1, err, kErrStagedRowWait)) { ok = false; break; }
+    // a warp whose wait expired goes on without new copies: its team meets once per row
+    ok = __all_sync(0xffffffffu, mbar_wait(&bars[team][stage], phase, err, kErrStagedRowWait) && ok);
     const uint8_t* st = buf + stage * stage_bytes;
     const float2 r2 = make_float2(r, r);
     // pass 1: dot = mean(dh w xhat)
     float2 dot2 = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < MAX_VEC; ++j) {
-      const int i = lane + j * 32;
-      if (i < nvec) {
+      const int i = v0 + lane + j * 32;
+      if (i < v1) {
         const float4 xv = reinterpret_cast<const float4*>(st)[i];
         const uint2 dv = reinterpret_cast<const uint2*>(st + off_dh)[i];
         const float2 a = bf2_to_f2(dv.x), b = bf2_to_f2(dv.y);
@@ -349,14 +365,23 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
         dot2 = fma2(mul2(b, make_float2(wv[j].z, wv[j].w)), make_float2(xv.z, xv.w), dot2);
       }
     }
-    const float dot = warp_sum(dot2.x + dot2.y) * r / D;
+    float dot = warp_sum(dot2.x + dot2.y);
+    if (T > 1) {
+      if (lane == 0) s_dot[team][k & 1][part] = dot;
+      asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(T * 32) : "memory");
+      dot = 0.f;
+#pragma unroll
+      for (int p = 0; p < T; ++p) dot += s_dot[team][k & 1][p];
+      if (part == 0 && ok && ahead < M) issue(ahead, free_stage);
+    }
+    dot = dot * r / D;
     const float2 nd2 = make_float2(-dot, -dot);
     // pass 2: dx = r (dh w - xhat dot) (+ dx_in), dw += dh xhat
     const int64_t off = static_cast<int64_t>(row) * D;
 #pragma unroll
     for (int j = 0; j < MAX_VEC; ++j) {
-      const int i = lane + j * 32;
-      if (i < nvec) {
+      const int i = v0 + lane + j * 32;
+      if (i < v1) {
         const float4 xv = reinterpret_cast<const float4*>(st)[i];
         const uint2 dv = reinterpret_cast<const uint2*>(st + off_dh)[i];
         const float2 a = bf2_to_f2(dv.x), b = bf2_to_f2(dv.y);
@@ -375,24 +400,26 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
       }
     }
     __syncwarp();   // every lane is done with this buffer before the next iteration's copies overwrite it
+    if (++stage == stages) { stage = 0; phase ^= 1; }
+    if (T == 1 && !ok) break;
   }
   if (!ok) {
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
   }
-  // warps -> one partial per column in shared memory (the row buffers are free now) -> one vector reduction per four
+  // teams -> one partial per column in shared memory (the row buffers are free now) -> one vector reduction per four
   // columns per CTA
   __syncthreads();
   float* red = reinterpret_cast<float*>(rn_smem);
 #pragma unroll
   for (int j = 0; j < MAX_VEC; ++j) {
-    const int i = lane + j * 32;
-    if (i < nvec) reinterpret_cast<float4*>(red + wid * D)[i] = dw_acc[j];
+    const int i = v0 + lane + j * 32;
+    if (i < v1) reinterpret_cast<float4*>(red + team * D)[i] = dw_acc[j];
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int kk = 0; kk < warps; ++kk) {
+    for (int kk = 0; kk < teams; ++kk) {
       const float4 v = reinterpret_cast<const float4*>(red + kk * D)[i];
       acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
     }
@@ -1009,7 +1036,7 @@ ce_softmax_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ldl, const in
       if (threadIdx.x == 0) {
         s_stats[0] = gm;
         s_stats[1] = gs;
-        if constexpr (MODE == CE_FUSED) {
+        if constexpr (MODE != CE_STATS) {
           row_loss[row] = gm + __logf(gs) - (label >= 0 ? __bfloat162float(lr[label]) : 0.f);
         } else {
           const int64_t n_rows = gridDim.x;
@@ -1122,17 +1149,25 @@ void rmsnorm_bwd(const __nv_bfloat16* dh, const float* x, const float* w, const 
                  float* dx, __nv_bfloat16* dx_bf16, float* dw, int M, int D, int num_sms, int* err, cudaStream_t stream,
                  int variant) {
   const bool aligned = D % 8 == 0 && ((reinterpret_cast<uintptr_t>(dh) | reinterpret_cast<uintptr_t>(x) |
-                                       reinterpret_cast<uintptr_t>(dx_in)) & 15) == 0;
-  if (variant != 1 && D <= 128 * 8 && M >= 4 * num_sms && aligned && err != nullptr) {
+                                       reinterpret_cast<uintptr_t>(dx_in)) & 15) == 0 &&
+                       (D <= 128 * 8 || (reinterpret_cast<uintptr_t>(dw) & 15) == 0);
+  if (variant != 1 && D <= 128 * 32 && (D > 128 * 8 || M >= 4 * num_sms) && aligned && err != nullptr) {
+    const int T = D <= 128 * 8 ? 1 : (D <= 128 * 16 ? 2 : 4);
     const int stage_bytes = D * (dx_in ? 10 : 6);
     const int budget = 200 * 1024;
-    const int stages = 2 * stage_bytes * RNB_MAX_WARPS <= budget ? 2 : 1;
-    const int warps = std::min(RNB_MAX_WARPS, budget / (stages * stage_bytes));
-    const int smem = std::max(warps * stages * stage_bytes, warps * D * 4);
-    if (warps >= 1 && ensure_dynamic_smem(reinterpret_cast<const void*>(rmsnorm_bwd_staged_kernel), smem)) {
-      const int grid = std::max(1, std::min((M + warps - 1) / warps, num_sms));
-      launch_pdl(rmsnorm_bwd_staged_kernel, dim3(grid), dim3(warps * 32), smem, stream, dh, x, w, rstd, dx_in, dx,
-                 dx_bf16, dw, M, D, stage_bytes, stages, err);
+    int teams = RNB_MAX_WARPS / T, stages = budget / (teams * stage_bytes);
+    if (T == 1) {
+      stages = stages >= 2 ? 2 : 1;
+      teams = std::min(teams, budget / (stages * stage_bytes));
+    } else {
+      stages = std::min(stages, RNB_MAX_STAGES);   // at least two: four rows of 20 KB, two of 40 KB
+    }
+    const int smem = teams * stages * stage_bytes;
+    auto kern = T == 1 ? rmsnorm_bwd_staged_kernel<1> : (T == 2 ? rmsnorm_bwd_staged_kernel<2> : rmsnorm_bwd_staged_kernel<4>);
+    if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) {
+      const int grid = std::max(1, std::min((M + teams - 1) / teams, num_sms));
+      launch_pdl(kern, dim3(grid), dim3(teams * T * 32), smem, stream, dh, x, w, rstd, dx_in, dx, dx_bf16, dw, M, D,
+                 stage_bytes, stages, err);
       return;
     }
   }
