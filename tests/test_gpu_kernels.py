@@ -281,6 +281,46 @@ def test_ce_softmax_grad(C, V):
     assert work[labels == -100].abs().sum() == 0
 
 
+@pytest.mark.parametrize("C,V", [(3, 17), (64, 1000), (130, 32003)])
+def test_ce_loss_alone(C, V):
+    """The loss of a pass without gradients: the bits of the fused step's, logits untouched, ignored rows zero."""
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(0)
+    ld = (V + 7) // 8 * 8
+    logits = (torch.randn(C, ld, device="cuda") * 3).bfloat16()[:, :V]
+    labels = torch.randint(0, V, (C,), device="cuda")
+    labels[::5] = -100
+    before = logits.clone()
+    alone, fused = torch.full((C,), 7.0, device="cuda"), torch.full((C,), 7.0, device="cuda")
+    kernels.ce_loss(logits, labels, alone, -100)
+    assert torch.equal(logits, before)
+    kernels.ce_softmax_grad_(logits, labels, fused, torch.ones(1, device="cuda"), -100)
+    assert torch.equal(alone, fused) and (alone[::5] == 0).all()
+    want = torch.nn.functional.cross_entropy(before.float(), labels, reduction="none")
+    torch.testing.assert_close(alone, want, rtol=1e-4, atol=1e-4)
+
+
+def test_linear_ce_without_gradients():
+    """no_grad with a weight that requires a gradient: same loss, no gradient work (one product and one loss per chunk)."""
+    from torchure_b200 import ops
+    from torchure_b200.loss import fused_linear_cross_entropy
+
+    torch.manual_seed(0)
+    h = torch.randn(300, 256, device="cuda").bfloat16()
+    w = (torch.randn(1000, 256, device="cuda") * 0.05).bfloat16().requires_grad_()
+    y = torch.randint(0, 1000, (300,), device="cuda")
+    y[3:40] = -100
+    full = fused_linear_cross_entropy(h, w, y, -100, 128)
+    with torch.no_grad():
+        before = ops.launches()
+        loss = fused_linear_cross_entropy(h, w, y, -100, 128)
+        assert ops.launches() - before == 2 * 3
+    assert not loss.requires_grad and torch.equal(loss, full.detach())
+    full.backward()
+    assert w.grad is not None
+
+
 @pytest.mark.parametrize("C,V,shards", [(64, 1024, 2), (300, 5008, 2), (256, 151936, 4)])   # shard rows stay 16-byte aligned
 def test_ce_vocabulary_sharded_passes(C, V, shards):
     """The two passes of the loss-parallel CE on column shards of one logits matrix (what the ranks of a

@@ -136,6 +136,11 @@ void ce_softmax_grad(torch::Tensor& logits, const torch::Tensor& labels, torch::
                       inv_n_valid.data_ptr<float>(), (int)logits.size(0), (int)logits.size(1), (int)ignore_index,
                       cur_stream());
 }
+void ce_loss(const torch::Tensor& logits, const torch::Tensor& labels, torch::Tensor& row_loss, int64_t ignore_index) {
+  TORCH_CHECK(logits.stride(1) == 1 && logits.stride(0) % 8 == 0, "ce: logits rows must be 16-byte aligned");
+  tb::ce_loss(bf(logits), logits.stride(0), labels.data_ptr<int64_t>(), row_loss.data_ptr<float>(), (int)logits.size(0),
+              (int)logits.size(1), (int)ignore_index, cur_stream());
+}
 void ce_row_stats(const torch::Tensor& logits, const torch::Tensor& labels, torch::Tensor& stats, int64_t vocab_lo,
                   int64_t ignore_index) {
   TORCH_CHECK(logits.stride(1) == 1 && logits.stride(0) % 8 == 0, "ce: logits rows must be 16-byte aligned");
@@ -262,6 +267,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      pybind11::arg("scale"), pybind11::arg("sq_delta"), pybind11::arg("blocks"),
      pybind11::arg("ids_scratch") = c10::nullopt);
   m.def("ce_softmax_grad", &ce_softmax_grad);
+  m.def("ce_loss", &ce_loss);
   m.def("ce_row_stats", &ce_row_stats);
   m.def("ce_grad_from_lse", &ce_grad_from_lse);
   m.def("cast_to_bf16", &cast_to_bf16);

@@ -160,6 +160,12 @@ def ce_softmax_grad_(logits, labels, row_loss, inv_n_valid, ignore_index):
     ops.count_launch()
 
 
+def ce_loss(logits, labels, row_loss, ignore_index):
+    """row_loss of ``ce_softmax_grad_`` alone; the logits are left as they are."""
+    _C().ce_loss(logits, labels, row_loss, ignore_index)
+    ops.count_launch()
+
+
 def ce_row_stats_(logits, labels, stats, vocab_lo, ignore_index):
     """Vocabulary-sharded CE, first pass: stats (fp32 [3, rows]) <- row maximum, sum of exponentials relative to it,
     target logit (0 when the target lies outside columns [vocab_lo, vocab_lo + V))."""

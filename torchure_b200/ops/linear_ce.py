@@ -14,6 +14,9 @@ V/n rows of the head, and step 2 becomes ``ce_row_stats`` (row maximum, sum of e
 rank's columns), two all-reduces over (chunk,)-sized fp32 vectors (maxima; rescaled sums packed with the target
 logits) and ``ce_grad_from_lse``; ``dH`` is summed over the axis once after the loop.
 
+Without gradients (``no_grad``, or neither input requires one) step 2 is ``ce_loss``, which only reads the logits, and
+steps 3 and 4 fall away.
+
 ``n_valid`` is counted on the device before the loop, so the mean is folded into step 2 and backward only has
 to multiply by the incoming gradient, which a conditional kernel skips when it is exactly 1.
 """
@@ -30,7 +33,7 @@ BF16 = torch.bfloat16
 class _LinearCESm100(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, labels, ignore_index, chunk_size, w_bf16, engine, loss_scale, sink_dest,
-                normalizer=None, vocab_parallel=None):
+                normalizer=None, vocab_parallel=None, want_grad=True):
         N, D = hidden.shape
         V_all = w_bf16.shape[0]   # a sharded strategy may have released the fp32 weight's own storage
         v0, V = 0, V_all
@@ -48,8 +51,9 @@ class _LinearCESm100(torch.autograd.Function):
         n_valid = (labels != ignore_index).sum().clamp_min(1) if normalizer is None else normalizer
         inv_n = (loss_scale / n_valid.float()).reshape(1)
         row_loss = torch.empty(N, dtype=torch.float32, device=dev)
-        need_dh = ctx.needs_input_grad[0]
-        need_dw = ctx.needs_input_grad[1]
+        # under no_grad the parameter still counts as an input that needs a gradient; nothing will ever ask for it
+        need_dh = want_grad and ctx.needs_input_grad[0]
+        need_dw = want_grad and ctx.needs_input_grad[1]
         d_hidden = torch.empty(N, D, dtype=BF16, device=dev) if need_dh else None
         acc0 = False
         if need_dw and sink_dest is not None:
@@ -70,7 +74,9 @@ class _LinearCESm100(torch.autograd.Function):
             hc = h[lo:hi]
             logits = logits_buf[: hi - lo, :V]
             K.gemm(hc, w_bf16, out=logits)
-            if vocab_parallel is None:
+            if vocab_parallel is None and not (need_dh or need_dw):
+                K.ce_loss(logits, labels[lo:hi], row_loss[lo:hi], ignore_index)
+            elif vocab_parallel is None:
                 K.ce_softmax_grad_(logits, labels[lo:hi], row_loss[lo:hi], inv_n, ignore_index)
             else:
                 yc = labels[lo:hi]
@@ -82,7 +88,8 @@ class _LinearCESm100(torch.autograd.Function):
                 all_reduce(packed, *vocab_parallel, "sum")
                 lse = mx + torch.log(packed[0])
                 row_loss[lo:hi] = torch.where(yc != ignore_index, lse - packed[1], torch.zeros_like(lse))
-                K.ce_grad_from_lse_(logits, yc, lse, inv_n, v0, ignore_index)
+                if need_dh or need_dw:
+                    K.ce_grad_from_lse_(logits, yc, lse, inv_n, v0, ignore_index)
             if need_dh:
                 K.gemm(logits, w_bf16, b_mn=True, out=d_hidden[lo:hi])
             if need_dw:
@@ -129,7 +136,7 @@ class _LinearCESm100(torch.autograd.Function):
             elif ctx.in_sink:
                 eng.model._grad_sink.grad_written(eng.model.lm_head.weight)
                 d_weight = None
-        return d_hidden, d_weight, None, None, None, None, None, None, None, None, None
+        return d_hidden, d_weight, None, None, None, None, None, None, None, None, None, None
 
 
 def linear_ce_sm100(hidden, weight, labels, ignore_index, chunk_size, loss_scale=1.0, normalizer=None,
@@ -147,4 +154,4 @@ def linear_ce_sm100(hidden, weight, labels, ignore_index, chunk_size, loss_scale
     else:
         w_bf16 = K.cast_to_bf16(weight.detach().contiguous()) if weight.dtype != BF16 else weight.detach()
     return _LinearCESm100.apply(hidden, weight, labels, ignore_index, chunk_size, w_bf16, eng, float(loss_scale),
-                                sink_dest, normalizer, vocab_parallel)
+                                sink_dest, normalizer, vocab_parallel, torch.is_grad_enabled())
