@@ -144,7 +144,7 @@ class Checkpointer:
 
     def _write_now(self, payload, step: int, name: str) -> None:
         final = self.step_dir(step, create=True) / name
-        tmp = final.with_name(final.name + ".tmp")
+        tmp = final.with_name(f"{final.name}.{os.getpid()}.tmp")   # ranks that share a data coordinate write the same file
         torch.save(payload, tmp)
         os.replace(tmp, final)
 
