@@ -260,6 +260,96 @@ def test_swiglu_fwd_bwd():
     assert relerr(kernels.swiglu_bwd(d, gu), ga.grad) < 5e-3
 
 
+@pytest.mark.parametrize("M,F,K", [(4096, 1536, 256), (4000, 1544, 192), (2304, 2184, 72), (1100, 3080, 520)])
+def test_linear_swiglu_epilogue(M, F, K):
+    """The activation in the product's epilogue: the bits of the product followed by the pass over it, with ragged rows,
+    ragged last column tiles (whose gate half must not spill into the up half) and a ragged last k block."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import debug
+    from torchure_b200.ops import kernels as k
+
+    torch.manual_seed(0)
+    x = torch.randn(M, K, device="cuda").bfloat16()
+    w = (torch.randn(2 * F, K, device="cuda") * 0.2).bfloat16()
+    gu_ref = k.gemm(x, w)
+    act_ref = k.swiglu(gu_ref)
+    debug.enable(True)
+    try:
+        before = ops.launches()
+        gu, act = k.linear_swiglu(x, w)
+        assert ops.launches() - before == 1, "expected the fused kernel"
+        none, alone = k.linear_swiglu(x, w, want_gu=False)
+        assert none is None
+        debug.verify()
+    finally:
+        debug.enable(False)
+    k.check_error()
+    assert torch.equal(gu, gu_ref) and torch.equal(act, act_ref) and torch.equal(alone, act_ref)
+    # few tiles: another kernel and a pass of its own
+    gu, act = k.linear_swiglu(x[:64], w)
+    assert torch.equal(act, k.swiglu(gu))
+
+
+@pytest.mark.parametrize("M,F,K", [(4096, 1536, 2048), (2000, 3088, 2056), (1100, 6160, 2112)])
+def test_swiglu_dgrad_epilogue(M, F, K):
+    """d(gate) and d(up) in the epilogue of d(act) = dy W against fp64 on the same operands; ragged rows, last column tiles of
+    16 columns, a ragged last k block.  Only the results are rounded: 2^-9 relative per element."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import debug
+    from torchure_b200.ops import kernels as k
+
+    torch.manual_seed(0)
+    dy, gu = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(M, 2 * F, device="cuda") * 2).bfloat16()
+    gu[0, :64] = torch.linspace(-200, 200, 64, device="cuda")
+    w = (torch.randn(K, F, device="cuda") * 0.2).bfloat16()
+    debug.enable(True)
+    try:
+        before = ops.launches()
+        got = k.swiglu_dgrad(dy, w, gu)
+        assert ops.launches() - before == 1, "expected the fused kernel"
+        debug.verify()
+    finally:
+        debug.enable(False)
+    k.check_error()
+    two = k.swiglu_bwd(k.linear_dgrad(dy, w), gu)
+    d, g, u = dy.double() @ w.double(), gu[:, :F].double(), gu[:, F:].double()
+    s = torch.sigmoid(g)
+    want = torch.cat([d * u * s * (1 + g * (1 - s)), d * g * s], 1)
+    err = ((got.double() - want).norm() / want.norm()).item()
+    assert err < 2e-3 and err <= ((two.double() - want).norm() / want.norm()).item()
+    # few tiles: the product and a pass of its own
+    assert torch.equal(k.swiglu_dgrad(dy[:64], w, gu[:64]), k.swiglu_bwd(k.linear_dgrad(dy[:64], w), gu[:64]))
+
+
+@pytest.mark.parametrize("C,V,K", [(512, 50257, 128), (300, 32003, 200), (4096, 2056, 64), (257, 65544, 72)])
+def test_gemm_ce_statistics(C, V, K):
+    """Loss from the product's epilogue against the loss pass over stored logits and fp64, over ragged vocabularies (last tile
+    of 1, 3, 8 columns), ragged rows, ignored and out-of-range labels."""
+    from torchure_b200.ops import kernels as k
+
+    torch.manual_seed(0)
+    h = torch.randn(C, K, device="cuda").bfloat16()
+    w = (torch.randn(V, K, device="cuda") * 0.5).bfloat16()
+    y = torch.randint(0, V, (C,), device="cuda")
+    y[0], y[1], y[2::7], y[3] = V - 1, 0, -100, V + 5
+    logits = torch.zeros(C, (V + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")[:, :V]
+    k.gemm(h, w, out=logits)
+    target = torch.full((C,), 7.0, device="cuda")
+    tiles = k.gemm_ce(h, w, y, target)
+    assert tiles is not None, "expected the CTA-pair kernel"
+    lse = torch.logsumexp(tiles[..., 0].double() + tiles[..., 1].double().log(), 0)
+    # fp32 sums of at most 256 terms (2^-24 x 16 relative), exp2 approximate to 2^-22
+    torch.testing.assert_close(lse, torch.logsumexp(logits.double(), 1), rtol=1e-6, atol=2e-6)
+    live = (y >= 0) & (y < V)
+    assert torch.equal(target[live], logits[live].gather(1, y[live, None])[:, 0].float()) and (target[~live] == 7).all()
+    a, b = torch.full((C,), 7.0, device="cuda"), torch.full((C,), 7.0, device="cuda")
+    k.ce_loss_tiles(tiles, target, y, a, V, -100)
+    k.ce_loss(logits, y, b, -100)
+    k.check_error()
+    torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-5)
+    assert (a[2::7] == 0).all()
+
+
 @pytest.mark.parametrize("C,V", [(64, 1000), (300, 5000), (512, 151936), (600, 50264), (130, 32000)])
 def test_ce_softmax_grad(C, V):
     from torchure_b200.ops import kernels

@@ -37,6 +37,19 @@ int gemm_pair_capacity();
 int gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
                bool a_mn, bool b_mn, int out_mode, int splits, int* err, int num_sms, cudaStream_t stream,
                int64_t slice_rows);
+// act [M, F] = silu(A Wg^T) * (A Wu^T) with W [2F, K] = [Wg; Wu]; gu [M, 2F] (optional) receives both factors.  The CTA-pair
+// kernel with another epilogue, for problems gemm_plan gives to it.
+int gemm2_swiglu(const void* A, const void* W, void* gu, void* act, int M, int F, int K, int64_t lda, int64_t ldw, int* err,
+                 int num_sms, cudaStream_t stream);
+// dgu [M, 2F] = d(gate) | d(up) of the SwiGLU unit from d(act) = dy [M, K] W, W [K, F], and the stored gu [M, 2F]; F a multiple
+// of 16, gu 32-byte aligned.  d(act) itself is not stored.
+int gemm2_swiglu_bwd(const void* dy, const void* W, const void* gu, void* dgu, int M, int F, int K, int64_t lda, int64_t ldw,
+                     int* err, int num_sms, cudaStream_t stream);
+// Row statistics of a softmax over A B^T, which is not stored: per row and 256 columns of the product, rounded to bf16, its
+// maximum and the sum of exponentials relative to it, stats [ceil(N / 256)][M] pairs; target [M] receives the logit of each
+// row's label (untouched where the label lies outside [0, N)).
+int gemm2_ce(const void* A, const void* B, int M, int N, int K, int64_t lda, int64_t ldb, const int64_t* labels, float* stats,
+             float* target, int* err, int num_sms, cudaStream_t stream);
 // The kernel for few output tiles (tiles of 128 x tile_n, K slices reduced inside a cluster): tile_n 64, 128 or 256,
 // splits a power of two up to 8 and at most the number of 64-wide k-blocks.
 int gemm_small_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
@@ -83,6 +96,9 @@ void ce_softmax_grad(__nv_bfloat16* logits, int64_t ldl, const int64_t* labels, 
 // row_loss alone, the logits stay as they are
 void ce_loss(const __nv_bfloat16* logits, int64_t ldl, const int64_t* labels, float* row_loss, int C, int V,
              int ignore_index, cudaStream_t stream);
+// row_loss from what gemm2_ce left
+void ce_loss_tiles(const float* tiles, const float* target, const int64_t* labels, float* row_loss, int C, int V,
+                   int ignore_index, cudaStream_t stream);
 // ce_softmax_grad for a vocabulary sharded over ranks (this rank's logits hold columns [vocab_lo, vocab_lo + V)):
 // ce_row_stats writes each row's maximum, sum of exponentials relative to it and target logit (0 when the target is
 // another rank's) to stats[0 / 1 / 2][C]; ce_grad_from_lse, given the log-sum-exp over ALL ranks' columns, overwrites

@@ -61,6 +61,69 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   TORCH_CHECK(rc == 0, "gemm_bf16 failed with code ", rc);
 }
 
+// False (nothing launched) when the problem belongs to another kernel than the CTA-pair one: the caller then runs the
+// product and the element-wise pass.
+bool gemm_swiglu(const torch::Tensor& x, const torch::Tensor& w, c10::optional<torch::Tensor> gu, torch::Tensor& act) {
+  TORCH_CHECK(x.scalar_type() == torch::kBFloat16 && w.scalar_type() == torch::kBFloat16 &&
+                  act.scalar_type() == torch::kBFloat16, "gemm_swiglu: bf16 tensors");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && act.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && act.is_contiguous(),
+              "gemm_swiglu: 2-D operands with innermost stride 1");
+  const int64_t M = x.size(0), K = x.size(1), F = act.size(1);
+  TORCH_CHECK(w.size(0) == 2 * F && w.size(1) == K && act.size(0) == M, "gemm_swiglu: shapes");
+  const bool has_gu = gu.has_value() && gu->defined();
+  TORCH_CHECK(!has_gu || (gu->is_contiguous() && gu->scalar_type() == torch::kBFloat16 && gu->size(0) == M &&
+                          gu->size(1) == 2 * F), "gemm_swiglu: gu must be contiguous bf16 [M, 2F]");
+  if (F % 8 != 0 || M == 0 ||
+      tb::gemm_plan((int)M, (int)(2 * F), (int)K, 0, num_sms(), 0, 0).kind != tb::GemmPlan::kPair)
+    return false;
+  c10::cuda::CUDAGuard guard(x.device());
+  const int rc = tb::gemm2_swiglu(x.data_ptr(), w.data_ptr(), has_gu ? gu->data_ptr() : nullptr, act.data_ptr(), (int)M,
+                                  (int)F, (int)K, x.stride(0), w.stride(0), err_word().data_ptr<int>(), num_sms(),
+                                  cur_stream());
+  TORCH_CHECK(rc == 0, "gemm2_swiglu failed with code ", rc);
+  return true;
+}
+
+// As above.
+bool gemm_swiglu_bwd(const torch::Tensor& dy, const torch::Tensor& w, const torch::Tensor& gu, torch::Tensor& dgu) {
+  TORCH_CHECK(dy.scalar_type() == torch::kBFloat16 && w.scalar_type() == torch::kBFloat16 &&
+                  gu.scalar_type() == torch::kBFloat16 && dgu.scalar_type() == torch::kBFloat16, "gemm_swiglu_bwd: bf16 tensors");
+  TORCH_CHECK(dy.dim() == 2 && w.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && gu.is_contiguous() &&
+                  dgu.is_contiguous(), "gemm_swiglu_bwd: 2-D operands with innermost stride 1");
+  const int64_t M = dy.size(0), K = dy.size(1), F = w.size(1);
+  TORCH_CHECK(w.size(0) == K && gu.size(0) == M && gu.size(1) == 2 * F && dgu.size(0) == M && dgu.size(1) == 2 * F,
+              "gemm_swiglu_bwd: shapes");
+  // below 2048 the epilogue takes longer than the products it should hide behind (figures at the kernel)
+  if (K < 2048 || F % 16 != 0 || M == 0 || (reinterpret_cast<uintptr_t>(gu.data_ptr()) & 31) != 0 ||
+      tb::gemm_plan((int)M, (int)F, (int)K, 0, num_sms(), 0, 0).kind != tb::GemmPlan::kPair)
+    return false;
+  c10::cuda::CUDAGuard guard(dy.device());
+  const int rc = tb::gemm2_swiglu_bwd(dy.data_ptr(), w.data_ptr(), gu.data_ptr(), dgu.data_ptr(), (int)M, (int)F, (int)K,
+                                      dy.stride(0), w.stride(0), err_word().data_ptr<int>(), num_sms(), cur_stream());
+  TORCH_CHECK(rc == 0, "gemm2_swiglu_bwd failed with code ", rc);
+  return true;
+}
+
+// As above.  stats: fp32 [ceil(N / 256), M, 2], target: fp32 [M].
+bool gemm_ce(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& labels, torch::Tensor& stats,
+             torch::Tensor& target) {
+  TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm_ce: bf16 operands");
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && a.size(1) == b.size(1),
+              "gemm_ce: 2-D operands with innermost stride 1");
+  const int64_t M = a.size(0), N = b.size(0), K = a.size(1);
+  TORCH_CHECK(labels.scalar_type() == torch::kInt64 && labels.is_contiguous() && labels.numel() == M, "gemm_ce: labels");
+  TORCH_CHECK(stats.scalar_type() == torch::kFloat32 && stats.is_contiguous() && stats.numel() >= 2 * M * ((N + 255) / 256) &&
+                  target.scalar_type() == torch::kFloat32 && target.is_contiguous() && target.numel() >= M,
+              "gemm_ce: stats must be fp32 [ceil(N / 256), M, 2], target fp32 [M]");
+  if (M == 0 || tb::gemm_plan((int)M, (int)N, (int)K, 0, num_sms(), 0, 0).kind != tb::GemmPlan::kPair) return false;
+  c10::cuda::CUDAGuard guard(a.device());
+  const int rc = tb::gemm2_ce(a.data_ptr(), b.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
+                              labels.data_ptr<int64_t>(), stats.data_ptr<float>(), target.data_ptr<float>(),
+                              err_word().data_ptr<int>(), num_sms(), cur_stream());
+  TORCH_CHECK(rc == 0, "gemm2_ce failed with code ", rc);
+  return true;
+}
+
 void add_rmsnorm_fwd(c10::optional<torch::Tensor> x, c10::optional<torch::Tensor> y, c10::optional<torch::Tensor> ids,
                      c10::optional<torch::Tensor> table, const torch::Tensor& w, c10::optional<torch::Tensor> x_out,
                      torch::Tensor& h, torch::Tensor& rstd, double eps) {
@@ -140,6 +203,11 @@ void ce_loss(const torch::Tensor& logits, const torch::Tensor& labels, torch::Te
   TORCH_CHECK(logits.stride(1) == 1 && logits.stride(0) % 8 == 0, "ce: logits rows must be 16-byte aligned");
   tb::ce_loss(bf(logits), logits.stride(0), labels.data_ptr<int64_t>(), row_loss.data_ptr<float>(), (int)logits.size(0),
               (int)logits.size(1), (int)ignore_index, cur_stream());
+}
+void ce_loss_tiles(const torch::Tensor& tiles, const torch::Tensor& target, const torch::Tensor& labels,
+                   torch::Tensor& row_loss, int64_t V, int64_t ignore_index) {
+  tb::ce_loss_tiles(tiles.data_ptr<float>(), target.data_ptr<float>(), labels.data_ptr<int64_t>(),
+                    row_loss.data_ptr<float>(), (int)labels.numel(), (int)V, (int)ignore_index, cur_stream());
 }
 void ce_row_stats(const torch::Tensor& logits, const torch::Tensor& labels, torch::Tensor& stats, int64_t vocab_lo,
                   int64_t ignore_index) {
@@ -268,6 +336,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
      pybind11::arg("ids_scratch") = c10::nullopt);
   m.def("ce_softmax_grad", &ce_softmax_grad);
   m.def("ce_loss", &ce_loss);
+  m.def("gemm_swiglu", &gemm_swiglu);
+  m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd);
+  m.def("gemm_ce", &gemm_ce);
+  m.def("ce_loss_tiles", &ce_loss_tiles);
   m.def("ce_row_stats", &ce_row_stats);
   m.def("ce_grad_from_lse", &ce_grad_from_lse);
   m.def("cast_to_bf16", &cast_to_bf16);

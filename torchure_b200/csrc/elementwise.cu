@@ -1084,6 +1084,25 @@ ce_softmax_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ldl, const in
   }
 }
 
+// The loss from the row statistics that a product left behind (gemm2_ce), without logits: one warp per row.
+__global__ void __launch_bounds__(256)
+ce_loss_tiles_kernel(const float2* __restrict__ tiles, const float* __restrict__ target, const int64_t* __restrict__ labels,
+                     float* __restrict__ row_loss, int rows, int num_tiles, int V, int ignore_index) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int64_t label = labels[row];
+  float m = -INFINITY, s = 0.f;
+  for (int i = lane; i < num_tiles; i += 32) {
+    const float2 t = tiles[static_cast<int64_t>(i) * rows + row];
+    if (t.x > m) { s = s * __expf(m - t.x) + t.y; m = t.x; }
+    else s += t.y * __expf(t.x - m);
+  }
+  const float gm = warp_max(m);
+  const float gs = warp_sum(m == -INFINITY ? 0.f : s * __expf(m - gm));
+  if (lane == 0)
+    row_loss[row] = label == ignore_index ? 0.f : gm + __logf(gs) - (label >= 0 && label < V ? target[row] : 0.f);
+}
+
 __global__ void __launch_bounds__(256)
 cast_f32_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, int64_t n) {
   const int64_t nvec = n >> 2;
@@ -1269,6 +1288,12 @@ void ce_softmax_grad(__nv_bfloat16* logits, int64_t ldl, const int64_t* labels, 
                      const float* inv_n_valid, int C, int V, int ignore_index, cudaStream_t stream) {
   ce_softmax_grad_kernel<CE_FUSED><<<C, CE_THREADS, 0, stream>>>(logits, ldl, labels, row_loss, inv_n_valid, V,
                                                                  ignore_index, 0, nullptr, nullptr);
+}
+
+void ce_loss_tiles(const float* tiles, const float* target, const int64_t* labels, float* row_loss, int C, int V,
+                   int ignore_index, cudaStream_t stream) {
+  ce_loss_tiles_kernel<<<(C + 7) / 8, 256, 0, stream>>>(reinterpret_cast<const float2*>(tiles), target, labels, row_loss, C,
+                                                        (V + 255) / 256, V, ignore_index);
 }
 
 void ce_loss(const __nv_bfloat16* logits, int64_t ldl, const int64_t* labels, float* row_loss, int C, int V,

@@ -8,8 +8,8 @@ Forward of a block (all bf16 GEMMs on tcgen05, fp32 residual stream)::
     o       = attention(qk, qkv.v)               # causal GQA flash attention, emits LSE
     y_a     = o @ Wo^T
     x2, h2  = add_rmsnorm(x, y_a)
-    gu      = h2 @ [Wgate; Wup]^T                # gate and up as ONE GEMM (N = 2F)
-    y_out   = swiglu(gu) @ Wdown^T               # returned unadded: the next block's norm adds it
+    gu, act = h2 @ [Wgate; Wup]^T, swiglu(gu)    # gate and up as ONE GEMM (N = 2F), the activation in its epilogue
+    y_out   = act @ Wdown^T                      # returned unadded: the next block's norm adds it
 
 Each block returns ``(x2, y_out)``; the sum is never materialised on its own.  Backward mirrors it
 with dgrad (B operand read MN-major, no transposes) and wgrad (both operands MN-major, fp32 output)
@@ -160,6 +160,8 @@ class Sm100Engine:
         B, S = ids.shape
         x, y = None, None
         flat_ids = ids.reshape(-1)
+        # under no_grad the parameters still count as inputs that need gradients
+        want_grad = torch.is_grad_enabled()
         if self.pre_block is not None:
             self.pre_block(-1)
         for i, (block, sh) in enumerate(zip(m.blocks, self.layers)):
@@ -173,7 +175,8 @@ class Sm100Engine:
                 self, sh, i, B, S, flat_ids if first else None,
                 m.token_emb.weight if first else None, x, y,
                 block.norm1.weight, g.q_proj.weight, g.k_proj.weight, g.v_proj.weight, g.o_proj.weight, qn, kn,
-                block.norm2.weight, block.ffn.gate_proj.weight, block.ffn.up_proj.weight, block.ffn.down_proj.weight)
+                block.norm2.weight, block.ffn.gate_proj.weight, block.ffn.up_proj.weight, block.ffn.down_proj.weight,
+                want_grad)
         h = _FinalNormFn.apply(x, y, m.norm.weight, m.norm.eps, self)
         if self.tied and torch.is_grad_enabled() and m.token_emb.weight.requires_grad:
             self.expect_tied_grad = True
@@ -188,7 +191,8 @@ class Sm100Engine:
 
 class _BlockFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, eng, sh, layer_idx, B, S, ids, table, x_in, y_in, w1, wq, wk, wv, wo, qn, kn, w2, wg, wu, wd):
+    def forward(ctx, eng, sh, layer_idx, B, S, ids, table, x_in, y_in, w1, wq, wk, wv, wo, qn, kn, w2, wg, wu, wd,
+                want_grad=True):
         cfg = eng.cfg
         Hq, Hkv, hd, eps = cfg["num_heads"], cfg["num_kv_heads"], cfg["head_dim"], cfg["norm_eps"]
         use_norm = cfg["qk_norm"]
@@ -200,7 +204,7 @@ class _BlockFn(torch.autograd.Function):
             x, h1, rstd1 = K.add_rmsnorm(x_in, y_in, w1, eps)
         qkv = K.linear_fwd(h1, sh.wqkv)
         qk = K.qknorm_rope(qkv, qn, kn, cos, sin, S, Hq, Hkv, eps, use_norm)
-        need_grad = any(ctx.needs_input_grad)
+        need_grad = want_grad and any(ctx.needs_input_grad)
         if eng.cp is not None:
             from torchure_b200.parallel.context_parallel import ring_fwd_sm100
 
@@ -214,8 +218,7 @@ class _BlockFn(torch.autograd.Function):
         if eng.tp is not None:
             eng.tp.all_reduce_(y_a)        # row-parallel: sum the partial products of the ranks' heads
         x2, h2, rstd2 = K.add_rmsnorm(x, y_a, w2, eps)
-        gu = K.linear_fwd(h2, sh.wgu)
-        act = K.swiglu(gu)
+        gu, act = K.linear_swiglu(h2, sh.wgu, want_gu=need_grad)
         y_out = K.linear_fwd(act, sh.wd)
         if eng.tp is not None:
             eng.tp.all_reduce_(y_out)      # ... and of their FFN columns
@@ -242,10 +245,8 @@ class _BlockFn(torch.autograd.Function):
             dx2 = dy.float()
         dy = dy.contiguous()
         # ---- MLP
-        d_act = K.linear_dgrad(dy, sh.wd)
+        d_gu = K.swiglu_dgrad(dy, sh.wd, gu)
         out.wgrad((P["wd"],), dy, act)
-        d_gu = K.swiglu_bwd(d_act, gu)
-        del d_act
         d_h2 = K.linear_dgrad(d_gu, sh.wgu)
         if eng.tp is not None:
             eng.tp.all_reduce_(d_h2)       # column-parallel input gradient: every rank contributes its columns
@@ -329,7 +330,7 @@ class _BlockFn(torch.autograd.Function):
                 dx0 if want_prev else None, dx0_b if want_prev else None,
                 g(P["w1"]), g(P["wq"]), g(P["wk"]), g(P["wv"]), g(P["wo"]),
                 g(P["qn"]) if use_norm else None, g(P["kn"]) if use_norm else None,
-                g(P["w2"]), g(P["wg"]), g(P["wu"]), g(P["wd"]))
+                g(P["w2"]), g(P["wg"]), g(P["wu"]), g(P["wd"]), None)
 
 
 class _GradOut:

@@ -130,9 +130,36 @@ def swiglu(gu):
     return act
 
 
+def linear_swiglu(x, w, want_gu=True):
+    """(gu, act) with gu = x @ w^T (w [2F, K] = gate rows | up rows) and act = silu(gate) * up: one kernel where the product
+    runs on CTA pairs, the product and a pass over it otherwise.  gu is None when it is not wanted (no backward pass)."""
+    M, F = x.shape[0], w.shape[0] // 2
+    act = new_output("linear_swiglu.act", M, F, dtype=BF16, device=x.device)
+    gu = new_output("linear_swiglu.gu", M, 2 * F, dtype=BF16, device=x.device) if want_gu else None
+    if _C().gemm_swiglu(x, w, gu, act):
+        ops.count_launch()
+        return gu, act
+    gu = gemm(x, w, out=gu)
+    _C().swiglu_fwd(gu, act)
+    ops.count_launch()
+    return gu if want_gu else None, act
+
+
 def swiglu_bwd(dact, gu):
     dgu = new_output("swiglu_bwd", gu.shape, dtype=gu.dtype, device=gu.device)
     _C().swiglu_bwd(dact, gu, dgu)
+    ops.count_launch()
+    return dgu
+
+
+def swiglu_dgrad(dy, w, gu):
+    """d(gate) | d(up) [M, 2F] from dy [M, K], the down projection w [K, F] and the stored gu: one kernel where the product
+    d(act) = dy @ w runs on CTA pairs with a long k loop, the product and a pass over it otherwise."""
+    dgu = new_output("swiglu_dgrad", gu.shape, dtype=gu.dtype, device=gu.device)
+    if _C().gemm_swiglu_bwd(dy, w, gu, dgu):
+        ops.count_launch()
+        return dgu
+    _C().swiglu_bwd(linear_dgrad(dy, w), gu, dgu)
     ops.count_launch()
     return dgu
 
@@ -157,6 +184,23 @@ def embedding_scatter_(sources, dtable, M, scale=1.0, sq_delta=None, blocks=592,
 
 def ce_softmax_grad_(logits, labels, row_loss, inv_n_valid, ignore_index):
     _C().ce_softmax_grad(logits, labels, row_loss, inv_n_valid, ignore_index)
+    ops.count_launch()
+
+
+def gemm_ce(a, b, labels, target):
+    """Partial softmax statistics of the rows of a @ b^T, [ceil(N / 256), M, 2] fp32 (maximum and sum of exponentials per 256
+    columns), and the labels' logits in `target`; the product is not stored.  None when the problem runs on another kernel
+    than the CTA-pair one (nothing was launched)."""
+    stats = torch.empty((b.shape[0] + 255) // 256, a.shape[0], 2, dtype=torch.float32, device=a.device)
+    if not _C().gemm_ce(a, b, labels, stats, target):
+        return None
+    ops.count_launch()
+    return stats
+
+
+def ce_loss_tiles(tiles, target, labels, row_loss, vocab, ignore_index):
+    """``ce_loss`` from the statistics and label logits of ``gemm_ce``."""
+    _C().ce_loss_tiles(tiles, target, labels, row_loss, vocab, ignore_index)
     ops.count_launch()
 
 

@@ -14,8 +14,9 @@ V/n rows of the head, and step 2 becomes ``ce_row_stats`` (row maximum, sum of e
 rank's columns), two all-reduces over (chunk,)-sized fp32 vectors (maxima; rescaled sums packed with the target
 logits) and ``ce_grad_from_lse``; ``dH`` is summed over the axis once after the loop.
 
-Without gradients (``no_grad``, or neither input requires one) step 2 is ``ce_loss``, which only reads the logits, and
-steps 3 and 4 fall away.
+Without gradients (``no_grad``, or neither input requires one) steps 3 and 4 fall away, step 1 leaves only the rows'
+softmax statistics and label logits (``gemm_ce``) and step 2 combines them; a chunk too small for the CTA-pair kernel
+stores its logits and runs ``ce_loss`` over them.
 
 ``n_valid`` is counted on the device before the loop, so the mean is folded into step 2 and backward only has
 to multiply by the incoming gradient, which a conditional kernel skips when it is exactly 1.
@@ -47,7 +48,7 @@ class _LinearCESm100(torch.autograd.Function):
             w_bf16 = w_bf16[v0:v0 + V]
         dev = hidden.device
         h = hidden if hidden.dtype == BF16 else hidden.to(BF16)
-        h = h.contiguous()
+        h, labels = h.contiguous(), labels.contiguous()
         n_valid = (labels != ignore_index).sum().clamp_min(1) if normalizer is None else normalizer
         inv_n = (loss_scale / n_valid.float()).reshape(1)
         row_loss = torch.empty(N, dtype=torch.float32, device=dev)
@@ -68,13 +69,21 @@ class _LinearCESm100(torch.autograd.Function):
             d_weight = d_weight[v0:v0 + V]
         chunk = min(chunk_size, N)
         ldl = (V + 7) // 8 * 8
-        logits_buf = torch.empty(chunk, ldl, dtype=BF16, device=dev)
+        logits_buf = None       # allocated by the first chunk that keeps its logits
+        target = torch.empty(chunk, dtype=torch.float32, device=dev) if not (need_dh or need_dw) else None
         for lo in range(0, N, chunk):
             hi = min(N, lo + chunk)
             hc = h[lo:hi]
+            if target is not None and vocab_parallel is None:
+                tiles = K.gemm_ce(hc, w_bf16, labels[lo:hi], target[: hi - lo])
+                if tiles is not None:       # the logits never leave the chip
+                    K.ce_loss_tiles(tiles, target, labels[lo:hi], row_loss[lo:hi], V, ignore_index)
+                    continue
+            if logits_buf is None:
+                logits_buf = torch.empty(chunk, ldl, dtype=BF16, device=dev)
             logits = logits_buf[: hi - lo, :V]
             K.gemm(hc, w_bf16, out=logits)
-            if vocab_parallel is None and not (need_dh or need_dw):
+            if vocab_parallel is None and target is not None:
                 K.ce_loss(logits, labels[lo:hi], row_loss[lo:hi], ignore_index)
             elif vocab_parallel is None:
                 K.ce_softmax_grad_(logits, labels[lo:hi], row_loss[lo:hi], inv_n, ignore_index)
