@@ -605,8 +605,13 @@ GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_spl
   float best = pair ? 6.9f + 0.30f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits)
                     : 5.f + 0.36f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits);
   if (p.splits > 1 && out_mode == 1) best += 3.f;     // C is cleared first
+  // A bf16 product feeds another layer, and sums in another order round differently: it is split only over a K that no block
+  // has (the loss head's dH over the vocabulary, 600 x 512 x 50257: 226 us in one slice, 36 in ten).  The blocks' products then
+  // add up in one order however many rows come along; what splitting them would gain is little (128 x 1024 x 3072: 10.4 us
+  // in one slice, 8.9 in four; 128 x 1024 x 2048: no difference).
+  const bool may_split = out_mode != 0 || num_kb >= 256;
   // K slices through a workspace: only where the tiles leave most of the chip idle for a long K
-  if (pair && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
+  if (may_split && pair && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
     const int s = static_cast<int>(workers / tiles) < num_kb / 16 ? static_cast<int>(workers / tiles) : num_kb / 16;
     if (s > 1) {
       const float run = std::max(0.30f * ceil_div(num_kb, s), cold ? tiles * num_kb * 65536.f / 8.5e6f : 0.f);
@@ -619,7 +624,7 @@ GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_spl
   for (int i = 0; i < 3; ++i) {
     const int64_t t_small = static_cast<int64_t>(ceil_div(M, BM)) * ceil_div(N, kTile[i]);
     if (t_small > 2 * num_sms) continue;
-    for (int s = 1, lg = 0; s <= 8 && s <= num_kb; s *= 2, ++lg) {
+    for (int s = 1, lg = 0; s <= (may_split ? 8 : 1) && s <= num_kb; s *= 2, ++lg) {
       // clusters of 4 and 8 leave SMs of a GPC over
       const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 15 / 16 : num_sms * 7 / 8);
       const int waves = ceil_div(t_small * s, slots);
