@@ -21,6 +21,7 @@ struct GemmPlan {
   int tile_n;         // kSmall: 64, 128 or 256
   int splits;         // K slices
   size_t workspace;   // kSlices: bytes the caller provides
+  bool b_is_old;      // B was not written by the kernel launched just before: kSmall may read it ahead of that one's end
 };
 // The kernel and the K split for a problem.  force_splits > 0 fixes the number of K slices; force_tile_n > 0 selects the
 // kernel for few tiles with that tile width, force_tile_n < 0 the slices through a workspace.
@@ -53,7 +54,8 @@ int gemm2_ce(const void* A, const void* B, int M, int N, int K, int64_t lda, int
 // The kernel for few output tiles (tiles of 128 x tile_n, K slices reduced inside a cluster): tile_n 64, 128 or 256,
 // splits a power of two up to 8 and at most the number of 64-wide k-blocks.
 int gemm_small_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-                    bool a_mn, bool b_mn, int out_mode, int tile_n, int splits, int* err, cudaStream_t stream);
+                    bool a_mn, bool b_mn, int out_mode, int tile_n, int splits, int* err, cudaStream_t stream,
+                    bool b_is_old = false);
 
 // ---- elementwise / normalisation -------------------------------------------------------------
 // h = rmsnorm(x_new) * w with x_new = x (+ y); optional gather x = table[ids].  Writes x_new when y or ids

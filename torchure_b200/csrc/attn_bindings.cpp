@@ -1,5 +1,6 @@
 // Python bindings of the attention kernels.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
 #include <cuda_bf16.h>
@@ -7,6 +8,16 @@
 #include "attn_api.h"
 
 torch::Tensor attn_err_word();
+
+namespace {
+void check_whole(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t B, int64_t Sq, int64_t Skv,
+                 int64_t Hq, int64_t Hkv) {
+  for (const auto* t : {&q, &k, &v})
+    TORCH_CHECK(t->is_contiguous() && t->scalar_type() == torch::kBFloat16, "attention: contiguous bf16 operands");
+  TORCH_CHECK(q.numel() == B * Sq * Hq * 128 && k.numel() == B * Skv * Hkv * 128 && v.numel() == k.numel(),
+              "attention: operand sizes");
+}
+}  // namespace
 
 void register_attn(pybind11::module_& m) {
   m.def("attn_fwd", [](const torch::Tensor& qk, const torch::Tensor& qkv, torch::Tensor& o, torch::Tensor& lse,
@@ -131,6 +142,47 @@ void register_attn(pybind11::module_& m) {
                                       nlse2.data_ptr<float>(), (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal,
                                       attn_err_word().data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream(), &lay);
     TORCH_CHECK(rc == 0, "attn_bwd_pair failed with code ", rc);
+  });
+  // flash_attention's two passes over whole tensors, each as one call: what the entry points above do one at a time
+  // (allocations included), without a round trip through Python per launch
+  m.def("attn_whole_fwd", [](const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t B, int64_t Sq,
+                             int64_t Skv, int64_t Hq, int64_t Hkv, bool causal) {
+    check_whole(q, k, v, B, Sq, Skv, Hq, Hkv);
+    c10::cuda::CUDAGuard guard(q.device());
+    torch::Tensor o = torch::empty({B * Sq, Hq * 128}, q.options());
+    torch::Tensor lse = torch::empty({B, Hq, Sq}, q.options().dtype(torch::kFloat32));
+    const int rc = tb::attn_fwd_pair({q.data_ptr(), Hq * 128, 0}, {k.data_ptr(), Hkv * 128, 0}, {v.data_ptr(), Hkv * 128, 0},
+                                     o.data_ptr(), lse.data_ptr<float>(), (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv,
+                                     B * Sq, (int)Sq, 0, B * Skv, (int)Skv, 0, causal, attn_err_word().data_ptr<int>(),
+                                     at::cuda::getCurrentCUDAStream().stream());
+    TORCH_CHECK(rc == 0, "attn_fwd_pair failed with code ", rc);
+    return std::make_tuple(o, lse);
+  });
+  m.def("attn_whole_bwd", [](const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, const torch::Tensor& o,
+                             const torch::Tensor& lse, const torch::Tensor& d_o, int64_t B, int64_t Sq, int64_t Skv,
+                             int64_t Hq, int64_t Hkv, bool causal) {
+    check_whole(q, k, v, B, Sq, Skv, Hq, Hkv);
+    TORCH_CHECK(d_o.is_contiguous() && d_o.scalar_type() == torch::kBFloat16 && d_o.numel() == q.numel() &&
+                o.is_contiguous() && o.numel() == q.numel() && lse.is_contiguous() && lse.numel() == B * Hq * Sq,
+                "attention backward: operands");
+    c10::cuda::CUDAGuard guard(q.device());
+    auto stream = at::cuda::getCurrentCUDAStream().stream();
+    torch::Tensor stats = torch::empty({2, B * Hq * Sq}, lse.options());
+    torch::Tensor dq_acc = torch::empty({B * Sq, Hq * 128}, lse.options());      // [B, Hq, Sq, 128]
+    torch::Tensor dq = torch::empty({B * Sq, Hq * 128}, q.options());
+    torch::Tensor dk = torch::empty({B * Skv, Hkv * 128}, q.options()), dv = torch::empty({B * Skv, Hkv * 128}, q.options());
+    float* nds = stats.data_ptr<float>();
+    float* nlse2 = nds + B * Hq * Sq;
+    int rc = tb::attn_bwd_stats(d_o.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), nds, nlse2, dq_acc.data_ptr<float>(),
+                                (int)B, (int)Sq, (int)Hq, stream);
+    TORCH_CHECK(rc == 0, "attn_bwd_stats failed with code ", rc);
+    rc = tb::attn_bwd_fused({q.data_ptr(), Hq * 128, 0}, {k.data_ptr(), Hkv * 128, 0}, {v.data_ptr(), Hkv * 128, 0},
+                            d_o.data_ptr(), dq_acc.data_ptr<float>(), dk.data_ptr(), dv.data_ptr(), Hkv * 128, nds, nlse2,
+                            (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, attn_err_word().data_ptr<int>(), stream);
+    TORCH_CHECK(rc == 0, "attn_bwd_fused failed with code ", rc);
+    rc = tb::attn_dq_convert(dq_acc.data_ptr<float>(), dq.data_ptr(), Hq * 128, (int)B, (int)Sq, (int)Hq, stream);
+    TORCH_CHECK(rc == 0, "dq conversion failed with code ", rc);
+    return std::make_tuple(dq, dk, dv);
   });
   m.def("attn_dq_convert", [](const torch::Tensor& dq_acc, torch::Tensor& dst, int64_t B, int64_t S, int64_t Hq) {
     TORCH_CHECK(dq_acc.is_contiguous() && dst.dim() == 2 && dst.stride(1) == 1 && dst.size(0) == B * S);

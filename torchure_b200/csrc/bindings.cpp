@@ -4,6 +4,7 @@
 #include <torch/extension.h>
 
 #include "api.h"
+#include "bind_common.h"
 #include "comm_api.h"
 #include "attn_api.h"
 
@@ -39,7 +40,7 @@ T* opt_mptr(c10::optional<torch::Tensor>& t) {
 }
 
 void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
-          int64_t splits, int64_t tile_n) {
+          int64_t splits, int64_t tile_n, bool b_is_old = false) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda(), "gemm: CUDA tensors required");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm: bf16 operands");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2, "gemm: 2-D tensors");
@@ -51,7 +52,8 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   TORCH_CHECK(out_mode == 0 ? out.scalar_type() == torch::kBFloat16 : out.scalar_type() == torch::kFloat32,
               "gemm: output dtype does not match out_mode");
   c10::cuda::CUDAGuard guard(a.device());
-  const tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, (int)out_mode, num_sms(), (int)splits, (int)tile_n);
+  tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, (int)out_mode, num_sms(), (int)splits, (int)tile_n);
+  plan.b_is_old = b_is_old;
   torch::Tensor ws;
   if (plan.workspace > 0) ws = torch::empty({(int64_t)plan.workspace}, a.options().dtype(torch::kUInt8));
   const int rc = tb::gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0),
@@ -281,12 +283,25 @@ torch::Tensor error_word() { return err_word(); }
 }  // namespace
 
 torch::Tensor attn_err_word() { return err_word(); }
+int bind_num_sms() { return num_sms(); }
+void bind_gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
+               int64_t splits, int64_t tile_n, bool b_is_old) {
+  gemm(a, b, out, a_mn, b_mn, out_mode, splits, tile_n, b_is_old);
+}
+bool bind_gemm_swiglu(const torch::Tensor& x, const torch::Tensor& w, c10::optional<torch::Tensor> gu, torch::Tensor& act) {
+  return gemm_swiglu(x, w, gu, act);
+}
+bool bind_gemm_swiglu_bwd(const torch::Tensor& dy, const torch::Tensor& w, const torch::Tensor& gu, torch::Tensor& dgu) {
+  return gemm_swiglu_bwd(dy, w, gu, dgu);
+}
 
 void register_comm(pybind11::module_& m);
 void register_attn(pybind11::module_& m);
+void register_block(pybind11::module_& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("gemm", &gemm, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
+  m.def("gemm", [](const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
+                   int64_t splits, int64_t tile_n) { gemm(a, b, out, a_mn, b_mn, out_mode, splits, tile_n); }, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
         pybind11::arg("b"), pybind11::arg("out"), pybind11::arg("a_mn"), pybind11::arg("b_mn"), pybind11::arg("out_mode"),
         pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0);
   m.def("set_sm_reserve", [](int64_t n) { g_sm_reserve = (int)n; }, "persistent kernels use (SM count - n) CTAs");
@@ -357,4 +372,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bucket_pack_multi", &bucket_pack_multi);
   register_comm(m);
   register_attn(m);
+  register_block(m);
 }

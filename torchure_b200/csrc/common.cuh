@@ -6,6 +6,8 @@
 // the host can report which wait expired.
 #pragma once
 
+#include "pdl.h"
+
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -31,7 +33,7 @@ inline bool pdl_enabled() {
     const char* e = std::getenv("TORCHURE_B200_PDL");
     return e && e[0] == '1';
   }();
-  return on;
+  return on || t_pdl_scope;
 }
 
 template <typename... KArgs, typename... Args>

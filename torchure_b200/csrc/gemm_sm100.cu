@@ -650,7 +650,8 @@ int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_
   if (M <= 0 || N <= 0 || K <= 0) return -1;
   int splits = plan.splits;
   if (plan.kind == GemmPlan::kSmall)
-    return gemm_small_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, plan.tile_n, splits, err, stream);
+    return gemm_small_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, plan.tile_n, splits, err, stream,
+                           plan.b_is_old);
   if (plan.kind == GemmPlan::kSlices) {
     const int64_t slice_rows = static_cast<int64_t>((M + 2 * BM - 1) / (2 * BM)) * 2 * BM, ldw = (N + 3) / 4 * 4;
     if (workspace == nullptr) return -4;

@@ -87,9 +87,15 @@ __device__ __forceinline__ void put(void* C, int64_t at, float (&f)[VEC], int n)
 template <bool A_MN, bool B_MN, int OUT, int BN>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, void* C, int64_t ldc, int M, int N, int K, int splits, int* err) {
-  pdl_wait();
-  pdl_launch_dependents();
+                  const __grid_constant__ CUtensorMap tmC, void* C, int64_t ldc, int M, int N, int K, int splits, int early_b,
+                  int* err) {
+  // early_b: launched while the kernel before still runs, which has not written B.  Set-up and the first B tiles (weights that
+  // come from memory when the problem is small) then run under that kernel's tail; A, and with it everything that
+  // follows, waits for its end in the producer thread.
+  if (!early_b) {
+    pdl_wait();
+    pdl_launch_dependents();
+  }
   using P = Plan<BN>;
   constexpr int STAGES = P::STAGES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -135,11 +141,28 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
+      auto load_b = [&](int st, int k0) {
+        uint8_t* sB = smem + st * P::STAGE_BYTES + A_BYTES;
+        if (!B_MN) {
+          tma_load_2d(sB, &tmB, &full[st], k0, n0);
+        } else {
+#pragma unroll
+          for (int j = 0; j < BN / 64; ++j) tma_load_2d(sB + j * 8192, &tmB, &full[st], n0 + j * 64, k0);
+        }
+      };
+      const int ahead = early_b ? min(kb1, kb0 + STAGES) : kb0;     // k-blocks whose B is on its way
+      if (early_b) {
+        for (int kb = kb0; kb < ahead; ++kb) {
+          mbar_expect_tx(&full[kb - kb0], P::STAGE_BYTES);
+          load_b(kb - kb0, kb * BK);
+        }
+        pdl_wait();
+        pdl_launch_dependents();
+      }
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, err, kErrProducerEmptyWait)) break;
         uint8_t* sA = smem + stage * P::STAGE_BYTES;
-        uint8_t* sB = sA + A_BYTES;
-        mbar_expect_tx(&full[stage], P::STAGE_BYTES);
+        if (kb >= ahead) mbar_expect_tx(&full[stage], P::STAGE_BYTES);
         const int k0 = kb * BK;
         if (!A_MN) {
           tma_load_2d(sA, &tmA, &full[stage], k0, m0);
@@ -147,12 +170,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
           for (int j = 0; j < BM / 64; ++j) tma_load_2d(sA + j * 8192, &tmA, &full[stage], m0 + j * 64, k0);
         }
-        if (!B_MN) {
-          tma_load_2d(sB, &tmB, &full[stage], k0, n0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < BN / 64; ++j) tma_load_2d(sB + j * 8192, &tmB, &full[stage], n0 + j * 64, k0);
-        }
+        if (kb >= ahead) load_b(stage, k0);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
@@ -287,7 +305,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
 template <bool A_MN, bool B_MN, int OUT, int BN>
 int launch_small(const CUtensorMap& ta, const CUtensorMap& tb_, const CUtensorMap& tc, void* C, int64_t ldc, int M, int N,
-                 int K, int splits, int* err, cudaStream_t stream) {
+                 int K, int splits, int* err, cudaStream_t stream, bool b_is_old) {
   auto kern = gemm_small_kernel<A_MN, B_MN, OUT, BN>;
   if (!ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Plan<BN>::SMEM_BYTES)) return -20;
   cudaLaunchConfig_t cfg{};
@@ -304,13 +322,17 @@ int launch_small(const CUtensorMap& ta, const CUtensorMap& tb_, const CUtensorMa
   attr[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kern, ta, tb_, tc, C, ldc, M, N, K, splits, err) == cudaSuccess ? 0 : -21;
+  return cudaLaunchKernelEx(&cfg, kern, ta, tb_, tc, C, ldc, M, N, K, splits, b_is_old && pdl_enabled() ? 1 : 0, err) ==
+                 cudaSuccess
+             ? 0
+             : -21;
 }
 
 }  // namespace
 
 int gemm_small_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
-                    bool a_mn, bool b_mn, int out_mode, int tile_n, int splits, int* err, cudaStream_t stream) {
+                    bool a_mn, bool b_mn, int out_mode, int tile_n, int splits, int* err, cudaStream_t stream,
+                    bool b_is_old) {
   const int num_kb = (K + BK - 1) / BK;
   if (splits < 1 || splits > 8 || (splits & (splits - 1)) || splits > num_kb) return -3;
   CUtensorMap ta, tb_, tc;
@@ -322,7 +344,7 @@ int gemm_small_bf16(const void* A, const void* B, void* C, int M, int N, int K, 
   r = out_mode == 0 ? make_tmap_2d(&tc, C, 2, M, N, ldc, 32, 64) : make_tmap_2d(&tc, C, 4, M, N, ldc, 32, 32);
   if (r) return r - 200;
 #define TB_SMALL_BN(AM, BMN, O, W) \
-  if (tile_n == W) return launch_small<AM, BMN, O, W>(ta, tb_, tc, C, ldc, M, N, K, splits, err, stream);
+  if (tile_n == W) return launch_small<AM, BMN, O, W>(ta, tb_, tc, C, ldc, M, N, K, splits, err, stream, b_is_old);
 #define TB_SMALL_CASE(AM, BMN, O)                    \
   if (a_mn == AM && b_mn == BMN && out_mode == O) {  \
     TB_SMALL_BN(AM, BMN, O, 64)                      \

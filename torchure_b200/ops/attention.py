@@ -90,6 +90,11 @@ def attn_fwd(qk, qkv, B, S, Hq, Hkv, hd, need_grad=True):
     return out.transpose(1, 2).reshape(B * S, Hq * hd), AttnState("sdpa")
 
 
+def single_pass(state) -> bool:
+    """True when ``attn_bwd`` would run the single-pass kernel on this forward's state."""
+    return isinstance(state, AttnState) and state.impl == "sm100" and _BWD == "fused"
+
+
 def attn_bwd(d_o, qk, qkv, state: AttnState, B, S, Hq, Hkv, hd, keep_dq_fp32: bool = False):
     """Returns dqkv (M, (Hq+2Hkv)*hd) bf16 = [dq (post-rope) | dk (post-rope) | dv].
 
@@ -137,16 +142,14 @@ def _rows(t: torch.Tensor) -> torch.Tensor:
 
 class _FlashAttention(torch.autograd.Function):
     """Full-sequence attention on separate q / k / v tensors through the block-pair entry points of the sm_100a
-    kernels: ``attn_fwd_pair`` forward, ``attn_bwd_stats`` + ``attn_bwd_pair`` + ``attn_dq_convert`` backward."""
+    kernels, each pass one native call: the forward kernel, then statistics, single-pass backward and dQ conversion."""
 
     @staticmethod
     def forward(ctx, q, k, v, causal):
         B, Sq, Hq, _ = q.shape
         Skv, Hkv = k.shape[1], k.shape[2]
         q2, k2, v2 = _rows(q), _rows(k), _rows(v)
-        o = torch.empty(B * Sq, Hq * 128, dtype=torch.bfloat16, device=q.device)
-        lse = torch.empty(B, Hq, Sq, dtype=torch.float32, device=q.device)
-        ops.ext().attn_fwd_pair(q2, 0, k2, 0, v2, 0, o, lse, B, Sq, Skv, Hq, Hkv, Sq, 0, Skv, 0, bool(causal))
+        o, lse = ops.ext().attn_whole_fwd(q2, k2, v2, B, Sq, Skv, Hq, Hkv, bool(causal))
         ops.count_launch()
         ctx.save_for_backward(q2, k2, v2, o, lse)
         ctx.dims = (B, Sq, Skv, Hq, Hkv, bool(causal))
@@ -156,19 +159,8 @@ class _FlashAttention(torch.autograd.Function):
     def backward(ctx, d_o):
         q2, k2, v2, o, lse = ctx.saved_tensors
         B, Sq, Skv, Hq, Hkv, causal = ctx.dims
-        ext = ops.ext()
         d_o2 = _rows(d_o.to(torch.bfloat16))
-        dev = q2.device
-        nds = torch.empty(B, Hq, Sq, dtype=torch.float32, device=dev)
-        nlse2 = torch.empty_like(nds)
-        dq_acc = torch.empty(B, Hq, Sq, 128, dtype=torch.float32, device=dev)
-        ext.attn_bwd_stats(d_o2, o, lse, nds, nlse2, dq_acc, B, Sq, Hq)
-        dk = torch.empty(B * Skv, Hkv * 128, dtype=torch.bfloat16, device=dev)
-        dv = torch.empty_like(dk)
-        ext.attn_bwd_pair(q2, 0, k2, 0, v2, 0, d_o2, dq_acc, dk, dv, nds, nlse2, B, Sq, Skv, Hq, Hkv, Sq, 0, Skv, 0, Sq, 0,
-                          causal)
-        dq = torch.empty(B * Sq, Hq * 128, dtype=torch.bfloat16, device=dev)
-        ext.attn_dq_convert(dq_acc, dq, B, Sq, Hq)
+        dq, dk, dv = ops.ext().attn_whole_bwd(q2, k2, v2, o, lse, d_o2, B, Sq, Skv, Hq, Hkv, causal)
         ops.count_launch(3)
         return dq.view(B, Sq, Hq, 128), dk.view(B, Skv, Hkv, 128), dv.view(B, Skv, Hkv, 128), None
 

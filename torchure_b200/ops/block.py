@@ -27,7 +27,9 @@ import weakref
 
 import torch
 
+from torchure_b200 import ops
 from torchure_b200.ops import attention as attn_ops
+from torchure_b200.ops import debug
 from torchure_b200.ops import kernels as K
 
 BF16 = torch.bfloat16
@@ -60,11 +62,24 @@ class _LayerShadow:
                            wo=g.o_proj.weight, qn=g.q_norm.weight if g.qk_norm else None,
                            kn=g.k_norm.weight if g.qk_norm else None, w2=block.norm2.weight,
                            wg=f.gate_proj.weight, wu=f.up_proj.weight, wd=f.down_proj.weight, table=None)
+        self._modules = (block.norm1, g.q_proj, g.k_proj, g.v_proj, g.o_proj, g.q_norm if g.qk_norm else None,
+                         g.k_norm if g.qk_norm else None, block.norm2, f.gate_proj, f.up_proj, f.down_proj)
         self.pairs = [
             (g.q_proj.weight, self.wqkv[:nq]), (g.k_proj.weight, self.wqkv[nq:nq + nkv]),
             (g.v_proj.weight, self.wqkv[nq + nkv:]), (g.o_proj.weight, self.wo),
             (f.gate_proj.weight, self.wgu[:F_]), (f.up_proj.weight, self.wgu[F_:]), (f.down_proj.weight, self.wd),
         ]
+
+
+    def inputs(self, dummy):
+        """The block's parameters in the order of ``_BlockFn``, as the modules hold them now; without QK-norm its gains are
+        the engine's dummy.  Read from the modules' tables: attribute look-ups through ``Module.__getattr__`` cost a short
+        forward pass 7 us per block."""
+        out = []
+        for m in self._modules:
+            w = dummy if m is None else m._parameters.get("weight")
+            out.append(m.weight if w is None else w)
+        return out
 
 
 class Sm100Engine:
@@ -164,18 +179,14 @@ class Sm100Engine:
         want_grad = torch.is_grad_enabled()
         if self.pre_block is not None:
             self.pre_block(-1)
-        for i, (block, sh) in enumerate(zip(m.blocks, self.layers)):
+        for i, sh in enumerate(self.layers):
             if self.pre_block is not None:
                 self.pre_block(i)
-            g = block.gqa
-            qn = g.q_norm.weight if g.qk_norm else self.dummy
-            kn = g.k_norm.weight if g.qk_norm else self.dummy
             first = i == 0
             x, y = _BlockFn.apply(
                 self, sh, i, B, S, flat_ids if first else None,
                 m.token_emb.weight if first else None, x, y,
-                block.norm1.weight, g.q_proj.weight, g.k_proj.weight, g.v_proj.weight, g.o_proj.weight, qn, kn,
-                block.norm2.weight, block.ffn.gate_proj.weight, block.ffn.up_proj.weight, block.ffn.down_proj.weight,
+                *sh.inputs(self.dummy),
                 want_grad)
         h = _FinalNormFn.apply(x, y, m.norm.weight, m.norm.eps, self)
         if self.tied and torch.is_grad_enabled() and m.token_emb.weight.requires_grad:
@@ -197,31 +208,38 @@ class _BlockFn(torch.autograd.Function):
         Hq, Hkv, hd, eps = cfg["num_heads"], cfg["num_kv_heads"], cfg["head_dim"], cfg["norm_eps"]
         use_norm = cfg["qk_norm"]
         cos, sin = eng.rope_tables(S, w1.device)
-        if ids is not None:
-            x, h1, rstd1 = K.add_rmsnorm(None, None, w1, eps, ids=ids,
-                                         table=eng.emb_shadow if eng.bf16_embedding else table)
-        else:
-            x, h1, rstd1 = K.add_rmsnorm(x_in, y_in, w1, eps)
-        qkv = K.linear_fwd(h1, sh.wqkv)
-        qk = K.qknorm_rope(qkv, qn, kn, cos, sin, S, Hq, Hkv, eps, use_norm)
         need_grad = want_grad and any(ctx.needs_input_grad)
-        if eng.cp is not None:
-            from torchure_b200.parallel.context_parallel import ring_fwd_sm100
-
-            # q is used where it lies in `qk`; K and V travel around the ring, so they get buffers of their own
-            k2, v2 = qk[:, Hq * hd:].contiguous(), qkv[:, (Hq + Hkv) * hd:].contiguous()
-            o, lse = ring_fwd_sm100(qk, 0, k2, v2, B, S, Hq, Hkv, *eng.cp)
-            st = (k2, v2, lse)
+        table_used = eng.emb_shadow if eng.bf16_embedding else table
+        if eng.cp is None and eng.tp is None and not debug.enabled() and attn_ops.kernel_supported(S, Hq, Hkv, hd):
+            (x, h1, rstd1, qkv, qk, o, lse, x2, h2, rstd2, gu, act, y_out), n = ops.ext().block_forward(
+                x_in, y_in, ids, table_used, w1, sh.wqkv, qn, kn, cos, sin, sh.wo, w2, sh.wgu, sh.wd, B, S, Hq, Hkv, eps,
+                use_norm, need_grad)
+            ops.count_launch(n)
+            st = attn_ops.AttnState("sm100", o, lse)
         else:
-            o, st = attn_ops.attn_fwd(qk, qkv, B, S, Hq, Hkv, hd, need_grad=need_grad)
-        y_a = K.linear_fwd(o, sh.wo)
-        if eng.tp is not None:
-            eng.tp.all_reduce_(y_a)        # row-parallel: sum the partial products of the ranks' heads
-        x2, h2, rstd2 = K.add_rmsnorm(x, y_a, w2, eps)
-        gu, act = K.linear_swiglu(h2, sh.wgu, want_gu=need_grad)
-        y_out = K.linear_fwd(act, sh.wd)
-        if eng.tp is not None:
-            eng.tp.all_reduce_(y_out)      # ... and of their FFN columns
+            if ids is not None:
+                x, h1, rstd1 = K.add_rmsnorm(None, None, w1, eps, ids=ids, table=table_used)
+            else:
+                x, h1, rstd1 = K.add_rmsnorm(x_in, y_in, w1, eps)
+            qkv = K.linear_fwd(h1, sh.wqkv)
+            qk = K.qknorm_rope(qkv, qn, kn, cos, sin, S, Hq, Hkv, eps, use_norm)
+            if eng.cp is not None:
+                from torchure_b200.parallel.context_parallel import ring_fwd_sm100
+
+                # q is used where it lies in `qk`; K and V travel around the ring, so they get buffers of their own
+                k2, v2 = qk[:, Hq * hd:].contiguous(), qkv[:, (Hq + Hkv) * hd:].contiguous()
+                o, lse = ring_fwd_sm100(qk, 0, k2, v2, B, S, Hq, Hkv, *eng.cp)
+                st = (k2, v2, lse)
+            else:
+                o, st = attn_ops.attn_fwd(qk, qkv, B, S, Hq, Hkv, hd, need_grad=need_grad)
+            y_a = K.linear_fwd(o, sh.wo)
+            if eng.tp is not None:
+                eng.tp.all_reduce_(y_a)        # row-parallel: sum the partial products of the ranks' heads
+            x2, h2, rstd2 = K.add_rmsnorm(x, y_a, w2, eps)
+            gu, act = K.linear_swiglu(h2, sh.wgu, want_gu=need_grad)
+            y_out = K.linear_fwd(act, sh.wd)
+            if eng.tp is not None:
+                eng.tp.all_reduce_(y_out)      # ... and of their FFN columns
         ctx.eng, ctx.sh, ctx.dims = eng, sh, (B, S, Hq, Hkv, hd, eps, use_norm)
         ctx.attn_state = st
         ctx.first = ids is not None
@@ -243,64 +261,85 @@ class _BlockFn(torch.autograd.Function):
             dy = dx2.to(BF16)
         if dx2 is None:
             dx2 = dy.float()
-        dy = dy.contiguous()
-        # ---- MLP
-        d_gu = K.swiglu_dgrad(dy, sh.wd, gu)
-        out.wgrad((P["wd"],), dy, act)
-        d_h2 = K.linear_dgrad(d_gu, sh.wgu)
-        if eng.tp is not None:
-            eng.tp.all_reduce_(d_h2)       # column-parallel input gradient: every rank contributes its columns
-        out.wgrad((P["wg"], P["wu"]), d_gu, h2)
-        del d_gu
-        dw2 = out.small(P["w2"])
-        dx1, dx1_b = K.rmsnorm_bwd(d_h2, x2, w2, rstd2, dx2, dw2)
-        out.done(P["w2"])
-        del d_h2
-        # ---- attention
-        d_o = K.linear_dgrad(dx1_b, sh.wo)
-        out.wgrad((P["wo"],), dx1_b, o)
-        if eng.cp is not None:
-            from torchure_b200.parallel.context_parallel import ring_bwd_sm100
-
-            k2, v2, lse = ctx.attn_state
-            dq_acc, dk, dv = ring_bwd_sm100(qk, 0, k2, v2, o, lse, d_o, B, S, Hq, Hkv, *eng.cp)
-            dqkv = torch.empty(B * S, nq + 2 * nkv, dtype=BF16, device=d_o.device)   # q columns: read from dq_acc
-            dqkv[:, nq:nq + nkv].copy_(dk.view(B * S, nkv))
-            dqkv[:, nq + nkv:].copy_(dv.view(B * S, nkv))
-            del k2, v2, lse, dk, dv
-        else:
-            dqkv, dq_acc = attn_ops.attn_bwd(d_o, qk, qkv, ctx.attn_state, B, S, Hq, Hkv, hd, keep_dq_fp32=True)
-        ctx.attn_state = None
-        del d_o
-        if use_norm:
-            dqn, dkn = out.small(P["qn"]), out.small(P["kn"])
-        else:
-            dqn = dkn = eng.dummy
-        if use_norm and eng.tp is not None:
-            # the gains are shared by all heads while each rank sees only its own: this backward's contribution is
-            # summed over the axis before it joins the (possibly running) destination
-            part = torch.zeros(2, dqn.numel(), dtype=torch.float32, device=dqn.device)
-            K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, part[0], part[1], S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc)
-            eng.tp.all_reduce_(part)
-            dqn.add_(part[0])
-            dkn.add_(part[1])
-        else:
-            K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, dqn, dkn, S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc)
-        del dq_acc
-        if use_norm:
-            out.done(P["qn"])
-            out.done(P["kn"])
-        d_h1 = K.linear_dgrad(dqkv, sh.wqkv)
-        if eng.tp is not None:
-            eng.tp.all_reduce_(d_h1)
-        out.wgrad((P["wq"], P["wk"], P["wv"]), dqkv, h1)
-        del dqkv
-        dw1 = out.small(P["w1"])
+        dy, dx2 = dy.contiguous(), dx2.contiguous()
         want_prev = not ctx.first
         early = ctx.first and eng.pending_tied_grad is EARLY_TABLE
         # with the row exchange, dx0 is written where the other ranks can read it
         dx_out = out.sink.embed_rows_dest(x.shape[0], x.shape[1]) if early else None
-        dx0, dx0_b = K.rmsnorm_bwd(d_h1, x, w1, rstd1, dx1, dw1, want_bf16=want_prev, dx_out=dx_out)
+        dests = None
+        # ranks that reduce gradients under the backward pass are told of each one as it is launched (the other branch)
+        if (eng.cp is None and eng.tp is None and not debug.enabled() and attn_ops.single_pass(ctx.attn_state)
+                and (out.sink is None or getattr(out.sink, "world", 0) == 1)):
+            dests = [out.dest(ps) for ps in ((P["wd"],), (P["wg"], P["wu"]), (P["wo"],), (P["wq"], P["wk"], P["wv"]))]
+        if dests is not None and None not in dests:
+            (dwd, add_d), (dwgu, add_gu), (dwo, add_o), (dwqkv, add_qkv) = dests
+            gains = [P["w2"]] + ([P["qn"], P["kn"]] if use_norm else []) + [P["w1"]]
+            small = out.smalls(gains)
+            dw2, dw1 = small[0], small[-1]
+            dqn, dkn = small[1:3] if use_norm else (eng.dummy, eng.dummy)
+            dx1, dx1_b, n_mlp = ops.ext().block_backward_mlp(dx2, dy, gu, act, h2, x2, w2, rstd2, sh.wgu, sh.wd, dwd, add_d, dwgu,
+                                                             add_gu, dw2)
+            out.written((P["wd"], P["wg"], P["wu"], P["w2"]))
+            dx0, dx0_b, n_attn = ops.ext().block_backward_attn(
+                dx1, dx1_b, o, ctx.attn_state.lse, qk, qkv, h1, x, w1, rstd1, qn, kn, cos, sin, sh.wqkv, sh.wo, dwo, add_o,
+                dwqkv, add_qkv, dqn, dkn, dw1, dx_out, want_prev, B, S, Hq, Hkv, eps, use_norm)
+            out.written((P["wo"], P["wq"], P["wk"], P["wv"], *gains[1:-1]))
+            ctx.attn_state = None
+            ops.count_launch(n_mlp + n_attn)
+        else:
+            # ---- MLP
+            d_gu = K.swiglu_dgrad(dy, sh.wd, gu)
+            out.wgrad((P["wd"],), dy, act)
+            d_h2 = K.linear_dgrad(d_gu, sh.wgu)
+            if eng.tp is not None:
+                eng.tp.all_reduce_(d_h2)       # column-parallel input gradient: every rank contributes its columns
+            out.wgrad((P["wg"], P["wu"]), d_gu, h2)
+            del d_gu
+            dw2 = out.small(P["w2"])
+            dx1, dx1_b = K.rmsnorm_bwd(d_h2, x2, w2, rstd2, dx2, dw2)
+            out.done(P["w2"])
+            del d_h2
+            # ---- attention
+            d_o = K.linear_dgrad(dx1_b, sh.wo)
+            out.wgrad((P["wo"],), dx1_b, o)
+            if eng.cp is not None:
+                from torchure_b200.parallel.context_parallel import ring_bwd_sm100
+
+                k2, v2, lse = ctx.attn_state
+                dq_acc, dk, dv = ring_bwd_sm100(qk, 0, k2, v2, o, lse, d_o, B, S, Hq, Hkv, *eng.cp)
+                dqkv = torch.empty(B * S, nq + 2 * nkv, dtype=BF16, device=d_o.device)   # q columns: read from dq_acc
+                dqkv[:, nq:nq + nkv].copy_(dk.view(B * S, nkv))
+                dqkv[:, nq + nkv:].copy_(dv.view(B * S, nkv))
+                del k2, v2, lse, dk, dv
+            else:
+                dqkv, dq_acc = attn_ops.attn_bwd(d_o, qk, qkv, ctx.attn_state, B, S, Hq, Hkv, hd, keep_dq_fp32=True)
+            ctx.attn_state = None
+            del d_o
+            if use_norm:
+                dqn, dkn = out.small(P["qn"]), out.small(P["kn"])
+            else:
+                dqn = dkn = eng.dummy
+            if use_norm and eng.tp is not None:
+                # the gains are shared by all heads while each rank sees only its own: this backward's contribution is
+                # summed over the axis before it joins the (possibly running) destination
+                part = torch.zeros(2, dqn.numel(), dtype=torch.float32, device=dqn.device)
+                K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, part[0], part[1], S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc)
+                eng.tp.all_reduce_(part)
+                dqn.add_(part[0])
+                dkn.add_(part[1])
+            else:
+                K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, dqn, dkn, S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc)
+            del dq_acc
+            if use_norm:
+                out.done(P["qn"])
+                out.done(P["kn"])
+            d_h1 = K.linear_dgrad(dqkv, sh.wqkv)
+            if eng.tp is not None:
+                eng.tp.all_reduce_(d_h1)
+            out.wgrad((P["wq"], P["wk"], P["wv"]), dqkv, h1)
+            del dqkv
+            dw1 = out.small(P["w1"])
+            dx0, dx0_b = K.rmsnorm_bwd(d_h1, x, w1, rstd1, dx1, dw1, want_bf16=want_prev, dx_out=dx_out)
         out.done(P["w1"])
         if early:
             eng.pending_tied_grad = None
@@ -369,6 +408,36 @@ class _GradOut:
                 at += r
         for p in params:
             self.sink.grad_written(p)
+
+    def dest(self, params: tuple):
+        """(fp32 destination of the whole fused matrix, accumulate?); None when a sink keeps its parts apart."""
+        if self.sink is None:
+            rows = [p.shape[0] for p in params]
+            dw = torch.empty(sum(rows), params[0].shape[1], dtype=torch.float32, device=self.device)
+            for p, part in zip(params, dw.split(rows)):
+                self.grads[p] = part
+            return dw, False
+        dests = [self.sink.grad_dest(p) for p in params]
+        first, acc = dests[0]
+        for (a, acc_a), (b, acc_b) in zip(dests, dests[1:]):
+            if a.data_ptr() + a.numel() * 4 != b.data_ptr() or acc_a != acc_b:
+                return None
+        rows = sum(d[0].shape[0] for d in dests)
+        return torch.as_strided(first, (rows, first.shape[1]), (first.shape[1], 1)), acc
+
+    def written(self, params) -> None:
+        if self.sink is not None:
+            for p in params:
+                self.sink.grad_written(p)
+
+    def smalls(self, params) -> list[torch.Tensor]:
+        """``small`` of several gains; fresh ones share one cleared buffer."""
+        if self.sink is not None:
+            return [self.small(p) for p in params]
+        parts = torch.zeros(sum(p.numel() for p in params), dtype=torch.float32, device=self.device).split(
+            [p.numel() for p in params])
+        self.grads.update(zip(params, parts))
+        return list(parts)
 
     def small(self, p: torch.Tensor) -> torch.Tensor:
         """Zeroed (or running) fp32 destination for a gain gradient that a kernel accumulates with atomics."""

@@ -21,31 +21,44 @@ def available() -> bool:
     return ops.available()
 
 
+def _addresses(columns) -> tuple:
+    """Five address columns, the missing ones null."""
+    ptrs = [tuple(t.data_ptr() if t is not None else 0 for t in col) for col in columns]
+    return tuple(ptrs + [(0,) * len(columns[0])] * (5 - len(ptrs)))
+
+
 class TensorTable:
-    def __init__(self, columns: list[list[torch.Tensor | None]], flags: list[int] | None = None):
-        """columns: up to 5 equally long tensor lists (None entries become null pointers)."""
+    def __init__(self, columns: list[list[torch.Tensor | None]], flags: list[int] | None = None,
+                 ptrs: tuple | None = None, like: "TensorTable | None" = None):
+        """columns: up to 5 equally long tensor lists (None entries become null pointers).  `ptrs`: their addresses when
+        the caller has them already.  `like`: a table of the same sizes and flags, whose device copies of everything but
+        the addresses are shared: fresh gradients then cost one upload instead of five."""
         n = len(columns[0])
         assert n > 0 and all(len(c) == n for c in columns)
         dev = next(t for t in columns[0] if t is not None).device
-        ptrs = [[(t.data_ptr() if t is not None else 0) for t in col] for col in columns]
-        while len(ptrs) < 5:
-            ptrs.append([0] * n)
-        numel = [t.numel() for t in columns[0]]
-        import numpy as np
+        self.key = ptrs if ptrs is not None else _addresses(columns)
 
-        chunks = [(ne + CHUNK - 1) // CHUNK for ne in numel]
-        bt = np.repeat(np.arange(n, dtype=np.int32), chunks)
-        bc = np.concatenate([np.arange(c, dtype=np.int32) for c in chunks]) if chunks else np.zeros(0, np.int32)
-        self.key = tuple(tuple(p) for p in ptrs)
         # uploads go through pinned staging that lives as long as the table: an asynchronous copy from pinned memory
         # is legal while a stream is being captured (the copy node re-reads the same, unchanged, host bytes)
-        host = [torch.tensor(ptrs, dtype=torch.int64), torch.tensor(numel, dtype=torch.int64),
-                torch.tensor(flags if flags is not None else [0] * n, dtype=torch.int32),
-                torch.from_numpy(bt), torch.from_numpy(bc)]
-        if dev.type == "cuda":
-            host = [h.pin_memory() for h in host]
-        self.host = host
-        self.ptrs, self.numel, self.flags, self.bt, self.bc = (h.to(dev, non_blocking=True) for h in host)
+        def upload(host):
+            host = host.pin_memory() if dev.type == "cuda" else host
+            return host, host.to(dev, non_blocking=True)
+
+        if like is None:
+            import numpy as np
+
+            numel = [t.numel() for t in columns[0]]
+            chunks = [(ne + CHUNK - 1) // CHUNK for ne in numel]
+            bt = np.repeat(np.arange(n, dtype=np.int32), chunks)
+            bc = np.concatenate([np.arange(c, dtype=np.int32) for c in chunks]) if chunks else np.zeros(0, np.int32)
+            sizes = [torch.tensor(numel, dtype=torch.int64),
+                     torch.tensor(flags if flags is not None else [0] * n, dtype=torch.int32),
+                     torch.from_numpy(bt), torch.from_numpy(bc)]
+            self.sizes = [upload(h) for h in sizes]
+        else:
+            self.sizes = like.sizes
+        self.numel, self.flags, self.bt, self.bc = (d for _, d in self.sizes)
+        self.host_ptrs, self.ptrs = upload(torch.tensor(self.key, dtype=torch.int64))
 
     def args(self):
         return self.ptrs, self.numel, self.flags, self.bt, self.bc
@@ -58,14 +71,12 @@ def _table(tag: str, columns, flags=None) -> TensorTable:
     first = columns[0]
     slot = (tag, len(columns), tuple(t.numel() for t in first), tuple(flags) if flags is not None else (),
             first[0].device.index)
-    ptrs = [tuple((t.data_ptr() if t is not None else 0) for t in col) for col in columns]
-    while len(ptrs) < 5:
-        ptrs.append((0,) * len(first))
+    ptrs = _addresses(columns)
     tab = _CACHE.get(slot)
-    if tab is None or tab.key != tuple(ptrs):
+    if tab is None or tab.key != ptrs:
         if len(_CACHE) > 256:
             _CACHE.clear()
-        tab = TensorTable(columns, flags)   # replaces (and thereby drops) the slot's previous table
+        tab = TensorTable(columns, flags, ptrs, tab)   # replaces (and thereby drops) the slot's previous table
         _CACHE[slot] = tab
     return tab
 
