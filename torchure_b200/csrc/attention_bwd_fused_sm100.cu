@@ -26,6 +26,12 @@
 // below, which also clears the dQ accumulator).  The accumulator is head-major ([B, Hq, Sq, 128] fp32) so that the
 // 32 reductions of a thread differ by compile-time offsets.
 //
+// With few key blocks (short sequences, few KV heads) one CTA per block leaves most of the chip idle and the longest block's
+// chain of iterations is the kernel's time.  A cluster of `parts` CTAs then shares a key block, each with a contiguous part of
+// the iterations, and the partial dV and dK tiles are summed, in a fixed order, through distributed shared memory (the operand
+// stages are free by then).  Measured on B200, before and now: 384 x 896 tokens, 8 / 2 heads, batch 2 39 -> 23 us; 1024, 8 / 4
+// heads 51 -> 25; 2048, 16 / 4 heads 178 -> 97; 8192, 2 / 1 heads 342 -> 177; 2048, 16 / 8 heads (128 blocks, not split) 93.
+//
 // `causal`: query block qb sees key blocks <= qb (Sq == Skv); otherwise every query sees every key (the off-diagonal
 // steps of ring attention).  Because partial dQ tiles are added in whatever order CTAs finish, dQ is not bitwise
 // reproducible from run to run; the two-kernel backward (attention_bwd_dq/dkv) is.
@@ -90,9 +96,21 @@ struct FusedArgs {
   // rows of batch b: q / dO at b * q_bstride + q_row0, k / v at b * kv_bstride + kv_row0; the statistics and the dQ
   // accumulator are [B, Hq, stat_stride(, 128)] with this call's queries starting at stat_row0
   int q_bstride, q_row0, kv_bstride, kv_row0, stat_stride, stat_row0;
-  int causal;
+  int causal, parts;
   float scale, scale_log2;
 };
+
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes into the shared memory of CTA `rank` of the cluster, at the place that has the address `local` here
+__device__ __forceinline__ void st_cluster_v4(uint32_t local, uint32_t rank, const uint32_t* v) {
+  asm volatile(
+      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\t"
+      "st.shared::cluster.v4.b32 [a], {%2, %3, %4, %5};\n\t}" ::"r"(local),
+      "r"(rank), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+      : "memory");
+}
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -120,14 +138,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int nqb = a.Sq / 128;
   const int ratio = a.Hq / a.Hkv;
   const int groups = a.B * a.Hkv;
-  const int kblk = static_cast<int>(blockIdx.x) / groups;   // causal: block 0 sees the most query blocks, it goes first
-  const int g = static_cast<int>(blockIdx.x) % groups;
+  const int part = static_cast<int>(blockIdx.x) % a.parts;   // == rank in the cluster
+  const int tile = static_cast<int>(blockIdx.x) / a.parts;
+  const int kblk = tile / groups;            // causal: block 0 sees the most query blocks, it goes first
+  const int g = tile % groups;
   const int kvh = g % a.Hkv, b = g / a.Hkv;
   const int krow0 = b * a.Skv + kblk * 128;                          // in the dK / dV outputs
   const int krow_in = b * a.kv_bstride + a.kv_row0 + kblk * 128;     // in the k / v tensors
   const int qb0 = a.causal ? kblk : 0;       // first visible query block
   const int n_qb = nqb - qb0;
-  const int n_iter = n_qb * ratio;           // iteration = (query head of the group, query block)
+  // iteration = (query head of the group, query block); this CTA's are [it0, it0 + n_iter), possibly none
+  const int it0 = n_qb * ratio * part / a.parts;
+  const int n_iter = n_qb * ratio * (part + 1) / a.parts - it0;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ);
@@ -159,7 +181,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (elect_one()) {
+    if (n_iter > 0 && elect_one()) {
       const int kcol = a.k_col0 + kvh * HD, vcol = a.v_col0 + kvh * HD;
       mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES);
       tma_load_2d(sK, &tmK, &bars->kv_full, kcol, krow_in);
@@ -170,8 +192,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const int s = it % Q_STAGES;
         const uint32_t ph = (it / Q_STAGES) & 1;
         if (!mbar_wait(&bars->q_empty[s], ph ^ 1, err, kErrAttnWait)) break;
-        const int h = kvh * ratio + it / n_qb;
-        const int qb = qb0 + it % n_qb;
+        const int h = kvh * ratio + (it0 + it) / n_qb;
+        const int qb = qb0 + (it0 + it) % n_qb;
         const int qrow = b * a.q_bstride + a.q_row0 + qb * 128;
         uint8_t* sQ = sStage + s * STAGE_BYTES;
         uint8_t* sDO = sQ + TILE_BYTES;
@@ -188,7 +210,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (elect_one()) {
+    if (n_iter > 0 && elect_one()) {
       constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, false, false);   // S^T / dP^T halves: N = 64 queries
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, false, true);  // A in TMEM, B MN-major, N = 128 (hd)
       constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, true, true);     // K^T (MN-major) x dS^T (MN-major)
@@ -337,7 +359,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     };
     for (int it = 0; it < n_iter && ok; ++it) {
       const int s = it % Q_STAGES;
-      const bool diag = a.causal && (it % n_qb) == 0;     // query block == key block
+      const bool diag = a.causal && ((it0 + it) % n_qb) == 0;     // query block == key block
       const float* sStat = reinterpret_cast<const float*>(sStage + s * STAGE_BYTES + 2 * TILE_BYTES);
       if (!mbar_wait(&bars->st_full[grp], it & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
@@ -354,15 +376,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bars->dq_drained[grp]);
-      const int h = kvh * ratio + it / n_qb;
-      const int qb = qb0 + it % n_qb;
+      const int h = kvh * ratio + (it0 + it) / n_qb;
+      const int qb = qb0 + (it0 + it) % n_qb;
       float* dst = a.dq_acc +
                    ((static_cast<int64_t>(b) * a.Hq + h) * a.stat_stride + a.stat_row0 + qb * 128 + grp * 64 + cg * 32) * HD + row;
 #pragma unroll
       for (int j = 0; j < 32; ++j) red_add_unordered(dst + j * HD, __uint_as_float(v[j]));
     }
-    if (ok && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait)) {
+    if (n_iter > 0) {
+      ok = ok && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait);
       tc_fence_after();
+    }
+    if (ok && a.parts == 1) {
       // group 0 writes dV, group 1 dK: this warp's 64 of the 128 head-dim columns, one key row per lane, straight to
       // global memory
       {
@@ -385,6 +410,56 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
         }
       }
+    }
+  }
+
+  if (a.parts > 1) {
+    __syncwarp();
+    cluster_sync_all();        // the products of every CTA are done: its operand stages may be written
+    const int cw = 256 / a.parts;                    // columns of dV | dK that this CTA sums: 32 and more
+    const int log_cw = 31 - __clz(cw);
+    const uint32_t slots = smem_u32(sStage);         // [part][128 rows][cw] fp32: 128 KB, groups of 16 bytes XORed by the row
+    if (warp >= 2) {
+      const int quarter = warp & 3, row = quarter * 32 + lane;
+      const int c0 = ((warp - 2) >> 2) * 64;         // this warp's 64 of the 256 columns
+#pragma unroll 1
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t v[32];
+        if (n_iter > 0) {
+          tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 256 + c0 + c, v);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
+        }
+        const int owner = (c0 + c) >> log_cw;
+        const uint32_t base = slots + static_cast<uint32_t>(part * 128 + row) * cw * 4;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int vec = (((c0 + c) & (cw - 1)) >> 2) + j;
+          st_cluster_v4(base + (static_cast<uint32_t>(vec ^ (row & 7)) << 4), owner, v + 4 * j);
+        }
+      }
+    }
+    cluster_sync_all();        // all partials have arrived; no remote access after this point
+    const int items = cw >> 3;                       // eight columns each
+    for (int i = threadIdx.x; i < 128 * items; i += NUM_THREADS) {
+      const int r = i / items, c = (i - r * items) * 8;
+      float acc[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+      for (int s2 = 0; s2 < a.parts; ++s2) {
+        const uint8_t* src = sStage + static_cast<size_t>(s2 * 128 + r) * cw * 4;
+#pragma unroll
+        for (int h2 = 0; h2 < 2; ++h2) {
+          const float4 x = *reinterpret_cast<const float4*>(src + ((((c >> 2) + h2) ^ (r & 7)) << 4));
+          acc[4 * h2] += x.x; acc[4 * h2 + 1] += x.y; acc[4 * h2 + 2] += x.z; acc[4 * h2 + 3] += x.w;
+        }
+      }
+      const int col = part * cw + c;
+      __nv_bfloat16* dst = (col < HD ? a.dv : a.dk) + static_cast<int64_t>(krow0 + r) * a.ld_dkv + kvh * HD + (col & (HD - 1));
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
+                                                  pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
     }
   }
 
@@ -491,6 +566,18 @@ int attn_bwd_stats(const void* d_o, const void* o, const float* lse, float* nds,
              : -21;
 }
 
+// CTAs per key block, from a model of the kernel's time fitted on B200: 7 us + 2.7 us per iteration of the longest block, + 4 us
+// for the exchange in a cluster of two, 7.5 in one of four.  All clusters have to run at once (74 pairs; fours leave SMs of a
+// GPC over).  Clusters of eight cost 20 us and more: sixteen of them did not fit at once.
+static int bwd_parts(int tiles, int longest) {
+  const float one = 2.7f * longest, two = 2.7f * ((longest + 1) / 2) + 4.f, four = 2.7f * ((longest + 3) / 4) + 7.5f;
+  int parts = 1;
+  float best = one;
+  if (tiles <= 74 && two < best) { parts = 2; best = two; }
+  if (tiles <= 32 && four < best) parts = 4;
+  return parts;
+}
+
 int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc,
                    void* dk, void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv,
                    int Hq, int Hkv, bool causal, int* err, cudaStream_t stream, const AttnPairLayout* lay) {
@@ -528,10 +615,23 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   a.stat_stride = lay->stat_stride; a.stat_row0 = lay->stat_row0;
   a.scale = 1.f / sqrtf(static_cast<float>(HD));
   a.scale_log2 = a.scale * 1.4426950408889634f;
-  const int grid = (Skv / 128) * B * Hkv;
-  if (launch_pdl(attn_bwd_fused_kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, stream, tq, tk, tv, tdo, a, err) !=
-      cudaSuccess)
-    return -21;
+  const int tiles = (Skv / 128) * B * Hkv;
+  a.parts = bwd_parts(tiles, (Sq / 128) * (Hq / Hkv));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles * a.parts);
+  cfg.blockDim = dim3(NUM_THREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = a.parts;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = a.parts > 1 ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, attn_bwd_fused_kernel, tq, tk, tv, tdo, a, err) != cudaSuccess) return -21;
   return 0;
 }
 
