@@ -478,6 +478,21 @@ def test_multi_tensor_adamw_norm_scale():
         torch.testing.assert_close(x, wv)
 
 
+def test_multi_tensor_tables_follow_moved_tensors():
+    """Tensors of the same sizes at new addresses reuse the table's sizes and upload only their addresses."""
+    from torchure_b200.ops import multi_tensor
+
+    torch.manual_seed(0)
+    keep = []
+    for _ in range(4):
+        ts = [torch.randn(n, device="cuda") for n in (5, 40000, 16384, 1)]
+        keep.append(ts)
+        want = sum(t.double().pow(2).sum() for t in ts)
+        torch.testing.assert_close(multi_tensor.sq_norm(ts).double(), want, rtol=1e-5, atol=1e-4)
+    multi_tensor.zero_(keep[0])
+    assert all((t == 0).all() for t in keep[0]) and all((t != 0).any() for ts in keep[1:] for t in ts)
+
+
 def test_bucket_pack():
     from torchure_b200.ops import multi_tensor
 

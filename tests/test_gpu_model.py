@@ -189,3 +189,41 @@ def test_uncovered_shapes_are_loud():
     with pytest.warns(UserWarning, match="PyTorch path"):
         out = small(torch.randint(0, 512, (1, 100), device="cuda"))
     assert out.shape == (1, 100, 512)
+
+
+@pytest.mark.parametrize("B,S,qk_norm", [(1, 128, True), (3, 384, False), (2, 1152, True)])
+def test_native_block_calls_equal_the_wrappers(B, S, qk_norm):
+    """The block's native forward and backward calls against the same kernels launched one wrapper at a time (what the poison
+    mode does), on both sides of the size up to which launches overlap.  The forward repeats bit for bit; gradients differ by
+    the order of the fp32 dQ additions, which can flip single bf16 roundings behind them (2^-9 each)."""
+    from torchure_b200.models import build_model
+    from torchure_b200.ops import debug, kernels
+
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        model = build_model("qwen3_dense" if qk_norm else "llama3_2",
+                            dict(num_layers=3, num_heads=4, num_kv_heads=2, emb_dim=640, head_dim=128, vocab_size=1000,
+                                 ffn_dim=1096))
+        model.init_weights()
+    ids = torch.randint(0, 1000, (B, S), device="cuda")
+    g = torch.randn(B, S, 640, device="cuda").bfloat16()
+
+    def run():
+        model.zero_grad()
+        h = model(ids, return_final_hidden=True)
+        h.backward(g)
+        return h.detach(), {n: p.grad.clone() for n, p in model.named_parameters() if p.grad is not None}
+
+    debug.enable(True)
+    try:
+        want, want_grads = run()
+    finally:
+        debug.enable(False)
+    got, got_grads = run()
+    assert torch.equal(got, want) and got_grads.keys() == want_grads.keys() and len(got_grads) > 20
+    for n, w in want_grads.items():
+        assert ((got_grads[n] - w).norm() / w.norm()).item() < 1e-2, n
+    with torch.no_grad():
+        for _ in range(20):
+            assert torch.equal(model(ids, return_final_hidden=True), want)
+    kernels.check_error()
