@@ -13,6 +13,8 @@
 
 namespace {
 
+// Up to here the launches of a block's forward overlap.  Measured on B200: a prompt of 128 tokens through 28 blocks 2.08 ms
+// without, 1.79 with; from some thousand rows on a kernel outlasts the launch of the next and nothing is gained.
 constexpr int64_t PDL_MAX_ROWS = 2048;
 
 using torch::Tensor;

@@ -23,8 +23,9 @@ namespace tb {
 // ---- programmatic dependent launch ----------------------------------------------------------------
 // Kernels launched through launch_pdl may be scheduled while the previous kernel of the stream is still draining;
 // each of them executes pdl_wait() before its first global-memory access, which blocks until that previous kernel
-// has completed and its writes are visible.  Only the launch latency overlaps.  Off unless TORCHURE_B200_PDL=1: on
-// this stack the step is bound by the host's enqueue rate, not by the device-side launch gap, and it measured no gain.
+// has completed and its writes are visible.  Only the launch latency overlaps.  A whole training step is bound by its kernels
+// and gained nothing (51.86 against 51.36 ms), so it is off unless TORCHURE_B200_PDL=1 or a launch sequence turns it on for
+// itself (pdl.h; the block's forward with few tokens).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
