@@ -28,6 +28,8 @@ def _addresses(columns) -> tuple:
 
 
 class TensorTable:
+    captured = False     # made while a stream was being captured
+
     def __init__(self, columns: list[list[torch.Tensor | None]], flags: list[int] | None = None,
                  ptrs: tuple | None = None, like: "TensorTable | None" = None):
         """columns: up to 5 equally long tensor lists (None entries become null pointers).  `ptrs`: their addresses when
@@ -76,7 +78,11 @@ def _table(tag: str, columns, flags=None) -> TensorTable:
     if tab is None or tab.key != ptrs:
         if len(_CACHE) > 256:
             _CACHE.clear()
-        tab = TensorTable(columns, flags, ptrs, tab)   # replaces (and thereby drops) the slot's previous table
+        # tables of a captured step stand alone: their uploads run when the graph does, in memory of its pool
+        captured = first[0].is_cuda and torch.cuda.is_current_stream_capturing()
+        like = None if tab is None or captured or tab.captured else tab
+        tab = TensorTable(columns, flags, ptrs, like)   # replaces (and thereby drops) the slot's previous table
+        tab.captured = captured
         _CACHE[slot] = tab
     return tab
 
