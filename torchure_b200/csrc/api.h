@@ -65,7 +65,7 @@ void add_rmsnorm_fwd(const float* x, const __nv_bfloat16* y, const int64_t* ids,
                      const __nv_bfloat16* table_bf16, const float* w, float* x_out, __nv_bfloat16* h, float* rstd, int M,
                      int D, float eps, cudaStream_t stream);
 // dx = dx_in + d rmsnorm; dw += sum_rows(dh * xhat).  dx_bf16 (optional) receives a bf16 copy of dx.
-// variant 0: rows staged through shared memory when the shape allows (D <= 1024); 1: the register-resident kernels
+// variant 0: rows staged through shared memory when the shape allows (D <= 4096); 1: the register-resident kernels
 void rmsnorm_bwd(const __nv_bfloat16* dh, const float* x, const float* w, const float* rstd, const float* dx_in,
                  float* dx, __nv_bfloat16* dx_bf16, float* dw, int M, int D, int num_sms, int* err, cudaStream_t stream,
                  int variant = 0);
