@@ -493,6 +493,28 @@ def test_multi_tensor_tables_follow_moved_tensors():
     assert all((t == 0).all() for t in keep[0]) and all((t != 0).any() for ts in keep[1:] for t in ts)
 
 
+def test_multi_tensor_tables_belong_to_their_stream():
+    """Equal sizes on two streams, at the same and at moved addresses: no device copy is shared, a stream finds its own
+    table again, and moved tensors share the sizes of their own stream's table only."""
+    from torchure_b200.ops import multi_tensor
+
+    new = lambda: [torch.zeros(n, device="cuda") for n in (7, 40000)]
+    first, moved = new(), new()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    here = multi_tensor._table("streams", [first])
+    with torch.cuda.stream(side):
+        there = multi_tensor._table("streams", [first])
+        there_moved = multi_tensor._table("streams", [moved])
+        assert multi_tensor._table("streams", [moved]) is there_moved
+    assert multi_tensor._table("streams", [first]) is here
+    here_moved = multi_tensor._table("streams", [moved])
+    copies = lambda tabs: {t.data_ptr() for tab in tabs for t in tab.args()}
+    assert not copies([here, here_moved]) & copies([there, there_moved])
+    assert here_moved.bt is here.bt and there_moved.bt is there.bt
+    torch.cuda.synchronize()
+
+
 def test_bucket_pack():
     from torchure_b200.ops import multi_tensor
 

@@ -4,8 +4,10 @@ A ``TensorTable`` records, for a fixed list of tensors, up to five pointer colum
 per-tensor flags and the (tensor, chunk) assignment of every thread block.  It is uploaded once; while the
 underlying storages stay where they are (parameters, optimizer state, bucket views), every later launch
 reuses it.  Tables are rebuilt only when a pointer changes (fresh autograd grads).  A table holds addresses, not
-tensors: it keeps nothing alive, and there is one live table per (operation, tensor sizes, flags) slot, so fresh
-gradients arriving at new addresses every step replace the previous table instead of piling up.
+tensors: it keeps nothing alive, and there is one live table per (operation, tensor sizes, flags, stream) slot, so fresh
+gradients arriving at new addresses every step replace the previous table instead of piling up.  A table belongs to the
+stream that was current when it was made: its uploads are ordered before the kernels that read it, and its memory goes
+back to that stream's pool, only there.
 """
 
 from __future__ import annotations
@@ -33,8 +35,8 @@ class TensorTable:
     def __init__(self, columns: list[list[torch.Tensor | None]], flags: list[int] | None = None,
                  ptrs: tuple | None = None, like: "TensorTable | None" = None):
         """columns: up to 5 equally long tensor lists (None entries become null pointers).  `ptrs`: their addresses when
-        the caller has them already.  `like`: a table of the same sizes and flags, whose device copies of everything but
-        the addresses are shared: fresh gradients then cost one upload instead of five."""
+        the caller has them already.  `like`: a table of the same sizes and flags made on this stream, whose device
+        copies of everything but the addresses are shared: fresh gradients then cost one upload instead of five."""
         n = len(columns[0])
         assert n > 0 and all(len(c) == n for c in columns)
         dev = next(t for t in columns[0] if t is not None).device
@@ -69,10 +71,15 @@ class TensorTable:
 _CACHE: dict[tuple, TensorTable] = {}
 
 
+def _stream(device: torch.device) -> int:
+    """Handle of the device's current stream."""
+    return torch.cuda.current_stream(device).cuda_stream if device.type == "cuda" else 0
+
+
 def _table(tag: str, columns, flags=None) -> TensorTable:
     first = columns[0]
     slot = (tag, len(columns), tuple(t.numel() for t in first), tuple(flags) if flags is not None else (),
-            first[0].device.index)
+            first[0].device.index, _stream(first[0].device))
     ptrs = _addresses(columns)
     tab = _CACHE.get(slot)
     if tab is None or tab.key != ptrs:
