@@ -515,6 +515,56 @@ def test_multi_tensor_tables_belong_to_their_stream():
     torch.cuda.synchronize()
 
 
+def test_multi_tensor_tables_of_a_capture():
+    """A captured step and calls around it on the same and on moved tensors: neither uses the other's tables, replays read
+    host bytes that nobody else has been given meanwhile, and these go with the graph."""
+    import gc
+    import time
+
+    from torchure_b200 import ops
+    from torchure_b200.ops import multi_tensor
+
+    sizes = (5, 40000)
+    new = lambda v: [torch.full((n,), v, device="cuda") for n in sizes]
+    factor = lambda v: torch.tensor(v, device="cuda")
+    half, two, one = factor(0.5), factor(2.0), factor(1.0)
+    start = ops.ext().graph_keeps()
+    a = new(8.0)
+    eager = multi_tensor._table("scale", [a], [0, 0])        # a table of these addresses is there before the capture
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        inside = multi_tensor._table("scale", [a], [0, 0])
+        multi_tensor.scale_(a, half)
+        norm = multi_tensor.sq_norm(a)
+        assert multi_tensor._table("scale", [a], [0, 0]) is inside
+    assert inside is not eager and multi_tensor._table("scale", [a], [0, 0]) is eager
+    assert ops.ext().graph_keeps() == start + 2
+    staging = {t.data_ptr() for t in inside.host()}
+    b = new(3.0)
+    multi_tensor.scale_(b, two)         # moved: replaces the eager table
+    multi_tensor.scale_(a, one)         # ... and moved back, before the first replay
+    del inside, eager
+    multi_tensor._CAPTURES.clear()
+    gc.collect()
+    torch.cuda.synchronize()
+    taken = [torch.zeros(n, dtype=torch.int64).pin_memory() for n in (2, 10) for _ in range(8)]
+    assert not staging & {t.data_ptr() for t in taken}
+    for want in (4.0, 2.0, 1.0):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all((t == want).all() for t in a) and all((t == 6.0).all() for t in b)
+        assert norm.item() == want * want * sum(sizes)
+    graph.reset()
+    del graph
+    torch.cuda.synchronize()
+    for _ in range(200):                # CUDA calls back from a thread of its own
+        if ops.ext().graph_keeps() == start:
+            break
+        time.sleep(0.01)
+    assert ops.ext().graph_keeps() == start
+
+
 def test_bucket_pack():
     from torchure_b200.ops import multi_tensor
 

@@ -3,6 +3,9 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "api.h"
 #include "bind_common.h"
 #include "comm_api.h"
@@ -280,6 +283,58 @@ void bucket_pack_multi(const torch::Tensor& ptrs, const torch::Tensor& numel, co
 
 torch::Tensor error_word() { return err_word(); }
 
+// Tensors that a captured graph reads at every replay (the host bytes of copy nodes) are owned by the graph: CUDA calls back
+// when neither the graph nor an executable made from it is left.  The callback may not call CUDA, as releasing pinned memory
+// does, so it only hands the tensors over; they go when a table is next asked for.
+using Kept = std::vector<torch::Tensor>;
+std::mutex g_gone_mutex;
+std::vector<Kept*> g_gone;
+std::atomic<int> g_any_gone{0}, g_graph_keeps{0};
+
+void CUDART_CB graph_gone(void* kept) {
+  std::lock_guard<std::mutex> lock(g_gone_mutex);
+  g_gone.push_back(static_cast<Kept*>(kept));
+  g_any_gone = 1;
+}
+
+void release_gone() {
+  if (g_any_gone == 0) return;
+  std::vector<Kept*> gone;
+  {
+    std::lock_guard<std::mutex> lock(g_gone_mutex);
+    gone.swap(g_gone);
+    g_any_gone = 0;
+  }
+  g_graph_keeps -= static_cast<int>(gone.size());
+  for (Kept* k : gone) delete k;
+}
+
+// (current stream, id of the capture it is in, 0 outside of one)
+std::pair<int64_t, int64_t> stream_place(int64_t device) {
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+  cudaStreamCaptureStatus status;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id));
+  if (status == cudaStreamCaptureStatusNone) release_gone();
+  return {(int64_t) reinterpret_cast<uintptr_t>(stream), status == cudaStreamCaptureStatusNone ? 0 : (int64_t)id + 1};
+}
+
+void keep_with_graph(Kept tensors) {
+  cudaStreamCaptureStatus status;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(cur_stream(), &status, &id, &graph));
+  TORCH_CHECK(status == cudaStreamCaptureStatusActive && graph != nullptr, "keep_with_graph: no capture on the current stream");
+  auto kept = std::make_unique<Kept>(std::move(tensors));
+  cudaUserObject_t owner = nullptr;
+  C10_CUDA_CHECK(cudaUserObjectCreate(&owner, kept.get(), graph_gone, 1, cudaUserObjectNoDestructorSync));
+  kept.release();      // the callback has it from here on
+  ++g_graph_keeps;
+  const cudaError_t rc = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (rc != cudaSuccess) cudaUserObjectRelease(owner, 1);
+  C10_CUDA_CHECK(rc);
+}
+
 }  // namespace
 
 torch::Tensor attn_err_word() { return err_word(); }
@@ -306,6 +361,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0);
   m.def("set_sm_reserve", [](int64_t n) { g_sm_reserve = (int)n; }, "persistent kernels use (SM count - n) CTAs");
   m.def("gemm_pair_capacity", &tb::gemm_pair_capacity, "CTA pairs (2-SM clusters) resident at once; 0 before the first launch");
+  m.def("stream_place", &stream_place, "(current stream of a device, id of the capture it is in or 0)");
+  m.def("keep_with_graph", &keep_with_graph, "the graph being captured on the current stream owns these tensors");
+  m.def("graph_keeps", [] { release_gone(); return g_graph_keeps.load(); }, "how many keep_with_graph sets are alive");
   m.def("error_word", &error_word, "device int32[4]; [0] is set when a bounded wait of a kernel expired");
   m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd, pybind11::arg("dh"), pybind11::arg("x"), pybind11::arg("w"), pybind11::arg("rstd"),

@@ -8,6 +8,10 @@ tensors: it keeps nothing alive, and there is one live table per (operation, ten
 gradients arriving at new addresses every step replace the previous table instead of piling up.  A table belongs to the
 stream that was current when it was made: its uploads are ordered before the kernels that read it, and its memory goes
 back to that stream's pool, only there.
+
+A capture has tables of its own.  Their uploads are nodes of the graph, so the device copies hold nothing before the
+first replay and every replay reads the host bytes again: no call outside the capture is given such a table, and the
+host bytes stay until the graph is gone, whatever becomes of the table.
 """
 
 from __future__ import annotations
@@ -30,8 +34,6 @@ def _addresses(columns) -> tuple:
 
 
 class TensorTable:
-    captured = False     # made while a stream was being captured
-
     def __init__(self, columns: list[list[torch.Tensor | None]], flags: list[int] | None = None,
                  ptrs: tuple | None = None, like: "TensorTable | None" = None):
         """columns: up to 5 equally long tensor lists (None entries become null pointers).  `ptrs`: their addresses when
@@ -42,8 +44,8 @@ class TensorTable:
         dev = next(t for t in columns[0] if t is not None).device
         self.key = ptrs if ptrs is not None else _addresses(columns)
 
-        # uploads go through pinned staging that lives as long as the table: an asynchronous copy from pinned memory
-        # is legal while a stream is being captured (the copy node re-reads the same, unchanged, host bytes)
+        # uploads go through pinned staging: an asynchronous copy from pinned memory is legal while a stream is being
+        # captured
         def upload(host):
             host = host.pin_memory() if dev.type == "cuda" else host
             return host, host.to(dev, non_blocking=True)
@@ -64,33 +66,42 @@ class TensorTable:
         self.numel, self.flags, self.bt, self.bc = (d for _, d in self.sizes)
         self.host_ptrs, self.ptrs = upload(torch.tensor(self.key, dtype=torch.int64))
 
+    def host(self) -> list[torch.Tensor]:
+        """The staging buffers the uploads read."""
+        return [h for h, _ in self.sizes] + [self.host_ptrs]
+
     def args(self):
         return self.ptrs, self.numel, self.flags, self.bt, self.bc
 
 
 _CACHE: dict[tuple, TensorTable] = {}
+_CAPTURES: dict[int, dict[tuple, TensorTable]] = {}     # capture id -> tables made in it; the newest few captures
 
 
-def _stream(device: torch.device) -> int:
-    """Handle of the device's current stream."""
-    return torch.cuda.current_stream(device).cuda_stream if device.type == "cuda" else 0
+def _place(device: torch.device) -> tuple[int, int]:
+    """(handle of the device's current stream, id of the capture it is in or 0)."""
+    return ops.ext().stream_place(device.index) if device.type == "cuda" else (0, 0)
 
 
 def _table(tag: str, columns, flags=None) -> TensorTable:
     first = columns[0]
+    stream, capture = _place(first[0].device)
     slot = (tag, len(columns), tuple(t.numel() for t in first), tuple(flags) if flags is not None else (),
-            first[0].device.index, _stream(first[0].device))
+            first[0].device.index, stream)
     ptrs = _addresses(columns)
-    tab = _CACHE.get(slot)
+    cache = _CACHE
+    if capture:
+        if capture not in _CAPTURES and len(_CAPTURES) >= 4:
+            _CAPTURES.clear()
+        cache = _CAPTURES.setdefault(capture, {})
+    tab = cache.get(slot)
     if tab is None or tab.key != ptrs:
-        if len(_CACHE) > 256:
-            _CACHE.clear()
-        # tables of a captured step stand alone: their uploads run when the graph does, in memory of its pool
-        captured = first[0].is_cuda and torch.cuda.is_current_stream_capturing()
-        like = None if tab is None or captured or tab.captured else tab
-        tab = TensorTable(columns, flags, ptrs, like)   # replaces (and thereby drops) the slot's previous table
-        tab.captured = captured
-        _CACHE[slot] = tab
+        if len(cache) > 256:
+            cache.clear()
+        tab = TensorTable(columns, flags, ptrs, tab)   # replaces (and thereby drops) the slot's previous table
+        if capture:
+            ops.ext().keep_with_graph(tab.host())
+        cache[slot] = tab
     return tab
 
 
