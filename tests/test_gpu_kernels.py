@@ -99,6 +99,22 @@ def test_gemm_few_tile_kernels(M, N, K, tile_n, splits):
         assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("M,N,K,tile_n,splits", [(600, 512, 50257, 0, 0), (130, 64, 16400, 0, 0), (300, 520, 2500, 64, 4),
+                                                 (1, 8, 520, 128, 2), (257, 136, 1000, 256, 1)])
+def test_gemm_transposed_a_row_major_b(M, N, K, tile_n, splits):
+    """A [K, M] with B [N, K], bf16 output, at few tiles and a long K: by the plan and on each width of the few-tile kernel.
+    The output is rounded to bf16 once (2^-9)."""
+    from torchure_b200 import ops
+
+    torch.manual_seed(0)
+    pad = lambda n: (n + 7) // 8 * 8
+    a = torch.randn(K, pad(M), device="cuda").bfloat16()[:, :M]
+    b = torch.randn(N, pad(K), device="cuda").bfloat16()[:, :K]
+    out = torch.zeros(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N]
+    ops.ext().gemm(a, b, out, True, False, 0, splits, tile_n)
+    assert relerr(out.double(), a.double().t() @ b.double().t()) < 4e-3
+
+
 def test_gemm_strided_views():
     from torchure_b200.ops import kernels
 

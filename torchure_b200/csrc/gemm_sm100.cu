@@ -561,7 +561,7 @@ static int sum_slices(const float* ws, int64_t stride, int slices, int64_t ldw, 
 // slices: 13.1 us, as the other terms say).
 // Narrow tiles win while the problem is one wave of them (1024 x 512 x 512: 4.8 against 9.1 us; 2048 x 1024 x 4096: 16.2
 // against 25.4), the pair kernel as soon as it fills its 74 SM pairs (4096 x 1024 x 6144: 37.1 against 38.7).
-GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_splits, int force_tile_n) {
+GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, int force_splits, int force_tile_n) {
   GemmPlan p{};
   p.splits = 1;
   const int num_kb = (K + BK - 1) / BK;
@@ -610,8 +610,9 @@ GemmPlan gemm_plan(int M, int N, int K, int out_mode, int num_sms, int force_spl
   // add up in one order however many rows come along; what splitting them would gain is little (128 x 1024 x 3072: 10.4 us
   // in one slice, 8.9 in four; 128 x 1024 x 2048: no difference).
   const bool may_split = out_mode != 0 || num_kb >= 256;
-  // K slices through a workspace: only where the tiles leave most of the chip idle for a long K
-  if (may_split && pair && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
+  // K slices through a workspace: only where the tiles leave most of the chip idle for a long K.  The slices are fp32 products,
+  // which no kernel has for A [K, M] with B [N, K].
+  if (may_split && pair && !(a_mn && !b_mn) && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
     const int s = static_cast<int>(workers / tiles) < num_kb / 16 ? static_cast<int>(workers / tiles) : num_kb / 16;
     if (s > 1) {
       const float run = std::max(0.30f * ceil_div(num_kb, s), cold ? tiles * num_kb * 65536.f / 8.5e6f : 0.f);
