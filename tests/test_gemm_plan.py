@@ -1,5 +1,8 @@
 """The choice of a kernel for a product (``gemm_plan``), which needs no GPU."""
 
+import subprocess
+import sys
+
 import pytest
 
 from torchure_b200 import ops
@@ -15,3 +18,15 @@ SIZES = [(600, 512, 50257), (130, 64, 151936), (300, 520, 2500), (129, 128, 1638
 def test_transposed_a_with_row_major_b_is_not_sliced(M, N, K):
     """A [K, M] with B [N, K] exists with bf16 output only: slices of K, which are fp32 products, cannot run it."""
     assert _C.gemm_plan(M, N, K, a_mn=True, b_mn=False)[0] != "slices"
+
+
+def test_empty_products_are_planned():
+    """A size of zero is left to the launcher's argument check (an integer division by zero would end the process, hence
+    the child)."""
+    code = ("from torchure_b200 import _C\n"
+            "for M, N, K in ((256, 0, 8192), (0, 256, 8192), (256, 256, 0), (0, 0, 0), (256, 0, 32768)):\n"
+            "    for mode in (0, 1, 2):\n"
+            "        kind, _, splits, ws = _C.gemm_plan(M, N, K, out_mode=mode)\n"
+            "        assert splits == 1 and ws == 0 and kind != 'slices'\n")
+    res = subprocess.run([sys.executable, "-c", "import torch\n" + code], capture_output=True, text=True, timeout=240)
+    assert res.returncode == 0, (res.returncode, res.stderr[-500:])

@@ -564,6 +564,7 @@ static int sum_slices(const float* ws, int64_t stride, int slices, int64_t ldw, 
 GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, int force_splits, int force_tile_n) {
   GemmPlan p{};
   p.splits = 1;
+  if (M <= 0 || N <= 0 || K <= 0) return p;      // an argument error of gemm_bf16
   const int num_kb = (K + BK - 1) / BK;
   auto ceil_div = [](int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); };
   const bool pair = pair_enabled() && M > BM && num_sms >= 2;
