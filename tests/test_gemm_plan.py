@@ -30,3 +30,21 @@ def test_empty_products_are_planned():
             "        assert splits == 1 and ws == 0 and kind != 'slices'\n")
     res = subprocess.run([sys.executable, "-c", "import torch\n" + code], capture_output=True, text=True, timeout=240)
     assert res.returncode == 0, (res.returncode, res.stderr[-500:])
+
+
+@pytest.mark.parametrize("free", [16, 40, 100])
+def test_reserved_sms_stay_free(free):
+    """With SMs reserved no product starts more CTAs than the others hold: the kernel for few tiles is not persistent, so its
+    tiles have to fit at once (the other kernels take the number of SMs they may use)."""
+    sms = 148 - free
+    two_waves = 0
+    for m in (1, 100, 128, 300, 1024, 1408, 2048, 2304, 4096):
+        for n in (64, 512, 1024, 2048, 3072, 6144):
+            for k in (64, 512, 4096, 20000):
+                for mode in (0, 1):
+                    def ctas(**kw):
+                        kind, tile, splits, _ = _C.gemm_plan(m, n, k, out_mode=mode, **kw)
+                        return -(-m // 128) * -(-n // tile) * splits if kind == "small" else 0
+                    assert ctas(num_sms=sms, sms_reserved=True) <= sms, (m, n, k, mode)
+                    two_waves += ctas(num_sms=sms) > sms
+    assert two_waves > 0

@@ -1,5 +1,8 @@
 """GPU numerics: each sm_100a kernel against a plain PyTorch fp32 statement of the same op."""
 
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -113,6 +116,30 @@ def test_gemm_transposed_a_row_major_b(M, N, K, tile_n, splits):
     out = torch.zeros(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N]
     ops.ext().gemm(a, b, out, True, False, 0, splits, tile_n)
     assert relerr(out.double(), a.double().t() @ b.double().t()) < 4e-3
+
+
+def test_gemm_with_reserved_sms():
+    """Products with most SMs reserved and after the reservation was lifted, in a fresh process whose first launch has it:
+    right in both states, and the pairs that the device holds are counted without it."""
+    code = """
+import torch
+from torchure_b200 import ops
+from torchure_b200.ops import kernels as K
+torch.manual_seed(0)
+a, b = torch.randn(2304, 512, device="cuda").bfloat16(), torch.randn(1024, 512, device="cuda").bfloat16()
+ref = a.double() @ b.double().t()
+outs = []
+for free in (120, 16, 0):
+    ops.set_compute_sm_reserve(free)
+    outs.append(K.gemm(a, b))
+    assert (outs[-1].double() - ref).norm() / ref.norm() < 4e-3
+assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+wide = K.gemm(a, torch.randn(8192, 512, device="cuda").bfloat16())
+assert ops.ext().gemm_pair_capacity() > 40, ops.ext().gemm_pair_capacity()
+K.check_error()
+"""
+    res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=240)
+    assert res.returncode == 0, res.stderr[-1000:]
 
 
 def test_gemm_strided_views():

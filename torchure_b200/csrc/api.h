@@ -24,14 +24,16 @@ struct GemmPlan {
   bool b_is_old;      // B was not written by the kernel launched just before: kSmall may read it ahead of that one's end
 };
 // The kernel and the K split for a problem.  force_splits > 0 fixes the number of K slices; force_tile_n > 0 selects the
-// kernel for few tiles with that tile width, force_tile_n < 0 the slices through a workspace.
-GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, int force_splits, int force_tile_n);
+// kernel for few tiles with that tile width, force_tile_n < 0 the slices through a workspace.  sms_reserved: num_sms is less
+// than the device has, and the others are to stay free of GEMM CTAs.
+GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, int force_splits,
+                   int force_tile_n);
 // Returns 0 or a negative code for an argument error.  `err` is a device int that a kernel sets when
 // one of its bounded waits expires.
 int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,
               bool a_mn, bool b_mn, int out_mode, const GemmPlan& plan, void* workspace, int* err, int num_sms,
               cudaStream_t stream);
-// CTA pairs the device holds at once (0 before the first pair launch of this process).
+// CTA pairs the whole device holds at once (0 before the first pair launch of this process).
 int gemm_pair_capacity();
 // The CTA-pair kernel behind gemm_bf16 (tiles of 256 x 256 on two SMs).  slice_rows > 0: K slice s stores its tile at row
 // s * slice_rows of C (a multiple of 256) instead of adding into a shared tile.

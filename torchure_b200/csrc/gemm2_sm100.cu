@@ -536,14 +536,19 @@ int launch_pairs(void (*kern)(Params...), int units, int num_sms, cudaStream_t s
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   if (g_pair_capacity == 0) {
-    cfg.gridDim = dim3(2 * (num_sms / 2));
+    int dev = 0, all_sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&all_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return -23;
+    cfg.gridDim = dim3(2 * (all_sms / 2));
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) return -23;
-    g_pair_capacity = n < num_sms / 2 ? n : num_sms / 2;
+    g_pair_capacity = n < all_sms / 2 ? n : all_sms / 2;
   }
-  const int clusters = units < g_pair_capacity ? units : g_pair_capacity;
+  const int pairs = g_pair_capacity < num_sms / 2 ? g_pair_capacity : num_sms / 2;    // num_sms: without the reserved ones
+  const int clusters = units < pairs ? units : pairs;
   cfg.gridDim = dim3(2 * clusters);
   cfg.stream = stream;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -561,14 +561,16 @@ static int sum_slices(const float* ws, int64_t stride, int slices, int64_t ldw, 
 // slices: 13.1 us, as the other terms say).
 // Narrow tiles win while the problem is one wave of them (1024 x 512 x 512: 4.8 against 9.1 us; 2048 x 1024 x 4096: 16.2
 // against 25.4), the pair kernel as soon as it fills its 74 SM pairs (4096 x 1024 x 6144: 37.1 against 38.7).
-GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, int force_splits, int force_tile_n) {
+GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, int force_splits,
+                   int force_tile_n) {
   GemmPlan p{};
   p.splits = 1;
   if (M <= 0 || N <= 0 || K <= 0) return p;      // an argument error of gemm_bf16
   const int num_kb = (K + BK - 1) / BK;
   auto ceil_div = [](int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); };
   const bool pair = pair_enabled() && M > BM && num_sms >= 2;
-  const int workers = pair ? (gemm_pair_capacity() > 0 ? gemm_pair_capacity() : num_sms / 2) : num_sms;
+  const int capacity = gemm_pair_capacity();
+  const int workers = !pair ? num_sms : (capacity > 0 && capacity < num_sms / 2 ? capacity : num_sms / 2);
   const int64_t tiles = static_cast<int64_t>(ceil_div(M, (pair ? 2 : 1) * BM)) * ceil_div(N, BN);
   const int64_t slice_rows = static_cast<int64_t>(ceil_div(M, 2 * BM)) * 2 * BM;
   auto use_slices = [&](int s) {
@@ -627,6 +629,8 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
     const int64_t t_small = static_cast<int64_t>(ceil_div(M, BM)) * ceil_div(N, kTile[i]);
     if (t_small > 2 * num_sms) continue;
     for (int s = 1, lg = 0; s <= (may_split ? 8 : 1) && s <= num_kb; s *= 2, ++lg) {
+      // the grid is not persistent: a second wave of CTAs would run on the SMs that are to stay free
+      if (sms_reserved && t_small * s > num_sms) break;
       // clusters of 4 and 8 leave SMs of a GPC over
       const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 15 / 16 : num_sms * 7 / 8);
       const int waves = ceil_div(t_small * s, slots);
