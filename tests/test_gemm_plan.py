@@ -17,7 +17,7 @@ SIZES = [(600, 512, 50257), (130, 64, 151936), (300, 520, 2500), (129, 128, 1638
 @pytest.mark.parametrize("M,N,K", SIZES)
 def test_transposed_a_with_row_major_b_is_not_sliced(M, N, K):
     """A [K, M] with B [N, K] exists with bf16 output only: slices of K, which are fp32 products, cannot run it."""
-    assert _C.gemm_plan(M, N, K, a_mn=True, b_mn=False)[0] != "slices"
+    assert _C.gemm_plan(M, N, K, a_mn=True, b_mn=False, may_split=True)[0] != "slices"
 
 
 def test_empty_products_are_planned():
@@ -43,8 +43,23 @@ def test_reserved_sms_stay_free(free):
             for k in (64, 512, 4096, 20000):
                 for mode in (0, 1):
                     def ctas(**kw):
-                        kind, tile, splits, _ = _C.gemm_plan(m, n, k, out_mode=mode, **kw)
+                        kind, tile, splits, _ = _C.gemm_plan(m, n, k, out_mode=mode, may_split=True, **kw)
                         return -(-m // 128) * -(-n // tile) * splits if kind == "small" else 0
                     assert ctas(num_sms=sms, sms_reserved=True) <= sms, (m, n, k, mode)
                     two_waves += ctas(num_sms=sms) > sms
     assert two_waves > 0
+
+
+@pytest.mark.parametrize("K", [512, 4096, 16384, 19456, 28672])
+@pytest.mark.parametrize("N", [64, 1024, 2048, 2560])
+def test_bf16_products_are_split_only_on_request(N, K):
+    """A block's product (2 ffn_dim of the input gradient, ffn_dim of the down projection) keeps one order of additions for
+    any number of rows; a head's may be split."""
+    for M in (1, 128, 129, 256, 600, 1024, 4096):
+        assert _C.gemm_plan(M, N, K, b_mn=True)[2] == 1, M
+
+
+def test_head_products_are_split():
+    assert _C.gemm_plan(600, 512, 50257, b_mn=True, may_split=True)[2] > 1
+    assert _C.gemm_plan(128, 1024, 151936, b_mn=True, may_split=True)[2] > 1
+    assert _C.gemm_plan(600, 512, 8192, b_mn=True, may_split=True)[2] == 1

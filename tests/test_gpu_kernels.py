@@ -114,8 +114,39 @@ def test_gemm_transposed_a_row_major_b(M, N, K, tile_n, splits):
     a = torch.randn(K, pad(M), device="cuda").bfloat16()[:, :M]
     b = torch.randn(N, pad(K), device="cuda").bfloat16()[:, :K]
     out = torch.zeros(M, pad(N), device="cuda", dtype=torch.bfloat16)[:, :N]
-    ops.ext().gemm(a, b, out, True, False, 0, splits, tile_n)
+    ops.ext().gemm(a, b, out, True, False, 0, splits, tile_n, may_split=True)
     assert relerr(out.double(), a.double().t() @ b.double().t()) < 4e-3
+
+
+@pytest.mark.parametrize("K", [16384, 19456])       # 2 ffn_dim of the 1B and 4B blocks
+def test_block_gradient_rows_do_not_depend_on_their_number(K):
+    """The input gradient of a wide block, bf16: a row has the same bits among 128, 256 and 1024 rows."""
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(0)
+    dy, w = torch.randn(1024, K, device="cuda").bfloat16(), torch.randn(K, 2048, device="cuda").bfloat16()
+    whole = kernels.linear_dgrad(dy, w)
+    for M in (128, 256):
+        assert torch.equal(kernels.linear_dgrad(dy[:M], w), whole[:M]), M
+
+
+@pytest.mark.parametrize("M,N,K", [(262, 384, 32245), (600, 512, 50257), (211, 256, 141510), (150, 1024, 20000)])
+def test_head_gradient_in_slices_is_no_further_off(M, N, K):
+    """dH of a head from softmax gradients, against 64 bits: summing K in slices is at least as close as one long fp32 sum,
+    whose additions round K / 64 times as often (both end in a rounding to bf16, 2^-9 / sqrt(3) = 1.1e-3 on average)."""
+    from torchure_b200 import ops
+
+    torch.manual_seed(0)
+    p = torch.softmax(torch.randn(M, (K + 7) // 8 * 8, device="cuda"), 1)
+    p[torch.arange(M), torch.randint(0, K, (M,), device="cuda")] -= 1
+    p, w = p.bfloat16()[:, :K], (torch.randn(K, N, device="cuda") * 0.02).bfloat16()
+    want = p.double() @ w.double()
+    errs = []
+    for kw in (dict(splits=1), dict(may_split=True)):
+        out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        ops.ext().gemm(p, w, out, False, True, 0, **kw)
+        errs.append(((out.double() - want).norm() / want.norm()).item())
+    assert errs[1] <= errs[0] * 1.001 and errs[0] < 4e-3, errs
 
 
 def test_gemm_with_reserved_sms():

@@ -25,9 +25,10 @@ struct GemmPlan {
 };
 // The kernel and the K split for a problem.  force_splits > 0 fixes the number of K slices; force_tile_n > 0 selects the
 // kernel for few tiles with that tile width, force_tile_n < 0 the slices through a workspace.  sms_reserved: num_sms is less
-// than the device has, and the others are to stay free of GEMM CTAs.
-GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, int force_splits,
-                   int force_tile_n);
+// than the device has, and the others are to stay free of GEMM CTAs.  may_split: a bf16 product may be split over a long K,
+// so that its rounding depends on the number of rows.
+GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, bool may_split,
+                   int force_splits, int force_tile_n);
 // Returns 0 or a negative code for an argument error.  `err` is a device int that a kernel sets when
 // one of its bounded waits expires.
 int gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64_t lda, int64_t ldb, int64_t ldc,

@@ -43,7 +43,7 @@ T* opt_mptr(c10::optional<torch::Tensor>& t) {
 }
 
 void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
-          int64_t splits, int64_t tile_n, bool b_is_old = false) {
+          int64_t splits, int64_t tile_n, bool b_is_old = false, bool may_split = false) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda(), "gemm: CUDA tensors required");
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm: bf16 operands");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2, "gemm: 2-D tensors");
@@ -55,7 +55,7 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   TORCH_CHECK(out_mode == 0 ? out.scalar_type() == torch::kBFloat16 : out.scalar_type() == torch::kFloat32,
               "gemm: output dtype does not match out_mode");
   c10::cuda::CUDAGuard guard(a.device());
-  tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, num_sms(), g_sm_reserve > 0, (int)splits, (int)tile_n);
+  tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, num_sms(), g_sm_reserve > 0, may_split, (int)splits, (int)tile_n);
   plan.b_is_old = b_is_old;
   torch::Tensor ws;
   if (plan.workspace > 0) ws = torch::empty({(int64_t)plan.workspace}, a.options().dtype(torch::kUInt8));
@@ -79,7 +79,7 @@ bool gemm_swiglu(const torch::Tensor& x, const torch::Tensor& w, c10::optional<t
   TORCH_CHECK(!has_gu || (gu->is_contiguous() && gu->scalar_type() == torch::kBFloat16 && gu->size(0) == M &&
                           gu->size(1) == 2 * F), "gemm_swiglu: gu must be contiguous bf16 [M, 2F]");
   if (F % 8 != 0 || M == 0 ||
-      tb::gemm_plan((int)M, (int)(2 * F), (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, 0, 0).kind != tb::GemmPlan::kPair)
+      tb::gemm_plan((int)M, (int)(2 * F), (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind != tb::GemmPlan::kPair)
     return false;
   c10::cuda::CUDAGuard guard(x.device());
   const int rc = tb::gemm2_swiglu(x.data_ptr(), w.data_ptr(), has_gu ? gu->data_ptr() : nullptr, act.data_ptr(), (int)M,
@@ -100,7 +100,7 @@ bool gemm_swiglu_bwd(const torch::Tensor& dy, const torch::Tensor& w, const torc
               "gemm_swiglu_bwd: shapes");
   // below 2048 the epilogue takes longer than the products it should hide behind (figures at the kernel)
   if (K < 2048 || F % 16 != 0 || M == 0 || (reinterpret_cast<uintptr_t>(gu.data_ptr()) & 31) != 0 ||
-      tb::gemm_plan((int)M, (int)F, (int)K, false, true, 0, num_sms(), g_sm_reserve > 0, 0, 0).kind != tb::GemmPlan::kPair)
+      tb::gemm_plan((int)M, (int)F, (int)K, false, true, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind != tb::GemmPlan::kPair)
     return false;
   c10::cuda::CUDAGuard guard(dy.device());
   const int rc = tb::gemm2_swiglu_bwd(dy.data_ptr(), w.data_ptr(), gu.data_ptr(), dgu.data_ptr(), (int)M, (int)F, (int)K,
@@ -120,7 +120,7 @@ bool gemm_ce(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor
   TORCH_CHECK(stats.scalar_type() == torch::kFloat32 && stats.is_contiguous() && stats.numel() >= 2 * M * ((N + 255) / 256) &&
                   target.scalar_type() == torch::kFloat32 && target.is_contiguous() && target.numel() >= M,
               "gemm_ce: stats must be fp32 [ceil(N / 256), M, 2], target fp32 [M]");
-  if (M == 0 || tb::gemm_plan((int)M, (int)N, (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, 0, 0).kind != tb::GemmPlan::kPair) return false;
+  if (M == 0 || tb::gemm_plan((int)M, (int)N, (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind != tb::GemmPlan::kPair) return false;
   c10::cuda::CUDAGuard guard(a.device());
   const int rc = tb::gemm2_ce(a.data_ptr(), b.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
                               labels.data_ptr<int64_t>(), stats.data_ptr<float>(), target.data_ptr<float>(),
@@ -356,17 +356,20 @@ void register_block(pybind11::module_& m);
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", [](const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bool a_mn, bool b_mn, int64_t out_mode,
-                   int64_t splits, int64_t tile_n) { gemm(a, b, out, a_mn, b_mn, out_mode, splits, tile_n); }, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
+                   int64_t splits, int64_t tile_n, bool may_split) {
+    gemm(a, b, out, a_mn, b_mn, out_mode, splits, tile_n, false, may_split);
+  }, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
         pybind11::arg("b"), pybind11::arg("out"), pybind11::arg("a_mn"), pybind11::arg("b_mn"), pybind11::arg("out_mode"),
-        pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0);
-  m.def("gemm_plan", [](int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved) {
-    const tb::GemmPlan p = tb::gemm_plan(M, N, K, a_mn, b_mn, out_mode, num_sms, sms_reserved, 0, 0);
+        pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0, pybind11::arg("may_split") = false);
+  m.def("gemm_plan", [](int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved,
+                        bool may_split) {
+    const tb::GemmPlan p = tb::gemm_plan(M, N, K, a_mn, b_mn, out_mode, num_sms, sms_reserved, may_split, 0, 0);
     static const char* const kinds[] = {"single", "pair", "small", "slices"};
     return std::make_tuple(kinds[p.kind], p.tile_n, p.splits, p.workspace);
   }, "(kernel, tile width, K slices, workspace bytes) a product would run with on so many SMs", pybind11::arg("M"),
      pybind11::arg("N"), pybind11::arg("K"), pybind11::arg("a_mn") = false, pybind11::arg("b_mn") = false,
      pybind11::arg("out_mode") = 0, pybind11::arg("num_sms") = 148,
-     pybind11::arg("sms_reserved") = false);
+     pybind11::arg("sms_reserved") = false, pybind11::arg("may_split") = false);
   m.def("set_sm_reserve", [](int64_t n) { g_sm_reserve = (int)n; }, "persistent kernels use (SM count - n) CTAs");
   m.def("gemm_pair_capacity", &tb::gemm_pair_capacity, "CTA pairs (2-SM clusters) resident at once; 0 before the first launch");
   m.def("stream_place", &stream_place, "(current stream of a device, id of the capture it is in or 0)");

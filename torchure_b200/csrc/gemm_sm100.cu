@@ -561,8 +561,8 @@ static int sum_slices(const float* ws, int64_t stride, int slices, int64_t ldw, 
 // slices: 13.1 us, as the other terms say).
 // Narrow tiles win while the problem is one wave of them (1024 x 512 x 512: 4.8 against 9.1 us; 2048 x 1024 x 4096: 16.2
 // against 25.4), the pair kernel as soon as it fills its 74 SM pairs (4096 x 1024 x 6144: 37.1 against 38.7).
-GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, int force_splits,
-                   int force_tile_n) {
+GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved, bool may_split,
+                   int force_splits, int force_tile_n) {
   GemmPlan p{};
   p.splits = 1;
   if (M <= 0 || N <= 0 || K <= 0) return p;      // an argument error of gemm_bf16
@@ -608,11 +608,12 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
   float best = pair ? 6.9f + 0.30f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits)
                     : 5.f + 0.36f * ceil_div(tiles * p.splits, workers) * ceil_div(num_kb, p.splits);
   if (p.splits > 1 && out_mode == 1) best += 3.f;     // C is cleared first
-  // A bf16 product feeds another layer, and sums in another order round differently: it is split only over a K that no block
-  // has (the loss head's dH over the vocabulary, 600 x 512 x 50257: 226 us in one slice, 36 in ten).  The blocks' products then
-  // add up in one order however many rows come along; what splitting them would gain is little (128 x 1024 x 3072: 10.4 us
-  // in one slice, 8.9 in four; 128 x 1024 x 2048: no difference).
-  const bool may_split = out_mode != 0 || num_kb >= 256;
+  // A bf16 product feeds another layer, and sums in another order round differently: it is split only where the caller allows
+  // it, which the products of a head over its vocabulary do (the loss head's dH, 600 x 512 x 50257: 226 us in one slice, 36
+  // in ten), and there over a long K.  The blocks' products add up in one order however many rows come along, also over the
+  // 2 ffn_dim (16384 and more) of a wide block's input gradient; what splitting them would gain is little (128 x 1024 x 3072:
+  // 10.4 us in one slice, 8.9 in four; 128 x 1024 x 2048: no difference).
+  may_split = out_mode != 0 || (may_split && num_kb >= 256);
   // K slices through a workspace: only where the tiles leave most of the chip idle for a long K.  The slices are fp32 products,
   // which no kernel has for A [K, M] with B [N, K].
   if (may_split && pair && !(a_mn && !b_mn) && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {

@@ -490,6 +490,6 @@ class _LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, shadow = ctx.saved_tensors
         dy = dy.contiguous().to(BF16)
-        dx = K.linear_dgrad(dy, shadow) if ctx.needs_input_grad[0] else None
+        dx = K.linear_dgrad(dy, shadow, may_split=True) if ctx.needs_input_grad[0] else None
         dw = K.linear_wgrad(dy, x, out_dtype=torch.float32) if ctx.needs_input_grad[1] else None
         return dx, dw, None

@@ -47,10 +47,11 @@ def check_comm_error(rank: int | None = None) -> None:
 
 # ---- GEMM ---------------------------------------------------------------------------------------
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
-         out_dtype=BF16, accumulate: bool = False, splits: int = 0) -> torch.Tensor:
+         out_dtype=BF16, accumulate: bool = False, splits: int = 0, may_split: bool = False) -> torch.Tensor:
     """out[M,N] (+)= A * B^T on tcgen05 tensor cores, fp32 accumulation.
 
-    a: [M,K] (or [K,M] when a_mn), b: [N,K] (or [K,N] when b_mn); bf16, innermost stride 1.
+    a: [M,K] (or [K,M] when a_mn), b: [N,K] (or [K,N] when b_mn); bf16, innermost stride 1.  may_split: a bf16 product
+    with few rows and a long K may be summed in slices of K, so that the rounding of a row depends on how many there are.
     """
     M = a.shape[1] if a_mn else a.shape[0]
     N = b.shape[1] if b_mn else b.shape[0]
@@ -59,7 +60,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         out = new_output("gemm", M, N, dtype=out_dtype, device=a.device)
     mode = 0 if out.dtype == BF16 else (2 if accumulate else 1)
     assert not (accumulate and out.dtype == BF16), "accumulation needs an fp32 output"
-    _C().gemm(a, b, out, a_mn, b_mn, mode, splits)
+    _C().gemm(a, b, out, a_mn, b_mn, mode, splits, may_split=may_split)
     ops.count_launch()
     return out
 
@@ -69,9 +70,9 @@ def linear_fwd(x: torch.Tensor, w: torch.Tensor, out=None) -> torch.Tensor:
     return gemm(x, w, out=out)
 
 
-def linear_dgrad(dy: torch.Tensor, w: torch.Tensor, out=None) -> torch.Tensor:
+def linear_dgrad(dy: torch.Tensor, w: torch.Tensor, out=None, may_split: bool = False) -> torch.Tensor:
     """dx[M,K] = dy[M,N] @ w[N,K]   (w is the MN-major B operand)"""
-    return gemm(dy, w, b_mn=True, out=out)
+    return gemm(dy, w, b_mn=True, out=out, may_split=may_split)
 
 
 def linear_wgrad(dy: torch.Tensor, x: torch.Tensor, out=None, out_dtype=BF16, accumulate=False) -> torch.Tensor:

@@ -100,7 +100,7 @@ class _LinearCESm100(torch.autograd.Function):
                 if need_dh or need_dw:
                     K.ce_grad_from_lse_(logits, yc, lse, inv_n, v0, ignore_index)
             if need_dh:
-                K.gemm(logits, w_bf16, b_mn=True, out=d_hidden[lo:hi])
+                K.gemm(logits, w_bf16, b_mn=True, out=d_hidden[lo:hi], may_split=True)
             if need_dw:
                 K.gemm(logits, hc, a_mn=True, b_mn=True, out=d_weight, accumulate=acc0 or lo > 0)
         if vocab_parallel is not None and need_dh:
