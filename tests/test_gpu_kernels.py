@@ -485,6 +485,30 @@ def test_linear_ce_without_gradients():
     assert w.grad is not None
 
 
+# statistics from the product (300 rows) and a pass over stored logits (100)
+@pytest.mark.parametrize("rows,lo,hi", [(300, 16400, 17000), (100, 16400, 17000), (300, 256, 512), (300, 0, 1), (100, 0, 1)])
+def test_linear_ce_without_gradients_infinite_logits(rows, lo, hi):
+    """Vocabulary rows whose logits are all -inf (the last tiles of 256 columns, the first ones, one column) add nothing to the
+    loss; NaN in the same places makes it NaN."""
+    from torchure_b200.loss import fused_linear_cross_entropy
+
+    torch.manual_seed(0)
+    h = (torch.rand(rows, 128, device="cuda") + 0.5).bfloat16()
+    w = (torch.randn(17000, 128, device="cuda") * 0.1).bfloat16()
+    y = torch.randint(512, 16400, (rows,), device="cuda")
+    if (lo, hi) == (256, 512):
+        w[:256] = -3e38
+    w[lo:hi] = -3e38                    # times h beyond the range of fp32
+    with torch.no_grad():
+        loss = fused_linear_cross_entropy(h, w, y, -100, 300)
+        logits = (h.float() @ w.float().t()).bfloat16().double()
+        assert (logits == -float("inf")).any()
+        # logits rounded to bf16 from sums in another order: single ones differ by 2^-8 of their value, at most 2
+        torch.testing.assert_close(loss.double(), torch.nn.functional.cross_entropy(logits, y), rtol=1e-3, atol=0)
+        w[lo:hi] = float("nan")
+        assert fused_linear_cross_entropy(h, w, y, -100, 300).isnan()
+
+
 @pytest.mark.parametrize("C,V,shards", [(64, 1024, 2), (300, 5008, 2), (256, 151936, 4)])   # shard rows stay 16-byte aligned
 def test_ce_vocabulary_sharded_passes(C, V, shards):
     """The two passes of the loss-parallel CE on column shards of one logits matrix (what the ranks of a

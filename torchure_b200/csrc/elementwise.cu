@@ -1095,10 +1095,10 @@ ce_loss_tiles_kernel(const float2* __restrict__ tiles, const float* __restrict__
   for (int i = lane; i < num_tiles; i += 32) {
     const float2 t = tiles[static_cast<int64_t>(i) * rows + row];
     if (t.x > m) { s = s * __expf(m - t.x) + t.y; m = t.x; }
-    else s += t.y * __expf(t.x - m);
+    else s += t.x == -INFINITY ? t.y : t.y * __expf(t.x - m);     // a tile of -inf adds 0, one of NaN its NaN
   }
   const float gm = warp_max(m);
-  const float gs = warp_sum(m == -INFINITY ? 0.f : s * __expf(m - gm));
+  const float gs = warp_sum(m == -INFINITY ? s : s * __expf(m - gm));
   if (lane == 0)
     row_loss[row] = label == ignore_index ? 0.f : gm + __logf(gs) - (label >= 0 && label < V ? target[row] : 0.f);
 }

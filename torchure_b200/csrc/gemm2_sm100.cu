@@ -434,7 +434,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
               lm = fmaxf(lm, fmaxf(x, y));
             }
             if (lm > ce_m) { ce_s *= ex2_approx((ce_m - lm) * kLog2e); ce_m = lm; }
-            const float nm = -ce_m * kLog2e;
+            const float nm = ce_m == -INFINITY ? 0.f : -ce_m * kLog2e;    // only -inf so far: they add nothing
             float s0 = 0.f, s1 = 0.f;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
