@@ -192,12 +192,23 @@ def test_uncovered_shapes_are_loud():
 
 
 @pytest.mark.parametrize("B,S,qk_norm", [(1, 128, True), (3, 384, False), (2, 1152, True)])
-def test_native_block_calls_equal_the_wrappers(B, S, qk_norm):
-    """The block's native forward and backward calls against the same kernels launched one wrapper at a time (what the poison
-    mode does), on both sides of the size up to which launches overlap.  The forward repeats bit for bit; gradients differ by
-    the order of the fp32 dQ additions, which can flip single bf16 roundings behind them (2^-9 each)."""
+def test_native_block_calls_equal_the_wrappers(monkeypatch, B, S, qk_norm):
+    """The block's native forward and backward calls against the same kernels launched one wrapper at a time (what a
+    tensor-parallel axis does, here one whose sums are the terms), on both sides of the size up to which launches overlap.
+    The forward repeats bit for bit; gradients differ by the order of the fp32 dQ additions, which can flip single bf16
+    roundings behind them (2^-9 each).  Neither leaves an element of an output unwritten."""
+    from types import SimpleNamespace
+
+    from torchure_b200 import ops
     from torchure_b200.models import build_model
     from torchure_b200.ops import debug, kernels
+
+    native = []
+    for name in ("block_forward", "block_backward_mlp", "block_backward_attn"):
+        def call(*args, _f=getattr(ops.ext(), name), _name=name):
+            native.append(_name)
+            return _f(*args)
+        monkeypatch.setattr(ops.ext(), name, call)
 
     torch.manual_seed(0)
     with torch.device("cuda"):
@@ -216,10 +227,20 @@ def test_native_block_calls_equal_the_wrappers(B, S, qk_norm):
 
     debug.enable(True)
     try:
+        model.engine().tp = SimpleNamespace(all_reduce_=lambda t: t)
         want, want_grads = run()
+        assert not native and debug.verify() > 3 * 20
+        model.engine().tp = None
+        got, got_grads = run()
+        assert len(native) == 3 * 3
+        names = {n for n, _ in debug._pending}
+        assert {"block_forward.qkv", "block_forward.gu", "block_forward.y", "block_backward.dgu", "block_backward.dqkv",
+                "block_backward.dq_acc", "block_backward.dx0", "wgrad"} <= names
+        assert debug.verify() > 3 * 20
     finally:
         debug.enable(False)
-    got, got_grads = run()
+    again, _ = run()
+    assert torch.equal(again, got)
     assert torch.equal(got, want) and got_grads.keys() == want_grads.keys() and len(got_grads) > 20
     for n, w in want_grads.items():
         assert ((got_grads[n] - w).norm() / w.norm()).item() < 1e-2, n

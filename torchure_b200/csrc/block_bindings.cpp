@@ -20,6 +20,17 @@ constexpr int64_t PDL_MAX_ROWS = 2048;
 
 using torch::Tensor;
 
+// Allocates the outputs.  In the poison mode (ops/debug.py) `track` gets every one before its kernel runs, fills it with NaN and
+// looks later whether one was left.
+struct Outputs {
+  const pybind11::object& track;
+  Tensor operator()(const char* name, c10::IntArrayRef size, const at::TensorOptions& options) const {
+    Tensor t = torch::empty(size, options);
+    if (!track.is_none()) track(name, t);
+    return t;
+  }
+};
+
 __nv_bfloat16* bf(const Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
 
 // Returns the tensors ops/block.py keeps for backward and hands on, and the number of kernels launched:
@@ -28,7 +39,8 @@ std::tuple<std::vector<c10::optional<Tensor>>, int64_t> block_forward(
     const c10::optional<Tensor>& x_in, const c10::optional<Tensor>& y_in, const c10::optional<Tensor>& ids,
     const c10::optional<Tensor>& table, const Tensor& w1, const Tensor& wqkv, const Tensor& qn, const Tensor& kn,
     const Tensor& cos, const Tensor& sin, const Tensor& wo, const Tensor& w2, const Tensor& wgu, const Tensor& wd, int64_t B,
-    int64_t S, int64_t Hq, int64_t Hkv, double eps, bool use_norm, bool want_gu) {
+    int64_t S, int64_t Hq, int64_t Hkv, double eps, bool use_norm, bool want_gu, const pybind11::object& track) {
+  const Outputs make{track};
   c10::cuda::CUDAGuard guard(wqkv.device());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const int64_t M = B * S, D = w1.numel(), F = wd.size(1);
@@ -59,33 +71,34 @@ std::tuple<std::vector<c10::optional<Tensor>>, int64_t> block_forward(
                         b16_table ? bf(*tab) : nullptr, w.data_ptr<float>(), xo, bf(h), rstd.data_ptr<float>(), (int)M, (int)D,
                         (float)eps, stream);
   };
-  Tensor x = has_ids || has_y ? torch::empty({M, D}, f32) : *x_in;
-  Tensor h1 = torch::empty({M, D}, b16), rstd1 = torch::empty({M}, f32);
+  Tensor x = has_ids || has_y ? make("block_forward.x", {M, D}, f32) : *x_in;
+  Tensor h1 = make("block_forward.h1", {M, D}, b16), rstd1 = make("block_forward.rstd1", {M}, f32);
   add_norm(has_x ? x_in->data_ptr<float>() : nullptr, has_y ? bf(*y_in) : nullptr, has_ids ? ids->data_ptr<int64_t>() : nullptr,
            has_ids ? &*table : nullptr, w1, has_ids || has_y ? x.data_ptr<float>() : nullptr, h1, rstd1);
-  Tensor qkv = torch::empty({M, (Hq + 2 * Hkv) * 128}, b16);
+  Tensor qkv = make("block_forward.qkv", {M, (Hq + 2 * Hkv) * 128}, b16);
   product(h1, wqkv, qkv);
-  Tensor qk = torch::empty({M, (Hq + Hkv) * 128}, b16);
+  Tensor qk = make("block_forward.qk", {M, (Hq + Hkv) * 128}, b16);
   tb::qknorm_rope_fwd(bf(qkv), qn.data_ptr<float>(), kn.data_ptr<float>(), cos.data_ptr<float>(), sin.data_ptr<float>(), bf(qk),
                       (int)M, (int)S, (int)Hq, (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, stream);
-  Tensor o = torch::empty({M, Hq * 128}, b16), lse = torch::empty({B, Hq, S}, f32);
+  Tensor o = make("block_forward.o", {M, Hq * 128}, b16), lse = make("block_forward.lse", {B, Hq, S}, f32);
   const int rc = tb::attn_fwd(qk.data_ptr(), qkv.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), (int)B, (int)S, (int)Hq,
                               (int)Hkv, attn_err_word().data_ptr<int>(), stream);
   TORCH_CHECK(rc == 0, "attn_fwd failed with code ", rc);
-  Tensor y_a = torch::empty({M, D}, b16);
+  Tensor y_a = make("block_forward.y_a", {M, D}, b16);
   product(o, wo, y_a);
-  Tensor x2 = torch::empty({M, D}, f32), h2 = torch::empty({M, D}, b16), rstd2 = torch::empty({M}, f32);
+  Tensor x2 = make("block_forward.x2", {M, D}, f32), h2 = make("block_forward.h2", {M, D}, b16);
+  Tensor rstd2 = make("block_forward.rstd2", {M}, f32);
   add_norm(x.data_ptr<float>(), bf(y_a), nullptr, nullptr, w2, x2.data_ptr<float>(), h2, rstd2);
-  Tensor act = torch::empty({M, F}, b16);
+  Tensor act = make("block_forward.act", {M, F}, b16);
   c10::optional<Tensor> gu;
-  if (want_gu) gu = torch::empty({M, 2 * F}, b16);
+  if (want_gu) gu = make("block_forward.gu", {M, 2 * F}, b16);
   if (!bind_gemm_swiglu(h2, wgu, gu, act)) {
-    Tensor both = want_gu ? *gu : torch::empty({M, 2 * F}, b16);
+    Tensor both = want_gu ? *gu : make("block_forward.gu", {M, 2 * F}, b16);
     product(h2, wgu, both);
     tb::swiglu_fwd(bf(both), bf(act), (int)M, (int)F, stream);
     ++launches;
   }
-  Tensor y = torch::empty({M, D}, b16);
+  Tensor y = make("block_forward.y", {M, D}, b16);
   product(act, wd, y);
   return {{x, h1, rstd1, qkv, qk, o, lse, x2, h2, rstd2, gu, act, y}, launches};
 }
@@ -106,26 +119,29 @@ void norm_bwd(const Tensor& dh, const Tensor& x, const Tensor& w, const Tensor& 
 std::tuple<Tensor, Tensor, int64_t> block_backward_mlp(const Tensor& dx2, const Tensor& dy, const Tensor& gu, const Tensor& act,
                                                        const Tensor& h2, const Tensor& x2, const Tensor& w2,
                                                        const Tensor& rstd2, const Tensor& wgu, const Tensor& wd, Tensor dwd,
-                                                       bool add_d, Tensor dwgu, bool add_gu, Tensor dw2) {
+                                                       bool add_d, Tensor dwgu, bool add_gu, Tensor dw2,
+                                                       const pybind11::object& track) {
+  const Outputs make{track};
   c10::cuda::CUDAGuard guard(dy.device());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const int64_t M = dy.size(0), D = dy.size(1), F = wd.size(1);
   check_rows(dy, M, D, torch::kBFloat16, "block_backward: dy");
   check_rows(dx2, M, D, torch::kFloat32, "block_backward: dx2");
   int64_t launches = 5;
-  Tensor dgu = torch::empty({M, 2 * F}, dy.options());
+  Tensor dgu = make("block_backward.dgu", {M, 2 * F}, dy.options());
   if (!bind_gemm_swiglu_bwd(dy, wd, gu, dgu)) {
-    Tensor d_act = torch::empty({M, F}, dy.options());
+    Tensor d_act = make("block_backward.d_act", {M, F}, dy.options());
     bind_gemm(dy, wd, d_act, false, true, 0);
     tb::swiglu_bwd(bf(d_act), bf(gu), bf(dgu), (int)M, (int)F, stream);
     ++launches;
   }
   bind_gemm(dy, act, dwd, true, true, add_d ? 2 : 1);
-  Tensor d_h2 = torch::empty({M, D}, dy.options());
+  Tensor d_h2 = make("block_backward.d_h2", {M, D}, dy.options());
   bind_gemm(dgu, wgu, d_h2, false, true, 0);
   bind_gemm(dgu, h2, dwgu, true, true, add_gu ? 2 : 1);
   dgu = Tensor();
-  Tensor dx1 = torch::empty_like(dx2), dx1b = torch::empty({M, D}, dy.options());
+  Tensor dx1 = make("block_backward.dx1", {M, D}, dx2.options());
+  Tensor dx1b = make("block_backward.dx1b", {M, D}, dy.options());
   norm_bwd(d_h2, x2, w2, rstd2, dx2, dx1, dx1b, dw2, stream);
   return {dx1, dx1b, launches};
 }
@@ -136,7 +152,8 @@ std::tuple<Tensor, c10::optional<Tensor>, int64_t> block_backward_attn(
     const Tensor& h1, const Tensor& x, const Tensor& w1, const Tensor& rstd1, const Tensor& qn, const Tensor& kn,
     const Tensor& cos, const Tensor& sin, const Tensor& wqkv, const Tensor& wo, Tensor dwo, bool add_o, Tensor dwqkv,
     bool add_qkv, Tensor dqn, Tensor dkn, Tensor dw1, const c10::optional<Tensor>& dx_out, bool want_b16, int64_t B, int64_t S,
-    int64_t Hq, int64_t Hkv, double eps, bool use_norm) {
+    int64_t Hq, int64_t Hkv, double eps, bool use_norm, const pybind11::object& track) {
+  const Outputs make{track};
   c10::cuda::CUDAGuard guard(dx1.device());
   auto stream = at::cuda::getCurrentCUDAStream().stream();
   const int64_t M = dx1.size(0), D = dx1.size(1), nqkv = (Hq + 2 * Hkv) * 128;
@@ -146,11 +163,12 @@ std::tuple<Tensor, c10::optional<Tensor>, int64_t> block_backward_attn(
   TORCH_CHECK(M == B * S && lse.is_contiguous() && lse.numel() == B * Hq * S, "block_backward: sizes");
   TORCH_CHECK(cos.is_contiguous() && sin.is_contiguous() && cos.size(0) >= S && cos.size(-1) == 128, "block_backward: tables");
   int* err = attn_err_word().data_ptr<int>();
-  Tensor d_o = torch::empty({M, Hq * 128}, dx1b.options());
+  Tensor d_o = make("block_backward.d_o", {M, Hq * 128}, dx1b.options());
   bind_gemm(dx1b, wo, d_o, false, true, 0);
   bind_gemm(dx1b, o, dwo, true, true, add_o ? 2 : 1);
-  Tensor stats = torch::empty({2, M * Hq}, dx1.options()), dq_acc = torch::empty({M, Hq * 128}, dx1.options());
-  Tensor dqkv = torch::empty({M, nqkv}, dx1b.options());
+  Tensor stats = make("block_backward.stats", {2, M * Hq}, dx1.options());
+  Tensor dq_acc = make("block_backward.dq_acc", {M, Hq * 128}, dx1.options());
+  Tensor dqkv = make("block_backward.dqkv", {M, nqkv}, dx1b.options());
   float* nds = stats.data_ptr<float>();
   float* nlse2 = nds + M * Hq;
   int rc = tb::attn_bwd_stats(d_o.data_ptr(), o.data_ptr(), lse.data_ptr<float>(), nds, nlse2, dq_acc.data_ptr<float>(), (int)B,
@@ -167,13 +185,13 @@ std::tuple<Tensor, c10::optional<Tensor>, int64_t> block_backward_attn(
                            (int)S, (int)Hq, (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, bind_num_sms(), err, stream);
   TORCH_CHECK(rc == 0, "qknorm_rope_bwd failed with code ", rc);
   dq_acc = Tensor();
-  Tensor d_h1 = torch::empty({M, D}, dx1b.options());
+  Tensor d_h1 = make("block_backward.d_h1", {M, D}, dx1b.options());
   bind_gemm(dqkv, wqkv, d_h1, false, true, 0);
   bind_gemm(dqkv, h1, dwqkv, true, true, add_qkv ? 2 : 1);
-  Tensor dx0 = dx_out.has_value() && dx_out->defined() ? *dx_out : torch::empty_like(dx1);
+  Tensor dx0 = dx_out.has_value() && dx_out->defined() ? *dx_out : make("block_backward.dx0", {M, D}, dx1.options());
   check_rows(dx0, M, D, torch::kFloat32, "block_backward: dx_out");
   c10::optional<Tensor> dx0b;
-  if (want_b16) dx0b = torch::empty({M, D}, dx1b.options());
+  if (want_b16) dx0b = make("block_backward.dx0b", {M, D}, dx1b.options());
   norm_bwd(d_h1, x, w1, rstd1, dx1, dx0, dx0b, dw1, stream);
   return {dx0, dx0b, 8};
 }

@@ -210,10 +210,10 @@ class _BlockFn(torch.autograd.Function):
         cos, sin = eng.rope_tables(S, w1.device)
         need_grad = want_grad and any(ctx.needs_input_grad)
         table_used = eng.emb_shadow if eng.bf16_embedding else table
-        if eng.cp is None and eng.tp is None and not debug.enabled() and attn_ops.kernel_supported(S, Hq, Hkv, hd):
+        if eng.cp is None and eng.tp is None and attn_ops.kernel_supported(S, Hq, Hkv, hd):
             (x, h1, rstd1, qkv, qk, o, lse, x2, h2, rstd2, gu, act, y_out), n = ops.ext().block_forward(
                 x_in, y_in, ids, table_used, w1, sh.wqkv, qn, kn, cos, sin, sh.wo, w2, sh.wgu, sh.wd, B, S, Hq, Hkv, eps,
-                use_norm, need_grad)
+                use_norm, need_grad, debug.tracker())
             ops.count_launch(n)
             st = attn_ops.AttnState("sm100", o, lse)
         else:
@@ -268,7 +268,7 @@ class _BlockFn(torch.autograd.Function):
         dx_out = out.sink.embed_rows_dest(x.shape[0], x.shape[1]) if early else None
         dests = None
         # ranks that reduce gradients under the backward pass are told of each one as it is launched (the other branch)
-        if (eng.cp is None and eng.tp is None and not debug.enabled() and attn_ops.single_pass(ctx.attn_state)
+        if (eng.cp is None and eng.tp is None and attn_ops.single_pass(ctx.attn_state)
                 and (out.sink is None or getattr(out.sink, "world", 0) == 1)):
             dests = [out.dest(ps) for ps in ((P["wd"],), (P["wg"], P["wu"]), (P["wo"],), (P["wq"], P["wk"], P["wv"]))]
         if dests is not None and None not in dests:
@@ -278,11 +278,12 @@ class _BlockFn(torch.autograd.Function):
             dw2, dw1 = small[0], small[-1]
             dqn, dkn = small[1:3] if use_norm else (eng.dummy, eng.dummy)
             dx1, dx1_b, n_mlp = ops.ext().block_backward_mlp(dx2, dy, gu, act, h2, x2, w2, rstd2, sh.wgu, sh.wd, dwd, add_d, dwgu,
-                                                             add_gu, dw2)
+                                                             add_gu, dw2, debug.tracker())
             out.written((P["wd"], P["wg"], P["wu"], P["w2"]))
             dx0, dx0_b, n_attn = ops.ext().block_backward_attn(
                 dx1, dx1_b, o, ctx.attn_state.lse, qk, qkv, h1, x, w1, rstd1, qn, kn, cos, sin, sh.wqkv, sh.wo, dwo, add_o,
-                dwqkv, add_qkv, dqn, dkn, dw1, dx_out, want_prev, B, S, Hq, Hkv, eps, use_norm)
+                dwqkv, add_qkv, dqn, dkn, dw1, dx_out, want_prev, B, S, Hq, Hkv, eps, use_norm,
+                debug.tracker())
             out.written((P["wo"], P["wq"], P["wk"], P["wv"], *gains[1:-1]))
             ctx.attn_state = None
             ops.count_launch(n_mlp + n_attn)
@@ -413,7 +414,7 @@ class _GradOut:
         """(fp32 destination of the whole fused matrix, accumulate?); None when a sink keeps its parts apart."""
         if self.sink is None:
             rows = [p.shape[0] for p in params]
-            dw = torch.empty(sum(rows), params[0].shape[1], dtype=torch.float32, device=self.device)
+            dw = debug.new_output("wgrad", sum(rows), params[0].shape[1], dtype=torch.float32, device=self.device)
             for p, part in zip(params, dw.split(rows)):
                 self.grads[p] = part
             return dw, False

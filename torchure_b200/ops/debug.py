@@ -1,8 +1,8 @@
 """Poison-and-verify mode for the kernel wrappers (race / coverage detection without a sanitizer).
 
 With ``TORCHURE_B200_POISON=1`` (or ``enable()``), every output buffer that ``ops/kernels.py`` allocates for a kernel
-that must overwrite it completely is first filled with NaN and remembered; ``verify()`` synchronises and raises if
-any remembered buffer still holds a NaN, naming the wrapper that allocated it.  A kernel that skips a tile, a row or
+that must overwrite it completely, and every one that the native calls of a block allocate, is first filled with NaN and
+remembered; ``verify()`` synchronises and raises if any remembered buffer still holds a NaN, naming the wrapper that allocated it.  A kernel that skips a tile, a row or
 a tail element, or a consumer that runs before its producer, shows up as a surviving sentinel.  Inputs containing NaN
 are the caller's business: use finite test data.  Costs one fill per output, so it is a debugging mode only.
 """
@@ -31,10 +31,21 @@ def enabled() -> bool:
 def new_output(name: str, *shape, dtype, device) -> torch.Tensor:
     """``torch.empty`` for a kernel output; poisoned and tracked when the mode is on."""
     t = torch.empty(*shape, dtype=dtype, device=device)
-    if _enabled and t.is_floating_point():
+    if _enabled:
+        track(name, t)
+    return t
+
+
+def track(name: str, t: torch.Tensor) -> None:
+    """Poison a fresh output and remember it."""
+    if t.is_floating_point():
         t.fill_(float("nan"))
         _pending.append((name, t))
-    return t
+
+
+def tracker():
+    """What native code that allocates its outputs itself is given: ``track`` in this mode, else None."""
+    return track if _enabled else None
 
 
 def verify() -> int:
