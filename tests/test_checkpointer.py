@@ -4,6 +4,7 @@ step falls back, explicit torn step refused, non-numeric directories ignored).""
 
 import os
 
+import pytest
 import torch
 
 from tests.tiny import TINY
@@ -93,6 +94,49 @@ def test_complete_marker_semantics(tmp_path):
     ck.mark_complete(10)
     assert ck.latest() == 10
     assert not list((tmp_path / "run" / "10").glob("*.tmp"))
+
+
+def test_ranks_that_write_the_same_file(tmp_path, monkeypatch):
+    """Two writers of one file, the second from start to end inside the first's save (ranks of one data coordinate on two
+    hosts, process ids equal): both succeed, and nothing but the file is left."""
+    from torchure_b200.ckpt import Checkpointer
+
+    first, second = Checkpointer(str(tmp_path)), Checkpointer(str(tmp_path))
+    save, inside = torch.save, []
+
+    def interleaved(payload, path):
+        save(payload, path)
+        if not inside:
+            inside.append(path)
+            second.save_trainer({"step": 3, "by": "second"}, 3)
+
+    monkeypatch.setattr(torch, "save", interleaved)
+    first.save_trainer({"step": 3, "by": "first"}, 3)
+    assert inside and [p.name for p in (tmp_path / "3").iterdir()] == ["trainer.pt"]
+    assert first.load_trainer(3)["by"] == "first"
+
+
+def test_no_temporary_files_stay(tmp_path, monkeypatch):
+    """A failed write removes its temporary file; one that a killed writer left goes when the step is complete."""
+    from torchure_b200.ckpt import Checkpointer
+
+    ck = Checkpointer(str(tmp_path))
+    save = torch.save
+
+    def full_disk(payload, path):
+        save(payload, path)
+        raise OSError("no space left")
+
+    monkeypatch.setattr(torch, "save", full_disk)
+    with pytest.raises(OSError):
+        ck.save_trainer({"step": 4}, 4)
+    assert not list((tmp_path / "4").iterdir())
+    monkeypatch.setattr(torch, "save", save)
+    for name in ("trainer.pt.tmp", "trainer.pt.4711.tmp"):
+        (tmp_path / "4" / name).write_bytes(b"half a file")
+    ck.save_trainer({"step": 4}, 4)
+    ck.mark_complete(4)
+    assert sorted(p.name for p in (tmp_path / "4").iterdir()) == [".complete", "trainer.pt"]
 
 
 def test_prefetcher_position_is_exact(tmp_path):

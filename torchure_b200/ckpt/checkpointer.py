@@ -20,6 +20,7 @@ host snapshots while training goes on; the marker is only written once every ran
 from __future__ import annotations
 
 import os
+import uuid
 from pathlib import Path
 
 import torch
@@ -107,7 +108,12 @@ class Checkpointer:
         return d
 
     def mark_complete(self, step: int) -> None:
-        (self.step_dir(step, create=True) / MARKER).touch()
+        """Called when every rank's files of the step are on disk: a temporary file that is still there was left by a
+        writer that died in an earlier attempt at this step."""
+        d = self.step_dir(step, create=True)
+        for left in d.glob("*.tmp"):
+            left.unlink(missing_ok=True)
+        (d / MARKER).touch()
 
     def is_complete(self, step: int) -> bool:
         return (self.step_dir(step) / MARKER).exists()
@@ -144,9 +150,14 @@ class Checkpointer:
 
     def _write_now(self, payload, step: int, name: str) -> None:
         final = self.step_dir(step, create=True) / name
-        tmp = final.with_name(f"{final.name}.{os.getpid()}.tmp")   # ranks that share a data coordinate write the same file
-        torch.save(payload, tmp)
-        os.replace(tmp, final)
+        # ranks that share a data coordinate write the same file, from several hosts perhaps: a temporary file each
+        tmp = final.with_name(f"{final.name}.{uuid.uuid4().hex}.tmp")
+        try:
+            torch.save(payload, tmp)
+            os.replace(tmp, final)
+        except BaseException:
+            tmp.unlink(missing_ok=True)
+            raise
 
     def _read(self, step: int, name: str, weights_only: bool = True):
         return torch.load(self.step_dir(step) / name, map_location="cpu", weights_only=weights_only)
