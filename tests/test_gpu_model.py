@@ -191,6 +191,21 @@ def test_uncovered_shapes_are_loud():
     assert out.shape == (1, 100, 512)
 
 
+def test_blocks_and_norms_exchanged_after_the_first_pass():
+    """A model whose engine has run: a dropped block and an exchanged norm are those of the next pass."""
+    from torchure_b200.models.qwen3 import RMSNorm
+
+    fast, slow = _pair()
+    ids = torch.randint(0, CFG["vocab_size"], (1, 128), device="cuda")
+    with torch.no_grad():
+        assert relerr(fast(ids), slow(ids)) < 2e-2
+        for model in (fast, slow):
+            model.blocks = model.blocks[:1]
+            model.blocks[0].norm1 = RMSNorm(CFG["emb_dim"]).cuda()
+            model.blocks[0].norm1.weight.mul_(torch.linspace(-2, 2, CFG["emb_dim"], device="cuda"))
+        assert relerr(fast(ids), slow(ids)) < 2e-2
+
+
 @pytest.mark.parametrize("B,S,qk_norm", [(1, 128, True), (3, 384, False), (2, 1152, True)])
 def test_native_block_calls_equal_the_wrappers(monkeypatch, B, S, qk_norm):
     """The block's native forward and backward calls against the same kernels launched one wrapper at a time (what a

@@ -210,3 +210,45 @@ def test_llama3_registry_and_defaults():
     assert m.cfg["head_dim"] == 16 and m.cfg["qk_norm"] is False and m.cfg["rope_theta"] == 500_000.0
     assert not hasattr(m.blocks[0].gqa, "q_norm")
     assert m.lm_head.weight is m.token_emb.weight
+
+
+@pytest.mark.parametrize("qk_norm", [True, False])
+def test_engine_reads_the_modules_a_block_has_now(qk_norm):
+    """The parameters that the execution engine hands to a block are those of the modules in place at that call: exchanged
+    norms, projections and whole sub-modules are seen, parametrised weights too."""
+    from torchure_b200.models import Qwen3
+    from torchure_b200.models.qwen3 import RMSNorm, SwiGLU
+    from torchure_b200.ops.block import _LayerShadow
+
+    block = Qwen3(1, 4, 2, 64, 16, 32, ffn_dim=48, qk_norm=qk_norm).blocks[0]
+    sh, dummy = _LayerShadow(block, "cpu"), torch.zeros(1)
+
+    def want():
+        g, f = block.gqa, block.ffn
+        gains = [g.q_norm.weight, g.k_norm.weight] if g.qk_norm else [dummy, dummy]
+        return [block.norm1.weight, g.q_proj.weight, g.k_proj.weight, g.v_proj.weight, g.o_proj.weight, *gains,
+                block.norm2.weight, f.gate_proj.weight, f.up_proj.weight, f.down_proj.weight]
+
+    def check():
+        got = sh.inputs(block, dummy)
+        assert len(got) == 11 and all(a is b for a, b in zip(got, want()))
+
+    check()
+    check()
+    block.norm1 = RMSNorm(64)
+    check()
+    block.gqa.o_proj = torch.nn.Linear(64, 64, bias=False)
+    check()
+    block.ffn = SwiGLU(64, 48)
+    check()
+    block.norm2.weight = torch.nn.Parameter(torch.rand(64))
+    check()
+    block.gqa.qk_norm = False
+    check()
+
+    class Doubled(torch.nn.Module):
+        def forward(self, w):
+            return 2 * w
+
+    torch.nn.utils.parametrize.register_parametrization(block.ffn.up_proj, "weight", Doubled())
+    assert torch.equal(sh.inputs(block, dummy)[9], block.ffn.up_proj.weight)

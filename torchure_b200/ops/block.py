@@ -62,8 +62,7 @@ class _LayerShadow:
                            wo=g.o_proj.weight, qn=g.q_norm.weight if g.qk_norm else None,
                            kn=g.k_norm.weight if g.qk_norm else None, w2=block.norm2.weight,
                            wg=f.gate_proj.weight, wu=f.up_proj.weight, wd=f.down_proj.weight, table=None)
-        self._modules = (block.norm1, g.q_proj, g.k_proj, g.v_proj, g.o_proj, g.q_norm if g.qk_norm else None,
-                         g.k_norm if g.qk_norm else None, block.norm2, f.gate_proj, f.up_proj, f.down_proj)
+        self._seen = None
         self.pairs = [
             (g.q_proj.weight, self.wqkv[:nq]), (g.k_proj.weight, self.wqkv[nq:nq + nkv]),
             (g.v_proj.weight, self.wqkv[nq + nkv:]), (g.o_proj.weight, self.wo),
@@ -71,12 +70,20 @@ class _LayerShadow:
         ]
 
 
-    def inputs(self, dummy):
-        """The block's parameters in the order of ``_BlockFn``, as the modules hold them now; without QK-norm its gains are
+    def inputs(self, block, dummy):
+        """The block's parameters in the order of ``_BlockFn``, as its modules hold them now; without QK-norm its gains are
         the engine's dummy.  Read from the modules' tables: attribute look-ups through ``Module.__getattr__`` cost a short
-        forward pass 7 us per block."""
+        forward pass 7 us per block, so the modules are looked up again only when one was exchanged."""
+        seen = self._seen
+        if (seen is None or block._modules != seen[0] or seen[1]._modules != seen[2] or seen[3]._modules != seen[4]
+                or seen[1].qk_norm != seen[5]):
+            g, f = block.gqa, block.ffn
+            qk = g.qk_norm
+            modules = (block.norm1, g.q_proj, g.k_proj, g.v_proj, g.o_proj, g.q_norm if qk else None,
+                       g.k_norm if qk else None, block.norm2, f.gate_proj, f.up_proj, f.down_proj)
+            seen = self._seen = (dict(block._modules), g, dict(g._modules), f, dict(f._modules), qk, modules)
         out = []
-        for m in self._modules:
+        for m in seen[6]:
             w = dummy if m is None else m._parameters.get("weight")
             out.append(m.weight if w is None else w)
         return out
@@ -179,14 +186,14 @@ class Sm100Engine:
         want_grad = torch.is_grad_enabled()
         if self.pre_block is not None:
             self.pre_block(-1)
-        for i, sh in enumerate(self.layers):
+        for i, (block, sh) in enumerate(zip(m.blocks, self.layers)):
             if self.pre_block is not None:
                 self.pre_block(i)
             first = i == 0
             x, y = _BlockFn.apply(
                 self, sh, i, B, S, flat_ids if first else None,
                 m.token_emb.weight if first else None, x, y,
-                *sh.inputs(self.dummy),
+                *sh.inputs(block, self.dummy),
                 want_grad)
         h = _FinalNormFn.apply(x, y, m.norm.weight, m.norm.eps, self)
         if self.tied and torch.is_grad_enabled() and m.token_emb.weight.requires_grad:
