@@ -191,6 +191,25 @@ def test_uncovered_shapes_are_loud():
     assert out.shape == (1, 100, 512)
 
 
+def test_strided_token_ids():
+    """Tokens that are a strided view, one sequence (whose flat form is a view as well) and two: loss and table gradient of
+    the copied tokens."""
+    from torchure_b200.objectives import ARObjective
+
+    fast, _ = _pair()
+    obj = ARObjective(fused_linear_ce=True, ce_chunk_size=200)
+    for B in (1, 2):
+        wide = torch.randint(0, CFG["vocab_size"], (B, 256), device="cuda")
+        got = []
+        for ids in (wide[:, ::2], wide[:, ::2].contiguous()):
+            fast.zero_grad()
+            loss = obj.compute_loss(fast, {"input_ids": ids, "labels": ids})
+            loss.backward()
+            got.append((loss.item(), fast.token_emb.weight.grad.clone()))
+        assert got[0][0] == got[1][0]
+        assert relerr(got[0][1], got[1][1]) < 1e-2      # the order of the fp32 dQ additions is open
+
+
 def test_blocks_and_norms_exchanged_after_the_first_pass():
     """A model whose engine has run: a dropped block and an exchanged norm are those of the next pass."""
     from torchure_b200.models.qwen3 import RMSNorm

@@ -181,7 +181,7 @@ class Sm100Engine:
         self.refresh()
         B, S = ids.shape
         x, y = None, None
-        flat_ids = ids.reshape(-1)
+        flat_ids = ids.reshape(-1).contiguous()      # one strided sequence reshapes to a strided view
         # under no_grad the parameters still count as inputs that need gradients
         want_grad = torch.is_grad_enabled()
         if self.pre_block is not None:
