@@ -485,6 +485,54 @@ def test_linear_ce_without_gradients():
     assert w.grad is not None
 
 
+@pytest.mark.parametrize("rows,vocab,chunk,paths", [(1100, 50257, 512, [True, True, False]), (900, 20001, 300, [True] * 3),
+                                                    (300, 1000, 128, [False] * 3)])
+def test_linear_ce_without_gradients_chunk_by_chunk(monkeypatch, rows, vocab, chunk, paths):
+    """Chunks whose logits are not stored (more than 128 rows), a short last one that stores them, and only such: the loss
+    of every chunk's rows by themselves, ignored and out-of-range labels among them, is that of the pass with gradients.
+    The same logits, summed in another order: 2^-24 x 16 relative per row, as in the test of the statistics."""
+    from torchure_b200.loss import fused_linear_cross_entropy
+    from torchure_b200.ops import debug
+    from torchure_b200.ops import kernels as K
+
+    torch.manual_seed(0)
+    h = torch.randn(rows, 256, device="cuda").bfloat16()
+    w = (torch.randn(vocab, 256, device="cuda") * 0.2).bfloat16().requires_grad_()
+    y = torch.randint(0, vocab, (rows,), device="cuda")
+    y[::9] = -100
+    y[5] = vocab + 3
+    taken, gemm_ce = [], K.gemm_ce
+    monkeypatch.setattr(K, "gemm_ce", lambda *a: taken.append(gemm_ce(*a)) or taken[-1])
+    for lo in (0, *range(0, rows, chunk)):
+        part = y.clone() if not taken else torch.full_like(y, -100)
+        part[lo:lo + chunk] = y[lo:lo + chunk]
+        full = fused_linear_cross_entropy(h, w, part, -100, chunk)
+        before = len(taken)
+        with torch.no_grad():
+            loss = fused_linear_cross_entropy(h, w, part, -100, chunk)
+        assert [t is not None for t in taken[before:]] == paths
+        torch.testing.assert_close(loss, full.detach(), rtol=2e-6, atol=0)
+    debug.enable(True)
+    try:
+        with torch.no_grad():
+            fused_linear_cross_entropy(h, w, y, -100, chunk)
+        assert sum(n == "gemm_ce.stats" for n, _ in debug._pending) == sum(paths)
+        debug.verify()
+    finally:
+        debug.enable(False)
+
+
+def test_gemm_ce_decides_before_it_allocates():
+    from torchure_b200.ops import kernels as K
+
+    h, w = torch.zeros(128, 64, device="cuda").bfloat16(), torch.zeros(1 << 20, 64, device="cuda").bfloat16()
+    y, target = torch.zeros(128, dtype=torch.int64, device="cuda"), torch.empty(128, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    assert K.gemm_ce(h, w, y, target) is None and torch.cuda.max_memory_allocated() == before
+
+
 # statistics from the product (300 rows) and a pass over stored logits (100)
 @pytest.mark.parametrize("rows,lo,hi", [(300, 16400, 17000), (100, 16400, 17000), (300, 256, 512), (300, 0, 1), (100, 0, 1)])
 def test_linear_ce_without_gradients_infinite_logits(rows, lo, hi):

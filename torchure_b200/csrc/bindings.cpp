@@ -109,24 +109,27 @@ bool gemm_swiglu_bwd(const torch::Tensor& dy, const torch::Tensor& w, const torc
   return true;
 }
 
-// As above.  stats: fp32 [ceil(N / 256), M, 2], target: fp32 [M].
-bool gemm_ce(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& labels, torch::Tensor& stats,
-             torch::Tensor& target) {
+// The statistics, fp32 [ceil(N / 256), M, 2], or None (nothing launched or allocated) as above; target: fp32 [M].
+c10::optional<torch::Tensor> gemm_ce(const torch::Tensor& a, const torch::Tensor& b, const torch::Tensor& labels,
+                                     torch::Tensor& target, const pybind11::object& track) {
   TORCH_CHECK(a.scalar_type() == torch::kBFloat16 && b.scalar_type() == torch::kBFloat16, "gemm_ce: bf16 operands");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && a.size(1) == b.size(1),
               "gemm_ce: 2-D operands with innermost stride 1");
   const int64_t M = a.size(0), N = b.size(0), K = a.size(1);
   TORCH_CHECK(labels.scalar_type() == torch::kInt64 && labels.is_contiguous() && labels.numel() == M, "gemm_ce: labels");
-  TORCH_CHECK(stats.scalar_type() == torch::kFloat32 && stats.is_contiguous() && stats.numel() >= 2 * M * ((N + 255) / 256) &&
-                  target.scalar_type() == torch::kFloat32 && target.is_contiguous() && target.numel() >= M,
-              "gemm_ce: stats must be fp32 [ceil(N / 256), M, 2], target fp32 [M]");
-  if (M == 0 || tb::gemm_plan((int)M, (int)N, (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind != tb::GemmPlan::kPair) return false;
+  TORCH_CHECK(target.scalar_type() == torch::kFloat32 && target.is_contiguous() && target.numel() >= M,
+              "gemm_ce: target must be fp32 [M]");
+  if (M == 0 || tb::gemm_plan((int)M, (int)N, (int)K, false, false, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind !=
+                    tb::GemmPlan::kPair)
+    return c10::nullopt;
   c10::cuda::CUDAGuard guard(a.device());
+  torch::Tensor stats = torch::empty({(N + 255) / 256, M, 2}, target.options());
+  if (!track.is_none()) track("gemm_ce.stats", stats);
   const int rc = tb::gemm2_ce(a.data_ptr(), b.data_ptr(), (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
                               labels.data_ptr<int64_t>(), stats.data_ptr<float>(), target.data_ptr<float>(),
                               err_word().data_ptr<int>(), num_sms(), cur_stream());
   TORCH_CHECK(rc == 0, "gemm2_ce failed with code ", rc);
-  return true;
+  return stats;
 }
 
 void add_rmsnorm_fwd(c10::optional<torch::Tensor> x, c10::optional<torch::Tensor> y, c10::optional<torch::Tensor> ids,

@@ -9,6 +9,7 @@ from __future__ import annotations
 import torch
 
 from torchure_b200 import ops
+from torchure_b200.ops import debug
 from torchure_b200.ops.debug import new_output
 
 BF16 = torch.bfloat16
@@ -192,10 +193,9 @@ def gemm_ce(a, b, labels, target):
     """Partial softmax statistics of the rows of a @ b^T, [ceil(N / 256), M, 2] fp32 (maximum and sum of exponentials per 256
     columns), and the labels' logits in `target`; the product is not stored.  None when the problem runs on another kernel
     than the CTA-pair one (nothing was launched)."""
-    stats = torch.empty((b.shape[0] + 255) // 256, a.shape[0], 2, dtype=torch.float32, device=a.device)
-    if not _C().gemm_ce(a, b, labels, stats, target):
-        return None
-    ops.count_launch()
+    stats = _C().gemm_ce(a, b, labels, target, debug.tracker())
+    if stats is not None:
+        ops.count_launch()
     return stats
 
 
