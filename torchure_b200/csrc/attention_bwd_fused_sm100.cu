@@ -112,6 +112,9 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t local, uint32_t rank, con
       : "memory");
 }
 
+// SHARED: clusters of a.parts CTAs per key block, else one CTA each.  Two kernels, because the split's index arithmetic in
+// front of the first load costs a short problem 5 % (4 x 128 tokens, 16 / 8 heads: 14.6 us without it, 15.5 with).
+template <bool SHARED>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -138,8 +141,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int nqb = a.Sq / 128;
   const int ratio = a.Hq / a.Hkv;
   const int groups = a.B * a.Hkv;
-  const int part = static_cast<int>(blockIdx.x) % a.parts;   // == rank in the cluster
-  const int tile = static_cast<int>(blockIdx.x) / a.parts;
+  const int part = SHARED ? static_cast<int>(blockIdx.x) % a.parts : 0;   // == rank in the cluster
+  const int tile = SHARED ? static_cast<int>(blockIdx.x) / a.parts : static_cast<int>(blockIdx.x);
   const int kblk = tile / groups;            // causal: block 0 sees the most query blocks, it goes first
   const int g = tile % groups;
   const int kvh = g % a.Hkv, b = g / a.Hkv;
@@ -148,8 +151,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int qb0 = a.causal ? kblk : 0;       // first visible query block
   const int n_qb = nqb - qb0;
   // iteration = (query head of the group, query block); this CTA's are [it0, it0 + n_iter), possibly none
-  const int it0 = n_qb * ratio * part / a.parts;
-  const int n_iter = n_qb * ratio * (part + 1) / a.parts - it0;
+  const int it0 = SHARED ? n_qb * ratio * part / a.parts : 0;
+  const int n_iter = SHARED ? n_qb * ratio * (part + 1) / a.parts - it0 : n_qb * ratio;
+  const bool busy = !SHARED || n_iter > 0;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ);
@@ -181,7 +185,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (n_iter > 0 && elect_one()) {
+    if (busy && elect_one()) {
       const int kcol = a.k_col0 + kvh * HD, vcol = a.v_col0 + kvh * HD;
       mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES);
       tma_load_2d(sK, &tmK, &bars->kv_full, kcol, krow_in);
@@ -210,7 +214,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (n_iter > 0 && elect_one()) {
+    if (busy && elect_one()) {
       constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, false, false);   // S^T / dP^T halves: N = 64 queries
       constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, false, true);  // A in TMEM, B MN-major, N = 128 (hd)
       constexpr uint32_t idesc_dq = make_idesc_bf16(128, 64, true, true);     // K^T (MN-major) x dS^T (MN-major)
@@ -383,11 +387,11 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll
       for (int j = 0; j < 32; ++j) red_add_unordered(dst + j * HD, __uint_as_float(v[j]));
     }
-    if (n_iter > 0) {
+    if (busy) {
       ok = ok && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait);
       tc_fence_after();
     }
-    if (ok && a.parts == 1) {
+    if (!SHARED && ok) {
       // group 0 writes dV, group 1 dK: this warp's 64 of the 128 head-dim columns, one key row per lane, straight to
       // global memory
       {
@@ -413,7 +417,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   }
 
-  if (a.parts > 1) {
+  if constexpr (SHARED) {
     __syncwarp();
     cluster_sync_all();        // the products of every CTA are done: its operand stages may be written
     const int cw = 256 / a.parts;                    // columns of dV | dK that this CTA sums: 32 and more
@@ -425,7 +429,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 #pragma unroll 1
       for (int c = 0; c < 64; c += 32) {
         uint32_t v[32];
-        if (n_iter > 0) {
+        if (busy) {
           tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + 256 + c0 + c, v);
           tmem_ld_wait();
         } else {
@@ -598,7 +602,6 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   if (r) return r - 200;
   r = make_tmap_2d(&tdo, d_o, 2, Mq, static_cast<uint64_t>(Hq) * HD, static_cast<uint64_t>(Hq) * HD, 128, 64);
   if (r) return r - 300;
-  if (!ensure_dynamic_smem(reinterpret_cast<const void*>(attn_bwd_fused_kernel), SMEM_BYTES)) return -20;
   FusedArgs a{};
   a.dq_acc = dq_acc;
   a.dk = reinterpret_cast<__nv_bfloat16*>(dk);
@@ -617,6 +620,8 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   a.scale_log2 = a.scale * 1.4426950408889634f;
   const int tiles = (Skv / 128) * B * Hkv;
   a.parts = bwd_parts(tiles, (Sq / 128) * (Hq / Hkv));
+  const auto kern = a.parts > 1 ? attn_bwd_fused_kernel<true> : attn_bwd_fused_kernel<false>;
+  if (!ensure_dynamic_smem(reinterpret_cast<const void*>(kern), SMEM_BYTES)) return -20;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(tiles * a.parts);
   cfg.blockDim = dim3(NUM_THREADS);
@@ -631,7 +636,7 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = a.parts > 1 ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, attn_bwd_fused_kernel, tq, tk, tv, tdo, a, err) != cudaSuccess) return -21;
+  if (cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, a, err) != cudaSuccess) return -21;
   return 0;
 }
 
