@@ -273,187 +273,226 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
       const int m0 = (tile % num_m) * 2 * BM + static_cast<int>(rank) * BM;
       const int n0 = (tile / num_m) * TN;
       const int acc = it & 1;
-      uint32_t gv[2][16], uv[2][16];     // kEpiSwigluBwd: gate and up of 32 columns, two sets
-      auto load_gu = [&](int c, auto set_tag) {     // half `set` of slab c of this lane's row; zeros outside the matrix
-        constexpr int set = decltype(set_tag)::value;
-        const int gr = m0 + q * 32 + lane;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int col = n0 + c * 64 + set * 32 + j * 16;
-          const bool in = gr < M && col < N;
-          const __nv_bfloat16* p = ea.gu + static_cast<int64_t>(gr) * 2 * N + col;
-          if (in) {
-            load_sector(p, &gv[set][8 * j]);
-            load_sector(p + N, &uv[set][8 * j]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) gv[set][8 * j + i] = uv[set][8 * j + i] = 0u;
-          }
-        }
-      };
-      if constexpr (EPI == kEpiSwigluBwd) {
-        load_gu(0, std::integral_constant<int, 0>{});
-        load_gu(0, std::integral_constant<int, 1>{});
-      }
-      if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
-      tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
-      const bool rows_live = (m0 + q * 32) < M;
-      const uint32_t lead_tempty = map_to_cta(&tempty[acc], 0);
-      // 32 rows x 128 bytes of packed output, one row per lane, to columns `col` of a matrix
-      auto emit = [&](const uint32_t (&pk)[32], const CUtensorMap& tm, int col) {
-        uint8_t* buf = buf0 + (slab & 1) * EPI_BUF;
-        ++slab;
-        if (lane == 0) tma_wait_group_read<1>();  // the store that last used this buffer has read it
-        __syncwarp();
-        uint8_t* row = buf + lane * 128;
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-          *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (OUT == 2) tma_reduce_add_2d(&tm, buf, col, c_row + m0 + q * 32);
-          else tma_store_2d(&tm, buf, col, c_row + m0 + q * 32);
-          tma_commit_group();
-        }
-      };
-      if constexpr (EPI == kEpiSwiglu) {
+      if constexpr (EPI == kEpiStore) {
+        // In a branch of its own down to the wait: code of the other epilogues in the same loop body, never run here, cost the
+        // plain bf16 store 2 - 7 % of a short product (8192 x 3072 x 64 24.3 against 22.8 us, 1536 x 6144 x 256 13.55
+        // against 13.0).
+        if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+        const bool rows_live = (m0 + q * 32) < M;
+        const uint32_t lead_tempty = map_to_cta(&tempty[acc], 0);
 #pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-          uint32_t pg[32], pu[32], pa[32];
+        for (int c = 0; c < BN / COLS; ++c) {
+          uint32_t v[64];
+          if (OUT == 0) {
+            tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+            tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+          } else {
+            tmem_ld_32x32b_x32(t_row + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+          }
+          tmem_ld_wait();
+          if (c == BN / COLS - 1) {
+            // the accumulator is in registers: hand it back to the leader's MMA warp
+            tc_fence_before();
+            remote_arrive(lead_tempty);
+          }
+          if (rows_live && (n0 + c * COLS) < N) {
+            uint8_t* buf = buf0 + (slab & 1) * EPI_BUF;
+            ++slab;
+            if (lane == 0) tma_wait_group_read<1>();  // the store that last used this buffer has read it
+            __syncwarp();
+            uint8_t* row = buf + lane * 128;
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t g[32], u[32];
-            tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, g);
-            tmem_ld_32x32b_x32(t_row + BNH + c * 64 + hf * 32, u);
-            tmem_ld_wait();
-            if (c == 1 && hf == 1) {
-              tc_fence_before();
-              remote_arrive(lead_tempty);
+            for (int j = 0; j < 8; ++j) {
+              uint4 pk;
+              if (OUT == 0) {
+                pk.x = pack_bf16x2(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
+                pk.y = pack_bf16x2(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
+                pk.z = pack_bf16x2(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
+                pk.w = pack_bf16x2(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
+              } else {
+                pk.x = v[4 * j + 0]; pk.y = v[4 * j + 1]; pk.z = v[4 * j + 2]; pk.w = v[4 * j + 3];
+              }
+              *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = pk;
             }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const uint32_t gp = pack_bf16x2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
-              const uint32_t up = pack_bf16x2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
-              const float gx = __uint_as_float(gp << 16), gy = __uint_as_float(gp & 0xffff0000u);
-              const float ux = __uint_as_float(up << 16), uy = __uint_as_float(up & 0xffff0000u);
-              pg[hf * 16 + i] = gp;
-              pu[hf * 16 + i] = up;
-              pa[hf * 16 + i] = pack_bf16x2(__fdividef(gx, 1.f + __expf(-gx)) * ux, __fdividef(gy, 1.f + __expf(-gy)) * uy);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (OUT == 2) tma_reduce_add_2d(&tmC, buf, n0 + c * COLS, m0 + q * 32);
+              else tma_store_2d(&tmC, buf, n0 + c * COLS, c_row + m0 + q * 32);
+              tma_commit_group();
             }
           }
-          if (rows_live && (n0 + c * 64) < N) {
-            emit(pa, tmAct, n0 + c * 64);
-            if (ea.store) {
+        }
+      } else {
+        uint32_t gv[2][16], uv[2][16];     // kEpiSwigluBwd: gate and up of 32 columns, two sets
+        auto load_gu = [&](int c, auto set_tag) {     // half `set` of slab c of this lane's row; zeros outside the matrix
+          constexpr int set = decltype(set_tag)::value;
+          const int gr = m0 + q * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int col = n0 + c * 64 + set * 32 + j * 16;
+            const bool in = gr < M && col < N;
+            const __nv_bfloat16* p = ea.gu + static_cast<int64_t>(gr) * 2 * N + col;
+            if (in) {
+              load_sector(p, &gv[set][8 * j]);
+              load_sector(p + N, &uv[set][8 * j]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) gv[set][8 * j + i] = uv[set][8 * j + i] = 0u;
+            }
+          }
+        };
+        if constexpr (EPI == kEpiSwigluBwd) {
+          load_gu(0, std::integral_constant<int, 0>{});
+          load_gu(0, std::integral_constant<int, 1>{});
+        }
+        if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
+        const bool rows_live = (m0 + q * 32) < M;
+        const uint32_t lead_tempty = map_to_cta(&tempty[acc], 0);
+        // 32 rows x 128 bytes of packed output, one row per lane, to columns `col` of a matrix
+        auto emit = [&](const uint32_t (&pk)[32], const CUtensorMap& tm, int col) {
+          uint8_t* buf = buf0 + (slab & 1) * EPI_BUF;
+          ++slab;
+          if (lane == 0) tma_wait_group_read<1>();  // the store that last used this buffer has read it
+          __syncwarp();
+          uint8_t* row = buf + lane * 128;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(row + ((j ^ (lane & 7)) << 4)) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            tma_store_2d(&tm, buf, col, m0 + q * 32);
+            tma_commit_group();
+          }
+        };
+        if constexpr (EPI == kEpiSwiglu) {
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) {
+            uint32_t pg[32], pu[32], pa[32];
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+              uint32_t g[32], u[32];
+              tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, g);
+              tmem_ld_32x32b_x32(t_row + BNH + c * 64 + hf * 32, u);
+              tmem_ld_wait();
+              if (c == 1 && hf == 1) {
+                tc_fence_before();
+                remote_arrive(lead_tempty);
+              }
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint32_t gp = pack_bf16x2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1]));
+                const uint32_t up = pack_bf16x2(__uint_as_float(u[2 * i]), __uint_as_float(u[2 * i + 1]));
+                const float gx = __uint_as_float(gp << 16), gy = __uint_as_float(gp & 0xffff0000u);
+                const float ux = __uint_as_float(up << 16), uy = __uint_as_float(up & 0xffff0000u);
+                pg[hf * 16 + i] = gp;
+                pu[hf * 16 + i] = up;
+                pa[hf * 16 + i] = pack_bf16x2(__fdividef(gx, 1.f + __expf(-gx)) * ux, __fdividef(gy, 1.f + __expf(-gy)) * uy);
+              }
+            }
+            if (rows_live && (n0 + c * 64) < N) {
+              emit(pa, tmAct, n0 + c * 64);
+              if (ea.store) {
+                emit(pg, tmC, n0 + c * 64);
+                emit(pu, tmUp, n0 + c * 64);
+              }
+            }
+          }
+        } else if constexpr (EPI == kEpiSwigluBwd) {
+#pragma unroll 1
+          for (int c = 0; c < BN / 64; ++c) {
+            uint32_t pg[32], pu[32];
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+              uint32_t d[32];
+              tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, d);
+              tmem_ld_wait();
+              if (c == BN / 64 - 1 && hf == 1) {
+                tc_fence_before();
+                remote_arrive(lead_tempty);
+              }
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const uint32_t gp = gv[hf][i], up = uv[hf][i];
+                const float gx = __uint_as_float(gp << 16), gy = __uint_as_float(gp & 0xffff0000u);
+                const float ux = __uint_as_float(up << 16), uy = __uint_as_float(up & 0xffff0000u);
+                const float ex = __uint_as_float(d[2 * i]), ey = __uint_as_float(d[2 * i + 1]);
+                const float sx = __fdividef(1.f, 1.f + __expf(-gx)), sy = __fdividef(1.f, 1.f + __expf(-gy));
+                // d silu(g)/dg = s (1 + g (1 - s))
+                pg[hf * 16 + i] = pack_bf16x2(ex * ux * sx * (1.f + gx * (1.f - sx)), ey * uy * sy * (1.f + gy * (1.f - sy)));
+                pu[hf * 16 + i] = pack_bf16x2(ex * gx * sx, ey * gy * sy);
+              }
+              if (c < BN / 64 - 1) {
+                if (hf == 0) load_gu(c + 1, std::integral_constant<int, 0>{});
+                else load_gu(c + 1, std::integral_constant<int, 1>{});
+              }
+            }
+            if (rows_live && (n0 + c * 64) < N) {
               emit(pg, tmC, n0 + c * 64);
               emit(pu, tmUp, n0 + c * 64);
             }
           }
-        }
-        ++it;
-        continue;
-      }
-      if constexpr (EPI == kEpiSwigluBwd) {
+        } else {
+          // kEpiCe: running maximum and sum of this lane's row over the tile's columns
+          float ce_m = -INFINITY, ce_s = 0.f;
+          const int ce_row = m0 + q * 32 + lane;
+          int64_t ce_label = -1;
+          if (ce_row < M) ce_label = ea.labels[ce_row];
 #pragma unroll 1
-        for (int c = 0; c < BN / 64; ++c) {
-          uint32_t pg[32], pu[32];
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            uint32_t d[32];
-            tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, d);
+          for (int c = 0; c < BN / COLS; ++c) {
+            uint32_t v[64];
+            tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+            tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
             tmem_ld_wait();
-            if (c == BN / 64 - 1 && hf == 1) {
+            if (c == BN / COLS - 1) {
+              // the accumulator is in registers: hand it back to the leader's MMA warp
               tc_fence_before();
               remote_arrive(lead_tempty);
             }
+            if (rows_live && (n0 + c * COLS) < N) {
+              constexpr float kLog2e = 1.4426950408889634f;
+              const int left = N - (n0 + c * COLS);      // live columns of this slab (64 or more: all)
+              float lm = -INFINITY;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const uint32_t gp = gv[hf][i], up = uv[hf][i];
-              const float gx = __uint_as_float(gp << 16), gy = __uint_as_float(gp & 0xffff0000u);
-              const float ux = __uint_as_float(up << 16), uy = __uint_as_float(up & 0xffff0000u);
-              const float ex = __uint_as_float(d[2 * i]), ey = __uint_as_float(d[2 * i + 1]);
-              const float sx = __fdividef(1.f, 1.f + __expf(-gx)), sy = __fdividef(1.f, 1.f + __expf(-gy));
-              // d silu(g)/dg = s (1 + g (1 - s))
-              pg[hf * 16 + i] = pack_bf16x2(ex * ux * sx * (1.f + gx * (1.f - sx)), ey * uy * sy * (1.f + gy * (1.f - sy)));
-              pu[hf * 16 + i] = pack_bf16x2(ex * gx * sx, ey * gy * sy);
-            }
-            if (c < BN / 64 - 1) {
-              if (hf == 0) load_gu(c + 1, std::integral_constant<int, 0>{});
-              else load_gu(c + 1, std::integral_constant<int, 1>{});
-            }
-          }
-          if (rows_live && (n0 + c * 64) < N) {
-            emit(pg, tmC, n0 + c * 64);
-            emit(pu, tmUp, n0 + c * 64);
-          }
-        }
-        ++it;
-        continue;
-      }
-      // kEpiCe: running maximum and sum of this lane's row over the tile's columns
-      float ce_m = -INFINITY, ce_s = 0.f;
-      const int ce_row = m0 + q * 32 + lane;
-      int64_t ce_label = -1;
-      if (EPI == kEpiCe && ce_row < M) ce_label = ea.labels[ce_row];
-#pragma unroll 1
-      for (int c = 0; c < BN / COLS; ++c) {
-        uint32_t v[64];
-        if (OUT == 0) {
-          tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-          tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
-        } else {
-          tmem_ld_32x32b_x32(t_row + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-        }
-        tmem_ld_wait();
-        if (c == BN / COLS - 1) {
-          // the accumulator is in registers: hand it back to the leader's MMA warp
-          tc_fence_before();
-          remote_arrive(lead_tempty);
-        }
-        if (rows_live && (n0 + c * COLS) < N) {
-          uint32_t pk[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            pk[i] = OUT == 0 ? pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])) : v[i];
-          if (EPI != kEpiCe) emit(pk, tmC, n0 + c * COLS);
-          if constexpr (EPI == kEpiCe) {
-            constexpr float kLog2e = 1.4426950408889634f;
-            const int left = N - (n0 + c * COLS);      // live columns of this slab (64 or more: all)
-            float lm = -INFINITY;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              // from here on the rounded values; columns past the end count as -inf
-              float x = __uint_as_float(pk[i] << 16), y = __uint_as_float(pk[i] & 0xffff0000u);
-              if (left < COLS) {
-                if (2 * i >= left) x = -INFINITY;
-                if (2 * i + 1 >= left) y = -INFINITY;
+              for (int i = 0; i < 32; ++i) {
+                // from here on the rounded values; columns past the end count as -inf
+                const uint32_t xy = pack_bf16x2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]));
+                float x = __uint_as_float(xy << 16), y = __uint_as_float(xy & 0xffff0000u);
+                if (left < COLS) {
+                  if (2 * i >= left) x = -INFINITY;
+                  if (2 * i + 1 >= left) y = -INFINITY;
+                }
+                v[2 * i] = __float_as_uint(x);
+                v[2 * i + 1] = __float_as_uint(y);
+                lm = fmaxf(lm, fmaxf(x, y));
               }
-              v[2 * i] = __float_as_uint(x);
-              v[2 * i + 1] = __float_as_uint(y);
-              lm = fmaxf(lm, fmaxf(x, y));
-            }
-            if (lm > ce_m) { ce_s *= ex2_approx((ce_m - lm) * kLog2e); ce_m = lm; }
-            const float nm = ce_m == -INFINITY ? 0.f : -ce_m * kLog2e;    // only -inf so far: they add nothing
-            float s0 = 0.f, s1 = 0.f;
+              if (lm > ce_m) { ce_s *= ex2_approx((ce_m - lm) * kLog2e); ce_m = lm; }
+              const float nm = ce_m == -INFINITY ? 0.f : -ce_m * kLog2e;    // only -inf so far: they add nothing
+              float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              s0 += ex2_approx(fmaf(__uint_as_float(v[2 * i]), kLog2e, nm));
-              s1 += ex2_approx(fmaf(__uint_as_float(v[2 * i + 1]), kLog2e, nm));
-            }
-            ce_s += s0 + s1;
-            const int64_t at = ce_label - (n0 + c * COLS);
-            if (at >= 0 && at < COLS && at < left) {
-              float t = 0.f;
+              for (int i = 0; i < 32; ++i) {
+                s0 += ex2_approx(fmaf(__uint_as_float(v[2 * i]), kLog2e, nm));
+                s1 += ex2_approx(fmaf(__uint_as_float(v[2 * i + 1]), kLog2e, nm));
+              }
+              ce_s += s0 + s1;
+              const int64_t at = ce_label - (n0 + c * COLS);
+              if (at >= 0 && at < COLS && at < left) {
+                float t = 0.f;
 #pragma unroll
-              for (int i = 0; i < 64; ++i)
-                if (at == i) t = __uint_as_float(v[i]);
-              ea.target[ce_row] = t;
+                for (int i = 0; i < 64; ++i)
+                  if (at == i) t = __uint_as_float(v[i]);
+                ea.target[ce_row] = t;
+              }
             }
           }
+          if (ce_row < M) ea.stats[static_cast<int64_t>(tile / num_m) * M + ce_row] = make_float2(ce_m, ce_s);
         }
       }
-      if (EPI == kEpiCe && ce_row < M) ea.stats[static_cast<int64_t>(tile / num_m) * M + ce_row] = make_float2(ce_m, ce_s);
       ++it;
     }
     if (lane == 0) tma_wait_group<0>();
