@@ -63,3 +63,15 @@ def test_head_products_are_split():
     assert _C.gemm_plan(600, 512, 50257, b_mn=True, may_split=True)[2] > 1
     assert _C.gemm_plan(128, 1024, 151936, b_mn=True, may_split=True)[2] > 1
     assert _C.gemm_plan(600, 512, 8192, b_mn=True, may_split=True)[2] == 1
+
+
+def test_clusters_of_a_plan_run_at_once():
+    """Clusters of 4 and 8 CTAs do not fill every SM: 33 and 15 of them are resident on 148 SMs.  A problem that the few-tile
+    kernel could take in one wave of some form is not given to it in two waves of clusters."""
+    for m in (128, 256, 512, 1024, 2048):
+        for n in (64, 128, 256, 512, 1024):
+            for k in (2048, 4096, 8192, 16384, 65536):
+                for mode in (1, 2):
+                    kind, tile, splits, _ = _C.gemm_plan(m, n, k, a_mn=True, b_mn=True, out_mode=mode)
+                    if kind == "small" and splits >= 4:
+                        assert -(-m // 128) * -(-n // tile) <= {4: 33, 8: 15}[splits], (m, n, k, mode)

@@ -632,8 +632,9 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
     for (int s = 1, lg = 0; s <= (may_split ? 8 : 1) && s <= num_kb; s *= 2, ++lg) {
       // the grid is not persistent: a second wave of CTAs would run on the SMs that are to stay free
       if (sms_reserved && t_small * s > num_sms) break;
-      // clusters of 4 and 8 leave SMs of a GPC over
-      const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 15 / 16 : num_sms * 7 / 8);
+      // clusters of 4 and 8 leave SMs of a GPC over: 33 and 15 of them run at once on 148 SMs.  (One too many is a second wave:
+      // 1024 x 128 x 8192 in sixteen clusters of 8 took 20.7 us, in sixteen of 4 13.0, adding on SM pairs 12.5.)
+      const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 132 / 148 : num_sms * 120 / 148);
       const int waves = ceil_div(t_small * s, slots);
       const float bytes = static_cast<float>(t_small) * num_kb * (A_BYTES + 128 * kTile[i]);
       const float run = std::max(waves * kPerKb[i] * ceil_div(num_kb, s),
