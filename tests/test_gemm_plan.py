@@ -75,3 +75,11 @@ def test_clusters_of_a_plan_run_at_once():
                     kind, tile, splits, _ = _C.gemm_plan(m, n, k, a_mn=True, b_mn=True, out_mode=mode)
                     if kind == "small" and splits >= 4:
                         assert -(-m // 128) * -(-n // tile) <= {4: 33, 8: 15}[splits], (m, n, k, mode)
+
+
+@pytest.mark.parametrize("M,F,K,pays", [(8192, 8192, 2048, True), (4096, 9728, 2560, True), (2048, 9728, 2560, True),
+                                        (8192, 2048, 2048, True), (8192, 3072, 1024, False), (2048, 3072, 2048, False),
+                                        (512, 9728, 2560, False), (1408, 9728, 2560, False), (256, 9728, 4096, False)])
+def test_swiglu_gradient_is_fused_where_it_pays(M, F, K, pays):
+    """Long products with enough tiles that the last wave's epilogue, which nothing hides, does not decide."""
+    assert _C.gemm_swiglu_bwd_pays(M, F, K, 148) == pays

@@ -364,7 +364,7 @@ def test_linear_swiglu_epilogue(M, F, K):
     assert torch.equal(act, k.swiglu(gu))
 
 
-@pytest.mark.parametrize("M,F,K", [(4096, 1536, 2048), (2000, 3088, 2056), (1100, 6160, 2112)])
+@pytest.mark.parametrize("M,F,K", [(4096, 3856, 2048), (2000, 7696, 2056), (1100, 12304, 2112)])
 def test_swiglu_dgrad_epilogue(M, F, K):
     """d(gate) and d(up) in the epilogue of d(act) = dy W against fp64 on the same operands; ragged rows, last column tiles of
     16 columns, a ragged last k block.  Only the results are rounded: 2^-9 relative per element."""
@@ -391,7 +391,11 @@ def test_swiglu_dgrad_epilogue(M, F, K):
     want = torch.cat([d * u * s * (1 + g * (1 - s)), d * g * s], 1)
     err = ((got.double() - want).norm() / want.norm()).item()
     assert err < 2e-3 and err <= ((two.double() - want).norm() / want.norm()).item()
-    # few tiles: the product and a pass of its own
+    # few tiles, and few waves of them: the product and a pass of its own
+    before = ops.launches()
+    assert torch.equal(k.swiglu_dgrad(dy[:1024], w[:, :3072], gu[:1024, :6144].contiguous()),
+                       k.swiglu_bwd(k.linear_dgrad(dy[:1024], w[:, :3072]), gu[:1024, :6144].contiguous()))
+    assert ops.launches() - before == 4
     assert torch.equal(k.swiglu_dgrad(dy[:64], w, gu[:64]), k.swiglu_bwd(k.linear_dgrad(dy[:64], w), gu[:64]))
 
 

@@ -47,6 +47,7 @@ int gemm2_swiglu(const void* A, const void* W, void* gu, void* act, int M, int F
                  int num_sms, cudaStream_t stream);
 // dgu [M, 2F] = d(gate) | d(up) of the SwiGLU unit from d(act) = dy [M, K] W, W [K, F], and the stored gu [M, 2F]; F a multiple
 // of 16, gu 32-byte aligned.  d(act) itself is not stored.
+bool gemm2_swiglu_bwd_pays(int M, int F, int K, int num_sms);     // against the product and an element-wise pass
 int gemm2_swiglu_bwd(const void* dy, const void* W, const void* gu, void* dgu, int M, int F, int K, int64_t lda, int64_t ldw,
                      int* err, int num_sms, cudaStream_t stream);
 // Row statistics of a softmax over A B^T, which is not stored: per row and 256 columns of the product, rounded to bf16, its

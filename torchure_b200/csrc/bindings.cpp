@@ -98,8 +98,7 @@ bool gemm_swiglu_bwd(const torch::Tensor& dy, const torch::Tensor& w, const torc
   const int64_t M = dy.size(0), K = dy.size(1), F = w.size(1);
   TORCH_CHECK(w.size(0) == K && gu.size(0) == M && gu.size(1) == 2 * F && dgu.size(0) == M && dgu.size(1) == 2 * F,
               "gemm_swiglu_bwd: shapes");
-  // below 2048 the epilogue takes longer than the products it should hide behind (figures at the kernel)
-  if (K < 2048 || F % 16 != 0 || M == 0 || (reinterpret_cast<uintptr_t>(gu.data_ptr()) & 31) != 0 ||
+  if (!tb::gemm2_swiglu_bwd_pays((int)M, (int)F, (int)K, num_sms()) || F % 16 != 0 || M == 0 || (reinterpret_cast<uintptr_t>(gu.data_ptr()) & 31) != 0 ||
       tb::gemm_plan((int)M, (int)F, (int)K, false, true, 0, num_sms(), g_sm_reserve > 0, false, 0, 0).kind != tb::GemmPlan::kPair)
     return false;
   c10::cuda::CUDAGuard guard(dy.device());
@@ -364,6 +363,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, "bf16 tcgen05 GEMM: out = A * B^T (operand majors selectable)", pybind11::arg("a"),
         pybind11::arg("b"), pybind11::arg("out"), pybind11::arg("a_mn"), pybind11::arg("b_mn"), pybind11::arg("out_mode"),
         pybind11::arg("splits") = 0, pybind11::arg("tile_n") = 0, pybind11::arg("may_split") = false);
+  m.def("gemm_swiglu_bwd_pays", &tb::gemm2_swiglu_bwd_pays, "whether the SwiGLU gradient belongs in its product's epilogue");
   m.def("gemm_plan", [](int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int num_sms, bool sms_reserved,
                         bool may_split) {
     const tb::GemmPlan p = tb::gemm_plan(M, N, K, a_mn, b_mn, out_mode, num_sms, sms_reserved, may_split, 0, 0);

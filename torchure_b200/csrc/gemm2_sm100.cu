@@ -536,9 +536,8 @@ gemm2_swiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 }
 
 // Bound by its epilogue when K is short: 256 columns of two special-function operations, two loads and two stores per row
-// against K / 64 x 512 cycles of products.  Measured on B200, M x F x K, product + pass over it before, fused: 8192 x 8192 x
-// 2048 283, 253 us; 4096 x 9728 x 2560 227, 218; 8192 x 3072 x 1024 83.0, 85.8; 2048 x 3072 x 1024 30.3, 31.3; 8192 x 1024 x
-// 256 27.6, 25.2.  Hence the rule: K of 2048 and more.
+// against K / 64 x 512 cycles of products; and the last wave's epilogue has no products to hide behind.  It spares the passes
+// over d(act).  gemm2_swiglu_bwd_pays has the rule.
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_swiglu_bwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         const __grid_constant__ CUtensorMap tmGate, const __grid_constant__ CUtensorMap tmUp,
@@ -655,6 +654,20 @@ int gemm2_swiglu(const void* A, const void* W, void* gu, void* act, int M, int F
   ea.store = gu != nullptr ? 1 : 0;
   const int units = ((M + 2 * BM - 1) / (2 * BM)) * ((F + BNH - 1) / BNH);
   return launch_pairs(gemm2_swiglu_kernel, units, num_sms, stream, ta, tw, tg, tu, tact, ea, M, F, K, err);
+}
+
+// K of 2048 and more, and tiles for 3.25 waves of SM pairs and more.  Measured on B200, M x F x K (waves): product + pass over it,
+// fused, in us.
+//   K too short     8192 x 3072 x 512 (5.2) 74.9, 79.8; 8192 x 3072 x 1024 92.5, 93.6; 4096 x 9728 x 512 (8.2) 110.5, 114.1
+//   too few waves   2048 x 3072 x 2048 (1.3) 41.3, 45.4; 512 x 9728 x 2560 (1.03) 44.9, 49.3; 1024 x 9728 x 2048 (2.05) 57.9, 60.4;
+//                   1408 x 9728 x 2560 (3.08) 85.2, 87.0; 1024 x 14336 x 2048 (3.03) 77.3, 77.5
+//   taken           8192 x 2048 x 2048 (3.5) 80.4, 73.8; 6144 x 3072 x 2560 (3.9) 95.5, 92.0; 2048 x 9728 x 2560 (4.1) 106.3,
+//                   104.8; 4096 x 9728 x 2560 (8.2) 194, 185; 8192 x 8192 x 2048 (13.8) 273, 251, x 5120 657, 622
+// A few that are left out would gain by it: 8192 x 8192 x 1024 (13.8) 194, 178; 8192 x 1024 x 256 (1.7) 29.5, 28.8.
+bool gemm2_swiglu_bwd_pays(int M, int F, int K, int num_sms) {
+  const int64_t tiles = static_cast<int64_t>((M + 2 * BM - 1) / (2 * BM)) * ((F + BN - 1) / BN);
+  const int pairs = g_pair_capacity > 0 && g_pair_capacity < num_sms / 2 ? g_pair_capacity : num_sms / 2;
+  return K >= 2048 && tiles * 4 >= static_cast<int64_t>(pairs) * 13;
 }
 
 int gemm2_swiglu_bwd(const void* dy, const void* W, const void* gu, void* dgu, int M, int F, int K, int64_t lda, int64_t ldw,
