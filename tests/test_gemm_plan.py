@@ -10,6 +10,7 @@ from torchure_b200 import ops
 _C = ops.ext()
 pytestmark = pytest.mark.skipif(_C is None, reason="the CUDA extension is not built")
 
+ceil_div = lambda a, b: -(-a // b)
 SIZES = [(600, 512, 50257), (130, 64, 151936), (300, 520, 2500), (129, 128, 16384), (256, 256, 4096), (1, 8, 520),
          (128, 1024, 151936), (8192, 1024, 3072)]
 
@@ -83,3 +84,22 @@ def test_clusters_of_a_plan_run_at_once():
 def test_swiglu_gradient_is_fused_where_it_pays(M, F, K, pays):
     """Long products with enough tiles that the last wave's epilogue, which nothing hides, does not decide."""
     assert _C.gemm_swiglu_bwd_pays(M, F, K, 148) == pays
+
+
+def test_fp32_products_keep_their_slices_short():
+    """The tensor core's fp32 sums lose precision with every term: whichever kernel an fp32 product runs on, its slices of K
+    are no longer than those of the split by reduce-add, which gives SM pairs (SMs, up to 128 rows) the least wave time."""
+    for m in (64, 128, 256, 512, 1024, 3072, 8192):
+        for n in (64, 256, 512, 1024, 2560, 9728):
+            for k in (128, 600, 1024, 2048, 4224, 8192, 16384, 50257):
+                tile_m, workers = (256, 74) if m > 128 else (128, 148)
+                tiles, blocks = ceil_div(m, tile_m) * ceil_div(n, 256), ceil_div(k, 64)
+                longest = blocks
+                if blocks >= 32 and tiles < 2 * workers:
+                    # fp32 arithmetic of the plan: ties within 1e-6 go to fewer slices
+                    cost = lambda s: ceil_div(tiles * s, workers) / s + 0.02 * (s - 1)
+                    best = min(range(1, min(8, blocks // 8) + 1), key=lambda s: (round(cost(s), 5), s))
+                    longest = ceil_div(blocks, best)
+                for mode in (1, 2):
+                    _, _, splits, _ = _C.gemm_plan(m, n, k, a_mn=True, b_mn=True, out_mode=mode)
+                    assert ceil_div(blocks, splits) <= longest, (m, n, k, mode)

@@ -149,6 +149,27 @@ def test_head_gradient_in_slices_is_no_further_off(M, N, K):
     assert errs[1] <= errs[0] * 1.001 and errs[0] < 4e-3, errs
 
 
+@pytest.mark.parametrize("M,N,K", [(1024, 1024, 2048), (512, 512, 8192), (256, 512, 4096), (128, 128, 4096), (2048, 512, 2048)])
+def test_fp32_products_are_as_close_as_the_split_by_reduce_add(M, N, K):
+    """Weight gradients with few tiles against 64 bits: whichever kernel the plan takes, no further off than the split that
+    adds K slices into C (1 % for the order of the slices); about 1.03e-9 per term of the longest slice."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(0)
+    a, b = torch.randn(K, M, device="cuda").bfloat16(), torch.randn(K, N, device="cuda").bfloat16()
+    want = a.double().t() @ b.double()
+    err = lambda o: ((o.double() - want).norm() / want.norm()).item()
+    got = err(kernels.linear_wgrad(a, b, out_dtype=torch.float32))
+    tiles, workers = -(-M // 256) * -(-N // 256), 74
+    if M <= 128:
+        tiles, workers = -(-N // 256), 148
+    splits = min(range(1, 9), key=lambda s: (round(-(-tiles * s // workers) / s + 0.02 * (s - 1), 5), s))
+    out = torch.empty(M, N, device="cuda")
+    ops.ext().gemm(a, b, out, True, True, 1, splits)
+    assert got <= 1.01 * err(out) and got < 1.3e-9 * K / splits + 2e-7, (got, err(out))
+
+
 def test_gemm_with_reserved_sms():
     """Products with most SMs reserved and after the reservation was lifted, in a fresh process whose first launch has it:
     right in both states, and the pairs that the device holds are counted without it."""

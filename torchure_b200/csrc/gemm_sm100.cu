@@ -614,11 +614,15 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
   // 2 ffn_dim (16384 and more) of a wide block's input gradient; what splitting them would gain is little (128 x 1024 x 3072:
   // 10.4 us in one slice, 8.9 in four; 128 x 1024 x 2048: no difference).
   may_split = out_mode != 0 || (may_split && num_kb >= 256);
+  // The tensor core's fp32 accumulator loses about 1e-9 of the sum per term (relative error of an fp32 product of random
+  // operands: 600 terms in one slice 5.6e-7, 1024 1.0e-6, 2048 2.1e-6), sums of slices round to nearest: an fp32 output is
+  // not summed in longer slices than the split by reduce-add has.
+  const int longest = out_mode != 0 ? ceil_div(num_kb, p.splits) : num_kb;
   // K slices through a workspace: only where the tiles leave most of the chip idle for a long K.  The slices are fp32 products,
   // which no kernel has for A [K, M] with B [N, K].
   if (may_split && pair && !(a_mn && !b_mn) && out_mode != 2 && tiles * 2 <= workers && num_kb >= 64) {
     const int s = static_cast<int>(workers / tiles) < num_kb / 16 ? static_cast<int>(workers / tiles) : num_kb / 16;
-    if (s > 1) {
+    if (s > 1 && ceil_div(num_kb, s) <= longest) {
       const float run = std::max(0.30f * ceil_div(num_kb, s), cold ? tiles * num_kb * 65536.f / 8.5e6f : 0.f);
       const float t = 6.9f + run + 4.f + 2e-6f * s * static_cast<float>(M) * N;
       if (t < best) { best = t; use_slices(s); }
@@ -632,6 +636,7 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
     for (int s = 1, lg = 0; s <= (may_split ? 8 : 1) && s <= num_kb; s *= 2, ++lg) {
       // the grid is not persistent: a second wave of CTAs would run on the SMs that are to stay free
       if (sms_reserved && t_small * s > num_sms) break;
+      if (ceil_div(num_kb, s) > longest) continue;
       // clusters of 4 and 8 leave SMs of a GPC over: 33 and 15 of them run at once on 148 SMs.  (One too many is a second wave:
       // 1024 x 128 x 8192 in sixteen clusters of 8 took 20.7 us, in sixteen of 4 13.0, adding on SM pairs 12.5.)
       const int slots = s <= 2 ? num_sms : (s == 4 ? num_sms * 132 / 148 : num_sms * 120 / 148);
