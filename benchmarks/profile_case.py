@@ -2,7 +2,7 @@
 
     python -m benchmarks.profile_case <case> [--iters N]
 
-Cases: gemm_fwd, gemm_dgrad, gemm_wgrad, attn_fwd, attn_bwd (single pass), attn_bwd_split, attn_prep, rmsnorm, rmsnorm_bwd, qknorm_rope,
+Cases: gemm_fwd, gemm_dgrad, gemm_wgrad, gemm_small, gemm_swiglu, gemm_swiglu_bwd, gemm_ce, attn_fwd, attn_bwd (single pass), attn_bwd_split, attn_prep, rmsnorm, rmsnorm_bwd, qknorm_rope,
 qknorm_rope_bwd, qknorm_rope_bwd_acc, swiglu, swiglu_bwd, ce, adamw.  Each case builds inputs
 larger than the 126 MB L2 but well under a few GB, launches the kernel `iters` times (default 4) and prints the
 CUDA-event time of the last launch with the achieved FLOP/s or bytes/s, so the same command serves a plain timing run
@@ -45,6 +45,28 @@ def main(argv=None) -> None:
         out = torch.empty(2 * F_, D, dtype=torch.float32, device=dev)
         fn = lambda: K.gemm(a, b, a_mn=True, b_mn=True, out=out)
         flops = 2.0 * M * 2 * F_ * D
+    elif args.case == "gemm_small":    # dH of 128 rows over the vocabulary: few tiles, long K, slices of it in clusters
+        C, V = 128, 151936
+        a, b = torch.randn(C, V, device=dev).bfloat16(), torch.randn(V, D, device=dev).bfloat16()
+        out = torch.empty(C, D, dtype=torch.bfloat16, device=dev)
+        fn = lambda: K.gemm(a, b, b_mn=True, out=out, may_split=True)
+        flops = 2.0 * C * V * D
+    elif args.case == "gemm_swiglu":   # gate|up projection with the activation in its epilogue
+        a, b = torch.randn(M, D, device=dev).bfloat16(), torch.randn(2 * F_, D, device=dev).bfloat16()
+        fn = lambda: K.linear_swiglu(a, b)
+        flops = 2.0 * M * 2 * F_ * D
+    elif args.case == "gemm_swiglu_bwd":   # d(act) = dy W with d(gate) | d(up) in its epilogue, 1B sizes
+        W, F2 = 2048, 8192
+        dy, w = torch.randn(M, W, device=dev).bfloat16(), torch.randn(W, F2, device=dev).bfloat16()
+        gu = torch.randn(M, 2 * F2, device=dev).bfloat16()
+        fn = lambda: K.swiglu_dgrad(dy, w, gu)
+        flops = 2.0 * M * F2 * W
+    elif args.case == "gemm_ce":       # row statistics of the softmax over a head product that is not stored
+        C, V = 4096, 151936
+        a, b = torch.randn(C, D, device=dev).bfloat16(), (torch.randn(V, D, device=dev) * 0.02).bfloat16()
+        labels, target = torch.randint(0, V, (C,), device=dev), torch.empty(C, device=dev)
+        fn = lambda: K.gemm_ce(a, b, labels, target)
+        flops = 2.0 * C * V * D
     elif args.case in ("attn_fwd", "attn_bwd", "attn_bwd_split"):
         qk = torch.randn(M, (Hq + Hkv) * hd, device=dev).bfloat16()
         qkv = torch.randn(M, (Hq + 2 * Hkv) * hd, device=dev).bfloat16()

@@ -62,7 +62,8 @@ class _LayerShadow:
                            wo=g.o_proj.weight, qn=g.q_norm.weight if g.qk_norm else None,
                            kn=g.k_norm.weight if g.qk_norm else None, w2=block.norm2.weight,
                            wg=f.gate_proj.weight, wu=f.up_proj.weight, wd=f.down_proj.weight, table=None)
-        self._seen = None
+        self._no_gain = {"weight": None}       # stands for the table of a missing QK-norm
+        self._look_up(block)
         self.pairs = [
             (g.q_proj.weight, self.wqkv[:nq]), (g.k_proj.weight, self.wqkv[nq:nq + nkv]),
             (g.v_proj.weight, self.wqkv[nq + nkv:]), (g.o_proj.weight, self.wo),
@@ -70,23 +71,27 @@ class _LayerShadow:
         ]
 
 
+    def _look_up(self, block) -> None:
+        g, f = block.gqa, block.ffn
+        qk = g.qk_norm
+        modules = (block.norm1, g.q_proj, g.k_proj, g.v_proj, g.o_proj, g.q_norm if qk else None,
+                   g.k_norm if qk else None, block.norm2, f.gate_proj, f.up_proj, f.down_proj)
+        tables = [self._no_gain if m is None else m._parameters for m in modules]
+        self._seen = (dict(block._modules), g, dict(g._modules), f, dict(f._modules), qk, modules, tables)
+
     def inputs(self, block, dummy):
         """The block's parameters in the order of ``_BlockFn``, as its modules hold them now; without QK-norm its gains are
         the engine's dummy.  Read from the modules' tables: attribute look-ups through ``Module.__getattr__`` cost a short
         forward pass 7 us per block, so the modules are looked up again only when one was exchanged."""
-        seen = self._seen
-        if (seen is None or block._modules != seen[0] or seen[1]._modules != seen[2] or seen[3]._modules != seen[4]
-                or seen[1].qk_norm != seen[5]):
-            g, f = block.gqa, block.ffn
-            qk = g.qk_norm
-            modules = (block.norm1, g.q_proj, g.k_proj, g.v_proj, g.o_proj, g.q_norm if qk else None,
-                       g.k_norm if qk else None, block.norm2, f.gate_proj, f.up_proj, f.down_proj)
-            seen = self._seen = (dict(block._modules), g, dict(g._modules), f, dict(f._modules), qk, modules)
-        out = []
-        for m in seen[6]:
-            w = dummy if m is None else m._parameters.get("weight")
-            out.append(m.weight if w is None else w)
-        return out
+        subs, g, g_subs, f, f_subs, qk, modules, tables = self._seen
+        if block._modules != subs or g._modules != g_subs or f._modules != f_subs or g.qk_norm != qk:
+            self._look_up(block)
+            return self.inputs(block, dummy)
+        self._no_gain["weight"] = dummy
+        try:
+            return [t["weight"] for t in tables]
+        except KeyError:        # a parametrised weight is an attribute only
+            return [dummy if m is None else m.weight for m in modules]
 
 
 class Sm100Engine:

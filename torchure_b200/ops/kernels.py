@@ -61,7 +61,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         out = new_output("gemm", M, N, dtype=out_dtype, device=a.device)
     mode = 0 if out.dtype == BF16 else (2 if accumulate else 1)
     assert not (accumulate and out.dtype == BF16), "accumulation needs an fp32 output"
-    _C().gemm(a, b, out, a_mn, b_mn, mode, splits, may_split=may_split)
+    _C().gemm(a, b, out, a_mn, b_mn, mode, splits, 0, may_split)
     ops.count_launch()
     return out
 
