@@ -170,6 +170,28 @@ def test_fp32_products_are_as_close_as_the_split_by_reduce_add(M, N, K):
     assert got <= 1.01 * err(out) and got < 1.3e-9 * K / splits + 2e-7, (got, err(out))
 
 
+@pytest.mark.parametrize("M,D", [(130, 1032), (600, 1280), (1024, 2560), (3000, 2048), (2000, 4096)])
+def test_rmsnorm_bwd_of_wide_rows_is_as_close_as_unstaged(M, D):
+    """Rows shared by teams of warps against 64 bits, beside the kernels with one warp per row: dx no further off, the gain
+    gradient neither, up to the order in which the CTAs' sums are added (mean of eight inputs, 8 %)."""
+    from torchure_b200 import ops
+
+    errs = torch.zeros(2, 2, dtype=torch.float64)
+    for seed in range(8):
+        g = torch.Generator("cuda").manual_seed(seed)
+        rand = lambda *s: torch.randn(*s, device="cuda", generator=g)
+        x, dh, dx_in, w = rand(M, D), rand(M, D).bfloat16(), rand(M, D), rand(D).abs() + 0.5
+        rstd = torch.rsqrt(x.double().pow(2).mean(-1) + 1e-6).float()
+        xh, gw = x.double() * rstd.double()[:, None], dh.double() * w.double()
+        want = (dx_in.double() + rstd.double()[:, None] * (gw - xh * (gw * xh).mean(-1, keepdim=True)), (dh.double() * xh).sum(0))
+        for variant in (0, 1):
+            dx, dxb, dw = torch.empty_like(x), torch.empty_like(dh), torch.zeros(D, device="cuda")
+            ops.ext().rmsnorm_bwd(dh, x, w, rstd, dx_in, dx, dxb, dw, variant)
+            for i, (got, ref) in enumerate(zip((dx, dw), want)):
+                errs[variant, i] += (got.double() - ref).norm().cpu() / ref.norm().cpu()
+    assert errs[0, 0] <= errs[1, 0] and errs[0, 1] <= 1.08 * errs[1, 1], errs
+
+
 def test_gemm_with_reserved_sms():
     """Products with most SMs reserved and after the reservation was lifted, in a fresh process whose first launch has it:
     right in both states, and the pairs that the device holds are counted without it."""

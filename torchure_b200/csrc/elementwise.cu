@@ -285,7 +285,8 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dh, const float* __res
 // row before, so its buffer can take the next copy.
 // Bound by memory: 16 bytes per element with residual input and bf16 copy.  Measured on B200: 8192 x 1024 21 us (6.4
 // TB/s in a step); with one warp per row and both passes reading memory 8192 x 2048 took 96 us, now 45 (5.9 TB/s), 4096 x
-// 2560 62, now 29, 4096 x 4096 227, now 47, 512 x 2048 22, now 6.4.
+// 2560 62, now 29, 4096 x 4096 227, now 47.  Few rows are bound by the chain of one CTA's sixteen (see the launch): 600 x
+// 2048 22, now 12.5 (8.4 spread over every SM), 600 x 4096 62, now 21 (10).
 // ---------------------------------------------------------------------------------------------
 constexpr int RNB_MAX_WARPS = 8;
 constexpr int RNB_MAX_STAGES = 4;
@@ -386,11 +387,20 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
         const uint2 dv = reinterpret_cast<const uint2*>(st + off_dh)[i];
         const float2 a = bf2_to_f2(dv.x), b = bf2_to_f2(dv.y);
         const float2 xh0 = mul2(make_float2(xv.x, xv.y), r2), xh1 = mul2(make_float2(xv.z, xv.w), r2);
-        float2 o0 = mul2(fma2(xh0, nd2, mul2(a, make_float2(wv[j].x, wv[j].y))), r2);
-        float2 o1 = mul2(fma2(xh1, nd2, mul2(b, make_float2(wv[j].z, wv[j].w))), r2);
-        if (dx_in) {
+        const float2 t0 = fma2(xh0, nd2, mul2(a, make_float2(wv[j].x, wv[j].y)));
+        const float2 t1 = fma2(xh1, nd2, mul2(b, make_float2(wv[j].z, wv[j].w)));
+        float2 o0, o1;
+        if (T > 1 && dx_in) {      // one rounding, as the unstaged kernel has it (against 64 bits 3.8e-8, two 4.2e-8)
           const float4 p = reinterpret_cast<const float4*>(st + off_in)[i];
-          o0.x += p.x; o0.y += p.y; o1.x += p.z; o1.y += p.w;
+          o0 = fma2(t0, r2, make_float2(p.x, p.y));
+          o1 = fma2(t1, r2, make_float2(p.z, p.w));
+        } else {
+          o0 = mul2(t0, r2);
+          o1 = mul2(t1, r2);
+          if (dx_in) {
+            const float4 p = reinterpret_cast<const float4*>(st + off_in)[i];
+            o0.x += p.x; o0.y += p.y; o1.x += p.z; o1.y += p.w;
+          }
         }
         reinterpret_cast<float4*>(dx + off)[i] = make_float4(o0.x, o0.y, o1.x, o1.y);
         if (dx_bf16) reinterpret_cast<uint2*>(dx_bf16 + off)[i] = make_uint2(f2_to_bf2(o0.x, o0.y), f2_to_bf2(o1.x, o1.y));
@@ -1189,7 +1199,10 @@ void rmsnorm_bwd(const __nv_bfloat16* dh, const float* x, const float* w, const 
     const int smem = teams * stages * stage_bytes;
     auto kern = T == 1 ? rmsnorm_bwd_staged_kernel<1> : (T == 2 ? rmsnorm_bwd_staged_kernel<2> : rmsnorm_bwd_staged_kernel<4>);
     if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) {
-      const int grid = std::max(1, std::min((M + teams - 1) / teams, num_sms));
+      // T > 1: sixteen rows per CTA and more, as the unstaged kernel has them: the CTAs' partial gains are added one by one,
+      // and every addition rounds (600 x 1280 against 64 bits 1.4e-7 in 38 CTAs, 2.2e-7 in 148)
+      const int most = T == 1 ? num_sms : std::min(num_sms, (M + 15) / 16);
+      const int grid = std::max(1, std::min((M + teams - 1) / teams, most));
       launch_pdl(kern, dim3(grid), dim3(teams * T * 32), smem, stream, dh, x, w, rstd, dx_in, dx, dx_bf16, dw, M, D,
                  stage_bytes, stages, err);
       return;
