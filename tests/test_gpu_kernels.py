@@ -569,6 +569,26 @@ def test_linear_ce_without_gradients_chunk_by_chunk(monkeypatch, rows, vocab, ch
         debug.enable(False)
 
 
+@pytest.mark.parametrize("offset", [0.0, 60.0, 400.0])
+def test_loss_without_logits_is_as_close_as_with(offset):
+    """Row losses from the product's epilogue and from stored logits against 64 bits on the same rounded logits, whose level
+    lies around `offset`: the mean error of 512 rows is no larger (5 %), mostly the rounding of maximum + log."""
+    from torchure_b200.ops import kernels as K
+
+    torch.manual_seed(0)
+    C, V, D = 512, 40000, 128
+    h, w = torch.randn(C, D, device="cuda").bfloat16(), torch.randn(V, D, device="cuda").bfloat16()
+    h[:, 0], w[:, 0] = 1, offset
+    y = torch.randint(0, V, (C,), device="cuda")
+    logits = K.gemm(h, w)
+    want = torch.nn.functional.cross_entropy(logits.double(), y, reduction="none")
+    stored, fused, target = (torch.empty(C, device="cuda") for _ in range(3))
+    K.ce_loss(logits, y, stored, -100)
+    K.ce_loss_tiles(K.gemm_ce(h, w, y, target), target, y, fused, V, -100)
+    err = lambda t: (t.double() - want).abs().mean().item()
+    assert err(fused) <= 1.05 * err(stored), (err(fused), err(stored))
+
+
 def test_gemm_ce_decides_before_it_allocates():
     from torchure_b200.ops import kernels as K
 

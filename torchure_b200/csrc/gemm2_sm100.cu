@@ -472,14 +472,17 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
                 lm = fmaxf(lm, fmaxf(x, y));
               }
               if (lm > ce_m) { ce_s *= ex2_approx((ce_m - lm) * kLog2e); ce_m = lm; }
-              const float nm = ce_m == -INFINITY ? 0.f : -ce_m * kLog2e;    // only -inf so far: they add nothing
+              // 2^(x log2 e + nm) per column, nm = -max log2 e rounded; what the rounding took, the same for every column, is given
+              // back to their sum (0: only -inf so far, they add nothing)
+              const float nm = ce_m == -INFINITY ? 0.f : -ce_m * kLog2e;
+              const float left_out = ce_m == -INFINITY ? 0.f : fmaf(-ce_m, kLog2e, -nm);
               float s0 = 0.f, s1 = 0.f;
 #pragma unroll
               for (int i = 0; i < 32; ++i) {
                 s0 += ex2_approx(fmaf(__uint_as_float(v[2 * i]), kLog2e, nm));
                 s1 += ex2_approx(fmaf(__uint_as_float(v[2 * i + 1]), kLog2e, nm));
               }
-              ce_s += s0 + s1;
+              ce_s += fmaf(s0 + s1, left_out * 0.6931471805599453f, s0 + s1);
               const int64_t at = ce_label - (n0 + c * COLS);
               if (at >= 0 && at < COLS && at < left) {
                 float t = 0.f;
