@@ -4,9 +4,9 @@
 // What bounds such a problem is the serial chain of k-blocks of one tile, not the tensor cores: a 600 x 512 x 50257
 // product has six 256 x 256 tiles, so the pair kernel ran 786 k-blocks one after the other on 12 SMs, and the 128-row
 // products of a short prompt kept 4 to 16 SMs busy.  Narrow tiles and K slices put the same work on up to 148 SMs.
-// Measured on B200 (cold weights, pair or single-CTA kernel before -> this kernel): 128 x 1024 x 1024 9.1 -> 5.6 us,
-// 128 x 1024 x 3072 21.2 -> 9.2 (4 slices), 1024 x 512 x 512 9.1 -> 4.8, 512 x 512 x 8192 42.8 -> 13.1 (4 slices),
-// 2048 x 1024 x 4096 25.4 -> 16.2, 128 x 1024 x 151936 792 -> 75 (8 slices).
+// Measured on B200 (cold weights, pair or single-CTA kernel before -> this kernel), bf16: 128 x 1024 x 1024 9.1 -> 5.6 us,
+// 128 x 1024 x 3072 21.2 -> 10.4, 1024 x 512 x 512 9.1 -> 4.8, 2048 x 1024 x 4096 25.4 -> 16.2; in slices of K, which gemm_plan
+// takes for a head's gradient, 128 x 1024 x 151936 792 -> 75 (8 slices).
 //
 //   192 threads: warp 0 TMA producer, warp 1 TMEM allocator + MMA issuer, warps 2..5 epilogue (TMEM lanes), as in
 //   gemm_sm100.cu.  S > 1: when every CTA of the cluster has finished its MMAs (its operand stages are free then), each
