@@ -151,3 +151,70 @@ def test_backward_with_shared_key_blocks(B, Sq, Skv, Hq, Hkv, causal):
     for name, got, want in zip(("dq", "dk", "dv"), grads[0], (qf.grad, kf.grad, vf.grad)):
         # probabilities, score gradients and the output behind the row statistics are rounded to bf16, as in the tests above
         assert relerr(got, want.transpose(1, 2)) < 1.5e-2, (name, relerr(got, want.transpose(1, 2)))
+
+
+@pytest.mark.parametrize("B,Sq,Skv,Hq,Hkv,causal", [(8, 256, 256, 16, 8, True), (8, 640, 640, 16, 8, True), (4, 128, 1024, 16, 8, False),
+                                                    (2, 512, 640, 32, 8, False), (1, 2048, 2048, 16, 8, True)])
+def test_backward_on_cta_pairs(B, Sq, Skv, Hq, Hkv, causal):
+    """Two key blocks per CTA pair: an even and an odd number of them (the last one's partner is not there), two iterations and
+    many.  Gradients against fp64; dK and dV are summed in a fixed order, so a second run gives the same bits."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import kernels
+    from torchure_b200.ops.attention import flash_attention
+
+    assert ops.ext().attn_bwd_on_pairs(B, Sq, Skv, Hq, Hkv, causal)
+    torch.manual_seed(6)
+    q = torch.randn(B, Sq, Hq, 128, device="cuda").bfloat16().requires_grad_()
+    k, v = (torch.randn(B, Skv, Hkv, 128, device="cuda").bfloat16().requires_grad_() for _ in range(2))
+    g = torch.randn_like(q)
+    grads = [torch.autograd.grad(flash_attention(q, k, v, causal=causal), (q, k, v), g) for _ in range(2)]
+    kernels.check_error()
+    assert torch.equal(grads[0][1], grads[1][1]) and torch.equal(grads[0][2], grads[1][2])
+    qf, kf, vf = (t.detach().double().transpose(1, 2).requires_grad_() for t in (q, k, v))
+    s = qf @ kf.repeat_interleave(Hq // Hkv, 1).transpose(-1, -2) / 128 ** 0.5
+    if causal:
+        s = s.masked_fill(~torch.ones(Sq, Skv, dtype=torch.bool, device="cuda").tril(), float("-inf"))
+    (torch.softmax(s, -1) @ vf.repeat_interleave(Hq // Hkv, 1)).backward(g.double().transpose(1, 2))
+    for name, got, want in zip(("dq", "dk", "dv"), grads[0], (qf.grad, kf.grad, vf.grad)):
+        assert relerr(got, want.transpose(1, 2)) < 1.5e-2, (name, relerr(got, want.transpose(1, 2)))
+
+
+@pytest.mark.parametrize("Sq,Skv,causal", [(640, 640, True), (256, 640, False)])
+def test_backward_on_cta_pairs_inside_larger_tensors(Sq, Skv, causal):
+    """Queries and keys at row offsets of larger tensors, statistics and dQ accumulator of a longer sequence, as a step of ring
+    attention passes them: the same as on tensors of their own.  Everything outside holds NaN, which must not get in, least of
+    all through the partner that the odd last key block does not have."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import kernels
+
+    E = ops.ext()
+    B, Hq, Hkv, pad = 2, 16, 8, 128
+    assert E.attn_bwd_on_pairs(B, Sq, Skv, Hq, Hkv, causal)
+    torch.manual_seed(7)
+    q, g, o = (torch.randn(B, Sq, Hq * 128, device="cuda").bfloat16() for _ in range(3))
+    k, v = (torch.randn(B, Skv, Hkv * 128, device="cuda").bfloat16() for _ in range(2))
+    lse = torch.full((B, Hq, Sq), 12.0, device="cuda")
+
+    def inside(t):                                      # [B, pad + rows + pad, width], NaN around
+        big = torch.full((B, t.shape[1] + 2 * pad, t.shape[2]), float("nan"), dtype=t.dtype, device="cuda")
+        big[:, pad:pad + t.shape[1]] = t
+        return big.flatten(0, 1)
+
+    def run(qt, kt, vt, gt, rows_q, rows_k, off):
+        stats = torch.full((2, B, Hq, rows_q), float("nan"), device="cuda")
+        acc = torch.zeros(B, Hq, rows_q, 128, device="cuda")
+        nds, nlse2, ref = (torch.empty(n, device="cuda").view(B, Hq, Sq, -1) for n in (B * Hq * Sq, B * Hq * Sq, B * Hq * Sq * 128))
+        E.attn_bwd_stats(g.flatten(0, 1), o.flatten(0, 1), lse, nds, nlse2, ref, B, Sq, Hq)
+        stats[0, :, :, off:off + Sq], stats[1, :, :, off:off + Sq] = nds.squeeze(-1), nlse2.squeeze(-1)
+        dk, dv = (torch.empty(B * Skv, Hkv * 128, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        E.attn_bwd_pair(qt, 0, kt, 0, vt, 0, gt, acc, dk, dv, stats[0], stats[1], B, Sq, Skv, Hq, Hkv, rows_q, off, rows_k, off,
+                        rows_q, off, causal)
+        kernels.check_error()
+        return acc, dk, dv
+
+    a0, dk0, dv0 = run(*(t.flatten(0, 1) for t in (q, k, v, g)), Sq, Skv, 0)
+    a1, dk1, dv1 = run(*map(inside, (q, k, v, g)), Sq + 2 * pad, Skv + 2 * pad, pad)
+    assert torch.equal(dk0, dk1) and torch.equal(dv0, dv1)
+    assert not a1[:, :, :pad].any() and not a1[:, :, pad + Sq:].any()
+    # fp32 sums of up to five partial tiles in another order: a few units of 2^-24 of the terms
+    assert relerr(a1[:, :, pad:pad + Sq], a0) < 1e-6

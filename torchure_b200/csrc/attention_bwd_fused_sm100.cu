@@ -38,6 +38,8 @@
 #include "attn_api.h"
 #include "common.cuh"
 
+#include <algorithm>
+
 namespace tb {
 
 int make_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, uint64_t rows, uint64_t cols, uint64_t ld,
@@ -582,6 +584,39 @@ static int bwd_parts(int tiles, int longest) {
   return parts;
 }
 
+// Whether CTA pairs (attention_bwd_2cta_sm100.cu) take the call: they need fewer cycles per iteration, but there are half as many
+// of them, and clusters of single CTAs that share a key block are better still where a few long chains are all there is.  From a
+// model fitted on B200: a key block takes 10.5 us + 2.7 us per iteration, a pair of them 10.8 + 1.9; beyond one wave the SMs'
+// shares add up, and the last tile sticks out by half its time.  Measured, us, without and with pairs: taken 4096 tokens x 2, 16 / 8
+// heads 362, 291; 16384, 16 / 8 2633, 2102; 2048, 16 / 8 100, 75; 8 x 512 49.1, 45.4; 8 x 256 21.3, 18.4; 8 x 640 68.0, 66.4;
+// left 1024, 16 / 8 35.4 (shared by two), 41.1; 4096, 8 / 2 183, 251; 8 x 384 35.3, 36.0; 2 x 512 24.6, 25.4.
+bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal) {
+  const int nqb = Sq / 128, nkb = Skv / 128, ratio = Hq / Hkv;
+  const int64_t groups = static_cast<int64_t>(B) * Hkv;
+  if (nkb < 2) return false;
+  int64_t one = 0, two = 0;                     // iterations of all key blocks of a group, of all pairs of them
+  for (int kb = 0; kb < nkb; ++kb) {
+    one += (causal ? nqb - kb : nqb) * ratio;
+    if (kb % 2 == 0) two += (causal ? nqb - kb : nqb) * ratio;
+  }
+  const int64_t pairs = (nkb + 1) / 2;
+  const float longest = static_cast<float>(nqb * ratio);
+  const float last_one = static_cast<float>(causal ? ratio : nqb * ratio);
+  const float last_two = causal && nkb % 2 == 0 ? 2 * last_one : last_one;
+  auto wave = [&](float fixed, float each, int64_t tiles, int64_t iters, float last, int slots) {
+    const float all = (fixed * tiles + each * iters) * groups / slots;
+    return std::max(fixed + each * longest, tiles * groups > slots ? all + 0.5f * (fixed + each * last) : all);
+  };
+  const float t_two = wave(10.8f, 1.9f, pairs, two, last_two, 74);
+  const int parts = bwd_parts(static_cast<int>(nkb * groups), nqb * ratio);
+  if (parts > 1) return t_two < 9.f + 2.7f * ((nqb * ratio + parts - 1) / parts) + (parts == 2 ? 4.f : 7.5f);
+  return t_two < wave(10.5f, 2.7f, nkb, one, last_one, 148);
+}
+
+int attn_bwd_2cta(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc, void* dk,
+                  void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv, int Hq, int Hkv,
+                  bool causal, int* err, cudaStream_t stream, const AttnPairLayout& lay);
+
 int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc,
                    void* dk, void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv,
                    int Hq, int Hkv, bool causal, int* err, cudaStream_t stream, const AttnPairLayout* lay) {
@@ -592,6 +627,10 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   if (ld_dkv % 8 != 0 || (reinterpret_cast<uintptr_t>(dk) & 15) || (reinterpret_cast<uintptr_t>(dv) & 15) ||
       (reinterpret_cast<uintptr_t>(dq_acc) & 15))
     return -3;
+  const int tiles = (Skv / 128) * B * Hkv;
+  const int parts = bwd_parts(tiles, (Sq / 128) * (Hq / Hkv));
+  if (attn_bwd_on_pairs(B, Sq, Skv, Hq, Hkv, causal))
+    return attn_bwd_2cta(q, k, v, d_o, dq_acc, dk, dv, ld_dkv, nds, nlse2, B, Sq, Skv, Hq, Hkv, causal, err, stream, *lay);
   const uint64_t Mq = static_cast<uint64_t>(lay->q_rows), Mk = static_cast<uint64_t>(lay->kv_rows);
   CUtensorMap tq, tk, tv, tdo;
   int r = make_tmap_2d(&tq, q.ptr, 2, Mq, q.ld, q.ld, 128, 64);
@@ -618,8 +657,7 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
   a.stat_stride = lay->stat_stride; a.stat_row0 = lay->stat_row0;
   a.scale = 1.f / sqrtf(static_cast<float>(HD));
   a.scale_log2 = a.scale * 1.4426950408889634f;
-  const int tiles = (Skv / 128) * B * Hkv;
-  a.parts = bwd_parts(tiles, (Sq / 128) * (Hq / Hkv));
+  a.parts = parts;
   const auto kern = a.parts > 1 ? attn_bwd_fused_kernel<true> : attn_bwd_fused_kernel<false>;
   if (!ensure_dynamic_smem(reinterpret_cast<const void*>(kern), SMEM_BYTES)) return -20;
   cudaLaunchConfig_t cfg{};

@@ -52,7 +52,8 @@ struct AttnPairLayout {
   int stat_stride, stat_row0;
 };
 
-// Single-pass backward (attention_bwd_fused_sm100.cu): five tile products per block pair instead of seven.
+// Single-pass backward (attention_bwd_fused_sm100.cu, and attention_bwd_2cta_sm100.cu on CTA pairs where attn_bwd_on_pairs says
+// so): five tile products per block pair instead of seven.
 //   q [B*Sq rows], k / v [B*Skv rows], d_o [B*Sq, Hq*128] bf16
 //   nds / nlse2  [B, Hq, Sq] fp32 from attn_bwd_stats: -rowsum(dO*O)/sqrt(d) and -lse*log2(e)
 //   dq_acc  fp32 [B, Hq, Sq, 128] (head-major): every CTA ADDS its partial dQ tiles, so it must hold zeros (which
@@ -65,6 +66,7 @@ int attn_bwd_stats(const void* d_o, const void* o, const float* lse, float* nds,
 int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc,
                    void* dk, void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv,
                    int Hq, int Hkv, bool causal, int* err, cudaStream_t stream, const AttnPairLayout* lay = nullptr);
+bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal);
 // dst[(b S + s), 128 h + d] (bf16, row stride ld_dst elements) = dq_acc[b, h, s, d]
 int attn_dq_convert(const float* dq_acc, void* dst, int64_t ld_dst, int B, int S, int Hq, cudaStream_t stream);
 

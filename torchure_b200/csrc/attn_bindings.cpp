@@ -48,6 +48,9 @@ void register_attn(pybind11::module_& m) {
                           (int)Hq, (int)Hkv, err, stream);
     TORCH_CHECK(rc == 0, "attn_bwd_dkv failed with code ", rc);
   });
+  m.def("attn_bwd_on_pairs", [](int64_t B, int64_t Sq, int64_t Skv, int64_t Hq, int64_t Hkv, bool causal) {
+    return tb::attn_bwd_on_pairs((int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal);
+  });
   // single-pass backward: statistics (+ accumulator clear), fused kernel, conversion of dQ to bf16
   m.def("attn_bwd_fused", [](const torch::Tensor& d_o, const torch::Tensor& qk, const torch::Tensor& qkv,
                              const torch::Tensor& o, const torch::Tensor& lse, torch::Tensor& dqkv, int64_t B, int64_t S,

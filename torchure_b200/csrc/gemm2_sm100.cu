@@ -19,7 +19,7 @@
 // Every wait is bounded; the two CTAs meet at a cluster barrier before anyone touches a partner's barrier and again
 // before either releases its tensor memory.
 #include "api.h"
-#include "common.cuh"
+#include "cta_pair.cuh"
 
 #include <type_traits>
 
@@ -43,50 +43,6 @@ constexpr int BAR_BYTES = 256;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + BAR_BYTES + 1024;
 constexpr int NUM_THREADS = 192;
 constexpr uint32_t TMEM_COLS = 512;
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// the address, in the cluster's shared window, of `local` in the CTA of rank `rank`
-__device__ __forceinline__ uint32_t map_to_cta(const void* local, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(local)), "r"(rank));
-  return out;
-}
-__device__ __forceinline__ void remote_arrive(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-// tiled TMA load whose completion is counted on a barrier that may live in the partner CTA (no multicast)
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, uint32_t cluster_bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(cluster_bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-// D[tmem, both CTAs] (+)= A * B over the pair
-__device__ __forceinline__ void umma2_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                             uint32_t accumulate) {
-  const uint32_t zero = 0;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(zero)
-      : "memory");
-}
-// the barrier at this shared-memory offset, in both CTAs, gets one arrival when every MMA issued so far has completed
-__device__ __forceinline__ void umma2_commit_both(uint64_t* bar) {
-  const uint16_t mask = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   smem_u32(bar)),
-               "h"(mask)
-               : "memory");
-}
 
 // What the epilogue does beside storing the tile.
 //   kEpiStore   nothing
@@ -168,10 +124,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
     fence_barrier_init();
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    tmem_alloc_pair(tmem_slot, TMEM_COLS);
     tc_fence_before();
   }
   __syncthreads();
@@ -512,7 +465,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   cluster_sync_all();   // neither CTA retires while its partner may still signal its barriers or read its operands
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 
