@@ -362,6 +362,36 @@ def test_qknorm_rope_bwd_reads_dq_from_the_fp32_accumulator(Hq, Hkv):
         torch.testing.assert_close(dkw, outs[0][2], rtol=1e-4, atol=1e-3)
 
 
+@pytest.mark.parametrize("Hq,Hkv,M", [(2, 1, 1), (4, 2, 7), (6, 3, 130), (10, 5, 9), (16, 8, 129), (24, 6, 33), (2, 2, 5000)])
+@pytest.mark.parametrize("variant", [0, 1, 2])
+def test_qknorm_rope_chunks(Hq, Hkv, M, variant):
+    """Heads are worked on in chunks of eight (backward: also of four) of one kind or of both, rows by warps that take several:
+    chunks that are not full, a kind that fills none, rows that fill no CTA and more rows than warps."""
+    from torchure_b200 import ops
+    from torchure_b200.models.qwen3 import RotaryEmbedding
+    from torchure_b200.ops import kernels, oracle
+
+    torch.manual_seed(2)
+    hd = 128
+    qkv = torch.randn(M, (Hq + 2 * Hkv) * hd, device="cuda").bfloat16()
+    qw, kw = torch.rand(hd, device="cuda") + 0.5, torch.rand(hd, device="cuda") + 0.5
+    cos, sin = RotaryEmbedding(hd).tables(M, "cuda")
+    qa = qkv.float().requires_grad_()
+    qwa, kwa = qw.clone().requires_grad_(), kw.clone().requires_grad_()
+    ref = oracle.qknorm_rope(qa, qwa, kwa, cos, sin, 1, M, Hq, Hkv, hd, 1e-6, True)
+    assert relerr(kernels.qknorm_rope(qkv, qw, kw, cos, sin, M, Hq, Hkv, 1e-6, True), ref) < 8e-3
+    g = torch.randn(M, (Hq + 2 * Hkv) * hd, device="cuda").bfloat16()
+    ref.backward(g[:, :(Hq + Hkv) * hd].float())
+    acc = g[:, :Hq * hd].float().view(1, M, Hq, hd).permute(0, 2, 1, 3).contiguous()
+    for dq_acc in (None, acc):
+        d, dqw, dkw = g.clone(), torch.zeros(hd, device="cuda"), torch.zeros(hd, device="cuda")
+        ops.ext().qknorm_rope_bwd(d, qkv, qw, kw, cos, sin, dqw, dkw, M, Hq, Hkv, 1e-6, True, dq_acc, variant)
+        assert relerr(d[:, :(Hq + Hkv) * hd], qa.grad[:, :(Hq + Hkv) * hd]) < 8e-3
+        assert torch.equal(d[:, (Hq + Hkv) * hd:], g[:, (Hq + Hkv) * hd:])
+        # the forward of the reference rounds the normalised values to bf16, whose gradient passes unrounded: 5e-3 as above
+        assert relerr(dqw, qwa.grad) < 5e-3 and relerr(dkw, kwa.grad) < 5e-3
+
+
 def test_swiglu_fwd_bwd():
     from torchure_b200.ops import kernels, oracle
 

@@ -183,7 +183,7 @@ std::tuple<Tensor, c10::optional<Tensor>, int64_t> block_backward_attn(
   d_o = Tensor();
   rc = tb::qknorm_rope_bwd(bf(dqkv), bf(qkv), qn.data_ptr<float>(), kn.data_ptr<float>(), cos.data_ptr<float>(),
                            sin.data_ptr<float>(), dqn.data_ptr<float>(), dkn.data_ptr<float>(), dq_acc.data_ptr<float>(), (int)M,
-                           (int)S, (int)Hq, (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, bind_num_sms(), err, stream);
+                           (int)S, (int)Hq, (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, bind_num_sms(), stream);
   TORCH_CHECK(rc == 0, "qknorm_rope_bwd failed with code ", rc);
   dq_acc = Tensor();
   Tensor d_h1 = make("block_backward.d_h1", {M, D}, dx1b.options());

@@ -443,9 +443,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
 // the rotation pairs element i with i + 64, so both partners sit in the same lane and need no shuffle.  cos/sin of
 // the row and both gain vectors are loaded once per row and reused by all heads.
 // ---------------------------------------------------------------------------------------------
-constexpr int QK_UNROLL = 4;      // forward: head pairs in flight per warp
-constexpr int QKB_U = 2;         // backward: head pairs whose reductions are interleaved
-constexpr int QKB_MAX_WARPS = 8;  // backward: warps of the one persistent CTA per SM (see the kernel)
+constexpr int QK_UNROLL = 4;      // forward: head pairs of a warp, all in flight at once
 
 __device__ __forceinline__ void unpack4(const uint2& u, float (&f)[4]) {
   float2 a = bf2_to_f2(u.x), b = bf2_to_f2(u.y);
@@ -466,6 +464,12 @@ __device__ __forceinline__ void load4f(const float* p, float (&f)[4]) {
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w;
 }
 
+// blockIdx.y: which 2 * QK_UNROLL heads, of one kind (q, then k) if SPLIT, else of both.  A warp does one row of them, all loads up
+// front: a warp per row that went through its 24 heads in three rounds left the memory idle during each round's arithmetic.
+// SPLIT needs one kind's gains only and fewer registers; it is taken where it makes no more chunks.  Measured on B200, inputs from
+// memory, before -> now, us: 8192 rows of 16 + 8 heads (101 MB) 24.2 -> 22.6; 4096 of 32 + 8 23.6 -> 18.8; 128 of 16 + 8 6.2 -> 3.2;
+// 8192 of 2 + 1 8.0 -> 7.2 (in one chunk of both kinds; 9.4 in two).
+template <bool SPLIT>
 __global__ void __launch_bounds__(256)
 qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ qw,
                        const float* __restrict__ kw, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
@@ -477,286 +481,236 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __res
   const int lane = threadIdx.x & 31;
   if (row >= M) return;
   const int sub = lane & 15, hsel = lane >> 4;
+  constexpr int PER = 2 * QK_UNROLL;
+  const int q_chunks = (Hq + PER - 1) / PER, chunk = blockIdx.y;
+  const bool of_q = chunk < q_chunks;                       // SPLIT: the chunk's kind
+  const int first = !SPLIT || of_q ? chunk * PER : Hq + (chunk - q_chunks) * PER;
+  const int end = min(SPLIT && of_q ? Hq : heads, first + PER);
   const int in_ld = (Hq + 2 * Hkv) * 128, out_ld = heads * 128;
   const __nv_bfloat16* src = qkv + static_cast<int64_t>(row) * in_ld + sub * 4;
   __nv_bfloat16* dst = out + static_cast<int64_t>(row) * out_ld + sub * 4;
   const int pos = row % S;
+  uint2 ulo[QK_UNROLL], uhi[QK_UNROLL];
+#pragma unroll
+  for (int k = 0; k < QK_UNROLL; ++k) {
+    const int h = first + 2 * k + hsel;
+    ulo[k] = uhi[k] = make_uint2(0u, 0u);
+    if (h < end) {
+      ulo[k] = *reinterpret_cast<const uint2*>(src + h * 128);
+      uhi[k] = *reinterpret_cast<const uint2*>(src + h * 128 + 64);
+    }
+  }
   float c[4], sn[4], gq_lo[4], gq_hi[4], gk_lo[4], gk_hi[4];
   load4f(cos_t + static_cast<int64_t>(pos) * 128 + sub * 4, c);  // cos[i] == cos[i + 64]
   load4f(sin_t + static_cast<int64_t>(pos) * 128 + sub * 4, sn);
   if (use_norm) {
-    load4f(qw + sub * 4, gq_lo); load4f(qw + 64 + sub * 4, gq_hi);
-    load4f(kw + sub * 4, gk_lo); load4f(kw + 64 + sub * 4, gk_hi);
+    const float* w = !SPLIT || of_q ? qw : kw;
+    load4f(w + sub * 4, gq_lo); load4f(w + 64 + sub * 4, gq_hi);
+    if (!SPLIT) { load4f(kw + sub * 4, gk_lo); load4f(kw + 64 + sub * 4, gk_hi); }
   }
-  const int pairs = (heads + 1) >> 1;
-  for (int hp = 0; hp < pairs; hp += QK_UNROLL) {
-    uint2 ulo[QK_UNROLL], uhi[QK_UNROLL];
 #pragma unroll
-    for (int k = 0; k < QK_UNROLL; ++k) {
-      const int h = 2 * (hp + k) + hsel;
-      ulo[k] = uhi[k] = make_uint2(0u, 0u);
-      if (h < heads) {
-        ulo[k] = *reinterpret_cast<const uint2*>(src + h * 128);
-        uhi[k] = *reinterpret_cast<const uint2*>(src + h * 128 + 64);
-      }
-    }
+  for (int k = 0; k < QK_UNROLL; ++k) {
+    const int h = first + 2 * k + hsel;
+    float lo[4], hi[4];
+    unpack4(ulo[k], lo);
+    unpack4(uhi[k], hi);
+    if (use_norm) {
+      float ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < QK_UNROLL; ++k) {
-      const int h = 2 * (hp + k) + hsel;
-      float lo[4], hi[4];
-      unpack4(ulo[k], lo);
-      unpack4(uhi[k], hi);
-      if (use_norm) {
-        float ss = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
-        ss = group16_sum(ss);
-        const float r = rsqrtf(ss * (1.f / 128.f) + eps);
-        const bool is_q = h < Hq;
-        // the reference normalises in bf16 precision before RoPE (its q_norm returns bf16)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          lo[e] = lo[e] * r * (is_q ? gq_lo[e] : gk_lo[e]);
-          hi[e] = hi[e] * r * (is_q ? gq_hi[e] : gk_hi[e]);
-        }
-        const uint2 rl = pack4(lo), rh = pack4(hi);
-        unpack4(rl, lo);
-        unpack4(rh, hi);
-      }
-      float olo[4], ohi[4];
+      for (int e = 0; e < 4; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
+      ss = group16_sum(ss);
+      const float r = rsqrtf(ss * (1.f / 128.f) + eps);
+      const bool is_q = SPLIT || h < Hq;      // SPLIT: gq is the chunk's kind
+      // the reference normalises in bf16 precision before RoPE (its q_norm returns bf16)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        olo[e] = lo[e] * c[e] - hi[e] * sn[e];
-        ohi[e] = hi[e] * c[e] + lo[e] * sn[e];
+        lo[e] = lo[e] * r * (is_q ? gq_lo[e] : gk_lo[e]);
+        hi[e] = hi[e] * r * (is_q ? gq_hi[e] : gk_hi[e]);
       }
-      if (h < heads) {
-        *reinterpret_cast<uint2*>(dst + h * 128) = pack4(olo);
-        *reinterpret_cast<uint2*>(dst + h * 128 + 64) = pack4(ohi);
-      }
+      const uint2 rl = pack4(lo), rh = pack4(hi);
+      unpack4(rl, lo);
+      unpack4(rh, hi);
+    }
+    float olo[4], ohi[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      olo[e] = lo[e] * c[e] - hi[e] * sn[e];
+      ohi[e] = hi[e] * c[e] + lo[e] * sn[e];
+    }
+    if (h < end) {
+      *reinterpret_cast<uint2*>(dst + h * 128) = pack4(olo);
+      *reinterpret_cast<uint2*>(dst + h * 128 + 64) = pack4(ohi);
     }
   }
 }
 
-// Backward of QK-norm + RoPE, one warp per token row, rows staged through shared memory by the TMA unit.
+// Backward of QK-norm + RoPE.  blockIdx.y: which 2 U heads of one kind (q, then k) the CTA's warps work on, a token row at a time;
+// so a CTA holds one kind's gain-gradient partials, and leaves them with one 16-byte reduction per four columns.
 //
-// A row needs dq (from the q columns of dqkv, or, ACC, from the head-major fp32 accumulator [B, Hq, S, 128] of the
-// single-pass attention backward, which is rounded to bf16 here on the way in instead of by a conversion pass of its
-// own), dk, the forward inputs x of the same heads and 64 cos / sin values: 16 KB for 16 + 8 heads.  Loaded straight
-// into registers, the bytes a warp keeps in flight are bounded by its register budget and the kernel ran at about a
-// third of the copy bandwidth.  Here every warp owns two row buffers; while it works on one row, up to 32 bulk
-// copies (one per lane: a head of the accumulator, the dk columns, the x columns, cos, sin) fill the other and
-// signal an mbarrier, so that a persistent CTA of eight warps keeps 100 KB and more in flight at no register cost.
-// Results are written to dqkv with 8-byte stores (16 lanes cover the 128 contiguous bytes of half a head).
-// Eight warps of 128 registers use half of the SM's register file: the CTA also fits on an SM that hosts a 512-thread
-// CTA of a gradient all-reduce kernel, so a launch during a data-parallel backward pass does not wait for those SMs.
-// Measured on B200, 8192 rows of 16 + 8 heads: 39 us with bf16 dq (two buffers per warp), 52 us with the fp32
-// accumulator (16.9 KB rows: one buffer per warp); twelve warps would gain 3 us but fill the register file.
-struct QkBwdPlan {
-  int dq_bytes;      // Hq * 512 (ACC) or Hq * 256
-  int off_dk, off_x, off_cs, stage_bytes;
-  int stages;        // row buffers per warp: 2 (the next row loads during this one's arithmetic) or 1
-};
-
-template <bool ACC>
-__global__ void __launch_bounds__(QKB_MAX_WARPS * 32, 2)   // <= 128 registers
-qknorm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dqkv, const __nv_bfloat16* __restrict__ qkv,
-                       const float* __restrict__ qw, const float* __restrict__ kw, const float* __restrict__ cos_t,
-                       const float* __restrict__ sin_t, float* __restrict__ dqw, float* __restrict__ dkw,
-                       const float* __restrict__ dq_acc, int M, int S, int Hq, int Hkv, float eps, int use_norm,
-                       QkBwdPlan plan, int* err) {
-  pdl_wait();
-  pdl_launch_dependents();
-  extern __shared__ __align__(128) uint8_t qk_smem[];
-  __shared__ uint64_t bars[QKB_MAX_WARPS][2];
-  __shared__ __align__(16) float red[2][128];
-  const int heads = Hq + Hkv;
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+// A row needs dq (from the q columns of dqkv, or, ACC, from the head-major fp32 accumulator [B, Hq, S, 128] of the single-pass
+// attention backward, which is rounded to bf16 here on the way out), dk, the forward inputs x of the same heads and 64 cos / sin
+// values.  All of a warp's U head pairs are loaded before the first is used, up to 3 KB a warp, and enough warps fit to keep
+// the memory busy.  (One persistent CTA of eight warps per SM with whole rows staged in shared memory by bulk copies, the
+// kernel before, was bound by the latency of those eight warps.)  Measured on B200, 8192 rows of 16 + 8 heads: dq in the accumulator
+// 51.2 -> 41.5 us, in bf16 36.7 -> 33.1; 4096 of 32 + 8 46.7 -> 35.7; 128 of 16 + 8 10.0 -> 5.8; 8192 of 2 + 1 19.0 -> 13.5.
+// U: 4 where every chunk is full and dq comes from the accumulator (16 + 8 heads 41.5, with 2 41.7; 32 + 8 35.7, 37.1), else 2 (16 + 4
+// heads 36.0, with 4 38.8; bf16 16 + 8 33.1, 37.4).
+template <bool ACC, bool IS_Q, int U>
+__device__ __forceinline__ void qknorm_rope_bwd_rows(__nv_bfloat16* __restrict__ dqkv, const __nv_bfloat16* __restrict__ qkv,
+                                                     const float* __restrict__ w, const float* __restrict__ cos_t,
+                                                     const float* __restrict__ sin_t, const float* __restrict__ dq_acc,
+                                                     float (&red)[128], int M, int S, int Hq, int Hkv, float eps, int use_norm,
+                                                     int first, int end) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane & 15, hsel = lane >> 4;
   const int ld = (Hq + 2 * Hkv) * 128;
-  const int pairs = (heads + 1) >> 1;
-  uint8_t* buf = qk_smem + static_cast<size_t>(wid) * plan.stages * plan.stage_bytes;
-  if (lane == 0) {
-    mbar_init(&bars[wid][0], 1);
-    mbar_init(&bars[wid][1], 1);
-    fence_barrier_init();
-  }
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) (&red[0][0])[i] = 0.f;
-  __syncthreads();
   // gains and this lane's gain-gradient partials as fp32 pairs: [0], [1] elements 4*sub.., [2], [3] elements 64+4*sub..
-  float2 gq[4], gk[4], aq[4], ak[4];
+  float2 g[4], acc[4];
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    gq[e] = gk[e] = make_float2(1.f, 1.f);
-    aq[e] = ak[e] = make_float2(0.f, 0.f);
+    g[e] = make_float2(1.f, 1.f);
+    acc[e] = make_float2(0.f, 0.f);
   }
   if (use_norm) {
-    const float4 q0 = *reinterpret_cast<const float4*>(qw + sub * 4), q1 = *reinterpret_cast<const float4*>(qw + 64 + sub * 4);
-    const float4 k0 = *reinterpret_cast<const float4*>(kw + sub * 4), k1 = *reinterpret_cast<const float4*>(kw + 64 + sub * 4);
-    gq[0] = make_float2(q0.x, q0.y); gq[1] = make_float2(q0.z, q0.w); gq[2] = make_float2(q1.x, q1.y); gq[3] = make_float2(q1.z, q1.w);
-    gk[0] = make_float2(k0.x, k0.y); gk[1] = make_float2(k0.z, k0.w); gk[2] = make_float2(k1.x, k1.y); gk[3] = make_float2(k1.z, k1.w);
+    const float4 g0 = *reinterpret_cast<const float4*>(w + sub * 4), g1 = *reinterpret_cast<const float4*>(w + 64 + sub * 4);
+    g[0] = make_float2(g0.x, g0.y); g[1] = make_float2(g0.z, g0.w); g[2] = make_float2(g1.x, g1.y); g[3] = make_float2(g1.z, g1.w);
   }
-  const uint32_t tx_bytes = static_cast<uint32_t>(plan.dq_bytes + Hkv * 256 + (use_norm ? heads * 256 : 0) + 512);
-  // every lane issues the copies whose index it owns: [0, n_dq) accumulator heads (or one copy of the q columns),
-  // then dk, x, cos, sin
-  auto issue = [&](int row, int stage) {
-    uint8_t* dst = buf + stage * plan.stage_bytes;
-    uint64_t* bar = &bars[wid][stage];
-    if (lane == 0) mbar_expect_tx(bar, tx_bytes);
-    __syncwarp();
+  for (int row = blockIdx.x * 8 + wid; row < M; row += gridDim.x * 8) {
     const int pos = row % S;
-    const __nv_bfloat16* drow = dqkv + static_cast<int64_t>(row) * ld;
-    const int n_dq = ACC ? Hq : 1;
-    for (int i = lane; i < n_dq + 4; i += 32) {
-      if (i < n_dq) {
-        if (ACC)
-          bulk_load_1d(dst + i * 512, dq_acc + ((static_cast<int64_t>(row / S) * Hq + i) * S + pos) * 128, 512, bar);
-        else
-          bulk_load_1d(dst, drow, static_cast<uint32_t>(Hq * 256), bar);
-      } else if (i == n_dq) {
-        bulk_load_1d(dst + plan.off_dk, drow + Hq * 128, static_cast<uint32_t>(Hkv * 256), bar);
-      } else if (i == n_dq + 1) {
-        if (use_norm)
-          bulk_load_1d(dst + plan.off_x, qkv + static_cast<int64_t>(row) * ld, static_cast<uint32_t>(heads * 256), bar);
-      } else if (i == n_dq + 2) {
-        bulk_load_1d(dst + plan.off_cs, cos_t + static_cast<int64_t>(pos) * 128, 256, bar);   // cos[i] == cos[i + 64]
+    __nv_bfloat16* drow = dqkv + static_cast<int64_t>(row) * ld + sub * 4;
+    const __nv_bfloat16* xrow = qkv + static_cast<int64_t>(row) * ld + sub * 4;
+    float4 flo[U], fhi[U];            // ACC: dq in fp32
+    uint2 dlo[U], dhi[U], xlo[U], xhi[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int h = first + 2 * u + hsel;
+      const bool live = h < end;      // an idle pass still takes part in the shuffles
+      if (ACC && IS_Q) {
+        flo[u] = fhi[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live) {
+          const float* p = dq_acc + ((static_cast<int64_t>(row / S) * Hq + h) * S + pos) * 128 + sub * 4;
+          flo[u] = *reinterpret_cast<const float4*>(p);
+          fhi[u] = *reinterpret_cast<const float4*>(p + 64);
+        }
       } else {
-        bulk_load_1d(dst + plan.off_cs + 256, sin_t + static_cast<int64_t>(pos) * 128, 256, bar);
+        dlo[u] = dhi[u] = make_uint2(0u, 0u);
+        if (live) {
+          dlo[u] = *reinterpret_cast<const uint2*>(drow + h * 128);
+          dhi[u] = *reinterpret_cast<const uint2*>(drow + h * 128 + 64);
+        }
+      }
+      xlo[u] = xhi[u] = make_uint2(0u, 0u);
+      if (live && use_norm) {
+        xlo[u] = *reinterpret_cast<const uint2*>(xrow + h * 128);
+        xhi[u] = *reinterpret_cast<const uint2*>(xrow + h * 128 + 64);
       }
     }
-  };
-  const int row0 = blockIdx.x * warps + wid, row_step = gridDim.x * warps;
-  bool ok = true;
-  const bool two = plan.stages == 2;
-  if (two && row0 < M) issue(row0, 0);
-  int k = 0;
-  for (int row = row0; row < M; row += row_step, ++k) {
-    const int stage = two ? (k & 1) : 0;
-    if (!two) issue(row, 0);
-    else if (row + row_step < M) issue(row + row_step, stage ^ 1);
-    if (!mbar_wait(&bars[wid][stage], (two ? (k >> 1) : k) & 1, err, kErrStagedRowWait)) { ok = false; break; }
-    const uint8_t* st = buf + stage * plan.stage_bytes;
-    float2 c[2], sn[2], nsn[2];
-    {
-      const float4 cv = *reinterpret_cast<const float4*>(st + plan.off_cs + sub * 16);
-      const float4 sv = *reinterpret_cast<const float4*>(st + plan.off_cs + 256 + sub * 16);
-      c[0] = make_float2(cv.x, cv.y); c[1] = make_float2(cv.z, cv.w);
-      sn[0] = make_float2(sv.x, sv.y); sn[1] = make_float2(sv.z, sv.w);
-      nsn[0] = make_float2(-sv.x, -sv.y); nsn[1] = make_float2(-sv.z, -sv.w);
-    }
-    __nv_bfloat16* dptr = dqkv + static_cast<int64_t>(row) * ld + sub * 4;
-    // One call handles the head pairs [first, first + count) of one kind (q or k, so the gains are not selected per
-    // element), QKB_U pairs at a time with every step written across the group: their shuffle chains, the only long
-    // dependency of a pass, then overlap.  All arithmetic is on fp32 pairs.  With xh = x r the normalised input,
-    // t = n g and d = mean(t xh):  dx = r (t - xh d) = r (g n - (r d) x),  dgain += n xh = (n x) r.
-    auto run = [&](auto is_q_tag, int first, int count, const float2 (&g)[4], float2 (&acc)[4]) {
-      constexpr bool IS_Q = decltype(is_q_tag)::value;
-      for (int p0 = 0; p0 < count; p0 += QKB_U) {
-        float2 n[QKB_U][4], x[QKB_U][4], ssd[QKB_U][2];   // ssd: partial sums of x^2 and of g n x
-        bool live[QKB_U];
-        int hh[QKB_U];
+    const float4 cv = *reinterpret_cast<const float4*>(cos_t + static_cast<int64_t>(pos) * 128 + sub * 4);   // cos[i] == cos[i + 64]
+    const float4 sv = *reinterpret_cast<const float4*>(sin_t + static_cast<int64_t>(pos) * 128 + sub * 4);
+    const float2 c[2] = {make_float2(cv.x, cv.y), make_float2(cv.z, cv.w)};
+    const float2 sn[2] = {make_float2(sv.x, sv.y), make_float2(sv.z, sv.w)};
+    const float2 nsn[2] = {make_float2(-sv.x, -sv.y), make_float2(-sv.z, -sv.w)};
+    // Every step is written across two head pairs: their shuffle chains, the only long dependency, overlap.  All arithmetic is on
+    // fp32 pairs.  With xh = x r the normalised input, t = n g and d = mean(t xh):
+    // dx = r (t - xh d) = r (g n - (r d) x),  dgain += n xh = (n x) r.
+    constexpr int V = U < 2 ? U : 2;
 #pragma unroll
-        for (int u = 0; u < QKB_U; ++u) {
-          const int h = first + 2 * (p0 + u) + hsel;
-          live[u] = p0 + u < count && h < (IS_Q ? Hq : heads);   // an idle pass still takes part in the shuffles
-          hh[u] = h;
-          const int hs = live[u] ? h : first;
-          float2 d[4];
-          if (ACC && IS_Q) {
-            const float4 lo = *reinterpret_cast<const float4*>(st + hs * 512 + sub * 16);
-            const float4 hi = *reinterpret_cast<const float4*>(st + hs * 512 + 256 + sub * 16);
-            d[0] = make_float2(lo.x, lo.y); d[1] = make_float2(lo.z, lo.w);
-            d[2] = make_float2(hi.x, hi.y); d[3] = make_float2(hi.z, hi.w);
-          } else {
-            const uint8_t* src = IS_Q ? st + hs * 256 : st + plan.off_dk + (hs - Hq) * 256;
-            const uint2 lo = *reinterpret_cast<const uint2*>(src + sub * 8), hi = *reinterpret_cast<const uint2*>(src + 128 + sub * 8);
-            d[0] = bf2_to_f2(lo.x); d[1] = bf2_to_f2(lo.y); d[2] = bf2_to_f2(hi.x); d[3] = bf2_to_f2(hi.y);
-          }
-          // transpose of the rotation: n_lo = d_lo c + d_hi s, n_hi = d_hi c - d_lo s
+    for (int u0 = 0; u0 < U; u0 += V) {
+      float2 n[V][4], x[V][4];
+      float ss[V], dot[V];
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            n[u][e] = fma2(d[2 + e], sn[e], mul2(d[e], c[e]));
-            n[u][2 + e] = fma2(d[e], nsn[e], mul2(d[2 + e], c[e]));
-          }
-          if (use_norm) {
-            const uint8_t* xs = st + plan.off_x + hs * 256;
-            const uint2 lo = *reinterpret_cast<const uint2*>(xs + sub * 8), hi = *reinterpret_cast<const uint2*>(xs + 128 + sub * 8);
-            x[u][0] = bf2_to_f2(lo.x); x[u][1] = bf2_to_f2(lo.y); x[u][2] = bf2_to_f2(hi.x); x[u][3] = bf2_to_f2(hi.y);
-            ssd[u][0] = ssd[u][1] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              ssd[u][0] = fma2(x[u][e], x[u][e], ssd[u][0]);
-              ssd[u][1] = fma2(mul2(n[u][e], x[u][e]), g[e], ssd[u][1]);
-            }
-          }
+      for (int v = 0; v < V; ++v) {
+        const int u = u0 + v;
+        float2 d[4];
+        if (ACC && IS_Q) {
+          d[0] = make_float2(flo[u].x, flo[u].y); d[1] = make_float2(flo[u].z, flo[u].w);
+          d[2] = make_float2(fhi[u].x, fhi[u].y); d[3] = make_float2(fhi[u].z, fhi[u].w);
+        } else {
+          d[0] = bf2_to_f2(dlo[u].x); d[1] = bf2_to_f2(dlo[u].y); d[2] = bf2_to_f2(dhi[u].x); d[3] = bf2_to_f2(dhi[u].y);
         }
-        if (use_norm) {
-          float ss[QKB_U], dot[QKB_U];
+        // transpose of the rotation: n_lo = d_lo c + d_hi s, n_hi = d_hi c - d_lo s
 #pragma unroll
-          for (int u = 0; u < QKB_U; ++u) {
-            ss[u] = ssd[u][0].x + ssd[u][0].y;
-            dot[u] = ssd[u][1].x + ssd[u][1].y;
-          }
+        for (int e = 0; e < 2; ++e) {
+          n[v][e] = fma2(d[2 + e], sn[e], mul2(d[e], c[e]));
+          n[v][2 + e] = fma2(d[e], nsn[e], mul2(d[2 + e], c[e]));
+        }
+        x[v][0] = bf2_to_f2(xlo[u].x); x[v][1] = bf2_to_f2(xlo[u].y); x[v][2] = bf2_to_f2(xhi[u].x); x[v][3] = bf2_to_f2(xhi[u].y);
+        float2 s2 = make_float2(0.f, 0.f), d2 = make_float2(0.f, 0.f);      // partial sums of x^2 and of g n x
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) {
+        for (int e = 0; e < 4; ++e) {
+          s2 = fma2(x[v][e], x[v][e], s2);
+          d2 = fma2(mul2(n[v][e], x[v][e]), g[e], d2);
+        }
+        ss[v] = s2.x + s2.y;
+        dot[v] = d2.x + d2.y;
+      }
+      if (use_norm) {
 #pragma unroll
-            for (int u = 0; u < QKB_U; ++u) {
-              ss[u] += __shfl_xor_sync(0xffffffffu, ss[u], o);
-              dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
-            }
-          }
+        for (int o = 8; o > 0; o >>= 1) {
 #pragma unroll
-          for (int u = 0; u < QKB_U; ++u) {
-            const float r = rsqrtf(ss[u] * (1.f / 128.f) + eps);
-            const float nrd = -r * r * dot[u] * (1.f / 128.f);      // -(r d)
-            const float2 r2 = make_float2(r, r), nrd2 = make_float2(nrd, nrd);
-            const float2 ra = live[u] ? r2 : make_float2(0.f, 0.f);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              acc[e] = fma2(mul2(n[u][e], x[u][e]), ra, acc[e]);
-              n[u][e] = mul2(fma2(x[u][e], nrd2, mul2(n[u][e], g[e])), r2);
-            }
+          for (int v = 0; v < V; ++v) {
+            ss[v] += __shfl_xor_sync(0xffffffffu, ss[v], o);
+            dot[v] += __shfl_xor_sync(0xffffffffu, dot[v], o);
           }
         }
 #pragma unroll
-        for (int u = 0; u < QKB_U; ++u) {
-          if (live[u]) {
-            *reinterpret_cast<uint2*>(dptr + hh[u] * 128) =
-                make_uint2(f2_to_bf2(n[u][0].x, n[u][0].y), f2_to_bf2(n[u][1].x, n[u][1].y));
-            *reinterpret_cast<uint2*>(dptr + hh[u] * 128 + 64) =
-                make_uint2(f2_to_bf2(n[u][2].x, n[u][2].y), f2_to_bf2(n[u][3].x, n[u][3].y));
+        for (int v = 0; v < V; ++v) {
+          const float r = rsqrtf(ss[v] * (1.f / 128.f) + eps);
+          const float nrd = -r * r * dot[v] * (1.f / 128.f);      // -(r d)
+          const float2 r2 = make_float2(r, r), nrd2 = make_float2(nrd, nrd);
+          // an idle pass has x = 0 and adds n x = 0
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            acc[e] = fma2(mul2(n[v][e], x[v][e]), r2, acc[e]);
+            n[v][e] = mul2(fma2(x[v][e], nrd2, mul2(n[v][e], g[e])), r2);
           }
         }
       }
-    };
-    run(std::true_type{}, 0, (Hq + 1) >> 1, gq, aq);
-    run(std::false_type{}, Hq, (Hkv + 1) >> 1, gk, ak);
-    __syncwarp();   // every lane is done with this buffer before the next iteration's copies overwrite it
-  }
-  if (!ok) {
-    // a copy may still be landing in this CTA's shared memory: give it time before the CTA retires
-    const uint64_t t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const int h = first + 2 * (u0 + v) + hsel;
+        if (h < end) {
+          *reinterpret_cast<uint2*>(drow + h * 128) =
+              make_uint2(f2_to_bf2(n[v][0].x, n[v][0].y), f2_to_bf2(n[v][1].x, n[v][1].y));
+          *reinterpret_cast<uint2*>(drow + h * 128 + 64) =
+              make_uint2(f2_to_bf2(n[v][2].x, n[v][2].y), f2_to_bf2(n[v][3].x, n[v][3].y));
+        }
+      }
+    }
   }
   if (use_norm) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      atomicAdd(&red[0][sub * 4 + 2 * e], aq[e].x);
-      atomicAdd(&red[0][sub * 4 + 2 * e + 1], aq[e].y);
-      atomicAdd(&red[0][64 + sub * 4 + 2 * e], aq[2 + e].x);
-      atomicAdd(&red[0][64 + sub * 4 + 2 * e + 1], aq[2 + e].y);
-      atomicAdd(&red[1][sub * 4 + 2 * e], ak[e].x);
-      atomicAdd(&red[1][sub * 4 + 2 * e + 1], ak[e].y);
-      atomicAdd(&red[1][64 + sub * 4 + 2 * e], ak[2 + e].x);
-      atomicAdd(&red[1][64 + sub * 4 + 2 * e + 1], ak[2 + e].y);
+      atomicAdd(&red[sub * 4 + 2 * e], acc[e].x);
+      atomicAdd(&red[sub * 4 + 2 * e + 1], acc[e].y);
+      atomicAdd(&red[64 + sub * 4 + 2 * e], acc[2 + e].x);
+      atomicAdd(&red[64 + sub * 4 + 2 * e + 1], acc[2 + e].y);
     }
+  }
+}
+
+template <bool ACC, int U>
+__global__ void __launch_bounds__(256, U == 4 ? 2 : 3)
+qknorm_rope_bwd_kernel(__nv_bfloat16* __restrict__ dqkv, const __nv_bfloat16* __restrict__ qkv,
+                       const float* __restrict__ qw, const float* __restrict__ kw, const float* __restrict__ cos_t,
+                       const float* __restrict__ sin_t, float* __restrict__ dqw, float* __restrict__ dkw,
+                       const float* __restrict__ dq_acc, int M, int S, int Hq, int Hkv, float eps, int use_norm) {
+  pdl_wait();
+  pdl_launch_dependents();
+  __shared__ __align__(16) float red[128];
+  if (threadIdx.x < 128) red[threadIdx.x] = 0.f;
+  __syncthreads();
+  const int q_chunks = (Hq + 2 * U - 1) / (2 * U), chunk = blockIdx.y;
+  const bool is_q = chunk < q_chunks;
+  const int first = (is_q ? chunk : chunk - q_chunks) * 2 * U;
+  if (is_q)
+    qknorm_rope_bwd_rows<ACC, true, U>(dqkv, qkv, qw, cos_t, sin_t, dq_acc, red, M, S, Hq, Hkv, eps, use_norm, first, Hq);
+  else
+    qknorm_rope_bwd_rows<ACC, false, U>(dqkv, qkv, kw, cos_t, sin_t, dq_acc, red, M, S, Hq, Hkv, eps, use_norm, Hq + first,
+                                        Hq + Hkv);
+  if (use_norm) {
     __syncthreads();
-    // one 16-byte reduction per four columns per CTA
-    if (threadIdx.x < 64) {
-      const int which = threadIdx.x >> 5, i = threadIdx.x & 31;
-      const float4 v = *reinterpret_cast<const float4*>(&red[which][4 * i]);
-      red_add_v4((which ? dkw : dqw) + 4 * i, v);
-    }
+    if (threadIdx.x < 32) red_add_v4((is_q ? dqw : dkw) + 4 * threadIdx.x, *reinterpret_cast<const float4*>(&red[4 * threadIdx.x]));
   }
 }
 
@@ -1227,37 +1181,31 @@ void qknorm_rope_fwd(const __nv_bfloat16* qkv, const float* qw, const float* kw,
                      __nv_bfloat16* out, int M, int S, int Hq, int Hkv, int hd, float eps, int use_norm,
                      cudaStream_t stream) {
   (void)hd;  // 128 only (checked by the caller)
-  launch_pdl(qknorm_rope_fwd_kernel, dim3((M + 7) / 8), dim3(256), 0, stream, qkv, qw, kw, cos, sin, out, M, S, Hq, Hkv, eps, use_norm);
+  constexpr int per = 2 * QK_UNROLL;
+  const int split = (Hq + per - 1) / per + (Hkv + per - 1) / per, mixed = (Hq + Hkv + per - 1) / per;
+  const dim3 grid((M + 7) / 8, split == mixed ? split : mixed);
+  if (split == mixed)
+    launch_pdl(qknorm_rope_fwd_kernel<true>, grid, dim3(256), 0, stream, qkv, qw, kw, cos, sin, out, M, S, Hq, Hkv, eps, use_norm);
+  else
+    launch_pdl(qknorm_rope_fwd_kernel<false>, grid, dim3(256), 0, stream, qkv, qw, kw, cos, sin, out, M, S, Hq, Hkv, eps, use_norm);
 }
 
 int qknorm_rope_bwd(__nv_bfloat16* dqkv, const __nv_bfloat16* qkv, const float* qw, const float* kw, const float* cos,
                     const float* sin, float* dqw, float* dkw, const float* dq_acc, int M, int S, int Hq, int Hkv, int hd,
-                    float eps, int use_norm, int num_sms, int* err, cudaStream_t stream, int force_stages, int force_warps) {
+                    float eps, int use_norm, int num_sms, cudaStream_t stream, int force_pairs) {
   (void)hd;
+  // four head pairs in flight where that leaves none idle and dq comes from the accumulator
+  const int pairs = force_pairs > 0 ? force_pairs : (dq_acc != nullptr && Hq % 8 == 0 && Hkv % 8 == 0 ? 4 : 2);
+  const int per = 2 * pairs, chunks = (Hq + per - 1) / per + (Hkv + per - 1) / per;
+  auto go = [&](auto kern) {
+    const int ctas = num_sms * (pairs == 4 ? 2 : 3);               // resident at once
+    const int cols = std::max(1, std::min((M + 7) / 8, ctas / chunks));
+    return launch_pdl(kern, dim3(cols, chunks), dim3(256), 0, stream, dqkv, qkv, qw, kw, cos, sin, dqw, dkw, dq_acc, M, S, Hq, Hkv,
+                      eps, use_norm);
+  };
   const bool acc = dq_acc != nullptr;
-  QkBwdPlan plan;
-  plan.dq_bytes = Hq * (acc ? 512 : 256);
-  plan.off_dk = plan.dq_bytes;
-  plan.off_x = plan.off_dk + Hkv * 256;
-  plan.off_cs = plan.off_x + (Hq + Hkv) * 256;
-  plan.stage_bytes = plan.off_cs + 512;
-  // as many warps (two row buffers each) as fit into the shared memory of one persistent CTA per SM
-  const int budget = 220 * 1024;
-  // two buffers per warp when all warps can have them, else one (more warps beat deeper buffers)
-  plan.stages = force_stages > 0 ? force_stages : (2 * plan.stage_bytes * QKB_MAX_WARPS <= budget ? 2 : 1);
-  int warps = std::min(force_warps > 0 ? std::min(force_warps, QKB_MAX_WARPS) : QKB_MAX_WARPS,
-                       budget / (plan.stages * plan.stage_bytes));
-  if (warps < 1) return -1;
-  const int smem = warps * plan.stages * plan.stage_bytes;
-  const void* fn = acc ? reinterpret_cast<const void*>(qknorm_rope_bwd_kernel<true>)
-                       : reinterpret_cast<const void*>(qknorm_rope_bwd_kernel<false>);
-  if (!ensure_dynamic_smem(fn, smem)) return -2;
-  const int grid = std::max(1, std::min((M + warps - 1) / warps, num_sms));
-  const cudaError_t rc =
-      acc ? launch_pdl(qknorm_rope_bwd_kernel<true>, dim3(grid), dim3(warps * 32), smem, stream, dqkv, qkv, qw, kw, cos,
-                       sin, dqw, dkw, dq_acc, M, S, Hq, Hkv, eps, use_norm, plan, err)
-          : launch_pdl(qknorm_rope_bwd_kernel<false>, dim3(grid), dim3(warps * 32), smem, stream, dqkv, qkv, qw, kw, cos,
-                       sin, dqw, dkw, dq_acc, M, S, Hq, Hkv, eps, use_norm, plan, err);
+  const cudaError_t rc = pairs == 4 ? (acc ? go(qknorm_rope_bwd_kernel<true, 4>) : go(qknorm_rope_bwd_kernel<false, 4>))
+                                    : (acc ? go(qknorm_rope_bwd_kernel<true, 2>) : go(qknorm_rope_bwd_kernel<false, 2>));
   return rc == cudaSuccess ? 0 : -3;
 }
 
