@@ -362,6 +362,37 @@ def test_qknorm_rope_bwd_reads_dq_from_the_fp32_accumulator(Hq, Hkv):
         torch.testing.assert_close(dkw, outs[0][2], rtol=1e-4, atol=1e-3)
 
 
+@pytest.mark.parametrize("M,N,K", [(19074, 512, 128), (9600, 904, 72), (20000, 1504, 64), (5000, 4000, 64)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_tall_outputs_in_groups_of_tile_rows(M, N, K, a_mn, b_mn):
+    """Tall outputs go through groups of tile rows: a last group of fewer rows, ragged tiles at both edges, several groups and
+    one, every operand order and output mode of the CTA-pair kernel."""
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(8)
+
+    def operand(rows, k_major):
+        t = torch.randn(rows, K, device="cuda").bfloat16()
+        if k_major:
+            return t, t
+        wide = torch.zeros(K, (rows + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")
+        wide[:, :rows] = t.t()
+        return t, wide[:, :rows]
+
+    a, a_arg = operand(M, not a_mn)
+    b, b_arg = operand(N, not b_mn)
+    ref = a.float() @ b.float().t()
+    out = kernels.gemm(a_arg, b_arg, a_mn=a_mn, b_mn=b_mn)
+    assert relerr(out, ref) < 4e-3                    # rounded to bf16: 2^-9
+    if a_mn == b_mn or not a_mn:
+        acc = torch.ones(M, N, device="cuda")
+        if a_mn == b_mn:
+            kernels.gemm(a_arg, b_arg, a_mn=a_mn, b_mn=b_mn, out=acc, accumulate=True)
+            assert relerr(acc, ref + 1) < 1e-5
+        kernels.gemm(a_arg, b_arg, a_mn=a_mn, b_mn=b_mn, out=acc)
+        assert relerr(acc, ref) < 1e-5                # fp32 sums of at most 128 products
+
+
 @pytest.mark.parametrize("Hq,Hkv,M", [(2, 1, 1), (4, 2, 7), (6, 3, 130), (10, 5, 9), (16, 8, 129), (24, 6, 33), (2, 2, 5000)])
 @pytest.mark.parametrize("variant", [0, 1, 2])
 def test_qknorm_rope_chunks(Hq, Hkv, M, variant):

@@ -84,7 +84,7 @@ __device__ __forceinline__ float ex2_approx(float x) {
 template <bool A_MN, bool B_MN, int OUT, int EPI>
 __device__ __forceinline__ void
 gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmUp,
-           const CUtensorMap& tmAct, const EpiArgs& ea, int M, int N, int K, int splits, int slice_rows, int* err) {
+           const CUtensorMap& tmAct, const EpiArgs& ea, int M, int N, int K, int splits, int slice_rows, int group, int* err) {
   constexpr int TN = EPI == kEpiSwiglu ? BNH : BN;   // columns of C per tile
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
@@ -108,6 +108,19 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   // split-K: work unit u = (tile u % num_tiles, K slice u / num_tiles); slices add into C with TMA reduce-add
   const int num_units = num_tiles * splits;
   const int kb_per = (num_kb + splits - 1) / splits;
+  // Tiles go down the columns, one column of tiles after the other, or (gemm2_bf16) down `group` rows of tiles at a time, through
+  // all columns.
+  auto place = [&](int tile, int& tm, int& tn) {
+    if (EPI == kEpiStore && group > 0) {
+      const int g0 = tile / (group * num_n) * group;
+      const int rows = min(group, num_m - g0), at = tile - g0 * num_n;
+      tm = g0 + at % rows;
+      tn = at / rows;
+    } else {
+      tm = tile % num_m;
+      tn = tile / num_m;
+    }
+  };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA);
@@ -145,9 +158,11 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
         const int tile = unit % num_tiles;
         const int kb0 = (unit / num_tiles) * kb_per;
         const int kb1 = min(num_kb, kb0 + kb_per);
-        const int m0 = (tile % num_m) * 2 * BM + static_cast<int>(rank) * BM;
+        int tm, tn;
+        place(tile, tm, tn);
+        const int m0 = tm * 2 * BM + static_cast<int>(rank) * BM;
         // the leader holds the first 128 B rows of the tile
-        const int n0 = (tile / num_m) * TN + static_cast<int>(rank) * (EPI == kEpiSwiglu ? N : BNH);
+        const int n0 = tn * TN + static_cast<int>(rank) * (EPI == kEpiSwiglu ? N : BNH);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, err, kErrProducerEmptyWait)) { ok = false; break; }
           uint8_t* sA = smem + stage * STAGE_BYTES;
@@ -223,8 +238,10 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
       const int tile = unit % num_tiles;
       if ((unit / num_tiles) * kb_per >= num_kb) continue;  // empty K slice
       const int c_row = (unit / num_tiles) * slice_rows;    // each slice has rows of its own in a workspace
-      const int m0 = (tile % num_m) * 2 * BM + static_cast<int>(rank) * BM;
-      const int n0 = (tile / num_m) * TN;
+      int tm, tn;
+      place(tile, tm, tn);
+      const int m0 = tm * 2 * BM + static_cast<int>(rank) * BM;
+      const int n0 = tn * TN;
       const int acc = it & 1;
       if constexpr (EPI == kEpiStore) {
         // In a branch of its own down to the wait: code of the other epilogues in the same loop body, never run here, cost the
@@ -446,7 +463,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
               }
             }
           }
-          if (ce_row < M) ea.stats[static_cast<int64_t>(tile / num_m) * M + ce_row] = make_float2(ce_m, ce_s);
+          if (ce_row < M) ea.stats[static_cast<int64_t>(tn) * M + ce_row] = make_float2(ce_m, ce_s);
         }
       }
       ++it;
@@ -472,10 +489,10 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 template <bool A_MN, bool B_MN, int OUT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int splits, int slice_rows, int* err) {
+                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int splits, int slice_rows, int group, int* err) {
   pdl_wait();
   pdl_launch_dependents();
-  gemm2_body<A_MN, B_MN, OUT, kEpiStore>(tmA, tmB, tmC, tmC, tmC, EpiArgs{}, M, N, K, splits, slice_rows, err);
+  gemm2_body<A_MN, B_MN, OUT, kEpiStore>(tmA, tmB, tmC, tmC, tmC, EpiArgs{}, M, N, K, splits, slice_rows, group, err);
 }
 
 // Measured on B200, M x F x K, product + pass over it before, fused now, fused without storing gate and up: 8192 x 3072 x 1024
@@ -488,7 +505,7 @@ gemm2_swiglu_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     int* err) {
   pdl_wait();
   pdl_launch_dependents();
-  gemm2_body<false, false, 0, kEpiSwiglu>(tmA, tmB, tmGate, tmUp, tmAct, ea, M, F, K, 1, 0, err);
+  gemm2_body<false, false, 0, kEpiSwiglu>(tmA, tmB, tmGate, tmUp, tmAct, ea, M, F, K, 1, 0, 0, err);
 }
 
 // Bound by its epilogue when K is short: 256 columns of two special-function operations, two loads and two stores per row
@@ -500,7 +517,7 @@ gemm2_swiglu_bwd_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                         const __grid_constant__ EpiArgs ea, int M, int F, int K, int* err) {
   pdl_wait();
   pdl_launch_dependents();
-  gemm2_body<false, true, 0, kEpiSwigluBwd>(tmA, tmB, tmGate, tmUp, tmGate, ea, M, F, K, 1, 0, err);
+  gemm2_body<false, true, 0, kEpiSwigluBwd>(tmA, tmB, tmGate, tmUp, tmGate, ea, M, F, K, 1, 0, 0, err);
 }
 
 // Measured on B200, against the product and a loss pass over its output: 4096 x 151936 x 1024 834 + 238 us before, 773 + 17
@@ -510,7 +527,7 @@ gemm2_ce_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 const __grid_constant__ EpiArgs ea, int M, int N, int K, int* err) {
   pdl_wait();
   pdl_launch_dependents();
-  gemm2_body<false, false, 0, kEpiCe>(tmA, tmB, tmB, tmB, tmB, ea, M, N, K, 1, 0, err);
+  gemm2_body<false, false, 0, kEpiCe>(tmA, tmB, tmB, tmB, tmB, ea, M, N, K, 1, 0, 0, err);
 }
 
 // How many CTA pairs the device can hold at once.  The two CTAs of a pair sit on the two SMs of one TPC; a part with
@@ -571,12 +588,21 @@ int gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int64
   const uint64_t c_rows = slice_rows > 0 ? static_cast<uint64_t>(slice_rows) * splits : M;
   r = out_mode == 0 ? make_tmap_2d(&tc, C, 2, c_rows, N, ldc, 32, 64) : make_tmap_2d(&tc, C, 4, c_rows, N, ldc, 32, 32);
   if (r) return r - 200;
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-  const int units = tiles * splits;
+  // The order of the tiles, so that the clusters in flight cover a block of the output as square as can be and read A and B from
+  // memory once: a wide output column by column of tiles (all rows at a time), a tall one by groups of as many rows of tiles as one
+  // wave holds of whole rows.  Column by column a tall output read A once per column of tiles: the gradient of a head its 1.2 GB of
+  // logits four times.  Measured on B200, cold inputs, M x N x K, column by column, in groups, us: weight gradients 151936 x 1024 x 1024
+  // 307, 243; 19456 x 2560 x 4096 328, 264; 16384 x 2048 x 8192 408, 350; 50257 x 512 x 600 48.0, 43.6; bf16 16384 x 1024 x 2048
+  // 57.4, 52.9; 8192 x 2048 x 16384 388, 365; 8192 x 1024 x 3072 43.7, 41.6; wide ones, in groups slower: 2560 x 9728 x 4096 140, 149;
+  // 2048 x 8192 x 8192 180, 189; 4096 x 6144 x 2560 87.8, 88.8; about square, 8192 x 8192 x 2048, no difference.
+  const int pairs = g_pair_capacity > 0 && g_pair_capacity < num_sms / 2 ? g_pair_capacity : num_sms / 2;
+  const int num_m = (M + 2 * BM - 1) / (2 * BM), num_n = (N + BN - 1) / BN;
+  const int units = num_m * num_n * splits;
+  const int group = splits == 1 && num_n > 1 && num_m > num_n ? (pairs > 4 * num_n ? pairs / num_n : 4) : 0;
 #define TB_GEMM2_CASE(AM, BMN, O) \
   if (a_mn == AM && b_mn == BMN && out_mode == O) \
     return launch_pairs(gemm2_bf16_kernel<AM, BMN, O>, units, num_sms, stream, ta, tb_, tc, M, N, K, splits, \
-                        static_cast<int>(slice_rows), err);
+                        static_cast<int>(slice_rows), group, err);
   TB_GEMM2_CASE(false, false, 0)
   TB_GEMM2_CASE(false, false, 1)
   TB_GEMM2_CASE(false, false, 2)
