@@ -103,3 +103,17 @@ def test_fp32_products_keep_their_slices_short():
                 for mode in (1, 2):
                     _, _, splits, _ = _C.gemm_plan(m, n, k, a_mn=True, b_mn=True, out_mode=mode)
                     assert ceil_div(blocks, splits) <= longest, (m, n, k, mode)
+
+
+@pytest.mark.parametrize("M,N,K", [(4096, 2560, 151936), (2816, 1024, 151936), (4096, 1024, 151936), (8192, 4096, 151936),
+                                   (16384, 8192, 151936), (4096, 2560, 9728)])
+def test_slices_that_fill_the_waves(M, N, K):
+    """A head's dH with many tiles is sliced where the waves are partly empty: within 256 MB, without an empty slice, and on
+    request only."""
+    assert _C.gemm_plan(M, N, K, b_mn=True)[0] != "slices"
+    kind, _, splits, ws = _C.gemm_plan(M, N, K, b_mn=True, may_split=True)
+    if kind == "slices":
+        assert 1 < splits <= 8 and ws <= 256 << 20
+        per = ceil_div(ceil_div(K, 64), splits)
+        assert (splits - 1) * per < ceil_div(K, 64)
+    assert (kind == "slices") == ((M, N) in ((4096, 2560), (2816, 1024)) and K > 65536)
