@@ -282,3 +282,47 @@ def test_native_block_calls_equal_the_wrappers(monkeypatch, B, S, qk_norm):
         for _ in range(20):
             assert torch.equal(model(ids, return_final_hidden=True), want)
     kernels.check_error()
+
+
+@pytest.mark.parametrize("B,S,layers,qk_norm", [(1, 128, 1, True), (3, 384, 4, False), (2, 1152, 3, True)])
+def test_forward_without_gradients_in_one_call(monkeypatch, B, S, layers, qk_norm):
+    """The pass without gradients (one native call, the blocks' buffers used again and again) gives the bits of the pass with
+    them, for strided ids, an exchanged gain and on another stream; poisoned outputs keep it a block at a time."""
+    from torchure_b200 import ops
+    from torchure_b200.models import build_model
+    from torchure_b200.ops import debug, kernels
+
+    calls = []
+    whole = ops.ext().blocks_forward
+    monkeypatch.setattr(ops.ext(), "blocks_forward", lambda *a: calls.append(1) or whole(*a))
+    torch.manual_seed(1)
+    with torch.device("cuda"):
+        model = build_model("qwen3_dense" if qk_norm else "llama3_2",
+                            dict(num_layers=layers, num_heads=4, num_kv_heads=2, emb_dim=640, head_dim=128, vocab_size=1000,
+                                 ffn_dim=1096))
+        model.init_weights()
+    ids = torch.randint(0, 1000, (S, B), device="cuda").t()
+    want = model(ids, return_final_hidden=True).detach()
+    assert not calls
+    with torch.no_grad():
+        for _ in range(20):
+            assert torch.equal(model(ids, return_final_hidden=True), want)
+        assert len(calls) == 20
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            other = model(ids, return_final_hidden=True)
+        side.synchronize()
+        assert torch.equal(other, want)
+        model.blocks[-1].norm2.weight = torch.nn.Parameter(model.blocks[-1].norm2.weight * 2)
+    want = model(ids, return_final_hidden=True).detach()
+    with torch.no_grad():
+        assert torch.equal(model(ids, return_final_hidden=True), want)
+        n = len(calls)
+        debug.enable(True)
+        try:
+            assert torch.equal(model(ids, return_final_hidden=True), want) and debug.verify() > 10
+        finally:
+            debug.enable(False)
+        assert len(calls) == n
+    kernels.check_error()

@@ -27,8 +27,11 @@
 // cluster scope waits for the SM's reductions in flight, 1800 cycles.  Shared memory: K and V (own keys), K of all 256 keys cut
 // to the CTA's 64 head-dim columns, dS, dS on its way to the partner (one 16 KB bulk copy per block), dQ on its way to memory,
 // and a ring of 16 KB tiles in the order in which the products want them: 64 rows of Q or dO for S^T and dP^T, 64 columns of
-// them for dK and dV.  Shared memory is what bounds it now: of 128-byte accesses per block the products' operands take 1536, TMA
-// 512, the exchange and dS 512, dQ 512, the row statistics 256, 3300 of the 3600 cycles that an iteration measures.
+// them for dK and dV.
+//
+// What bounds it now is the chain of an iteration, 3600 cycles by clock marks: no unit is above 66 % busy (tensor pipe 65, shared
+// memory and L1 63, issue 36).  The row statistics queue behind the tensor core's operand reads, so S_i -> P_i takes 1300 cycles, as
+// long with its exp2 and conversions taken out; the exchange of dS takes 900 to 1600 of the 1030 that dK_i-1 and dP_i cover.
 //
 // Measured on B200, single-CTA kernel -> this one, us: 2 x 4096 tokens, 16 / 8 heads 362 -> 291; 16384, 16 / 8 2633 -> 2102 (1308
 // TFLOP/s of the five causal products); 4096, 32 / 8 384 -> 281; 3 x 1408, 16 / 8 87 -> 71; 8 x 1024, 16 / 8 136 -> 117.

@@ -26,6 +26,7 @@ from __future__ import annotations
 import weakref
 
 import torch
+from torch.autograd import forward_ad
 
 from torchure_b200 import ops
 from torchure_b200.ops import attention as attn_ops
@@ -189,6 +190,18 @@ class Sm100Engine:
         flat_ids = ids.reshape(-1).contiguous()      # one strided sequence reshapes to a strided view
         # under no_grad the parameters still count as inputs that need gradients
         want_grad = torch.is_grad_enabled()
+        if not want_grad and self._one_call(S):
+            cfg = self.cfg
+            cos, sin = self.rope_tables(S, ids.device)
+            layers = []
+            for block, sh in zip(m.blocks, self.layers):
+                w1, _, _, _, _, qn, kn, w2, _, _, _ = sh.inputs(block, self.dummy)
+                layers.append((w1, sh.wqkv, qn, kn, sh.wo, w2, sh.wgu, sh.wd))
+            h, n = ops.ext().blocks_forward(
+                flat_ids, self.emb_shadow if self.bf16_embedding else m.token_emb.weight, layers, cos, sin, m.norm.weight,
+                m.norm.eps, B, S, cfg["num_heads"], cfg["num_kv_heads"], cfg["norm_eps"], cfg["qk_norm"])
+            ops.count_launch(n)
+            return h.view(B, S, -1)
         if self.pre_block is not None:
             self.pre_block(-1)
         for i, (block, sh) in enumerate(zip(m.blocks, self.layers)):
@@ -204,6 +217,15 @@ class Sm100Engine:
         if self.tied and torch.is_grad_enabled() and m.token_emb.weight.requires_grad:
             self.expect_tied_grad = True
         return h.view(B, S, -1)
+
+    def _one_call(self, S: int) -> bool:
+        """True when a pass without gradients may run as one native call: no strategy acts between the kernels, no output is
+        poisoned, and nothing traces or transforms the autograd functions that the call passes by."""
+        cfg = self.cfg
+        return (len(self.layers) > 0 and self.pre_block is None and self.cp is None and self.tp is None and not debug.enabled()
+                and forward_ad._current_level < 0 and not torch._C._are_functorch_transforms_active()
+                and not torch.jit.is_tracing()
+                and attn_ops.kernel_supported(S, cfg["num_heads"], cfg["num_kv_heads"], cfg["head_dim"]))
 
     def lm_head(self, h: torch.Tensor) -> torch.Tensor:
         m = self.model
