@@ -117,3 +117,17 @@ def test_slices_that_fill_the_waves(M, N, K):
         per = ceil_div(ceil_div(K, 64), splits)
         assert (splits - 1) * per < ceil_div(K, 64)
     assert (kind == "slices") == ((M, N) in ((4096, 2560), (2816, 1024)) and K > 65536)
+
+
+@pytest.mark.parametrize("weight", [1 << 20, 1 << 28])
+def test_chunks_of_the_loss_head(weight):
+    """At most ``chunk_size`` rows, no more chunks than it asks for, every row in one; 4097 rows in two chunks of about half."""
+    from torchure_b200.ops.linear_ce import _chunk_rows
+
+    for chunk in (1, 100, 255, 256, 257, 512, 600, 1000, 1024, 4096, 10000):
+        for n in [1, 2, 127, 128, 129, 255, 256, 257, 511, 513, 600, 1100, 1531, 4096, 4097, 4224, 8192, 30000]:
+            rows = _chunk_rows(n, chunk, weight)
+            assert 0 < rows <= min(chunk, n) or (rows == chunk and n > chunk), (n, chunk, rows)
+            assert ceil_div(n, rows) <= ceil_div(n, chunk), (n, chunk, rows)
+    assert _chunk_rows(4097, 4096, 1 << 28) == 2304 and _chunk_rows(1531, 600, 1 << 28) == 512
+    assert _chunk_rows(1100, 1000, 1 << 20) == 1000 and _chunk_rows(8192, 4096, 1 << 28) == 4096
