@@ -10,8 +10,9 @@ Backward writes dq | dk | dv into one (M, (Hq+2Hkv)*hd) buffer laid out like ``q
 QK-norm/RoPE backward kernel then transforms in place and the QKV dgrad/wgrad GEMMs consume.
 
 ``impl="sm100"`` is the hand-written tcgen05 kernel set: ``csrc/attention_fwd_sm100.cu`` forward and, for
-backward, either the single-pass kernel ``csrc/attention_bwd_fused_sm100.cu`` (default: five tile products per
-block pair, dQ partial tiles added into an fp32 accumulator, so dQ is not bitwise repeatable) or the two-kernel
+backward, either a single-pass kernel (default: five tile products per block pair, dQ partial tiles added into an fp32
+accumulator, so dQ is not bitwise repeatable; ``csrc/attention_bwd_2cta_sm100.cu`` on CTA pairs, or
+``csrc/attention_bwd_fused_sm100.cu`` where few or short chains are all there is) or the two-kernel
 path ``csrc/attention_bwd_dq_sm100.cu`` + ``csrc/attention_bwd_dkv_sm100.cu`` (seven products, no atomics, bitwise
 repeatable; ``set_backward("split")`` or ``TORCHURE_B200_ATTN_BWD=split``).
 ``impl="sdpa"`` routes through ``torch.nn.functional.scaled_dot_product_attention``.  It exists for A/B comparison

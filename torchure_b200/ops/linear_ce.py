@@ -1,6 +1,6 @@
 """Chunked fused linear + cross-entropy on sm_100a kernels.
 
-Per chunk of ``chunk_size`` rows (reference algorithm: ``torchure/loss/fused_linear_ce.py:31-93``):
+Per chunk of at most ``chunk_size`` rows (reference algorithm: ``torchure/loss/fused_linear_ce.py:31-93``):
 
 1. ``logits = h_chunk @ W^T``         tcgen05 GEMM, bf16 out (the only (chunk, V) buffer, reused by every chunk)
 2. ``ce_softmax_grad``                one kernel: online max/sum, target gather, per-row loss and, in place,
