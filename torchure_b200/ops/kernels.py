@@ -199,6 +199,21 @@ def gemm_ce(a, b, labels, target):
     return stats
 
 
+def ce_inverse_count(labels, ignore_index, scale):
+    """fp32 (1,): scale / max(1, labels that are not ``ignore_index``).  Like ``ce_mean`` not among the counted launches, which are
+    those of a chunk."""
+    out = new_output("ce_inverse_count", 1, dtype=torch.float32, device=labels.device)
+    _C().ce_inverse_count(labels, out, ignore_index, scale)
+    return out
+
+
+def ce_mean(row_loss, inv_n):
+    """0-dim fp32: sum(row_loss) * inv_n."""
+    out = new_output("ce_mean", 1, dtype=torch.float32, device=row_loss.device)
+    _C().ce_mean(row_loss, inv_n, out)
+    return out.view(())
+
+
 def ce_loss_tiles(tiles, target, labels, row_loss, vocab, ignore_index):
     """``ce_loss`` from the statistics and label logits of ``gemm_ce``."""
     _C().ce_loss_tiles(tiles, target, labels, row_loss, vocab, ignore_index)

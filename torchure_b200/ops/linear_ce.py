@@ -40,6 +40,8 @@ def _chunk_rows(N: int, chunk_size: int, weight_elements: int) -> int:
     3000 x 2048 x 60000 (1000) 2544 -> 2291; 5000 x 1024 x 100000 (4096) 3255 -> 3086.  A last chunk of at most 128 rows, which has
     a kernel of its own, stays where dW fits the cache (64 MB): 1100 x 512 x 30000 (1000) 368, 389 in equal ones.
     """
+    if N <= 0 or chunk_size <= 0:       # refused by the loop over the chunks
+        return min(chunk_size, N)
     if 0 < N % chunk_size <= 128 and N > chunk_size and weight_elements <= 1 << 24:
         return chunk_size
     per = -(-N // -(-N // chunk_size))
@@ -65,8 +67,10 @@ class _LinearCESm100(torch.autograd.Function):
         dev = hidden.device
         h = hidden if hidden.dtype == BF16 else hidden.to(BF16)
         h, labels = h.contiguous(), labels.contiguous()
-        n_valid = (labels != ignore_index).sum().clamp_min(1) if normalizer is None else normalizer
-        inv_n = (loss_scale / n_valid.float()).reshape(1)
+        if normalizer is None:
+            inv_n = K.ce_inverse_count(labels, ignore_index, loss_scale)
+        else:
+            inv_n = (loss_scale / normalizer.float()).reshape(1)
         row_loss = torch.empty(N, dtype=torch.float32, device=dev)
         # under no_grad the parameter still counts as an input that needs a gradient; nothing will ever ask for it
         need_dh = want_grad and ctx.needs_input_grad[0]
@@ -121,7 +125,7 @@ class _LinearCESm100(torch.autograd.Function):
                 K.gemm(logits, hc, a_mn=True, b_mn=True, out=d_weight, accumulate=acc0 or lo > 0)
         if vocab_parallel is not None and need_dh:
             all_reduce(d_hidden, *vocab_parallel, "sum")     # each rank contributed its vocabulary rows
-        loss = row_loss.sum() * inv_n[0]
+        loss = K.ce_mean(row_loss, inv_n)
         ctx.stash = (d_hidden, d_weight_all)
         ctx.engine = engine
         ctx.in_sink = sink_dest is not None
