@@ -440,6 +440,32 @@ def test_qknorm_rope_chunks(Hq, Hkv, M, variant):
         assert relerr(dqw, qwa.grad) < 5e-3 and relerr(dkw, kwa.grad) < 5e-3
 
 
+@pytest.mark.parametrize("Hq,Hkv,M", [(2, 1, 130), (4, 2, 9), (6, 3, 130), (10, 5, 9), (16, 8, 129)])
+@pytest.mark.parametrize("variant", [0, 1, 2])
+def test_qknorm_rope_bwd_without_eps(Hq, Hkv, M, variant):
+    """eps = 0: the halves of a warp that have no head of their own (chunks that are not full) add nothing to the gain gradients."""
+    from torchure_b200 import ops
+    from torchure_b200.models.qwen3 import RotaryEmbedding
+    from torchure_b200.ops import oracle
+
+    torch.manual_seed(3)
+    hd = 128
+    qkv = torch.randn(M, (Hq + 2 * Hkv) * hd, device="cuda").bfloat16()
+    qw, kw = torch.rand(hd, device="cuda") + 0.5, torch.rand(hd, device="cuda") + 0.5
+    cos, sin = RotaryEmbedding(hd).tables(M, "cuda")
+    qa = qkv.float().requires_grad_()
+    qwa, kwa = qw.clone().requires_grad_(), kw.clone().requires_grad_()
+    g = torch.randn(M, (Hq + 2 * Hkv) * hd, device="cuda").bfloat16()
+    oracle.qknorm_rope(qa, qwa, kwa, cos, sin, 1, M, Hq, Hkv, hd, 0.0, True).backward(g[:, :(Hq + Hkv) * hd].float())
+    acc = g[:, :Hq * hd].float().view(1, M, Hq, hd).permute(0, 2, 1, 3).contiguous()
+    for dq_acc in (None, acc):
+        d, dqw, dkw = g.clone(), torch.zeros(hd, device="cuda"), torch.zeros(hd, device="cuda")
+        ops.ext().qknorm_rope_bwd(d, qkv, qw, kw, cos, sin, dqw, dkw, M, Hq, Hkv, 0.0, True, dq_acc, variant)
+        # as in test_qknorm_rope_chunks
+        assert relerr(d[:, :(Hq + Hkv) * hd], qa.grad[:, :(Hq + Hkv) * hd]) < 8e-3
+        assert relerr(dqw, qwa.grad) < 5e-3 and relerr(dkw, kwa.grad) < 5e-3
+
+
 def test_swiglu_fwd_bwd():
     from torchure_b200.ops import kernels, oracle
 
