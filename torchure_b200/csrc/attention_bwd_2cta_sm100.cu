@@ -372,9 +372,8 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
     int row = (b * a.Hq + kvh * ratio) * a.stat_stride + a.stat_row0 + (quarter >> 1) * 64;     // of the head's first query
     int qb = qb0;
     for (int it = 0; it < n_iter; ++it) {
-      if (!mbar_wait(&bars->dq_full, it & 1, err, kErrAttnWait)) break;
+      if (!mbar_wait_warp(&bars->dq_full, it & 1, err, kErrAttnWait)) break;
       tc_fence_after();
-      __syncwarp();
       uint32_t v[64];
       tmem_ld_32x32b_x32(t_dq, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
       tmem_ld_32x32b_x32(t_dq + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
@@ -418,10 +417,9 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
       const bool mask = phantom || (a.causal && qb <= kblk);
       const int hidden = phantom ? 64 : (kblk - qb) * 128 + row - half * 64;
       if (++qb == nqb) qb = qb0;
-      if (!mbar_wait(&bars->stat_full[it & 1], (it >> 1) & 1, err, kErrAttnWait) ||
-          !mbar_wait(&bars->s_full, it & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->stat_full[it & 1], (it >> 1) & 1, err, kErrAttnWait) ||
+          !mbar_wait_warp(&bars->s_full, it & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
-      __syncwarp();
       uint32_t p[64];                         // P^T in fp32, kept until dS^T
       tmem_ld_32x32b_x32(t_s, *reinterpret_cast<uint32_t(*)[32]>(&p[0]));
       tmem_ld_32x32b_x32(t_s + 32, *reinterpret_cast<uint32_t(*)[32]>(&p[32]));
@@ -429,6 +427,7 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive(lead_read);
+      __syncwarp();
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t pk[8];
@@ -454,9 +453,8 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) pair_arrive(lead_p);
-      if (!mbar_wait(&bars->dp_full, it & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->dp_full, it & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
-      __syncwarp();
       uint32_t pd[32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {           // dS^T goes where dP^T has been read already
@@ -477,7 +475,7 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         tmem_st_32x32b_x8(t_dp + 8 * c, *reinterpret_cast<const uint32_t(*)[8]>(&pd[8 * c]));
       }
       // the tensor core and the copy to the partner have read the dS^T tiles of the iteration before
-      if (it > 0 && !mbar_wait(&bars->dq_full, (it - 1) & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (it > 0 && !mbar_wait_warp(&bars->dq_full, (it - 1) & 1, err, kErrAttnWait)) { ok = false; break; }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
         *reinterpret_cast<uint4*>(ds_row + ((j ^ (row & 7)) << 4)) = make_uint4(pd[4 * j], pd[4 * j + 1], pd[4 * j + 2], pd[4 * j + 3]);
@@ -490,7 +488,7 @@ attn_bwd_2cta_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
         pair_arrive(lead_ds);
       }
     }
-    if (ok && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait) && !phantom) {
+    if (ok && mbar_wait_warp(&bars->acc_done, 0, err, kErrAttnWait) && !phantom) {
       // warps of half 0 write dV, of half 1 dK: one key row per lane
       tc_fence_after();
 #pragma unroll 1

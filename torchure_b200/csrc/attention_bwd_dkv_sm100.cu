@@ -200,7 +200,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
       const bool diag = (it % n_qb) == 0;     // query block == key block
       const float* sStat = reinterpret_cast<const float*>(sStage + s * STAGE_BYTES + 2 * TILE_BYTES);
       for (int hh = 0; hh < 2; ++hh) {
-        if (!mbar_wait(&bars->st_full[hh], it & 1, err, kErrAttnWait)) { ok = false; break; }
+        if (!mbar_wait_warp(&bars->st_full[hh], it & 1, err, kErrAttnWait)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tS = tmem_base + lane_sel + hh * 128;
         const uint32_t tP = tS + 64;
@@ -236,7 +236,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_const
         mbar_arrive(&bars->pds_ready[hh]);
       }
     }
-    if (ok && warp < 6 && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait)) {
+    if (ok && warp < 6 && mbar_wait_warp(&bars->acc_done, 0, err, kErrAttnWait)) {
       tc_fence_after();
       // stage 0's Q/dO tiles are dead: 4 warps x 8 KB of staging
       uint8_t* stage = sStage + quarter * 8192;

@@ -217,7 +217,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
     const float my_lse2 = lse2[stat], my_delta = delta[stat];
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(&bars->sd_full, j & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->sd_full, j & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
       const bool diag = j == n_kv - 1;
       const uint32_t tS = tmem_base + lane_sel + (j & 1) * 128;
@@ -253,7 +253,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQK, const __grid_consta
       tc_fence_before();
       mbar_arrive(&bars->ds_ready);
     }
-    if (ok && warp < 6 && mbar_wait(&bars->dq_done, 0, err, kErrAttnWait)) {
+    if (ok && warp < 6 && mbar_wait_warp(&bars->dq_done, 0, err, kErrAttnWait)) {
       tc_fence_after();
       uint8_t* stage = sQ + quarter * 8192;   // Q is dead once the last S tile has been produced
       const uint32_t tD = tmem_base + lane_sel + 384;

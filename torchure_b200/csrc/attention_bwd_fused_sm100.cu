@@ -367,14 +367,14 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const int s = it % Q_STAGES;
       const bool diag = a.causal && ((it0 + it) % n_qb) == 0;     // query block == key block
       const float* sStat = reinterpret_cast<const float*>(sStage + s * STAGE_BYTES + 2 * TILE_BYTES);
-      if (!mbar_wait(&bars->st_full[grp], it & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->st_full[grp], it & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
       if (diag) softmax_half(sStat, true);
       else softmax_half(sStat, false);
       // dQ^T of this half (the first product the tensor core runs on it): 32 query columns of this warp, one head-dim
       // index per lane.  The tile leaves TMEM first, which releases its columns for the next block's dP^T; the 32
       // fp32 reductions follow.  The accumulator is head-major, so they differ by compile-time offsets.
-      if (!mbar_wait(&bars->dq_full[grp], it & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->dq_full[grp], it & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
       uint32_t v[32];
       tmem_ld_32x32b_x32(tH + 64, v);
@@ -390,7 +390,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int j = 0; j < 32; ++j) red_add_unordered(dst + j * HD, __uint_as_float(v[j]));
     }
     if (busy) {
-      ok = ok && mbar_wait(&bars->acc_done, 0, err, kErrAttnWait);
+      ok = ok && mbar_wait_warp(&bars->acc_done, 0, err, kErrAttnWait);
       tc_fence_after();
     }
     if (!SHARED && ok) {

@@ -215,9 +215,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     float m_used = -1e30f, l = 0.f;
     bool ok = true;
     for (int j = 0; j < n_kv; ++j) {
-      if (!mbar_wait(&bars->s_full[t], j & 1, err, kErrAttnWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&bars->s_full[t], j & 1, err, kErrAttnWait)) { ok = false; break; }
       tc_fence_after();
-      __syncwarp();
       const bool diag = a.causal && j == n_kv - 1;
       // the whole score row (128 fp32) comes out of TMEM once: four loads in flight, one wait
       uint32_t sv[128];
@@ -245,9 +244,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       } else {
         const bool need = m_new > m_used + RESCALE_THRESHOLD;
         if (__any_sync(0xffffffffu, need)) {
-          if (!mbar_wait(&bars->o_done[t], (j - 1) & 1, err, kErrAttnWait)) { ok = false; break; }
+          if (!mbar_wait_warp(&bars->o_done[t], (j - 1) & 1, err, kErrAttnWait)) { ok = false; break; }
           tc_fence_after();
-          __syncwarp();
           const float alpha = need ? fast_exp2(m_used - m_new) : 1.f;
           uint32_t v[32];
 #pragma unroll 1
@@ -297,7 +295,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       if (lane == 0) mbar_arrive(&bars->p_ready[t]);
       __syncwarp();
     }
-    if (ok && mbar_wait(&bars->o_done[t], (n_kv - 1) & 1, err, kErrAttnWait)) {
+    if (ok && mbar_wait_warp(&bars->o_done[t], (n_kv - 1) & 1, err, kErrAttnWait)) {
       tc_fence_after();
       const float inv_l = 1.f / l;
       lse[(static_cast<int64_t>(b) * Hq + h0 + t) * S + qblk * BQ + row] = (m_used + log2f(l)) * 0.6931471805599453f;

@@ -142,6 +142,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   }
   return true;
 }
+// The same for a whole warp.  The lanes leave the poll apart, and what follows a wait is mostly warp-collective (tcgen05.ld, .st and
+// .wait are .sync.aligned, shuffles, __syncwarp): the vote brings them together again, and gives all of them one verdict, so that
+// no lane goes on when another gave up.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code)) != 0;
+}
 __device__ __forceinline__ void fence_barrier_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }

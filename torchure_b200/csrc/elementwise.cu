@@ -350,7 +350,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
     const float r = r_next;
     if (row + row_step < M) r_next = rstd[row + row_step];
     // a warp whose wait expired goes on without new copies: its team meets once per row
-    ok = __all_sync(0xffffffffu, mbar_wait(&bars[team][stage], phase, err, kErrStagedRowWait) && ok);
+    ok = mbar_wait_warp(&bars[team][stage], phase, err, kErrStagedRowWait) && ok;
     const uint8_t* st = buf + stage * stage_bytes;
     const float2 r2 = make_float2(r, r);
     // pass 1: dot = mean(dh w xhat)

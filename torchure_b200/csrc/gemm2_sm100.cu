@@ -247,7 +247,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
         // In a branch of its own down to the wait: code of the other epilogues in the same loop body, never run here, cost the
         // plain bf16 store 2 - 7 % of a short product (8192 x 3072 x 64 24.3 against 22.8 us, 1536 x 6144 x 256 13.55
         // against 13.0).
-        if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
         tc_fence_after();
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
         const bool rows_live = (m0 + q * 32) < M;
@@ -255,6 +255,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 #pragma unroll 1
         for (int c = 0; c < BN / COLS; ++c) {
           uint32_t v[64];
+          __syncwarp();      // one lane stored the slab before
           if (OUT == 0) {
             tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
             tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
@@ -318,7 +319,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
           load_gu(0, std::integral_constant<int, 0>{});
           load_gu(0, std::integral_constant<int, 1>{});
         }
-        if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
+        if (!mbar_wait_warp(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
         tc_fence_after();
         const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
         const bool rows_live = (m0 + q * 32) < M;
@@ -347,6 +348,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
               uint32_t g[32], u[32];
+              __syncwarp();
               tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, g);
               tmem_ld_32x32b_x32(t_row + BNH + c * 64 + hf * 32, u);
               tmem_ld_wait();
@@ -380,6 +382,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
               uint32_t d[32];
+              __syncwarp();
               tmem_ld_32x32b_x32(t_row + c * 64 + hf * 32, d);
               tmem_ld_wait();
               if (c == BN / 64 - 1 && hf == 1) {
@@ -416,6 +419,7 @@ gemm2_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
 #pragma unroll 1
           for (int c = 0; c < BN / COLS; ++c) {
             uint32_t v[64];
+            __syncwarp();    // the lane that holds the label took longer
             tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
             tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
             tmem_ld_wait();

@@ -317,13 +317,14 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tmA, const CUtensor
       int m0, n0;
       tile_coords(tile, m0, n0);
       const int acc = it & 1;
-      if (!mbar_wait(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
+      if (!mbar_wait_warp(&tfull[acc], (it >> 1) & 1, err, kErrEpilogueTmemFullWait)) { ok = false; break; }
       tc_fence_after();
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * BN;
       const bool rows_live = (m0 + q * 32) < M;
 #pragma unroll 1
       for (int c = 0; c < BN / COLS; ++c) {
         uint32_t v[64];
+        __syncwarp();      // one lane stored the slab before
         if (OUT == 0) {
           tmem_ld_32x32b_x32(t_row + c * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
           tmem_ld_32x32b_x32(t_row + c * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));

@@ -202,7 +202,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncwarp();
   bool ok = true;
   if (warp >= 2) {
-    ok = mbar_wait(tfull, 0, err, kErrEpilogueTmemFullWait);
+    ok = mbar_wait_warp(tfull, 0, err, kErrEpilogueTmemFullWait);
     tc_fence_after();
   }
   const int q = warp & 3;                 // TMEM lane quarter an epilogue warp may read
@@ -216,6 +216,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       for (int c = 0; c < BN / COLS; ++c) {
         if (n0 + c * COLS >= N) break;
         uint32_t v[64];
+        __syncwarp();      // one lane stored the slab before
         tmem_ld_32x32b_x32(t_row + c * COLS, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
         if (OUT == 0) tmem_ld_32x32b_x32(t_row + c * COLS + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
         tmem_ld_wait();
