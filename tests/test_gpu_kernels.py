@@ -636,6 +636,28 @@ def test_linear_ce_without_gradients():
     assert w.grad is not None
 
 
+def test_linear_ce_loss_changed_in_place():
+    """The loss is a tensor of its own, as on the CPU: a script may divide or add to it before backward, or detach it."""
+    from torchure_b200.loss import fused_linear_cross_entropy
+
+    torch.manual_seed(0)
+    h = torch.randn(300, 256, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(1000, 256, device="cuda") * 0.05).bfloat16()
+    y = torch.randint(0, 1000, (300,), device="cuda")
+    plain = fused_linear_cross_entropy(h, w, y, -100, 128)
+    plain.backward()
+    grad, h.grad = h.grad, None
+    loss = fused_linear_cross_entropy(h, w, y, -100, 128)
+    loss /= 4
+    loss += 1
+    assert abs(loss.item() - plain.item() / 4 - 1) < 1e-6      # two roundings to fp32
+    loss.backward()
+    assert torch.equal(h.grad, grad / 4)                       # a power of two: exact
+    loss = fused_linear_cross_entropy(h, w, y, -100, 128)
+    loss.detach_()
+    assert not loss.requires_grad and torch.equal(loss, plain.detach())
+
+
 @pytest.mark.parametrize("rows,vocab,chunk,paths", [(1100, 50257, 512, [True, True, False]), (900, 20001, 300, [True] * 3),
                                                     (300, 1000, 128, [False] * 3)])
 def test_linear_ce_without_gradients_chunk_by_chunk(monkeypatch, rows, vocab, chunk, paths):

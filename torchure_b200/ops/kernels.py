@@ -209,9 +209,9 @@ def ce_inverse_count(labels, ignore_index, scale):
 
 def ce_mean(row_loss, inv_n):
     """0-dim fp32: sum(row_loss) * inv_n."""
-    out = new_output("ce_mean", 1, dtype=torch.float32, device=row_loss.device)
+    out = new_output("ce_mean", (), dtype=torch.float32, device=row_loss.device)     # no view: a caller may change its loss in place
     _C().ce_mean(row_loss, inv_n, out)
-    return out.view(())
+    return out
 
 
 def ce_loss_tiles(tiles, target, labels, row_loss, vocab, ignore_index):
