@@ -326,3 +326,24 @@ def test_forward_without_gradients_in_one_call(monkeypatch, B, S, layers, qk_nor
             debug.enable(False)
         assert len(calls) == n
     kernels.check_error()
+
+
+@pytest.mark.parametrize("widths", [(1096, 512, 1096), (512, 2048, 512), (640, 640, 1280)])
+@pytest.mark.parametrize("S", [128, 512])
+def test_forward_without_gradients_blocks_of_other_widths(widths, S):
+    """Blocks whose MLPs differ in width (some were pruned): the pass without gradients gives the bits of the pass with them."""
+    from torchure_b200.models import Qwen3
+    from torchure_b200.models.qwen3 import SwiGLU
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(1)
+    model = Qwen3(num_layers=3, num_heads=4, num_kv_heads=2, emb_dim=640, head_dim=128, vocab_size=1000, ffn_dim=1096)
+    for block, width in zip(model.blocks, widths):
+        block.ffn = SwiGLU(640, width)
+    model = model.cuda()
+    model.init_weights()
+    ids = torch.randint(0, 1000, (2, S), device="cuda")
+    want = model(ids, return_final_hidden=True).detach()
+    with torch.no_grad():
+        assert torch.equal(model(ids, return_final_hidden=True), want)
+    kernels.check_error()

@@ -34,13 +34,16 @@ struct Outputs {
 
 __nv_bfloat16* bf(const Tensor& t) { return reinterpret_cast<__nv_bfloat16*>(t.data_ptr()); }
 
-// The same buffers for block after block: a pass without gradients keeps none of them.  An output's next writer is a block's length
-// of kernels behind its last reader, also where launches overlap (a kernel waits for the end of the one before).
+// The same buffers for block after block of the same widths (a pruned block has others): a pass without gradients keeps none of
+// them.  An output's next writer is a block's length of kernels behind its last reader, also where launches overlap (a kernel waits
+// for the end of the one before).
 struct Reused {
   mutable std::vector<std::pair<std::string, Tensor>> kept;
   Tensor operator()(const char* name, c10::IntArrayRef size, const at::TensorOptions& options) const {
     for (const auto& k : kept)
-      if (k.first == name) return k.second;
+      if (k.first == name && k.second.sizes() == size && k.second.scalar_type() == options.dtype().toScalarType() &&
+          k.second.device() == options.device())
+        return k.second;
     kept.emplace_back(name, torch::empty(size, options));
     return kept.back().second;
   }
