@@ -636,6 +636,31 @@ def test_linear_ce_without_gradients():
     assert w.grad is not None
 
 
+@pytest.mark.parametrize("rows", [100, 300])
+def test_linear_ce_with_a_count_kept_on_the_host(rows):
+    """A normalizer on the CPU gives what the same number on the GPU gives, with and without gradients."""
+    from torchure_b200.loss import fused_linear_cross_entropy
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(0)
+    h = torch.randn(rows, 256, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(17000, 256, device="cuda") * 0.05).bfloat16()
+    y = torch.randint(0, 17000, (rows,), device="cuda")
+    want, got = [], []
+    for out, n in ((want, torch.tensor(rows // 2, device="cuda")), (got, torch.tensor(rows // 2))):
+        with torch.no_grad():
+            out.append(fused_linear_cross_entropy(h, w, y, -100, 256, 1.0, n))
+        h.grad = None
+        loss = fused_linear_cross_entropy(h, w, y, -100, 256, 1.0, n)
+        loss.backward()
+        out += [loss.detach(), h.grad]
+    kernels.check_error()
+    for a, b in zip(got, want):
+        assert a.is_cuda and torch.equal(a, b)
+    with pytest.raises(RuntimeError, match="on the GPU"):
+        kernels.ce_mean(torch.zeros(4, device="cuda"), torch.ones(1))
+
+
 def test_linear_ce_loss_changed_in_place():
     """The loss is a tensor of its own, as on the CPU: a script may divide or add to it before backward, or detach it."""
     from torchure_b200.loss import fused_linear_cross_entropy

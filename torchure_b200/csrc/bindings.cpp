@@ -216,11 +216,13 @@ void ce_loss_tiles(const torch::Tensor& tiles, const torch::Tensor& target, cons
                     row_loss.data_ptr<float>(), (int)labels.numel(), (int)V, (int)ignore_index, cur_stream());
 }
 void ce_inverse_count(const torch::Tensor& labels, torch::Tensor& inv_n, int64_t ignore_index, double scale) {
-  TORCH_CHECK(labels.is_contiguous() && labels.scalar_type() == torch::kInt64, "ce: contiguous int64 labels");
+  TORCH_CHECK(labels.is_cuda() && labels.is_contiguous() && labels.scalar_type() == torch::kInt64,
+              "ce: contiguous int64 labels on the GPU");
   tb::ce_inverse_count(labels.data_ptr<int64_t>(), labels.numel(), ignore_index, (float)scale, inv_n.data_ptr<float>(), cur_stream());
 }
 void ce_mean(const torch::Tensor& row_loss, const torch::Tensor& inv_n, torch::Tensor& loss) {
-  TORCH_CHECK(row_loss.is_contiguous(), "ce: contiguous row losses");
+  TORCH_CHECK(row_loss.is_cuda() && inv_n.is_cuda() && loss.is_cuda() && row_loss.is_contiguous(),
+              "ce: contiguous row losses, their factor and the loss on the GPU");
   tb::ce_mean(row_loss.data_ptr<float>(), row_loss.numel(), inv_n.data_ptr<float>(), loss.data_ptr<float>(), cur_stream());
 }
 void ce_row_stats(const torch::Tensor& logits, const torch::Tensor& labels, torch::Tensor& stats, int64_t vocab_lo,

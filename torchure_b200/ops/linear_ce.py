@@ -70,7 +70,7 @@ class _LinearCESm100(torch.autograd.Function):
         if normalizer is None:
             inv_n = K.ce_inverse_count(labels, ignore_index, loss_scale)
         else:
-            inv_n = (loss_scale / normalizer.float()).reshape(1)
+            inv_n = (loss_scale / normalizer.to(dev).float()).reshape(1)      # read by kernels: a count kept on the host too
         row_loss = torch.empty(N, dtype=torch.float32, device=dev)
         # under no_grad the parameter still counts as an input that needs a gradient; nothing will ever ask for it
         need_dh = want_grad and ctx.needs_input_grad[0]
