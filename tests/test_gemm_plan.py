@@ -131,3 +131,30 @@ def test_chunks_of_the_loss_head(weight):
             assert ceil_div(n, rows) <= ceil_div(n, chunk), (n, chunk, rows)
     assert _chunk_rows(4097, 4096, 1 << 28) == 2304 and _chunk_rows(1531, 600, 1 << 28) == 512
     assert _chunk_rows(1100, 1000, 1 << 20) == 1000 and _chunk_rows(8192, 4096, 1 << 28) == 4096
+
+
+def test_chunks_of_a_sharded_loss_head(monkeypatch):
+    """With the vocabulary sharded, the products and dW of a chunk cover the rank's rows only: their size decides."""
+    import torch
+
+    from torchure_b200.ops import linear_ce
+
+    class Mesh:
+        def size(self, dim):
+            return 4
+
+        def coordinate(self, dim):
+            return 1
+
+    class Seen(Exception):
+        pass
+
+    def record(rows, chunk, weight_elements):
+        raise Seen(weight_elements)
+
+    monkeypatch.setattr(linear_ce, "_chunk_rows", record)
+    h, w = torch.zeros(1100, 64, dtype=torch.bfloat16), torch.zeros(4000, 64, dtype=torch.bfloat16)
+    y, one = torch.zeros(1100, dtype=torch.int64), torch.ones(())
+    for shard, elements in ((None, 4000 * 64), ((Mesh(), "tp"), 1000 * 64)):
+        with pytest.raises(Seen, match=f"^{elements}$"):
+            linear_ce._LinearCESm100.apply(h, w, y, -100, 1000, w, None, 1.0, None, one, shard, True)

@@ -87,7 +87,7 @@ class _LinearCESm100(torch.autograd.Function):
                 d_weight[:v0].zero_()
                 d_weight[v0 + V:].zero_()
             d_weight = d_weight[v0:v0 + V]
-        chunk = _chunk_rows(N, chunk_size, V_all * D)
+        chunk = _chunk_rows(N, chunk_size, V * D)      # equal slices of the vocabulary: every rank has the same chunks
         ldl = (V + 7) // 8 * 8
         logits_buf = None       # allocated by the first chunk that keeps its logits
         target = torch.empty(chunk, dtype=torch.float32, device=dev) if not (need_dh or need_dw) else None
