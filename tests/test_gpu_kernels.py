@@ -636,6 +636,34 @@ def test_linear_ce_without_gradients():
     assert w.grad is not None
 
 
+def test_product_in_slices_without_room_for_them():
+    """A dH whose K slices do not fit the memory that is left runs in one piece."""
+    from torchure_b200 import ops
+    from torchure_b200.ops import kernels as K
+
+    M, N, V = 1000, 2560, 66000
+    kind, _, _, workspace = ops.ext().gemm_plan(M, N, V, b_mn=True, may_split=True)
+    assert kind == "slices" and workspace > 16 << 20
+    torch.manual_seed(0)
+    a, b = torch.randn(M, V, device="cuda").bfloat16(), torch.randn(V, N, device="cuda").bfloat16()
+    want, out = K.gemm(a, b, b_mn=True), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    torch.cuda.empty_cache()
+    taken = []
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (4 << 20)) / torch.cuda.mem_get_info()[1])
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:               # free blocks among what earlier tests hold
+                taken.append(torch.empty(workspace, dtype=torch.uint8, device="cuda"))
+        K.gemm(a, b, b_mn=True, out=out, may_split=True)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        del taken
+    assert torch.equal(out, want)
+    K.gemm(a, b, b_mn=True, out=out, may_split=True)      # sums of slices round elsewhere: 2^-8 of the value, and rarely
+    assert not torch.equal(out, want) and relerr(out, want) < 4e-3
+    K.check_error()
+
+
 @pytest.mark.parametrize("rows", [100, 300])
 def test_linear_ce_with_a_count_kept_on_the_host(rows):
     """A normalizer on the CPU gives what the same number on the GPU gives, with and without gradients."""

@@ -58,7 +58,18 @@ void gemm(const torch::Tensor& a, const torch::Tensor& b, torch::Tensor& out, bo
   tb::GemmPlan plan = tb::gemm_plan((int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, num_sms(), g_sm_reserve > 0, may_split, (int)splits, (int)tile_n);
   plan.b_is_old = b_is_old;
   torch::Tensor ws;
-  if (plan.workspace > 0) ws = torch::empty({(int64_t)plan.workspace}, a.options().dtype(torch::kUInt8));
+  if (plan.workspace > 0) {
+    try {
+      ws = torch::empty({(int64_t)plan.workspace}, a.options().dtype(torch::kUInt8));
+    } catch (const c10::OutOfMemoryError&) {
+      // No room for the slices' partial sums (a head's dH: up to 256 MB where a step's memory peaks): a product that runs in one
+      // piece as well is not refused for them.
+      if (splits > 0 || tile_n != 0) throw;
+      plan = tb::gemm_plan((int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, num_sms(), g_sm_reserve > 0, false, 0, 0);
+      if (plan.workspace > 0) throw;
+      plan.b_is_old = b_is_old;
+    }
+  }
   const int rc = tb::gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), (int)M, (int)N, (int)K, a.stride(0),
                                b.stride(0), out.stride(0), a_mn, b_mn, (int)out_mode, plan,
                                plan.workspace > 0 ? ws.data_ptr() : nullptr, err_word().data_ptr<int>(), num_sms(),
