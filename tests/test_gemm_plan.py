@@ -1,4 +1,4 @@
-"""The choice of a kernel for a product (``gemm_plan``), which needs no GPU."""
+"""The choice of a kernel for a product (``gemm_plan``) and other rules of the launchers, which need no GPU."""
 
 import subprocess
 import sys
@@ -158,3 +158,16 @@ def test_chunks_of_a_sharded_loss_head(monkeypatch):
     for shard, elements in ((None, 4000 * 64), ((Mesh(), "tp"), 1000 * 64)):
         with pytest.raises(Seen, match=f"^{elements}$"):
             linear_ce._LinearCESm100.apply(h, w, y, -100, 1000, w, None, 1.0, None, one, shard, True)
+
+
+@pytest.mark.parametrize("Hq,Hkv", [(2, 1), (16, 4), (16, 8), (32, 8), (6, 3)])
+@pytest.mark.parametrize("acc", [True, False])
+def test_qknorm_backward_leaves_room_for_communication(Hq, Hkv, acc):
+    """All CTAs of the persistent QK-norm backward are resident at once where communication CTAs, which take half of an SM's
+    register file, are on some SMs: such an SM has room for one.  Without them the grid fills the chip."""
+    for sms, shared in ((148, 0), (148, 16), (148, 148), (132, 16), (148, 500)):
+        cols, chunks, per_sm = _C.qknorm_rope_bwd_grid(8192, Hq, Hkv, acc, sms, shared)
+        room = sms * per_sm - min(shared, sms) * (per_sm - 1)
+        assert room - chunks < cols * chunks <= room and 2 <= per_sm <= 3
+    assert _C.qknorm_rope_bwd_grid(9, Hq, Hkv, acc, 148, 16)[0] == 2          # eight rows per CTA
+    assert _C.qknorm_rope_bwd_grid(8192, 512, 64, acc, 8, 8)[0] == 1

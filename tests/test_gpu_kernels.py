@@ -1082,3 +1082,24 @@ def test_repeat_runs_are_bitwise_stable_under_poison():
     finally:
         debug.enable(False)
     K.check_error()
+
+
+@pytest.mark.parametrize("shared_sms", [0, 16, 148, 1000])
+def test_qknorm_rope_bwd_beside_communication(shared_sms):
+    """Fewer CTAs, more rows for each: the same gradients (the gains' partials are added in another order)."""
+    from torchure_b200.models.qwen3 import RotaryEmbedding
+    from torchure_b200.ops import kernels
+
+    torch.manual_seed(4)
+    M, Hq, Hkv, hd = 3001, 16, 8, 128
+    qkv, g = (torch.randn(M, (Hq + 2 * Hkv) * hd, device="cuda").bfloat16() for _ in range(2))
+    w = torch.rand(hd, device="cuda") + 0.5
+    cos, sin = RotaryEmbedding(hd).tables(M, "cuda")
+    outs = []
+    for shared in (0, shared_sms):
+        d, dq, dk = g.clone(), torch.zeros(hd, device="cuda"), torch.zeros(hd, device="cuda")
+        kernels.qknorm_rope_bwd_(d, qkv, w, w, cos, sin, dq, dk, M, Hq, Hkv, 1e-6, shared_sms=shared)
+        outs.append((d, dq, dk))
+    assert torch.equal(outs[0][0], outs[1][0])
+    # 48000 and 24000 terms in fp32, about 2^-24 x sqrt(terms) of their size
+    assert relerr(outs[1][1], outs[0][1]) < 1e-4 and relerr(outs[1][2], outs[0][2]) < 1e-4

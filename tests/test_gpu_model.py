@@ -347,3 +347,41 @@ def test_forward_without_gradients_blocks_of_other_widths(widths, S):
     with torch.no_grad():
         assert torch.equal(model(ids, return_final_hidden=True), want)
     kernels.check_error()
+
+
+@pytest.mark.parametrize("world,comm_sms", [(1, 16), (2, 16), (8, 40)])
+def test_qknorm_backward_is_told_of_communication_ctas(monkeypatch, world, comm_sms):
+    """With a gradient sink whose collectives run under the backward pass the QK-norm kernel gets the number of SMs they are
+    on, and gives the same gradients."""
+    from torchure_b200.ops import kernels
+
+    class Sink:
+        def __init__(self, params):
+            self.world, self.comm_sms = world, comm_sms
+            flat = torch.zeros(sum(p.numel() for p in params), device="cuda")
+            self.grads = {p: v.view_as(p) for p, v in zip(params, flat.split([p.numel() for p in params]))}
+
+        def grad_dest(self, p):
+            return self.grads[p], False
+
+        def grad_written(self, p):
+            pass
+
+    told = []
+    plain = kernels.qknorm_rope_bwd_
+    monkeypatch.setattr(kernels, "qknorm_rope_bwd_", lambda *a, **k: told.append(k["shared_sms"]) or plain(*a, **k))
+    model, _ = _pair(seed=5)
+    ids = torch.randint(0, CFG["vocab_size"], (2, 256), device="cuda")
+    g = torch.randn(2, 256, CFG["emb_dim"], device="cuda").bfloat16()
+    model(ids, return_final_hidden=True).backward(g)
+    want = {n: p.grad for n, p in model.named_parameters()}
+    model.zero_grad(set_to_none=True)
+    sink = Sink(list(model.parameters()))
+    model.set_grad_sink(sink)
+    model(ids, return_final_hidden=True).backward(g)
+    kernels.check_error()
+    assert told == ([] if world == 1 else [comm_sms] * CFG["num_layers"])      # one rank: native calls
+    for n, p in model.named_parameters():
+        if p.dim() == 1 or "proj" in n:
+            # gradients behind attention's fp32 additions, whose order differs from run to run
+            assert relerr(sink.grads[p], want[n]) < 1e-2, n

@@ -79,10 +79,16 @@ void qknorm_rope_fwd(const __nv_bfloat16* qkv, const float* qw, const float* kw,
                      cudaStream_t stream);
 // in place on the q/k column ranges of dqkv [M, (Hq+2Hkv)*hd]; dqw/dkw fp32 [hd] accumulate.  dq_acc (optional):
 // head-major fp32 [B, Hq, S, hd] holding dq instead of the q columns of dqkv (they are only written then).
-// Returns 0, or a negative code when the launch failed.
+// Returns 0, or a negative code when the launch failed.  shared_sms: SMs that CTAs of a communication kernel are on meanwhile.
 int qknorm_rope_bwd(__nv_bfloat16* dqkv, const __nv_bfloat16* qkv, const float* qw, const float* kw, const float* cos,
                     const float* sin, float* dqw, float* dkw, const float* dq_acc, int M, int S, int Hq, int Hkv, int hd,
-                    float eps, int use_norm, int num_sms, cudaStream_t stream, int force_pairs = 0);
+                    float eps, int use_norm, int num_sms, cudaStream_t stream, int shared_sms = 0, int force_pairs = 0);
+struct QkBwdGrid {
+  int pairs;            // head pairs of a warp
+  int chunks, cols;     // chunks of heads, CTAs that share the rows of each
+  int per_sm;           // CTAs of this variant that an SM holds
+};
+QkBwdGrid qknorm_rope_bwd_grid(int M, int Hq, int Hkv, bool acc, int num_sms, int shared_sms, int force_pairs = 0);
 void swiglu_fwd(const __nv_bfloat16* gu, __nv_bfloat16* act, int M, int F, cudaStream_t stream);
 void swiglu_bwd(const __nv_bfloat16* dact, const __nv_bfloat16* gu, __nv_bfloat16* dgu, int M, int F,
                 cudaStream_t stream);

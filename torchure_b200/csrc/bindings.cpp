@@ -24,6 +24,9 @@ int num_sms() {
   return usable > 8 ? usable : 8;
 }
 
+// of `n` SMs with a communication CTA those that compute kernels may use as well
+int unreserved_sms(int64_t n) { return n > g_sm_reserve ? (int)n - g_sm_reserve : 0; }
+
 // one error word per process (one process drives one GPU)
 torch::Tensor& err_word() {
   static torch::Tensor t;
@@ -177,7 +180,7 @@ void qknorm_rope_fwd(const torch::Tensor& qkv, const torch::Tensor& qw, const to
 void qknorm_rope_bwd(torch::Tensor& dqkv, const torch::Tensor& qkv, const torch::Tensor& qw, const torch::Tensor& kw,
                      const torch::Tensor& cos, const torch::Tensor& sin, torch::Tensor& dqw, torch::Tensor& dkw,
                      int64_t S, int64_t Hq, int64_t Hkv, double eps, bool use_norm,
-                     c10::optional<torch::Tensor> dq_acc, int64_t variant) {
+                     c10::optional<torch::Tensor> dq_acc, int64_t variant, int64_t shared_sms) {
   TORCH_CHECK(qkv.size(1) == (Hq + 2 * Hkv) * 128, "qknorm_rope: head_dim must be 128");
   if (dq_acc.has_value() && dq_acc->defined())
     TORCH_CHECK(dq_acc->scalar_type() == torch::kFloat32 && dq_acc->is_contiguous() &&
@@ -194,7 +197,8 @@ void qknorm_rope_bwd(torch::Tensor& dqkv, const torch::Tensor& qkv, const torch:
   const int rc = tb::qknorm_rope_bwd(bfm(dqkv), bf(qkv), qw.data_ptr<float>(), kw.data_ptr<float>(),
                                      cos.data_ptr<float>(), sin.data_ptr<float>(), dqw.data_ptr<float>(),
                                      dkw.data_ptr<float>(), opt_ptr<float>(dq_acc), (int)qkv.size(0), (int)S, (int)Hq,
-                                     (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, num_sms(), cur_stream(), 2 * (int)variant);
+                                     (int)Hkv, 128, (float)eps, use_norm ? 1 : 0, num_sms(), cur_stream(), unreserved_sms(shared_sms),
+                                     2 * (int)variant);
   TORCH_CHECK(rc == 0, "qknorm_rope_bwd failed with code ", rc);
 }
 
@@ -407,7 +411,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qknorm_rope_bwd", &qknorm_rope_bwd, pybind11::arg("dqkv"), pybind11::arg("qkv"), pybind11::arg("qw"),
         pybind11::arg("kw"), pybind11::arg("cos"), pybind11::arg("sin"), pybind11::arg("dqw"), pybind11::arg("dkw"),
         pybind11::arg("S"), pybind11::arg("Hq"), pybind11::arg("Hkv"), pybind11::arg("eps"), pybind11::arg("use_norm"),
-        pybind11::arg("dq_acc") = c10::nullopt, pybind11::arg("variant") = 0);
+        pybind11::arg("dq_acc") = c10::nullopt, pybind11::arg("variant") = 0, pybind11::arg("shared_sms") = 0);
+  m.def("qknorm_rope_bwd_grid", [](int M, int Hq, int Hkv, bool acc, int num_sms, int shared_sms) {
+    const tb::QkBwdGrid g = tb::qknorm_rope_bwd_grid(M, Hq, Hkv, acc, num_sms, shared_sms);
+    return std::make_tuple(g.cols, g.chunks, g.per_sm);
+  }, "CTAs per chunk of heads, chunks, CTAs that an SM holds");
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("embedding_bwd", &embedding_bwd);

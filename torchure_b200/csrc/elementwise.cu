@@ -1227,22 +1227,36 @@ void qknorm_rope_fwd(const __nv_bfloat16* qkv, const float* qw, const float* kw,
     launch_pdl(qknorm_rope_fwd_kernel<false>, grid, dim3(256), 0, stream, qkv, qw, kw, cos, sin, out, M, S, Hq, Hkv, eps, use_norm);
 }
 
+// The CTAs are persistent: as many as are resident at once, each with its share of the rows.  An SM that also hosts a CTA of a
+// gradient all-reduce (512 threads of 64 registers, half of the register file) has room for one of these; a grid that counts on
+// two or three leaves the others waiting for a first one to end, with a whole share still to do.  Measured on B200 with a kernel of that
+// footprint on 16 SMs in the place of the all-reduce, all SMs counted as free, those 16 counted as one CTA each, us: 8192 rows of 16 + 8
+// heads, dq in the accumulator 60, 52, in bf16 53, 41; of 16 + 4 52, 46; 4096 of 32 + 8 52, 49.  With nothing beside it the smaller grid
+// costs up to 2 us.  Several GPUs were not measured.
+QkBwdGrid qknorm_rope_bwd_grid(int M, int Hq, int Hkv, bool acc, int num_sms, int shared_sms, int force_pairs) {
+  QkBwdGrid g;
+  // four head pairs in flight where that leaves none idle and dq comes from the accumulator
+  g.pairs = force_pairs > 0 ? force_pairs : (acc && Hq % 8 == 0 && Hkv % 8 == 0 ? 4 : 2);
+  const int per = 2 * g.pairs;
+  g.chunks = (Hq + per - 1) / per + (Hkv + per - 1) / per;
+  g.per_sm = g.pairs == 4 ? 2 : 3;
+  const int ctas = num_sms * g.per_sm - std::min(std::max(shared_sms, 0), num_sms) * (g.per_sm - 1);
+  g.cols = std::max(1, std::min((M + 7) / 8, ctas / g.chunks));
+  return g;
+}
+
 int qknorm_rope_bwd(__nv_bfloat16* dqkv, const __nv_bfloat16* qkv, const float* qw, const float* kw, const float* cos,
                     const float* sin, float* dqw, float* dkw, const float* dq_acc, int M, int S, int Hq, int Hkv, int hd,
-                    float eps, int use_norm, int num_sms, cudaStream_t stream, int force_pairs) {
+                    float eps, int use_norm, int num_sms, cudaStream_t stream, int shared_sms, int force_pairs) {
   (void)hd;
-  // four head pairs in flight where that leaves none idle and dq comes from the accumulator
-  const int pairs = force_pairs > 0 ? force_pairs : (dq_acc != nullptr && Hq % 8 == 0 && Hkv % 8 == 0 ? 4 : 2);
-  const int per = 2 * pairs, chunks = (Hq + per - 1) / per + (Hkv + per - 1) / per;
-  auto go = [&](auto kern) {
-    const int ctas = num_sms * (pairs == 4 ? 2 : 3);               // resident at once
-    const int cols = std::max(1, std::min((M + 7) / 8, ctas / chunks));
-    return launch_pdl(kern, dim3(cols, chunks), dim3(256), 0, stream, dqkv, qkv, qw, kw, cos, sin, dqw, dkw, dq_acc, M, S, Hq, Hkv,
-                      eps, use_norm);
-  };
   const bool acc = dq_acc != nullptr;
-  const cudaError_t rc = pairs == 4 ? (acc ? go(qknorm_rope_bwd_kernel<true, 4>) : go(qknorm_rope_bwd_kernel<false, 4>))
-                                    : (acc ? go(qknorm_rope_bwd_kernel<true, 2>) : go(qknorm_rope_bwd_kernel<false, 2>));
+  const QkBwdGrid g = qknorm_rope_bwd_grid(M, Hq, Hkv, acc, num_sms, shared_sms, force_pairs);
+  auto go = [&](auto kern) {
+    return launch_pdl(kern, dim3(g.cols, g.chunks), dim3(256), 0, stream, dqkv, qkv, qw, kw, cos, sin, dqw, dkw, dq_acc, M, S, Hq,
+                      Hkv, eps, use_norm);
+  };
+  const cudaError_t rc = g.pairs == 4 ? (acc ? go(qknorm_rope_bwd_kernel<true, 4>) : go(qknorm_rope_bwd_kernel<false, 4>))
+                                      : (acc ? go(qknorm_rope_bwd_kernel<true, 2>) : go(qknorm_rope_bwd_kernel<false, 2>));
   return rc == cudaSuccess ? 0 : -3;
 }
 

@@ -363,7 +363,10 @@ class _BlockFn(torch.autograd.Function):
                 dqn.add_(part[0])
                 dkn.add_(part[1])
             else:
-                K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, dqn, dkn, S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc)
+                # buckets that are reduced under the backward pass have CTAs on these SMs
+                shared = getattr(out.sink, "comm_sms", 0) if getattr(out.sink, "world", 1) > 1 else 0
+                K.qknorm_rope_bwd_(dqkv, qkv, qn, kn, cos, sin, dqn, dkn, S, Hq, Hkv, eps, use_norm, dq_acc=dq_acc,
+                                   shared_sms=shared)
             del dq_acc
             if use_norm:
                 out.done(P["qn"])

@@ -117,10 +117,11 @@ def qknorm_rope(qkv, qw, kw, cos, sin, S, Hq, Hkv, eps, use_norm=True):
     return out
 
 
-def qknorm_rope_bwd_(dqkv, qkv, qw, kw, cos, sin, dqw, dkw, S, Hq, Hkv, eps, use_norm=True, dq_acc=None):
+def qknorm_rope_bwd_(dqkv, qkv, qw, kw, cos, sin, dqw, dkw, S, Hq, Hkv, eps, use_norm=True, dq_acc=None, shared_sms=0):
     """In place on the q / k columns of dqkv.  `dq_acc` (fp32 [B, Hq, S, 128]): dq is read from there instead of the
-    q columns (what the single-pass attention backward leaves behind), saving its conversion pass."""
-    _C().qknorm_rope_bwd(dqkv, qkv, qw, kw, cos, sin, dqw, dkw, S, Hq, Hkv, eps, use_norm, dq_acc)
+    q columns (what the single-pass attention backward leaves behind), saving its conversion pass.  `shared_sms`: SMs that
+    CTAs of a communication kernel may be on meanwhile."""
+    _C().qknorm_rope_bwd(dqkv, qkv, qw, kw, cos, sin, dqw, dkw, S, Hq, Hkv, eps, use_norm, dq_acc, 0, shared_sms)
     ops.count_launch()
     return dqkv
 
