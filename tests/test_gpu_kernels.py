@@ -1103,3 +1103,12 @@ def test_qknorm_rope_bwd_beside_communication(shared_sms):
     assert torch.equal(outs[0][0], outs[1][0])
     # 48000 and 24000 terms in fp32, about 2^-24 x sqrt(terms) of their size
     assert relerr(outs[1][1], outs[0][1]) < 1e-4 and relerr(outs[1][2], outs[0][2]) < 1e-4
+
+
+@pytest.mark.parametrize("variant", [-1, 3])
+def test_qknorm_rope_bwd_refuses_variants_it_does_not_have(variant):
+    from torchure_b200 import ops
+
+    t, w, table = torch.zeros(8, 512, device="cuda").bfloat16(), torch.ones(128, device="cuda"), torch.ones(8, 128, device="cuda")
+    with pytest.raises(RuntimeError, match="variant"):
+        ops.ext().qknorm_rope_bwd(t, t.clone(), w, w, table, table, w.clone(), w.clone(), 8, 2, 1, 1e-6, True, None, variant)

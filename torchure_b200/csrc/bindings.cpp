@@ -182,6 +182,7 @@ void qknorm_rope_bwd(torch::Tensor& dqkv, const torch::Tensor& qkv, const torch:
                      int64_t S, int64_t Hq, int64_t Hkv, double eps, bool use_norm,
                      c10::optional<torch::Tensor> dq_acc, int64_t variant, int64_t shared_sms) {
   TORCH_CHECK(qkv.size(1) == (Hq + 2 * Hkv) * 128, "qknorm_rope: head_dim must be 128");
+  TORCH_CHECK(variant >= 0 && variant <= 2, "qknorm_rope_bwd: variant 0 (the rule's), 1 or 2");
   if (dq_acc.has_value() && dq_acc->defined())
     TORCH_CHECK(dq_acc->scalar_type() == torch::kFloat32 && dq_acc->is_contiguous() &&
                     dq_acc->numel() == qkv.size(0) * Hq * 128,
