@@ -35,6 +35,7 @@
 // `causal`: query block qb sees key blocks <= qb (Sq == Skv); otherwise every query sees every key (the off-diagonal
 // steps of ring attention).  Because partial dQ tiles are added in whatever order CTAs finish, dQ is not bitwise
 // reproducible from run to run; the two-kernel backward (attention_bwd_dq/dkv) is.
+#include "api.h"
 #include "attn_api.h"
 #include "common.cuh"
 
@@ -572,15 +573,21 @@ int attn_bwd_stats(const void* d_o, const void* o, const float* lse, float* nds,
              : -21;
 }
 
+// CTA pairs that run at once on the SMs that are not reserved for communication
+static int sm_pairs(int num_sms) {
+  const int capacity = gemm_pair_capacity();
+  return capacity > 0 && capacity < num_sms / 2 ? capacity : num_sms / 2;
+}
+
 // CTAs per key block, from a model of the kernel's time fitted on B200: 7 us + 2.7 us per iteration of the longest block, + 4 us
-// for the exchange in a cluster of two, 7.5 in one of four.  All clusters have to run at once (74 pairs; fours leave SMs of a
-// GPC over).  Clusters of eight cost 20 us and more: sixteen of them did not fit at once.
-static int bwd_parts(int tiles, int longest) {
+// for the exchange in a cluster of two, 7.5 in one of four.  All clusters have to run at once (on 148 SMs 74 pairs; fours leave SMs of
+// a GPC over, 32 are sure to).  Clusters of eight cost 20 us and more: sixteen of them did not fit at once.
+int attn_bwd_parts(int tiles, int longest, int num_sms) {
   const float one = 2.7f * longest, two = 2.7f * ((longest + 1) / 2) + 4.f, four = 2.7f * ((longest + 3) / 4) + 7.5f;
   int parts = 1;
   float best = one;
-  if (tiles <= 74 && two < best) { parts = 2; best = two; }
-  if (tiles <= 32 && four < best) parts = 4;
+  if (tiles <= sm_pairs(num_sms) && two < best) { parts = 2; best = two; }
+  if (tiles <= num_sms * 32 / 148 && four < best) parts = 4;
   return parts;
 }
 
@@ -590,7 +597,7 @@ static int bwd_parts(int tiles, int longest) {
 // shares add up, and the last tile sticks out by half its time.  Measured, us, without and with pairs: taken 4096 tokens x 2, 16 / 8
 // heads 362, 291; 16384, 16 / 8 2633, 2102; 2048, 16 / 8 100, 75; 8 x 512 49.1, 45.4; 8 x 256 21.3, 18.4; 8 x 640 68.0, 66.4;
 // left 1024, 16 / 8 35.4 (shared by two), 41.1; 4096, 8 / 2 183, 251; 8 x 384 35.3, 36.0; 2 x 512 24.6, 25.4.
-bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal) {
+bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal, int num_sms) {
   const int nqb = Sq / 128, nkb = Skv / 128, ratio = Hq / Hkv;
   const int64_t groups = static_cast<int64_t>(B) * Hkv;
   if (nkb < 2) return false;
@@ -607,10 +614,10 @@ bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal) {
     const float all = (fixed * tiles + each * iters) * groups / slots;
     return std::max(fixed + each * longest, tiles * groups > slots ? all + 0.5f * (fixed + each * last) : all);
   };
-  const float t_two = wave(10.8f, 1.9f, pairs, two, last_two, 74);
-  const int parts = bwd_parts(static_cast<int>(nkb * groups), nqb * ratio);
+  const float t_two = wave(10.8f, 1.9f, pairs, two, last_two, sm_pairs(num_sms));
+  const int parts = attn_bwd_parts(static_cast<int>(nkb * groups), nqb * ratio, num_sms);
   if (parts > 1) return t_two < 9.f + 2.7f * ((nqb * ratio + parts - 1) / parts) + (parts == 2 ? 4.f : 7.5f);
-  return t_two < wave(10.5f, 2.7f, nkb, one, last_one, 148);
+  return t_two < wave(10.5f, 2.7f, nkb, one, last_one, num_sms);
 }
 
 int attn_bwd_2cta(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc, void* dk,
@@ -619,7 +626,7 @@ int attn_bwd_2cta(const AttnOperand& q, const AttnOperand& k, const AttnOperand&
 
 int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc,
                    void* dk, void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv,
-                   int Hq, int Hkv, bool causal, int* err, cudaStream_t stream, const AttnPairLayout* lay) {
+                   int Hq, int Hkv, bool causal, int num_sms, int* err, cudaStream_t stream, const AttnPairLayout* lay) {
   if (Sq % 128 != 0 || Skv % 128 != 0 || Hq % Hkv != 0 || B <= 0 || Sq <= 0 || Skv <= 0) return -1;
   AttnPairLayout whole{static_cast<int64_t>(B) * Sq, Sq, 0, static_cast<int64_t>(B) * Skv, Skv, 0, Sq, 0};
   if (lay == nullptr) lay = &whole;
@@ -628,8 +635,8 @@ int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand
       (reinterpret_cast<uintptr_t>(dq_acc) & 15))
     return -3;
   const int tiles = (Skv / 128) * B * Hkv;
-  const int parts = bwd_parts(tiles, (Sq / 128) * (Hq / Hkv));
-  if (attn_bwd_on_pairs(B, Sq, Skv, Hq, Hkv, causal))
+  const int parts = attn_bwd_parts(tiles, (Sq / 128) * (Hq / Hkv), num_sms);
+  if (attn_bwd_on_pairs(B, Sq, Skv, Hq, Hkv, causal, num_sms))
     return attn_bwd_2cta(q, k, v, d_o, dq_acc, dk, dv, ld_dkv, nds, nlse2, B, Sq, Skv, Hq, Hkv, causal, err, stream, *lay);
   const uint64_t Mq = static_cast<uint64_t>(lay->q_rows), Mk = static_cast<uint64_t>(lay->kv_rows);
   CUtensorMap tq, tk, tv, tdo;

@@ -65,8 +65,9 @@ int attn_bwd_stats(const void* d_o, const void* o, const float* lse, float* nds,
                    int S, int Hq, cudaStream_t stream);
 int attn_bwd_fused(const AttnOperand& q, const AttnOperand& k, const AttnOperand& v, const void* d_o, float* dq_acc,
                    void* dk, void* dv, int64_t ld_dkv, const float* nds, const float* nlse2, int B, int Sq, int Skv,
-                   int Hq, int Hkv, bool causal, int* err, cudaStream_t stream, const AttnPairLayout* lay = nullptr);
-bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal);
+                   int Hq, int Hkv, bool causal, int num_sms, int* err, cudaStream_t stream, const AttnPairLayout* lay = nullptr);
+bool attn_bwd_on_pairs(int B, int Sq, int Skv, int Hq, int Hkv, bool causal, int num_sms);
+int attn_bwd_parts(int key_blocks, int longest, int num_sms);     // CTAs that share one, where single CTAs take the call
 // dst[(b S + s), 128 h + d] (bf16, row stride ld_dst elements) = dq_acc[b, h, s, d]
 int attn_dq_convert(const float* dq_acc, void* dst, int64_t ld_dst, int B, int S, int Hq, cudaStream_t stream);
 

@@ -6,8 +6,7 @@
 #include <cuda_bf16.h>
 
 #include "attn_api.h"
-
-torch::Tensor attn_err_word();
+#include "bind_common.h"
 
 namespace {
 void check_whole(const torch::Tensor& q, const torch::Tensor& k, const torch::Tensor& v, int64_t B, int64_t Sq, int64_t Skv,
@@ -48,9 +47,11 @@ void register_attn(pybind11::module_& m) {
                           (int)Hq, (int)Hkv, err, stream);
     TORCH_CHECK(rc == 0, "attn_bwd_dkv failed with code ", rc);
   });
-  m.def("attn_bwd_on_pairs", [](int64_t B, int64_t Sq, int64_t Skv, int64_t Hq, int64_t Hkv, bool causal) {
-    return tb::attn_bwd_on_pairs((int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal);
-  });
+  m.def("attn_bwd_on_pairs", [](int64_t B, int64_t Sq, int64_t Skv, int64_t Hq, int64_t Hkv, bool causal, int num_sms) {
+    return tb::attn_bwd_on_pairs((int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, num_sms);
+  }, pybind11::arg("B"), pybind11::arg("Sq"), pybind11::arg("Skv"), pybind11::arg("Hq"), pybind11::arg("Hkv"),
+     pybind11::arg("causal"), pybind11::arg("num_sms") = 148);
+  m.def("attn_bwd_parts", &tb::attn_bwd_parts, pybind11::arg("key_blocks"), pybind11::arg("longest"), pybind11::arg("num_sms") = 148);
   // single-pass backward: statistics (+ accumulator clear), fused kernel, conversion of dQ to bf16
   m.def("attn_bwd_fused", [](const torch::Tensor& d_o, const torch::Tensor& qk, const torch::Tensor& qkv,
                              const torch::Tensor& o, const torch::Tensor& lse, torch::Tensor& dqkv, int64_t B, int64_t S,
@@ -70,7 +71,7 @@ void register_attn(pybind11::module_& m) {
     auto* out = reinterpret_cast<__nv_bfloat16*>(dqkv.data_ptr());
     rc = tb::attn_bwd_fused({qk.data_ptr(), wqk, 0}, {qk.data_ptr(), wqk, Hq * 128}, {qkv.data_ptr(), wqkv, (Hq + Hkv) * 128},
                             d_o.data_ptr(), dq_acc.data_ptr<float>(), out + Hq * 128, out + (Hq + Hkv) * 128, wqkv, nds,
-                            nlse2, (int)B, (int)S, (int)S, (int)Hq, (int)Hkv, true, err, stream);
+                            nlse2, (int)B, (int)S, (int)S, (int)Hq, (int)Hkv, true, bind_num_sms(), err, stream);
     TORCH_CHECK(rc == 0, "attn_bwd_fused failed with code ", rc);
     // convert_dq = false leaves dq in the returned head-major fp32 accumulator for a consumer that reads it there
     // (the QK-norm / RoPE backward); the q columns of dqkv are not written then
@@ -142,7 +143,7 @@ void register_attn(pybind11::module_& m) {
     const int rc = tb::attn_bwd_fused({q.data_ptr(), q.stride(0), q_col0}, {k.data_ptr(), k.stride(0), k_col0},
                                       {v.data_ptr(), v.stride(0), v_col0}, d_o.data_ptr(), dq_acc.data_ptr<float>(),
                                       dk.data_ptr(), dv.data_ptr(), Hkv * 128, nds.data_ptr<float>(),
-                                      nlse2.data_ptr<float>(), (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal,
+                                      nlse2.data_ptr<float>(), (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, bind_num_sms(),
                                       attn_err_word().data_ptr<int>(), at::cuda::getCurrentCUDAStream().stream(), &lay);
     TORCH_CHECK(rc == 0, "attn_bwd_pair failed with code ", rc);
   });
@@ -181,7 +182,8 @@ void register_attn(pybind11::module_& m) {
     TORCH_CHECK(rc == 0, "attn_bwd_stats failed with code ", rc);
     rc = tb::attn_bwd_fused({q.data_ptr(), Hq * 128, 0}, {k.data_ptr(), Hkv * 128, 0}, {v.data_ptr(), Hkv * 128, 0},
                             d_o.data_ptr(), dq_acc.data_ptr<float>(), dk.data_ptr(), dv.data_ptr(), Hkv * 128, nds, nlse2,
-                            (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, attn_err_word().data_ptr<int>(), stream);
+                            (int)B, (int)Sq, (int)Skv, (int)Hq, (int)Hkv, causal, bind_num_sms(),
+                            attn_err_word().data_ptr<int>(), stream);
     TORCH_CHECK(rc == 0, "attn_bwd_fused failed with code ", rc);
     rc = tb::attn_dq_convert(dq_acc.data_ptr<float>(), dq.data_ptr(), Hq * 128, (int)B, (int)Sq, (int)Hq, stream);
     TORCH_CHECK(rc == 0, "dq conversion failed with code ", rc);

@@ -230,7 +230,7 @@ std::tuple<Tensor, c10::optional<Tensor>, int64_t> block_backward_attn(
   const int64_t wqk = (Hq + Hkv) * 128;
   rc = tb::attn_bwd_fused({qk.data_ptr(), wqk, 0}, {qk.data_ptr(), wqk, Hq * 128}, {qkv.data_ptr(), nqkv, (Hq + Hkv) * 128},
                           d_o.data_ptr(), dq_acc.data_ptr<float>(), bf(dqkv) + Hq * 128, bf(dqkv) + (Hq + Hkv) * 128, nqkv,
-                          nds, nlse2, (int)B, (int)S, (int)S, (int)Hq, (int)Hkv, true, err, stream);
+                          nds, nlse2, (int)B, (int)S, (int)S, (int)Hq, (int)Hkv, true, bind_num_sms(), err, stream);
   TORCH_CHECK(rc == 0, "attn_bwd_fused failed with code ", rc);
   d_o = Tensor();
   rc = tb::qknorm_rope_bwd(bf(dqkv), bf(qkv), qn.data_ptr<float>(), kn.data_ptr<float>(), cos.data_ptr<float>(),
