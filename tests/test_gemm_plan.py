@@ -187,3 +187,14 @@ def test_attention_backward_counts_the_sms_it_has():
             parts = _C.attn_bwd_parts(tiles, 40, sms)
             assert parts in (1, 2, 4) and (parts == 1 or tiles * parts <= sms)
     assert [_C.attn_bwd_parts(t, 40, 148) for t in (32, 33, 74, 75)] == [4, 2, 2, 1]
+
+
+def test_chunks_that_are_said_to_change():
+    """The shapes whose times the rule quotes: it changes those that it is said to speed up, and no others."""
+    from torchure_b200.ops.linear_ce import _chunk_rows
+
+    for rows, dim, vocab, chunk, got in ((4224, 1024, 151936, 4096, 2304), (4224, 2048, 128256, 4096, 2304), (4097, 512, 50257, 4096, 2304),
+                                         (1531, 512, 50257, 600, 512), (5000, 1024, 100000, 4096, 2560)):
+        assert _chunk_rows(rows, chunk, dim * vocab) == got < min(chunk, rows)
+    for rows, dim, vocab, chunk in ((3500, 512, 20000, 512), (3000, 2048, 60000, 1000), (1100, 512, 30000, 1000)):
+        assert _chunk_rows(rows, chunk, dim * vocab) == chunk

@@ -1,6 +1,6 @@
 """Chunked fused linear + cross-entropy on sm_100a kernels.
 
-Per chunk of at most ``chunk_size`` rows (reference algorithm: ``torchure/loss/fused_linear_ce.py:31-93``):
+Per chunk of at most ``chunk_size`` rows (``_chunk_rows``; reference algorithm: ``torchure/loss/fused_linear_ce.py:31-93``):
 
 1. ``logits = h_chunk @ W^T``         tcgen05 GEMM, bf16 out (the only (chunk, V) buffer, reused by every chunk)
 2. ``ce_softmax_grad``                one kernel: online max/sum, target gather, per-row loss and, in place,
@@ -32,13 +32,16 @@ BF16 = torch.bfloat16
 
 
 def _chunk_rows(N: int, chunk_size: int, weight_elements: int) -> int:
-    """Rows per chunk: as many chunks as ``chunk_size`` asks for, of about equal size and in whole 256-row tiles of the products.
+    """Rows per chunk: as many chunks as ``chunk_size`` asks for, of about equal size, in whole 256-row tiles of the products where
+    such a size is no larger than ``chunk_size`` (3000 rows in chunks of at most 1000 stay three of 1000).
 
     A short last chunk costs nearly what a whole one does, since dW is read and written for it, and ragged ones run tiles that are
-    partly empty.  Measured on B200, loss head forward and backward, rows x dim x vocabulary (chunk size), last chunk short -> equal
-    ones, us: 4224 x 1024 x 151936 (4096) 3948 -> 3702; 4097 x 512 x 50257 (4096) 1085 -> 935; 3500 x 512 x 20000 (512) 800 -> 745;
-    3000 x 2048 x 60000 (1000) 2544 -> 2291; 5000 x 1024 x 100000 (4096) 3255 -> 3086.  A last chunk of at most 128 rows, which has
-    a kernel of its own, stays where dW fits the cache (64 MB): 1100 x 512 x 30000 (1000) 368, 389 in equal ones.
+    partly empty.  Measured on B200 with only this rule switched, loss head forward and backward, rows x dim x vocabulary (chunk
+    size), ``chunk_size`` as it is -> this rule, medians of two runs in us: 4224 x 1024 x 151936 (4096) 4053 -> 3790, 4216 -> 3913;
+    4224 x 2048 x 128256 (4096) 6630 -> 5934, 6602 -> 5881; 4097 x 512 x 50257 (4096) 1317 -> 1171, 1096 -> 912; 1531 x 512 x 50257
+    (600) 807 -> 760, 745 -> 704; 5000 x 1024 x 100000 (4096), whose last chunk is not that short, 3135 -> 3112, 3416 -> 3262, within
+    their spread.  A last chunk of at most 128 rows, which has a kernel of its own, stays where dW (``weight_elements``, this rank's
+    in a sharded head) fits the cache (64 MB): 1100 x 512 x 30000 (1000) 252, 258 in equal ones.
     """
     if N <= 0 or chunk_size <= 0:       # refused by the loop over the chunks
         return min(chunk_size, N)
