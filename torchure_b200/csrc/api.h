@@ -106,10 +106,10 @@ void ce_softmax_grad(__nv_bfloat16* logits, int64_t ldl, const int64_t* labels, 
 // row_loss alone, the logits stay as they are
 void ce_loss(const __nv_bfloat16* logits, int64_t ldl, const int64_t* labels, float* row_loss, int C, int V,
              int ignore_index, cudaStream_t stream);
-// row_loss from what gemm2_ce left
 // inv_n[0] = scale / max(1, labels other than ignore_index);  loss[0] = sum(row_loss) * inv_n[0]
 void ce_inverse_count(const int64_t* labels, int64_t n, int64_t ignore_index, float scale, float* inv_n, cudaStream_t stream);
 void ce_mean(const float* row_loss, int64_t n, const float* inv_n, float* loss, cudaStream_t stream);
+// row_loss from what gemm2_ce left
 void ce_loss_tiles(const float* tiles, const float* target, const int64_t* labels, float* row_loss, int C, int V,
                    int ignore_index, cudaStream_t stream);
 // ce_softmax_grad for a vocabulary sharded over ranks (this rank's logits hold columns [vocab_lo, vocab_lo + V)):

@@ -630,10 +630,13 @@ GemmPlan gemm_plan(int M, int N, int K, bool a_mn, bool b_mn, int out_mode, int 
     }
   }
   // ... or where they leave a good part of the waves empty and K is a vocabulary: s times as many units fill them better.  The
-  // slices' partial sums cost their traffic, and 256 MB at most; and since full waves run into the power cap, at 1420 TFLOP/s, it
-  // pays only where the model promises 15 %.  Measured on B200, dH of a head, one slice, sliced, us: taken 4096 x 2560 x 151936 (160
-  // tiles on 74 pairs) 2646, 2276; 2816 x 1024 x 151936 (44) 745, 606; 1000 x 2560 x 100000 (40) 481, 375; 4096 x 1536 x 70000 (96)
-  // 779, 632; left 4096 x 1024 x 151936 (64) 894, 922; 4096 x 2048 x 128256 (128) 1526, 1518.
+  // slices' partial sums cost their traffic, and 256 MB at most (a caller without that room runs in one piece); and since full waves
+  // run into the power cap, at 1420 TFLOP/s, it pays only where the model promises 15 %.  Measured on B200, dH of a head, product and sum
+  // of the slices, cache overwritten before, under the power cap, one slice, sliced, us: taken 4096 x 2560 x 151936 (160 tiles on 74
+  // pairs) 2635, 2260; 2816 x 1024 x 151936 (44) 1152, 810; 1000 x 2560 x 100000 (40) 693, 478; 4096 x 1536 x 70000 (96) 816, 617; left
+  // 4096 x 1024 x 151936 (64) 929, 939 in two and 888 in eight; 4096 x 2048 x 128256 (128) 1525, 1461 in four.  The line at K = 65536 is only
+  // where the first measurements ended: below it slices are faster as well (1000 x 2560 x 50257 345, 257 in five; 2048 x 2560 x 50257
+  // 548, 398 in six; 4096 x 1536 x 32000 349, 284 in three), which the plan does not take yet.
   if (may_split && pair && out_mode == 0 && !a_mn && tiles * 2 > workers && num_kb >= 1024) {
     float fill = 0.85f * best;
     for (int s = 2; s <= 8; ++s) {
