@@ -82,6 +82,15 @@ def test_whole_warps_do_not_poll_lane_by_lane():
             assert inside != bool(m.group(1)), f"{path.name}:{text.count(chr(10), 0, m.start()) + 1}"
 
 
+def test_named_barriers_take_whole_warps():
+    """``bar.sync`` is aligned too; it stands in one helper, behind a ``__syncwarp``."""
+    for path in [*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]:
+        text = _code(path.name)
+        for m in re.finditer(r'"bar\.(?:sync|arrive)', text):
+            body = text[text.rindex("{", 0, m.start()):m.start()]
+            assert path.name == "common.cuh" and "__syncwarp();" in body, f"{path.name}: {m.group()}"
+
+
 def test_the_check_sees_a_lane_that_is_apart():
     found = set()
     _walk("for (int i = 0; i < n; ++i) {\n tmem_ld_wait();\n if (lane == 0) store();\n}", None, 1, found)

@@ -287,8 +287,9 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t (&r)[
                : "r"(taddr)
                : "memory");
 }
-// named barrier over `threads` threads (a multiple of 32); id 0 is __syncthreads
+// named barrier over `threads` threads (a multiple of 32); id 0 is __syncthreads.  An aligned instruction: whole warps arrive
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
+  __syncwarp();
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 __device__ __forceinline__ void red_add_f32(float* p, float v) {

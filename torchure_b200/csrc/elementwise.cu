@@ -369,7 +369,7 @@ rmsnorm_bwd_staged_kernel(const __nv_bfloat16* __restrict__ dh, const float* __r
     float dot = warp_sum(dot2.x + dot2.y);
     if (T > 1) {
       if (lane == 0) s_dot[team][k & 1][part] = dot;
-      asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(T * 32) : "memory");
+      named_bar_sync(team + 1, T * 32);
       dot = 0.f;
 #pragma unroll
       for (int p = 0; p < T; ++p) dot += s_dot[team][k & 1][p];

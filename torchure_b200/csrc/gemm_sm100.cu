@@ -127,7 +127,7 @@ __device__ __forceinline__ void ag_copy_phase(const GemmComm* gc, int K, int tid
     }
     fence_proxy_async_all();  // the consumers read these bytes through TMA
     __threadfence_system();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    named_bar_sync(1, 128);
     if (tid < c.world && tid != c.rank) {
       uint32_t* flag = reinterpret_cast<uint32_t*>(c.peer_bufs[tid] + kAgReadyOffset) + mb * kAgSeg + seg;
       asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(flag), "r"(gc->epoch) : "memory");
